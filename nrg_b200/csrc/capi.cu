@@ -232,10 +232,17 @@ std::string build_dev_mech(const nrg::Mechanism& m, DevMech* d) {
     formula_elements(m.species[k], e);
     for (int q = 0; q < 3; ++q) d->elem[q][k] = e[q];
   }
+  d->RM = R;
+  for (int r = 0; r < R; ++r) d->m_of[r] = r;
   d->NI = N;
   for (int k = 0; k < N; ++k) d->full_of[k] = k;
   d->n_inert = 0;
   gear_coefficients(d->el, d->tq);
+  for (int q = 1; q <= nrg::kMaxOrd; ++q)
+    for (int i = 0; i < 3; ++i) {
+      const double x = d->tq[(q - 1) * 3 + i];
+      d->itq2[q][i] = x != 0.0 ? 1.0 / (x * x) : 0.0;
+    }
   d->eps = 1.0e-9;
   d->ewt = 1.0e-4;
   d->hmax = (double)1.0E-7f;  // single-precision literal in the reference
@@ -246,6 +253,48 @@ std::string build_dev_mech(const nrg::Mechanism& m, DevMech* d) {
   d->bp = std::pow(DBL_EPSILON, -0.15);
   d->facmin = std::pow(DBL_EPSILON, 0.78);
   return "";
+}
+
+// Reorders the reactions so that those whose reactant and product lists equal
+// an earlier one's come last (DevMech::RM, m_of).
+void merge_equal_reactions(DevMech* d) {
+  const DevMech in = *d;
+  auto equal = [&](int a, int b) {
+    return std::memcmp(in.left[a], in.left[b], sizeof in.left[a]) == 0 &&
+           std::memcmp(in.right[a], in.right[b], sizeof in.right[a]) == 0;
+  };
+  std::vector<int> order, repeats, to(in.R);
+  for (int r = 0; r < in.R; ++r) {
+    int f = 0;
+    while (!equal(f, r)) ++f;
+    (f == r ? order : repeats).push_back(r);
+    to[r] = f;
+  }
+  d->RM = (int)order.size();
+  std::vector<int> pos(in.R);
+  for (int q = 0; q < d->RM; ++q) pos[order[q]] = q;
+  order.insert(order.end(), repeats.begin(), repeats.end());
+  for (int q = 0; q < in.R; ++q) {
+    const int r = order[q];
+    d->m_of[q] = pos[to[r]];
+    d->type[q] = in.type[r];
+    d->nl[q] = in.nl[r];
+    d->nr[q] = in.nr[r];
+    std::memcpy(d->left[q], in.left[r], sizeof in.left[r]);
+    std::memcpy(d->right[q], in.right[r], sizeof in.right[r]);
+    d->nupd[q] = in.nupd[r];
+    std::memcpy(d->upd_k[q], in.upd_k[r], sizeof in.upd_k[r]);
+    std::memcpy(d->upd_prod[q], in.upd_prod[r], sizeof in.upd_prod[r]);
+    d->A[q] = in.A[r];
+    d->beta[q] = in.beta[r];
+    d->E[q] = in.E[r];
+    d->A_low[q] = in.A_low[r];
+    d->beta_low[q] = in.beta_low[r];
+    d->E_low[q] = in.E_low[r];
+    std::memcpy(d->troe[q], in.troe[r], sizeof in.troe[r]);
+    d->dnu[q] = in.dnu[r];
+    for (int k = 0; k < in.N; ++k) d->eff_t[k][q] = in.eff_t[k][r];
+  }
 }
 
 // Tables for the integrators that skip inert species: the reaction lists
@@ -278,6 +327,7 @@ void reduce_dev_mech(const DevMech& full, DevMech* d) {
     }
     for (int u = 0; u < d->nupd[r]; ++u) d->upd_k[r][u] = int_of[d->upd_k[r][u]];
   }
+  if (d->NI <= nrg::kMergeUpTo) merge_equal_reactions(d);
 }
 
 void free_staging(nrg_chem* h) {

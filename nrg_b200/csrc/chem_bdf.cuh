@@ -63,12 +63,12 @@ struct SmemStore {
     d = reinterpret_cast<double*>(smem) + tid;
     f = reinterpret_cast<LUT*>(smem + (size_t)kDoubles * 8 * BS) + tid;
   }
-  __device__ __forceinline__ double& yh(int j, int i) { return d[(kYH + j * N + i) * BS]; }
-  __device__ __forceinline__ double& kf(int r) { return d[(kKF + r) * BS]; }
-  __device__ __forceinline__ double& kr(int r) { return d[(kKR + r) * BS]; }
-  __device__ __forceinline__ double& z(int k) { return d[(kZ + k) * BS]; }
-  __device__ __forceinline__ double& zd(int k) { return d[(kZD + k) * BS]; }
-  __device__ __forceinline__ LUT& a(int j, int i) { return f[(j * N + i) * BS]; }  // A(i+1, j+1)
+  __device__ __forceinline__ double& yh(int j, int i) const { return d[(kYH + j * N + i) * BS]; }
+  __device__ __forceinline__ double& kf(int r) const { return d[(kKF + r) * BS]; }
+  __device__ __forceinline__ double& kr(int r) const { return d[(kKR + r) * BS]; }
+  __device__ __forceinline__ double& z(int k) const { return d[(kZ + k) * BS]; }
+  __device__ __forceinline__ double& zd(int k) const { return d[(kZD + k) * BS]; }
+  __device__ __forceinline__ LUT& a(int j, int i) const { return f[(j * N + i) * BS]; }  // A(i+1, j+1)
 };
 
 template <int N, int R, typename LUT, int BS, int NF = N, int SPEC = 0>
@@ -362,8 +362,8 @@ __device__ void rate_constants_fast(CS& c, double Tin) {
 
 // fun (chemical_kinetics_solver.f90:495-540): zd = dC/dt at z (both in the
 // cell's shared scratch), accumulated per reaction as the net rate f - b.
-template <int N, int R, class CS>
-__device__ __forceinline__ void rhs(CS& c) {
+template <int N, class CS>
+__device__ __forceinline__ void rhs(CS& c, int R) {
 #pragma unroll
   for (int k = 0; k < N; ++k) c.zd(k) = 0.0;
 // Fixed-trip inner loops (3 reactant and 3 product slots, unused and M
@@ -411,8 +411,8 @@ __device__ __forceinline__ void rhs_at(CS& c, const double (&v)[N], double (&out
 
 // Iteration matrix I + factor * J with J = dZdot/dZ of the mass-action rates
 // at z, written straight into the LU storage.
-template <int N, int R, class CS>
-__device__ void analytic_iteration_matrix(CS& c, double factor) {
+template <int N, class CS>
+__device__ void analytic_iteration_matrix(CS& c, double factor, int R) {
   using LUT_T = typename CS::lut_t;
 #pragma unroll
   for (int j = 0; j < N; ++j)
@@ -719,8 +719,19 @@ __device__ __noinline__ void nl_rhs(double* d, LUT* f) {
     static_assert(N == SpecOf<SPEC>::kN && R == SpecOf<SPEC>::kR, "specialised code is for another mechanism size");
     SpecOf<SPEC>::rhs(s);
   } else {
-    rhs<N, R>(s);
+    rhs<N>(s, R);
   }
+}
+
+// The generated iteration matrix into the LU storage, one column in registers
+// at a time.
+template <int SPEC, int N, typename LUT, int J, class S>
+__device__ __forceinline__ void spec_store_columns(const S& s, double factor) {
+  LUT v[N];
+  SpecOf<SPEC>::template column<J>(s, factor, v);
+#pragma unroll
+  for (int i = 0; i < N; ++i) s.a(J, i) = v[i];
+  if constexpr (J + 1 < N) spec_store_columns<SPEC, N, LUT, J + 1>(s, factor);
 }
 
 template <int N, int R, typename LUT, int BS, int SPEC>
@@ -730,9 +741,9 @@ __device__ __noinline__ void nl_analytic_matrix(double* d, LUT* f, double factor
   s.f = f;
   if constexpr (SPEC != 0) {
     static_assert(N == SpecOf<SPEC>::kN && R == SpecOf<SPEC>::kR, "specialised code is for another mechanism size");
-    SpecOf<SPEC>::template matrix<SmemStore<N, R, LUT, BS>, LUT>(s, factor);
+    spec_store_columns<SPEC, N, LUT, 0>(s, factor);
   } else {
-    analytic_iteration_matrix<N, R>(s, factor);
+    analytic_iteration_matrix<N>(s, factor, R);
   }
 }
 

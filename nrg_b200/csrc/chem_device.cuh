@@ -16,6 +16,7 @@ namespace nrg {
 constexpr int kMaxSpecies = 24;
 constexpr int kMaxReactions = 96;
 constexpr int kMaxOrd = 5;  // MXORD for Gear (MINT = 2)
+constexpr int kMergeUpTo = 8;  // integrated species up to which equal reactions are merged
 constexpr int kMaxSpecUpd = 64;  // reactions touching one species
 
 // Per-reaction update list entry: species (0-based) and whether the
@@ -41,6 +42,7 @@ struct DevMech {
   double h_ref[kMaxSpecies];   // h_k(T_ref)
   // integrator constants (host-computed so host and device agree bit-for-bit)
   double el[13 * 12], tq[3 * 12];
+  double itq2[kMaxOrd + 1][3];  // 1 / tq(i + 1, order)^2
   double eps, ewt, hmax, uround;
   double sqrt_uround, br, bl, bp, facmin;
   // per-species update lists in reaction order, entry-major so that lanes
@@ -60,6 +62,12 @@ struct DevMech {
   int full_of[kMaxSpecies];   // integrated index -> mechanism species
   int n_inert;
   int inert_of[kMaxSpecies];  // the inert species (mechanism index)
+  // The first RM reactions have distinct reactant and product lists; reaction
+  // r >= RM repeats the lists of reaction m_of[r], so the right-hand side and
+  // the iteration matrix walk RM reactions with the sums of the rate constants.
+  // (Full tables and tables of more than kMergeUpTo species: RM = R.)
+  int RM;
+  int m_of[kMaxReactions];
 };
 
 // Per-cell status byte written by the integrator.

@@ -1,6 +1,8 @@
 // Kernel templates of the chemistry step (included by the per-variant
 // translation units chem_k_*.cu, which instantiate them).
 //
+//   k_chem_pass   -- one thread per cell in passes (chem_pass.cuh): analytic
+//                    Jacobian, up to 8 integrated species.
 //   k_chem_plain  -- one thread per cell, grid covers all cells.
 //   k_chem_queue  -- persistent grid; every lane pulls cells from a device
 //                    work queue and is refilled as soon as its cell reaches
@@ -14,6 +16,7 @@
 
 #include "chem_bdf.cuh"
 #include "chem_kernels.hpp"
+#include "chem_pass.cuh"
 #include "chem_warp.cuh"
 
 namespace nrg {
@@ -132,6 +135,90 @@ static cudaError_t launch_bs(const StepArgs& a, const LaunchCfg& cfg, int* queue
 }
 
 
+// One cell per thread, integrated in passes (chem_pass.cuh).  LOCK: the warps of
+// the block go through the passes together, so that the loop's 50 to 80 KB of
+// code are fetched once for all of them.  QUEUE: the warps pull groups of 32
+// cells from the work queue; else the grid covers the cells.
+template <int N, int R, typename LUT, int BS, int NF, int SPEC, bool LOCK, bool QUEUE>
+__global__ void __launch_bounds__(BS, 256 / BS) k_chem_pass(StepArgs a, int* queue, int chunk,
+                                                            unsigned long long* counters) {
+  static_assert(!(LOCK && QUEUE), "the work queue serves warps on their own");
+  extern __shared__ __align__(16) char smem[];
+  const long nl = a.cell_list ? (long)(a.n_list_dev ? *a.n_list_dev : a.n_list) : a.n;
+  if (!QUEUE && (long)blockIdx.x * BS >= nl) return;
+  unsigned long long v[kCntSlots] = {0, 0, 0, 0, 0, 0};
+  PassStore<N, RateSlots<R, SPEC>::value, LUT, SPEC == 0> st;
+  st.bind(smem, threadIdx.x);
+  const int lane = threadIdx.x & 31;
+  long base = ((long)blockIdx.x * BS + threadIdx.x) & ~31L;
+  int left = 0;
+  for (;;) {
+    if (QUEUE) {
+      if (left == 0) {
+        int b = 0;
+        if (lane == 0) b = atomicAdd(queue, chunk);
+        base = 32L * __shfl_sync(0xffffffffu, b, 0);
+        left = chunk;
+      } else {
+        base += 32;
+      }
+      --left;
+      if (base >= nl) break;
+    }
+    const long li = base + lane;
+    const bool have = li < nl;
+    const long cid = have ? (a.cell_list ? (long)a.cell_list[li] : li) : 0;
+    PassResult<N, NF> res;
+#pragma unroll
+    for (int i = 0; i < N; ++i) res.y[i] = 0.0;
+    res.tout = a.dt;
+    bool live = false;
+    if (have) {
+      live = pass_begin<N, R, NF>(st, a, cid, res.y);
+      if (a.dt_cells) res.tout = a.dt_cells[cid];
+    }
+    const int status = pass_integrate<N, R, NF, SPEC, LOCK>(st, a, live, res.tout, res.y, v);
+    if (live) {
+      cell_finish<N, kJacAnalytic>(res, a, cid, status);
+      v[kCntCells] += 1;
+      v[kCntBad] += status != kCellOk;
+    }
+    if (!QUEUE) break;
+  }
+  if (counters) block_flush_counters(counters, v);
+}
+
+template <int N, int R, typename LUT, int BS, int NF, int SPEC, bool LOCK, bool QUEUE>
+static cudaError_t launch_pass_bs(const StepArgs& a, long grid, int* queue, int chunk, unsigned long long* counters,
+                                  cudaStream_t s) {
+  const auto kern = k_chem_pass<N, R, LUT, BS, NF, SPEC, LOCK, QUEUE>;
+  const int smem = BS * PassStore<N, RateSlots<R, SPEC>::value, LUT, SPEC == 0>::kBytesPerThread;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  if (e != cudaSuccess) return e;
+  if (grid > 0) kern<<<(unsigned)grid, BS, smem, s>>>(a, queue, chunk, counters);
+  return cudaGetLastError();
+}
+
+// Blocks of 128 threads in lockstep, two per SM, from kLockstepCells cells on
+// (one wave of them on 148 SMs); below, 64-thread blocks whose warps run on
+// their own: the cells then spread over more SMs and nothing waits for another
+// warp.  2048 x 2048 flame 32.1 ms on their own, 29.2 ms in lockstep; 512 x
+// 512 ignition field 22.1 and 18.8 ms; 64 x 64 random cells 1.15 and 1.29 ms.
+constexpr long kLockstepCells = 148L * 2 * 128;
+
+template <int N, int R, typename LUT, int NF, int SPEC>
+static cudaError_t launch_pass(const StepArgs& a, const LaunchCfg& cfg, int* queue, unsigned long long* counters,
+                               cudaStream_t s) {
+  if (cfg.kernel == kKernelThreadQueue)
+    return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, true>(a, cfg.grid > 0 ? cfg.grid : 148, queue, cfg.chunk,
+                                                                counters, s);
+  const long nl = a.cell_list ? (long)a.n_list : a.n;
+  if (nl < kLockstepCells)
+    return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, false>(a, (nl + 63) / 64, queue, 0, counters, s);
+  return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false>(a, (nl + 127) / 128, queue, 0, counters, s);
+}
+
 __host__ __device__ constexpr size_t warp_tables_bytes() { return (sizeof(DevMech) + 15) / 16 * 16; }
 
 // Warp-per-cell persistent kernel: every warp pulls `chunk` cells at a time
@@ -206,6 +293,23 @@ static cudaError_t launch_warp(const StepArgs& a, const LaunchCfg& cfg, int* que
   return cudaGetLastError();
 }
 
+// The thread-per-cell kernels: in passes where the Nordsieck array fits the
+// registers (up to 8 integrated species, analytic Jacobian; these choose their
+// blocks themselves), else routine by routine.
+template <int NF, int NI, int R, int JAC, typename LUT, int SPEC>
+static cudaError_t launch_thread(const StepArgs& a, const LaunchCfg& cfg, int* queue, unsigned long long* counters,
+                                 cudaStream_t s) {
+  if constexpr (JAC == kJacAnalytic && NI <= 8) {
+    return launch_pass<NI, R, LUT, NF, SPEC>(a, cfg, queue, counters, s);
+  } else {
+    switch (cfg.block) {
+      case 32: return launch_bs<NI, R, JAC, LUT, 32, NF, SPEC>(a, cfg, queue, counters, s);
+      case 64: return launch_bs<NI, R, JAC, LUT, 64, NF, SPEC>(a, cfg, queue, counters, s);
+      default: return cudaErrorInvalidValue;
+    }
+  }
+}
+
 // Launches one (JAC, LUT) variant: cfg.kernel selects thread-per-cell (grid
 // or work queue, 32- or 64-thread blocks) or warp-per-cell (128- or 256-thread
 // blocks).  With 32-thread blocks every warp is its own block, so an SM slot
@@ -225,11 +329,7 @@ static cudaError_t launch_variant(const StepArgs& a, const LaunchCfg& cfg, int* 
       default: return cudaErrorInvalidValue;
     }
   }
-  switch (cfg.block) {
-    case 32: return launch_bs<NI, R, JAC, LUT, 32, NF, SPEC>(a, cfg, queue, counters, s);
-    case 64: return launch_bs<NI, R, JAC, LUT, 64, NF, SPEC>(a, cfg, queue, counters, s);
-    default: return cudaErrorInvalidValue;
-  }
+  return launch_thread<NF, NI, R, JAC, LUT, SPEC>(a, cfg, queue, counters, s);
 }
 
 // The thread-per-cell grid kernel only (the shape used for the mechanisms
@@ -238,11 +338,7 @@ template <int NF, int NI, int R, int JAC, typename LUT, int SPEC = 0>
 static cudaError_t launch_grid(const StepArgs& a, const LaunchCfg& cfg, int* queue, unsigned long long* counters,
                                cudaStream_t s) {
   if (cfg.kernel != kKernelThreadGrid) return cudaErrorNotSupported;
-  switch (cfg.block) {
-    case 32: return launch_bs<NI, R, JAC, LUT, 32, NF, SPEC>(a, cfg, queue, counters, s);
-    case 64: return launch_bs<NI, R, JAC, LUT, 64, NF, SPEC>(a, cfg, queue, counters, s);
-    default: return cudaErrorInvalidValue;
-  }
+  return launch_thread<NF, NI, R, JAC, LUT, SPEC>(a, cfg, queue, counters, s);
 }
 
 }  // namespace nrg

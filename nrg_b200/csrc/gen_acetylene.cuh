@@ -327,833 +327,572 @@ __device__ __forceinline__ void spec_rhs(S& c) {
   c.zd(14) = d14;
 }
 
-// I + factor * J written into the LU storage: c.a(j, i) = A(i+1, j+1)
-template <class S, typename LUT>
-__device__ __forceinline__ void spec_matrix(S& c, double factor) {
-  const double z0 = c.z(0);
-  const double z1 = c.z(1);
-  const double z2 = c.z(2);
-  const double z3 = c.z(3);
-  const double z4 = c.z(4);
-  const double z5 = c.z(5);
-  const double z6 = c.z(6);
-  const double z7 = c.z(7);
-  const double z8 = c.z(8);
-  const double z9 = c.z(9);
-  const double z10 = c.z(10);
-  const double z11 = c.z(11);
-  const double z12 = c.z(12);
-  const double z13 = c.z(13);
-  const double z14 = c.z(14);
+// Column J of I + factor * J: v[i] = A(i+1, J+1), each element's terms in
+// reaction order.
+template <int J, class S, typename LUT>
+__device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[15]) {
   const double msf = -factor;
-  LUT a0_0 = (LUT)0, a0_1 = (LUT)0, a0_2 = (LUT)0, a0_3 = (LUT)0, a0_4 = (LUT)0, a0_5 = (LUT)0, a0_6 = (LUT)0, a0_7 = (LUT)0, a0_8 = (LUT)0, a0_9 = (LUT)0, a0_10 = (LUT)0, a0_11 = (LUT)0, a0_12 = (LUT)0, a0_13 = (LUT)0, a0_14 = (LUT)0, a1_0 = (LUT)0, a1_1 = (LUT)0, a1_2 = (LUT)0, a1_3 = (LUT)0, a1_4 = (LUT)0, a1_5 = (LUT)0, a1_6 = (LUT)0, a1_7 = (LUT)0, a1_8 = (LUT)0, a1_9 = (LUT)0, a1_10 = (LUT)0, a1_11 = (LUT)0, a1_12 = (LUT)0, a1_13 = (LUT)0, a1_14 = (LUT)0, a2_0 = (LUT)0, a2_1 = (LUT)0, a2_2 = (LUT)0, a2_3 = (LUT)0, a2_4 = (LUT)0, a2_5 = (LUT)0, a2_6 = (LUT)0, a2_7 = (LUT)0, a2_8 = (LUT)0, a2_9 = (LUT)0, a2_10 = (LUT)0, a2_11 = (LUT)0, a2_12 = (LUT)0, a2_13 = (LUT)0, a2_14 = (LUT)0, a3_0 = (LUT)0, a3_1 = (LUT)0, a3_2 = (LUT)0, a3_3 = (LUT)0, a3_4 = (LUT)0, a3_5 = (LUT)0, a3_6 = (LUT)0, a3_7 = (LUT)0, a3_8 = (LUT)0, a3_9 = (LUT)0, a3_10 = (LUT)0, a3_11 = (LUT)0, a3_12 = (LUT)0, a3_13 = (LUT)0, a3_14 = (LUT)0, a4_0 = (LUT)0, a4_1 = (LUT)0, a4_2 = (LUT)0, a4_3 = (LUT)0, a4_4 = (LUT)0, a4_5 = (LUT)0, a4_6 = (LUT)0, a4_7 = (LUT)0, a4_8 = (LUT)0, a4_9 = (LUT)0, a4_10 = (LUT)0, a4_11 = (LUT)0, a4_12 = (LUT)0, a4_13 = (LUT)0, a4_14 = (LUT)0, a5_0 = (LUT)0, a5_1 = (LUT)0, a5_2 = (LUT)0, a5_3 = (LUT)0, a5_4 = (LUT)0, a5_5 = (LUT)0, a5_6 = (LUT)0, a5_7 = (LUT)0, a5_8 = (LUT)0, a5_9 = (LUT)0, a5_10 = (LUT)0, a5_11 = (LUT)0, a5_12 = (LUT)0, a5_13 = (LUT)0, a5_14 = (LUT)0, a6_0 = (LUT)0, a6_1 = (LUT)0, a6_2 = (LUT)0, a6_3 = (LUT)0, a6_4 = (LUT)0, a6_5 = (LUT)0, a6_6 = (LUT)0, a6_7 = (LUT)0, a6_8 = (LUT)0, a6_9 = (LUT)0, a6_10 = (LUT)0, a6_11 = (LUT)0, a6_12 = (LUT)0, a6_13 = (LUT)0, a6_14 = (LUT)0, a7_0 = (LUT)0, a7_1 = (LUT)0, a7_2 = (LUT)0, a7_3 = (LUT)0, a7_4 = (LUT)0, a7_5 = (LUT)0, a7_6 = (LUT)0, a7_7 = (LUT)0, a7_8 = (LUT)0, a7_9 = (LUT)0, a7_10 = (LUT)0, a7_11 = (LUT)0, a7_12 = (LUT)0, a7_13 = (LUT)0, a7_14 = (LUT)0, a8_0 = (LUT)0, a8_1 = (LUT)0, a8_2 = (LUT)0, a8_3 = (LUT)0, a8_4 = (LUT)0, a8_5 = (LUT)0, a8_6 = (LUT)0, a8_7 = (LUT)0, a8_8 = (LUT)0, a8_9 = (LUT)0, a8_10 = (LUT)0, a8_11 = (LUT)0, a8_12 = (LUT)0, a8_13 = (LUT)0, a8_14 = (LUT)0, a9_0 = (LUT)0, a9_1 = (LUT)0, a9_2 = (LUT)0, a9_3 = (LUT)0, a9_4 = (LUT)0, a9_5 = (LUT)0, a9_6 = (LUT)0, a9_7 = (LUT)0, a9_8 = (LUT)0, a9_9 = (LUT)0, a9_10 = (LUT)0, a9_11 = (LUT)0, a9_12 = (LUT)0, a9_13 = (LUT)0, a9_14 = (LUT)0, a10_0 = (LUT)0, a10_1 = (LUT)0, a10_2 = (LUT)0, a10_3 = (LUT)0, a10_4 = (LUT)0, a10_5 = (LUT)0, a10_6 = (LUT)0, a10_7 = (LUT)0, a10_8 = (LUT)0, a10_9 = (LUT)0, a10_10 = (LUT)0, a10_11 = (LUT)0, a10_12 = (LUT)0, a10_13 = (LUT)0, a10_14 = (LUT)0, a11_0 = (LUT)0, a11_1 = (LUT)0, a11_2 = (LUT)0, a11_3 = (LUT)0, a11_4 = (LUT)0, a11_5 = (LUT)0, a11_6 = (LUT)0, a11_7 = (LUT)0, a11_8 = (LUT)0, a11_9 = (LUT)0, a11_10 = (LUT)0, a11_11 = (LUT)0, a11_12 = (LUT)0, a11_13 = (LUT)0, a11_14 = (LUT)0, a12_0 = (LUT)0, a12_1 = (LUT)0, a12_2 = (LUT)0, a12_3 = (LUT)0, a12_4 = (LUT)0, a12_5 = (LUT)0, a12_6 = (LUT)0, a12_7 = (LUT)0, a12_8 = (LUT)0, a12_9 = (LUT)0, a12_10 = (LUT)0, a12_11 = (LUT)0, a12_12 = (LUT)0, a12_13 = (LUT)0, a12_14 = (LUT)0, a13_0 = (LUT)0, a13_1 = (LUT)0, a13_2 = (LUT)0, a13_3 = (LUT)0, a13_4 = (LUT)0, a13_5 = (LUT)0, a13_6 = (LUT)0, a13_7 = (LUT)0, a13_8 = (LUT)0, a13_9 = (LUT)0, a13_10 = (LUT)0, a13_11 = (LUT)0, a13_12 = (LUT)0, a13_13 = (LUT)0, a13_14 = (LUT)0, a14_0 = (LUT)0, a14_1 = (LUT)0, a14_2 = (LUT)0, a14_3 = (LUT)0, a14_4 = (LUT)0, a14_5 = (LUT)0, a14_6 = (LUT)0, a14_7 = (LUT)0, a14_8 = (LUT)0, a14_9 = (LUT)0, a14_10 = (LUT)0, a14_11 = (LUT)0, a14_12 = (LUT)0, a14_13 = (LUT)0, a14_14 = (LUT)0;
   double d;
-  d = __dmul_rn(c.kf(0), z1);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_2 = (LUT)__dadd_rn((double)a3_2, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  d = __dmul_rn(c.kf(0), z3);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_2 = (LUT)__dadd_rn((double)a1_2, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  d = __dmul_rn(c.kr(0), z2);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_2 = (LUT)__dadd_rn((double)a4_2, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  d = __dmul_rn(c.kr(0), z4);
-  d = __dmul_rn(d, msf);
-  a2_1 = (LUT)__dsub_rn((double)a2_1, d);
-  a2_2 = (LUT)__dadd_rn((double)a2_2, d);
-  a2_3 = (LUT)__dsub_rn((double)a2_3, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  d = __dmul_rn(c.kf(1), z2);
-  d = __dmul_rn(d, factor);
-  a4_1 = (LUT)__dadd_rn((double)a4_1, d);
-  a4_2 = (LUT)__dsub_rn((double)a4_2, d);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  d = __dmul_rn(c.kf(1), z4);
-  d = __dmul_rn(d, factor);
-  a2_1 = (LUT)__dadd_rn((double)a2_1, d);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_3 = (LUT)__dadd_rn((double)a2_3, d);
-  a2_4 = (LUT)__dsub_rn((double)a2_4, d);
-  d = __dmul_rn(c.kr(1), z1);
-  d = __dmul_rn(d, msf);
-  a3_1 = (LUT)__dadd_rn((double)a3_1, d);
-  a3_2 = (LUT)__dsub_rn((double)a3_2, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  d = __dmul_rn(c.kr(1), z3);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_2 = (LUT)__dsub_rn((double)a1_2, d);
-  a1_3 = (LUT)__dadd_rn((double)a1_3, d);
-  a1_4 = (LUT)__dsub_rn((double)a1_4, d);
-  d = __dmul_rn(c.kf(2), z13);
-  d = __dmul_rn(d, factor);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  a4_13 = (LUT)__dsub_rn((double)a4_13, d);
-  d = __dmul_rn(c.kf(2), z4);
-  d = __dmul_rn(d, factor);
-  a13_3 = (LUT)__dadd_rn((double)a13_3, d);
-  a13_4 = (LUT)__dsub_rn((double)a13_4, d);
-  a13_5 = (LUT)__dadd_rn((double)a13_5, d);
-  a13_13 = (LUT)__dsub_rn((double)a13_13, d);
-  d = __dmul_rn(c.kr(2), z3);
-  d = __dmul_rn(d, msf);
-  a5_3 = (LUT)__dadd_rn((double)a5_3, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  a5_13 = (LUT)__dsub_rn((double)a5_13, d);
-  d = __dmul_rn(c.kr(2), z5);
-  d = __dmul_rn(d, msf);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  a3_5 = (LUT)__dadd_rn((double)a3_5, d);
-  a3_13 = (LUT)__dsub_rn((double)a3_13, d);
-  d = __dmul_rn(c.kf(3), z5);
-  d = __dmul_rn(d, factor);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  a2_5 = (LUT)__dsub_rn((double)a2_5, d);
-  d = __dmul_rn(c.kf(3), z2);
-  d = __dmul_rn(d, factor);
-  a5_2 = (LUT)__dsub_rn((double)a5_2, d);
-  a5_4 = (LUT)__dadd_rn((double)a5_4, d);
-  a5_4 = (LUT)__dadd_rn((double)a5_4, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  d = __dmul_rn(c.kr(3), z4);
-  d = __dmul_rn(d, msf);
-  a4_2 = (LUT)__dsub_rn((double)a4_2, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_5 = (LUT)__dsub_rn((double)a4_5, d);
-  d = __dmul_rn(c.kr(3), z4);
-  d = __dmul_rn(d, msf);
-  a4_2 = (LUT)__dsub_rn((double)a4_2, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_5 = (LUT)__dsub_rn((double)a4_5, d);
-  d = __dmul_rn(c.kf(4), z4);
-  d = __dmul_rn(d, factor);
-  a4_2 = (LUT)__dadd_rn((double)a4_2, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  d = __dmul_rn(c.kf(4), z4);
-  d = __dmul_rn(d, factor);
-  a4_2 = (LUT)__dadd_rn((double)a4_2, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  d = __dmul_rn(c.kr(4), z5);
-  d = __dmul_rn(d, msf);
-  a2_2 = (LUT)__dadd_rn((double)a2_2, d);
-  a2_4 = (LUT)__dsub_rn((double)a2_4, d);
-  a2_4 = (LUT)__dsub_rn((double)a2_4, d);
-  a2_5 = (LUT)__dadd_rn((double)a2_5, d);
-  d = __dmul_rn(c.kr(4), z2);
-  d = __dmul_rn(d, msf);
-  a5_2 = (LUT)__dadd_rn((double)a5_2, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  d = __dmul_rn(c.kf(5), z1);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_12 = (LUT)__dadd_rn((double)a3_12, d);
-  d = __dmul_rn(c.kf(5), z3);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_12 = (LUT)__dadd_rn((double)a1_12, d);
-  d = c.kr(5);
-  d = __dmul_rn(d, msf);
-  a12_1 = (LUT)__dsub_rn((double)a12_1, d);
-  a12_3 = (LUT)__dsub_rn((double)a12_3, d);
-  a12_12 = (LUT)__dadd_rn((double)a12_12, d);
-  d = __dmul_rn(c.kf(6), z3);
-  d = __dmul_rn(d, factor);
-  a12_3 = (LUT)__dsub_rn((double)a12_3, d);
-  a12_4 = (LUT)__dadd_rn((double)a12_4, d);
-  a12_4 = (LUT)__dadd_rn((double)a12_4, d);
-  a12_12 = (LUT)__dsub_rn((double)a12_12, d);
-  d = __dmul_rn(c.kf(6), z12);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_12 = (LUT)__dsub_rn((double)a3_12, d);
-  d = __dmul_rn(c.kr(6), z4);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_12 = (LUT)__dsub_rn((double)a4_12, d);
-  d = __dmul_rn(c.kr(6), z4);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_12 = (LUT)__dsub_rn((double)a4_12, d);
-  d = __dmul_rn(c.kf(7), z3);
-  d = __dmul_rn(d, factor);
-  a12_1 = (LUT)__dadd_rn((double)a12_1, d);
-  a12_3 = (LUT)__dsub_rn((double)a12_3, d);
-  a12_12 = (LUT)__dsub_rn((double)a12_12, d);
-  a12_13 = (LUT)__dadd_rn((double)a12_13, d);
-  d = __dmul_rn(c.kf(7), z12);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dadd_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_12 = (LUT)__dsub_rn((double)a3_12, d);
-  a3_13 = (LUT)__dadd_rn((double)a3_13, d);
-  d = __dmul_rn(c.kr(7), z1);
-  d = __dmul_rn(d, msf);
-  a13_1 = (LUT)__dadd_rn((double)a13_1, d);
-  a13_3 = (LUT)__dsub_rn((double)a13_3, d);
-  a13_12 = (LUT)__dsub_rn((double)a13_12, d);
-  a13_13 = (LUT)__dadd_rn((double)a13_13, d);
-  d = __dmul_rn(c.kr(7), z13);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_12 = (LUT)__dsub_rn((double)a1_12, d);
-  a1_13 = (LUT)__dadd_rn((double)a1_13, d);
-  d = __dmul_rn(c.kf(8), z4);
-  d = __dmul_rn(d, factor);
-  a12_1 = (LUT)__dadd_rn((double)a12_1, d);
-  a12_4 = (LUT)__dsub_rn((double)a12_4, d);
-  a12_5 = (LUT)__dadd_rn((double)a12_5, d);
-  a12_12 = (LUT)__dsub_rn((double)a12_12, d);
-  d = __dmul_rn(c.kf(8), z12);
-  d = __dmul_rn(d, factor);
-  a4_1 = (LUT)__dadd_rn((double)a4_1, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  a4_12 = (LUT)__dsub_rn((double)a4_12, d);
-  d = __dmul_rn(c.kr(8), z1);
-  d = __dmul_rn(d, msf);
-  a5_1 = (LUT)__dadd_rn((double)a5_1, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  a5_12 = (LUT)__dsub_rn((double)a5_12, d);
-  d = __dmul_rn(c.kr(8), z5);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_4 = (LUT)__dsub_rn((double)a1_4, d);
-  a1_5 = (LUT)__dadd_rn((double)a1_5, d);
-  a1_12 = (LUT)__dsub_rn((double)a1_12, d);
-  d = __dmul_rn(c.kf(9), z4);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  a3_5 = (LUT)__dadd_rn((double)a3_5, d);
-  d = __dmul_rn(c.kf(9), z3);
-  d = __dmul_rn(d, factor);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  d = c.kr(9);
-  d = __dmul_rn(d, msf);
-  a5_3 = (LUT)__dsub_rn((double)a5_3, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  d = c.kf(10);
-  d = __dmul_rn(d, factor);
-  a5_3 = (LUT)__dadd_rn((double)a5_3, d);
-  a5_4 = (LUT)__dadd_rn((double)a5_4, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  d = __dmul_rn(c.kr(10), z4);
-  d = __dmul_rn(d, msf);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_5 = (LUT)__dsub_rn((double)a3_5, d);
-  d = __dmul_rn(c.kr(10), z3);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_5 = (LUT)__dsub_rn((double)a4_5, d);
-  d = __dmul_rn(c.kf(11), z4);
-  d = __dmul_rn(d, factor);
-  a6_3 = (LUT)__dadd_rn((double)a6_3, d);
-  a6_4 = (LUT)__dsub_rn((double)a6_4, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_7 = (LUT)__dadd_rn((double)a6_7, d);
-  d = __dmul_rn(c.kf(11), z6);
-  d = __dmul_rn(d, factor);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_6 = (LUT)__dsub_rn((double)a4_6, d);
-  a4_7 = (LUT)__dadd_rn((double)a4_7, d);
-  d = __dmul_rn(c.kr(11), z3);
-  d = __dmul_rn(d, msf);
-  a7_3 = (LUT)__dadd_rn((double)a7_3, d);
-  a7_4 = (LUT)__dsub_rn((double)a7_4, d);
-  a7_6 = (LUT)__dsub_rn((double)a7_6, d);
-  a7_7 = (LUT)__dadd_rn((double)a7_7, d);
-  d = __dmul_rn(c.kr(11), z7);
-  d = __dmul_rn(d, msf);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  a3_6 = (LUT)__dsub_rn((double)a3_6, d);
-  a3_7 = (LUT)__dadd_rn((double)a3_7, d);
-  d = __dmul_rn(c.kf(12), z3);
-  d = __dmul_rn(d, factor);
-  a7_3 = (LUT)__dsub_rn((double)a7_3, d);
-  a7_4 = (LUT)__dadd_rn((double)a7_4, d);
-  a7_6 = (LUT)__dadd_rn((double)a7_6, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  d = __dmul_rn(c.kf(12), z7);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  a3_7 = (LUT)__dsub_rn((double)a3_7, d);
-  d = __dmul_rn(c.kr(12), z4);
-  d = __dmul_rn(d, msf);
-  a6_3 = (LUT)__dsub_rn((double)a6_3, d);
-  a6_4 = (LUT)__dadd_rn((double)a6_4, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_7 = (LUT)__dsub_rn((double)a6_7, d);
-  d = __dmul_rn(c.kr(12), z6);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_6 = (LUT)__dadd_rn((double)a4_6, d);
-  a4_7 = (LUT)__dsub_rn((double)a4_7, d);
-  d = __dmul_rn(c.kf(13), z1);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_1 = (LUT)__dsub_rn((double)a0_1, d);
-  a0_6 = (LUT)__dadd_rn((double)a0_6, d);
-  a0_8 = (LUT)__dadd_rn((double)a0_8, d);
-  d = __dmul_rn(c.kf(13), z0);
-  d = __dmul_rn(d, factor);
-  a1_0 = (LUT)__dsub_rn((double)a1_0, d);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_6 = (LUT)__dadd_rn((double)a1_6, d);
-  a1_8 = (LUT)__dadd_rn((double)a1_8, d);
-  d = __dmul_rn(c.kr(13), z6);
-  d = __dmul_rn(d, msf);
-  a8_0 = (LUT)__dsub_rn((double)a8_0, d);
-  a8_1 = (LUT)__dsub_rn((double)a8_1, d);
-  a8_6 = (LUT)__dadd_rn((double)a8_6, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(13), z8);
-  d = __dmul_rn(d, msf);
-  a6_0 = (LUT)__dsub_rn((double)a6_0, d);
-  a6_1 = (LUT)__dsub_rn((double)a6_1, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_8 = (LUT)__dadd_rn((double)a6_8, d);
-  d = __dmul_rn(c.kf(14), z2);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_2 = (LUT)__dsub_rn((double)a0_2, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  a0_10 = (LUT)__dadd_rn((double)a0_10, d);
-  d = __dmul_rn(c.kf(14), z0);
-  d = __dmul_rn(d, factor);
-  a2_0 = (LUT)__dsub_rn((double)a2_0, d);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_3 = (LUT)__dadd_rn((double)a2_3, d);
-  a2_10 = (LUT)__dadd_rn((double)a2_10, d);
-  d = __dmul_rn(c.kr(14), z3);
-  d = __dmul_rn(d, msf);
-  a10_0 = (LUT)__dsub_rn((double)a10_0, d);
-  a10_2 = (LUT)__dsub_rn((double)a10_2, d);
-  a10_3 = (LUT)__dadd_rn((double)a10_3, d);
-  a10_10 = (LUT)__dadd_rn((double)a10_10, d);
-  d = __dmul_rn(c.kr(14), z10);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_2 = (LUT)__dsub_rn((double)a3_2, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_10 = (LUT)__dadd_rn((double)a3_10, d);
-  d = __dmul_rn(c.kf(15), z4);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  a0_4 = (LUT)__dsub_rn((double)a0_4, d);
-  a0_9 = (LUT)__dadd_rn((double)a0_9, d);
-  d = __dmul_rn(c.kf(15), z0);
-  d = __dmul_rn(d, factor);
-  a4_0 = (LUT)__dsub_rn((double)a4_0, d);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_9 = (LUT)__dadd_rn((double)a4_9, d);
-  d = __dmul_rn(c.kr(15), z3);
-  d = __dmul_rn(d, msf);
-  a9_0 = (LUT)__dsub_rn((double)a9_0, d);
-  a9_3 = (LUT)__dadd_rn((double)a9_3, d);
-  a9_4 = (LUT)__dsub_rn((double)a9_4, d);
-  a9_9 = (LUT)__dadd_rn((double)a9_9, d);
-  d = __dmul_rn(c.kr(15), z9);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  a3_9 = (LUT)__dadd_rn((double)a3_9, d);
-  d = __dmul_rn(c.kf(16), z2);
-  d = __dmul_rn(d, factor);
-  a9_2 = (LUT)__dsub_rn((double)a9_2, d);
-  a9_4 = (LUT)__dadd_rn((double)a9_4, d);
-  a9_9 = (LUT)__dsub_rn((double)a9_9, d);
-  a9_10 = (LUT)__dadd_rn((double)a9_10, d);
-  d = __dmul_rn(c.kf(16), z9);
-  d = __dmul_rn(d, factor);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  a2_9 = (LUT)__dsub_rn((double)a2_9, d);
-  a2_10 = (LUT)__dadd_rn((double)a2_10, d);
-  d = __dmul_rn(c.kr(16), z4);
-  d = __dmul_rn(d, msf);
-  a10_2 = (LUT)__dsub_rn((double)a10_2, d);
-  a10_4 = (LUT)__dadd_rn((double)a10_4, d);
-  a10_9 = (LUT)__dsub_rn((double)a10_9, d);
-  a10_10 = (LUT)__dadd_rn((double)a10_10, d);
-  d = __dmul_rn(c.kr(16), z10);
-  d = __dmul_rn(d, msf);
-  a4_2 = (LUT)__dsub_rn((double)a4_2, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_9 = (LUT)__dsub_rn((double)a4_9, d);
-  a4_10 = (LUT)__dadd_rn((double)a4_10, d);
-  d = __dmul_rn(c.kf(17), z3);
-  d = __dmul_rn(d, factor);
-  a9_3 = (LUT)__dsub_rn((double)a9_3, d);
-  a9_6 = (LUT)__dadd_rn((double)a9_6, d);
-  a9_9 = (LUT)__dsub_rn((double)a9_9, d);
-  a9_14 = (LUT)__dadd_rn((double)a9_14, d);
-  d = __dmul_rn(c.kf(17), z9);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  a3_9 = (LUT)__dsub_rn((double)a3_9, d);
-  a3_14 = (LUT)__dadd_rn((double)a3_14, d);
-  d = __dmul_rn(c.kr(17), z6);
-  d = __dmul_rn(d, msf);
-  a14_3 = (LUT)__dsub_rn((double)a14_3, d);
-  a14_6 = (LUT)__dadd_rn((double)a14_6, d);
-  a14_9 = (LUT)__dsub_rn((double)a14_9, d);
-  a14_14 = (LUT)__dadd_rn((double)a14_14, d);
-  d = __dmul_rn(c.kr(17), z14);
-  d = __dmul_rn(d, msf);
-  a6_3 = (LUT)__dsub_rn((double)a6_3, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_9 = (LUT)__dsub_rn((double)a6_9, d);
-  a6_14 = (LUT)__dadd_rn((double)a6_14, d);
-  d = __dmul_rn(c.kf(18), z1);
-  d = __dmul_rn(d, factor);
-  a10_1 = (LUT)__dsub_rn((double)a10_1, d);
-  a10_4 = (LUT)__dadd_rn((double)a10_4, d);
-  a10_6 = (LUT)__dadd_rn((double)a10_6, d);
-  a10_6 = (LUT)__dadd_rn((double)a10_6, d);
-  a10_10 = (LUT)__dsub_rn((double)a10_10, d);
-  d = __dmul_rn(c.kf(18), z10);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  a1_6 = (LUT)__dadd_rn((double)a1_6, d);
-  a1_6 = (LUT)__dadd_rn((double)a1_6, d);
-  a1_10 = (LUT)__dsub_rn((double)a1_10, d);
-  d = __dmul_rn(__dmul_rn(c.kr(18), z6), z4);
-  d = __dmul_rn(d, msf);
-  a6_1 = (LUT)__dsub_rn((double)a6_1, d);
-  a6_4 = (LUT)__dadd_rn((double)a6_4, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_10 = (LUT)__dsub_rn((double)a6_10, d);
-  d = __dmul_rn(__dmul_rn(c.kr(18), z6), z4);
-  d = __dmul_rn(d, msf);
-  a6_1 = (LUT)__dsub_rn((double)a6_1, d);
-  a6_4 = (LUT)__dadd_rn((double)a6_4, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_10 = (LUT)__dsub_rn((double)a6_10, d);
-  d = __dmul_rn(__dmul_rn(c.kr(18), z6), z6);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_6 = (LUT)__dadd_rn((double)a4_6, d);
-  a4_6 = (LUT)__dadd_rn((double)a4_6, d);
-  a4_10 = (LUT)__dsub_rn((double)a4_10, d);
-  d = c.kf(19);
-  d = __dmul_rn(d, factor);
-  a8_3 = (LUT)__dadd_rn((double)a8_3, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  a8_11 = (LUT)__dadd_rn((double)a8_11, d);
-  d = __dmul_rn(c.kr(19), z3);
-  d = __dmul_rn(d, msf);
-  a11_3 = (LUT)__dadd_rn((double)a11_3, d);
-  a11_8 = (LUT)__dsub_rn((double)a11_8, d);
-  a11_11 = (LUT)__dadd_rn((double)a11_11, d);
-  d = __dmul_rn(c.kr(19), z11);
-  d = __dmul_rn(d, msf);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_8 = (LUT)__dsub_rn((double)a3_8, d);
-  a3_11 = (LUT)__dadd_rn((double)a3_11, d);
-  d = __dmul_rn(c.kf(20), z3);
-  d = __dmul_rn(d, factor);
-  a8_3 = (LUT)__dsub_rn((double)a8_3, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  a8_11 = (LUT)__dadd_rn((double)a8_11, d);
-  a8_13 = (LUT)__dadd_rn((double)a8_13, d);
-  d = __dmul_rn(c.kf(20), z8);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_8 = (LUT)__dsub_rn((double)a3_8, d);
-  a3_11 = (LUT)__dadd_rn((double)a3_11, d);
-  a3_13 = (LUT)__dadd_rn((double)a3_13, d);
-  d = __dmul_rn(c.kr(20), z13);
-  d = __dmul_rn(d, msf);
-  a11_3 = (LUT)__dsub_rn((double)a11_3, d);
-  a11_8 = (LUT)__dsub_rn((double)a11_8, d);
-  a11_11 = (LUT)__dadd_rn((double)a11_11, d);
-  a11_13 = (LUT)__dadd_rn((double)a11_13, d);
-  d = __dmul_rn(c.kr(20), z11);
-  d = __dmul_rn(d, msf);
-  a13_3 = (LUT)__dsub_rn((double)a13_3, d);
-  a13_8 = (LUT)__dsub_rn((double)a13_8, d);
-  a13_11 = (LUT)__dadd_rn((double)a13_11, d);
-  a13_13 = (LUT)__dadd_rn((double)a13_13, d);
-  d = __dmul_rn(c.kf(21), z4);
-  d = __dmul_rn(d, factor);
-  a8_4 = (LUT)__dsub_rn((double)a8_4, d);
-  a8_5 = (LUT)__dadd_rn((double)a8_5, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  a8_11 = (LUT)__dadd_rn((double)a8_11, d);
-  d = __dmul_rn(c.kf(21), z8);
-  d = __dmul_rn(d, factor);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  a4_8 = (LUT)__dsub_rn((double)a4_8, d);
-  a4_11 = (LUT)__dadd_rn((double)a4_11, d);
-  d = __dmul_rn(c.kr(21), z5);
-  d = __dmul_rn(d, msf);
-  a11_4 = (LUT)__dsub_rn((double)a11_4, d);
-  a11_5 = (LUT)__dadd_rn((double)a11_5, d);
-  a11_8 = (LUT)__dsub_rn((double)a11_8, d);
-  a11_11 = (LUT)__dadd_rn((double)a11_11, d);
-  d = __dmul_rn(c.kr(21), z11);
-  d = __dmul_rn(d, msf);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  a5_8 = (LUT)__dsub_rn((double)a5_8, d);
-  a5_11 = (LUT)__dadd_rn((double)a5_11, d);
-  d = c.kf(22);
-  d = __dmul_rn(d, factor);
-  a11_3 = (LUT)__dadd_rn((double)a11_3, d);
-  a11_6 = (LUT)__dadd_rn((double)a11_6, d);
-  a11_11 = (LUT)__dsub_rn((double)a11_11, d);
-  d = __dmul_rn(c.kr(22), z3);
-  d = __dmul_rn(d, msf);
-  a6_3 = (LUT)__dadd_rn((double)a6_3, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_11 = (LUT)__dsub_rn((double)a6_11, d);
-  d = __dmul_rn(c.kr(22), z6);
-  d = __dmul_rn(d, msf);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  a3_11 = (LUT)__dsub_rn((double)a3_11, d);
-  d = __dmul_rn(c.kf(23), z3);
-  d = __dmul_rn(d, factor);
-  a11_3 = (LUT)__dsub_rn((double)a11_3, d);
-  a11_6 = (LUT)__dadd_rn((double)a11_6, d);
-  a11_11 = (LUT)__dsub_rn((double)a11_11, d);
-  a11_13 = (LUT)__dadd_rn((double)a11_13, d);
-  d = __dmul_rn(c.kf(23), z11);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  a3_11 = (LUT)__dsub_rn((double)a3_11, d);
-  a3_13 = (LUT)__dadd_rn((double)a3_13, d);
-  d = __dmul_rn(c.kr(23), z13);
-  d = __dmul_rn(d, msf);
-  a6_3 = (LUT)__dsub_rn((double)a6_3, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_11 = (LUT)__dsub_rn((double)a6_11, d);
-  a6_13 = (LUT)__dadd_rn((double)a6_13, d);
-  d = __dmul_rn(c.kr(23), z6);
-  d = __dmul_rn(d, msf);
-  a13_3 = (LUT)__dsub_rn((double)a13_3, d);
-  a13_6 = (LUT)__dadd_rn((double)a13_6, d);
-  a13_11 = (LUT)__dsub_rn((double)a13_11, d);
-  a13_13 = (LUT)__dadd_rn((double)a13_13, d);
-  d = __dmul_rn(c.kf(24), z2);
-  d = __dmul_rn(d, factor);
-  a14_2 = (LUT)__dsub_rn((double)a14_2, d);
-  a14_3 = (LUT)__dadd_rn((double)a14_3, d);
-  a14_8 = (LUT)__dadd_rn((double)a14_8, d);
-  a14_14 = (LUT)__dsub_rn((double)a14_14, d);
-  d = __dmul_rn(c.kf(24), z14);
-  d = __dmul_rn(d, factor);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_3 = (LUT)__dadd_rn((double)a2_3, d);
-  a2_8 = (LUT)__dadd_rn((double)a2_8, d);
-  a2_14 = (LUT)__dsub_rn((double)a2_14, d);
-  d = __dmul_rn(c.kr(24), z3);
-  d = __dmul_rn(d, msf);
-  a8_2 = (LUT)__dsub_rn((double)a8_2, d);
-  a8_3 = (LUT)__dadd_rn((double)a8_3, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_14 = (LUT)__dsub_rn((double)a8_14, d);
-  d = __dmul_rn(c.kr(24), z8);
-  d = __dmul_rn(d, msf);
-  a3_2 = (LUT)__dsub_rn((double)a3_2, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  a3_14 = (LUT)__dsub_rn((double)a3_14, d);
-  a0_0 = a0_0 + 1;
-  a1_1 = a1_1 + 1;
-  a2_2 = a2_2 + 1;
-  a3_3 = a3_3 + 1;
-  a4_4 = a4_4 + 1;
-  a5_5 = a5_5 + 1;
-  a6_6 = a6_6 + 1;
-  a7_7 = a7_7 + 1;
-  a8_8 = a8_8 + 1;
-  a9_9 = a9_9 + 1;
-  a10_10 = a10_10 + 1;
-  a11_11 = a11_11 + 1;
-  a12_12 = a12_12 + 1;
-  a13_13 = a13_13 + 1;
-  a14_14 = a14_14 + 1;
-  c.a(0, 0) = a0_0;
-  c.a(0, 1) = a0_1;
-  c.a(0, 2) = a0_2;
-  c.a(0, 3) = a0_3;
-  c.a(0, 4) = a0_4;
-  c.a(0, 5) = a0_5;
-  c.a(0, 6) = a0_6;
-  c.a(0, 7) = a0_7;
-  c.a(0, 8) = a0_8;
-  c.a(0, 9) = a0_9;
-  c.a(0, 10) = a0_10;
-  c.a(0, 11) = a0_11;
-  c.a(0, 12) = a0_12;
-  c.a(0, 13) = a0_13;
-  c.a(0, 14) = a0_14;
-  c.a(1, 0) = a1_0;
-  c.a(1, 1) = a1_1;
-  c.a(1, 2) = a1_2;
-  c.a(1, 3) = a1_3;
-  c.a(1, 4) = a1_4;
-  c.a(1, 5) = a1_5;
-  c.a(1, 6) = a1_6;
-  c.a(1, 7) = a1_7;
-  c.a(1, 8) = a1_8;
-  c.a(1, 9) = a1_9;
-  c.a(1, 10) = a1_10;
-  c.a(1, 11) = a1_11;
-  c.a(1, 12) = a1_12;
-  c.a(1, 13) = a1_13;
-  c.a(1, 14) = a1_14;
-  c.a(2, 0) = a2_0;
-  c.a(2, 1) = a2_1;
-  c.a(2, 2) = a2_2;
-  c.a(2, 3) = a2_3;
-  c.a(2, 4) = a2_4;
-  c.a(2, 5) = a2_5;
-  c.a(2, 6) = a2_6;
-  c.a(2, 7) = a2_7;
-  c.a(2, 8) = a2_8;
-  c.a(2, 9) = a2_9;
-  c.a(2, 10) = a2_10;
-  c.a(2, 11) = a2_11;
-  c.a(2, 12) = a2_12;
-  c.a(2, 13) = a2_13;
-  c.a(2, 14) = a2_14;
-  c.a(3, 0) = a3_0;
-  c.a(3, 1) = a3_1;
-  c.a(3, 2) = a3_2;
-  c.a(3, 3) = a3_3;
-  c.a(3, 4) = a3_4;
-  c.a(3, 5) = a3_5;
-  c.a(3, 6) = a3_6;
-  c.a(3, 7) = a3_7;
-  c.a(3, 8) = a3_8;
-  c.a(3, 9) = a3_9;
-  c.a(3, 10) = a3_10;
-  c.a(3, 11) = a3_11;
-  c.a(3, 12) = a3_12;
-  c.a(3, 13) = a3_13;
-  c.a(3, 14) = a3_14;
-  c.a(4, 0) = a4_0;
-  c.a(4, 1) = a4_1;
-  c.a(4, 2) = a4_2;
-  c.a(4, 3) = a4_3;
-  c.a(4, 4) = a4_4;
-  c.a(4, 5) = a4_5;
-  c.a(4, 6) = a4_6;
-  c.a(4, 7) = a4_7;
-  c.a(4, 8) = a4_8;
-  c.a(4, 9) = a4_9;
-  c.a(4, 10) = a4_10;
-  c.a(4, 11) = a4_11;
-  c.a(4, 12) = a4_12;
-  c.a(4, 13) = a4_13;
-  c.a(4, 14) = a4_14;
-  c.a(5, 0) = a5_0;
-  c.a(5, 1) = a5_1;
-  c.a(5, 2) = a5_2;
-  c.a(5, 3) = a5_3;
-  c.a(5, 4) = a5_4;
-  c.a(5, 5) = a5_5;
-  c.a(5, 6) = a5_6;
-  c.a(5, 7) = a5_7;
-  c.a(5, 8) = a5_8;
-  c.a(5, 9) = a5_9;
-  c.a(5, 10) = a5_10;
-  c.a(5, 11) = a5_11;
-  c.a(5, 12) = a5_12;
-  c.a(5, 13) = a5_13;
-  c.a(5, 14) = a5_14;
-  c.a(6, 0) = a6_0;
-  c.a(6, 1) = a6_1;
-  c.a(6, 2) = a6_2;
-  c.a(6, 3) = a6_3;
-  c.a(6, 4) = a6_4;
-  c.a(6, 5) = a6_5;
-  c.a(6, 6) = a6_6;
-  c.a(6, 7) = a6_7;
-  c.a(6, 8) = a6_8;
-  c.a(6, 9) = a6_9;
-  c.a(6, 10) = a6_10;
-  c.a(6, 11) = a6_11;
-  c.a(6, 12) = a6_12;
-  c.a(6, 13) = a6_13;
-  c.a(6, 14) = a6_14;
-  c.a(7, 0) = a7_0;
-  c.a(7, 1) = a7_1;
-  c.a(7, 2) = a7_2;
-  c.a(7, 3) = a7_3;
-  c.a(7, 4) = a7_4;
-  c.a(7, 5) = a7_5;
-  c.a(7, 6) = a7_6;
-  c.a(7, 7) = a7_7;
-  c.a(7, 8) = a7_8;
-  c.a(7, 9) = a7_9;
-  c.a(7, 10) = a7_10;
-  c.a(7, 11) = a7_11;
-  c.a(7, 12) = a7_12;
-  c.a(7, 13) = a7_13;
-  c.a(7, 14) = a7_14;
-  c.a(8, 0) = a8_0;
-  c.a(8, 1) = a8_1;
-  c.a(8, 2) = a8_2;
-  c.a(8, 3) = a8_3;
-  c.a(8, 4) = a8_4;
-  c.a(8, 5) = a8_5;
-  c.a(8, 6) = a8_6;
-  c.a(8, 7) = a8_7;
-  c.a(8, 8) = a8_8;
-  c.a(8, 9) = a8_9;
-  c.a(8, 10) = a8_10;
-  c.a(8, 11) = a8_11;
-  c.a(8, 12) = a8_12;
-  c.a(8, 13) = a8_13;
-  c.a(8, 14) = a8_14;
-  c.a(9, 0) = a9_0;
-  c.a(9, 1) = a9_1;
-  c.a(9, 2) = a9_2;
-  c.a(9, 3) = a9_3;
-  c.a(9, 4) = a9_4;
-  c.a(9, 5) = a9_5;
-  c.a(9, 6) = a9_6;
-  c.a(9, 7) = a9_7;
-  c.a(9, 8) = a9_8;
-  c.a(9, 9) = a9_9;
-  c.a(9, 10) = a9_10;
-  c.a(9, 11) = a9_11;
-  c.a(9, 12) = a9_12;
-  c.a(9, 13) = a9_13;
-  c.a(9, 14) = a9_14;
-  c.a(10, 0) = a10_0;
-  c.a(10, 1) = a10_1;
-  c.a(10, 2) = a10_2;
-  c.a(10, 3) = a10_3;
-  c.a(10, 4) = a10_4;
-  c.a(10, 5) = a10_5;
-  c.a(10, 6) = a10_6;
-  c.a(10, 7) = a10_7;
-  c.a(10, 8) = a10_8;
-  c.a(10, 9) = a10_9;
-  c.a(10, 10) = a10_10;
-  c.a(10, 11) = a10_11;
-  c.a(10, 12) = a10_12;
-  c.a(10, 13) = a10_13;
-  c.a(10, 14) = a10_14;
-  c.a(11, 0) = a11_0;
-  c.a(11, 1) = a11_1;
-  c.a(11, 2) = a11_2;
-  c.a(11, 3) = a11_3;
-  c.a(11, 4) = a11_4;
-  c.a(11, 5) = a11_5;
-  c.a(11, 6) = a11_6;
-  c.a(11, 7) = a11_7;
-  c.a(11, 8) = a11_8;
-  c.a(11, 9) = a11_9;
-  c.a(11, 10) = a11_10;
-  c.a(11, 11) = a11_11;
-  c.a(11, 12) = a11_12;
-  c.a(11, 13) = a11_13;
-  c.a(11, 14) = a11_14;
-  c.a(12, 0) = a12_0;
-  c.a(12, 1) = a12_1;
-  c.a(12, 2) = a12_2;
-  c.a(12, 3) = a12_3;
-  c.a(12, 4) = a12_4;
-  c.a(12, 5) = a12_5;
-  c.a(12, 6) = a12_6;
-  c.a(12, 7) = a12_7;
-  c.a(12, 8) = a12_8;
-  c.a(12, 9) = a12_9;
-  c.a(12, 10) = a12_10;
-  c.a(12, 11) = a12_11;
-  c.a(12, 12) = a12_12;
-  c.a(12, 13) = a12_13;
-  c.a(12, 14) = a12_14;
-  c.a(13, 0) = a13_0;
-  c.a(13, 1) = a13_1;
-  c.a(13, 2) = a13_2;
-  c.a(13, 3) = a13_3;
-  c.a(13, 4) = a13_4;
-  c.a(13, 5) = a13_5;
-  c.a(13, 6) = a13_6;
-  c.a(13, 7) = a13_7;
-  c.a(13, 8) = a13_8;
-  c.a(13, 9) = a13_9;
-  c.a(13, 10) = a13_10;
-  c.a(13, 11) = a13_11;
-  c.a(13, 12) = a13_12;
-  c.a(13, 13) = a13_13;
-  c.a(13, 14) = a13_14;
-  c.a(14, 0) = a14_0;
-  c.a(14, 1) = a14_1;
-  c.a(14, 2) = a14_2;
-  c.a(14, 3) = a14_3;
-  c.a(14, 4) = a14_4;
-  c.a(14, 5) = a14_5;
-  c.a(14, 6) = a14_6;
-  c.a(14, 7) = a14_7;
-  c.a(14, 8) = a14_8;
-  c.a(14, 9) = a14_9;
-  c.a(14, 10) = a14_10;
-  c.a(14, 11) = a14_11;
-  c.a(14, 12) = a14_12;
-  c.a(14, 13) = a14_13;
-  c.a(14, 14) = a14_14;
+  if constexpr (J == 0) {
+    const double z1 = c.z(1), z2 = c.z(2), z4 = c.z(4);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(13), z1), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(14), z2), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a10 = (LUT)__dadd_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kf(15), z4), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    a0 = a0 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 1) {
+    const double z0 = c.z(0), z3 = c.z(3), z5 = c.z(5), z10 = c.z(10), z13 = c.z(13);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(0), z3), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(1), z3), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(5), z3), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a12 = (LUT)__dadd_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(c.kr(7), z13), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kr(8), z5), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(c.kf(13), z0), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(18), z10), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a10 = (LUT)__dsub_rn((double)a10, d);
+    a1 = a1 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 2) {
+    const double z0 = c.z(0), z4 = c.z(4), z5 = c.z(5), z9 = c.z(9), z14 = c.z(14);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(0), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(1), z4), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(3), z5), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(4), z5), msf);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(14), z0), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a10 = (LUT)__dadd_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kf(16), z9), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    a10 = (LUT)__dadd_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kf(24), z14), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a14 = (LUT)__dsub_rn((double)a14, d);
+    a2 = a2 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 3) {
+    const double z1 = c.z(1), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6), z7 = c.z(7), z8 = c.z(8), z9 = c.z(9), z10 = c.z(10), z11 = c.z(11), z12 = c.z(12);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(0), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(1), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(2), z5), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a13 = (LUT)__dsub_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kf(5), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a12 = (LUT)__dadd_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(c.kf(6), z12), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(c.kf(7), z12), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kf(9), z4), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(10), z4), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(11), z7), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a7 = (LUT)__dadd_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(12), z7), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(14), z10), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a10 = (LUT)__dadd_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kr(15), z9), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(17), z9), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    a14 = (LUT)__dadd_rn((double)a14, d);
+    d = __dmul_rn(__dmul_rn(c.kr(19), z11), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kf(20), z8), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kr(22), z6), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kf(23), z11), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kr(24), z8), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a14 = (LUT)__dsub_rn((double)a14, d);
+    a3 = a3 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 4) {
+    const double z0 = c.z(0), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4), z6 = c.z(6), z8 = c.z(8), z10 = c.z(10), z12 = c.z(12), z13 = c.z(13);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(0), z2), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(1), z2), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(2), z13), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a13 = (LUT)__dsub_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kr(3), z4), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(3), z4), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(4), z4), factor);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(4), z4), factor);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(6), z4), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(c.kr(6), z4), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(c.kf(8), z12), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(c.kf(9), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(10), z3), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(11), z6), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a7 = (LUT)__dadd_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(12), z6), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(15), z0), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(16), z10), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    a10 = (LUT)__dadd_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(18), z6), z6), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a10 = (LUT)__dsub_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kf(21), z8), factor);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    a4 = a4 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 5) {
+    const double z1 = c.z(1), z2 = c.z(2), z3 = c.z(3), z11 = c.z(11);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(2), z3), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a13 = (LUT)__dsub_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kf(3), z2), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(4), z2), msf);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(8), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    d = __dmul_rn(c.kr(9), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(c.kf(10), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(21), z11), msf);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    a5 = a5 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 6) {
+    const double z3 = c.z(3), z4 = c.z(4), z6 = c.z(6), z8 = c.z(8), z13 = c.z(13), z14 = c.z(14);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(11), z4), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a7 = (LUT)__dadd_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(12), z4), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(13), z8), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(17), z14), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    a14 = (LUT)__dadd_rn((double)a14, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(18), z6), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a10 = (LUT)__dsub_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(18), z6), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a10 = (LUT)__dsub_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kr(22), z3), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kr(23), z13), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    a6 = a6 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 7) {
+    const double z3 = c.z(3);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(11), z3), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a7 = (LUT)__dadd_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(12), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a7 = a7 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 8) {
+    const double z3 = c.z(3), z4 = c.z(4), z6 = c.z(6);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(13), z6), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(c.kf(19), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kf(20), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kf(21), z4), factor);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kr(24), z3), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a14 = (LUT)__dsub_rn((double)a14, d);
+    a8 = a8 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 9) {
+    const double z2 = c.z(2), z3 = c.z(3);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(15), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(16), z2), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    a10 = (LUT)__dadd_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kf(17), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    a14 = (LUT)__dadd_rn((double)a14, d);
+    a9 = a9 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 10) {
+    const double z1 = c.z(1), z3 = c.z(3), z4 = c.z(4);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(14), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a10 = (LUT)__dadd_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kr(16), z4), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    a10 = (LUT)__dadd_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kf(18), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a10 = (LUT)__dsub_rn((double)a10, d);
+    a10 = a10 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 11) {
+    const double z3 = c.z(3), z5 = c.z(5), z13 = c.z(13);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(19), z3), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kr(20), z13), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kr(21), z5), msf);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    d = __dmul_rn(c.kf(22), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kf(23), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    a11 = a11 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 12) {
+    const double z3 = c.z(3), z4 = c.z(4);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(c.kr(5), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a12 = (LUT)__dadd_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(c.kf(6), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(c.kf(7), z3), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kf(8), z4), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    a12 = a12 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 13) {
+    const double z1 = c.z(1), z4 = c.z(4), z6 = c.z(6), z11 = c.z(11);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(2), z4), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a13 = (LUT)__dsub_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kr(7), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kr(20), z11), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a11 = (LUT)__dadd_rn((double)a11, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    d = __dmul_rn(__dmul_rn(c.kr(23), z6), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    a13 = (LUT)__dadd_rn((double)a13, d);
+    a13 = a13 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
+  if constexpr (J == 14) {
+    const double z2 = c.z(2), z6 = c.z(6);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0, a13 = (LUT)0, a14 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(17), z6), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    a14 = (LUT)__dadd_rn((double)a14, d);
+    d = __dmul_rn(__dmul_rn(c.kf(24), z2), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a14 = (LUT)__dsub_rn((double)a14, d);
+    a14 = a14 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9; v[10] = a10; v[11] = a11; v[12] = a12; v[13] = a13; v[14] = a14;
+  }
 }
 
 }  // namespace gen_acetylene

@@ -23,48 +23,58 @@ struct SpecOf<kSpecKeromnes> {
   static constexpr int kN = gen_keromnes::kSpecN, kR = gen_keromnes::kSpecR;
   template <class S>
   __device__ static void rhs(S& c) { gen_keromnes::spec_rhs(c); }
-  template <class S, typename LUT>
-  __device__ static void matrix(S& c, double f) { gen_keromnes::spec_matrix<S, LUT>(c, f); }
+  template <int J, class S, typename LUT>
+  __device__ static void column(const S& c, double f, LUT (&v)[gen_keromnes::kSpecN]) {
+    gen_keromnes::spec_column<J>(c, f, v);
+  }
 };
 template <>
 struct SpecOf<kSpecZhang> {
   static constexpr int kN = gen_zhang::kSpecN, kR = gen_zhang::kSpecR;
   template <class S>
   __device__ static void rhs(S& c) { gen_zhang::spec_rhs(c); }
-  template <class S, typename LUT>
-  __device__ static void matrix(S& c, double f) { gen_zhang::spec_matrix<S, LUT>(c, f); }
+  template <int J, class S, typename LUT>
+  __device__ static void column(const S& c, double f, LUT (&v)[gen_zhang::kSpecN]) {
+    gen_zhang::spec_column<J>(c, f, v);
+  }
 };
 template <>
 struct SpecOf<kSpecTereza> {
   static constexpr int kN = gen_tereza::kSpecN, kR = gen_tereza::kSpecR;
   template <class S>
   __device__ static void rhs(S& c) { gen_tereza::spec_rhs(c); }
-  template <class S, typename LUT>
-  __device__ static void matrix(S& c, double f) { gen_tereza::spec_matrix<S, LUT>(c, f); }
+  template <int J, class S, typename LUT>
+  __device__ static void column(const S& c, double f, LUT (&v)[gen_tereza::kSpecN]) {
+    gen_tereza::spec_column<J>(c, f, v);
+  }
 };
 template <>
 struct SpecOf<kSpecKonnov> {
   static constexpr int kN = gen_konnov::kSpecN, kR = gen_konnov::kSpecR;
   template <class S>
   __device__ static void rhs(S& c) { gen_konnov::spec_rhs(c); }
-  template <class S, typename LUT>
-  __device__ static void matrix(S& c, double f) { gen_konnov::spec_matrix<S, LUT>(c, f); }
+  template <int J, class S, typename LUT>
+  __device__ static void column(const S& c, double f, LUT (&v)[gen_konnov::kSpecN]) {
+    gen_konnov::spec_column<J>(c, f, v);
+  }
 };
 template <>
 struct SpecOf<kSpecAcetylene> {
   static constexpr int kN = gen_acetylene::kSpecN, kR = gen_acetylene::kSpecR;
   template <class S>
   __device__ static void rhs(S& c) { gen_acetylene::spec_rhs(c); }
-  template <class S, typename LUT>
-  __device__ static void matrix(S& c, double f) { gen_acetylene::spec_matrix<S, LUT>(c, f); }
+  template <int J, class S, typename LUT>
+  __device__ static void column(const S& c, double f, LUT (&v)[gen_acetylene::kSpecN]) {
+    gen_acetylene::spec_column<J>(c, f, v);
+  }
 };
 
 // 0 when the reduced reaction lists match none of the generated codes.
 template <class M>
 inline int match_specialised_tables(const M& m) {
-  if (m.NI == gen_keromnes::kSpecN && m.R == gen_keromnes::kSpecR) {
+  if (m.NI == gen_keromnes::kSpecN && m.RM == gen_keromnes::kSpecR) {
     bool ok = true;
-    for (int r = 0; ok && r < m.R; ++r) {
+    for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_keromnes::kSpecNupd[r];
       for (int i = 0; ok && i < 3; ++i)
         ok = m.left[r][i] == gen_keromnes::kSpecLeft[r][i] && m.right[r][i] == gen_keromnes::kSpecRight[r][i];
@@ -73,9 +83,9 @@ inline int match_specialised_tables(const M& m) {
     }
     if (ok) return kSpecKeromnes;
   }
-  if (m.NI == gen_zhang::kSpecN && m.R == gen_zhang::kSpecR) {
+  if (m.NI == gen_zhang::kSpecN && m.RM == gen_zhang::kSpecR) {
     bool ok = true;
-    for (int r = 0; ok && r < m.R; ++r) {
+    for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_zhang::kSpecNupd[r];
       for (int i = 0; ok && i < 3; ++i)
         ok = m.left[r][i] == gen_zhang::kSpecLeft[r][i] && m.right[r][i] == gen_zhang::kSpecRight[r][i];
@@ -84,9 +94,9 @@ inline int match_specialised_tables(const M& m) {
     }
     if (ok) return kSpecZhang;
   }
-  if (m.NI == gen_tereza::kSpecN && m.R == gen_tereza::kSpecR) {
+  if (m.NI == gen_tereza::kSpecN && m.RM == gen_tereza::kSpecR) {
     bool ok = true;
-    for (int r = 0; ok && r < m.R; ++r) {
+    for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_tereza::kSpecNupd[r];
       for (int i = 0; ok && i < 3; ++i)
         ok = m.left[r][i] == gen_tereza::kSpecLeft[r][i] && m.right[r][i] == gen_tereza::kSpecRight[r][i];
@@ -95,9 +105,9 @@ inline int match_specialised_tables(const M& m) {
     }
     if (ok) return kSpecTereza;
   }
-  if (m.NI == gen_konnov::kSpecN && m.R == gen_konnov::kSpecR) {
+  if (m.NI == gen_konnov::kSpecN && m.RM == gen_konnov::kSpecR) {
     bool ok = true;
-    for (int r = 0; ok && r < m.R; ++r) {
+    for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_konnov::kSpecNupd[r];
       for (int i = 0; ok && i < 3; ++i)
         ok = m.left[r][i] == gen_konnov::kSpecLeft[r][i] && m.right[r][i] == gen_konnov::kSpecRight[r][i];
@@ -106,9 +116,9 @@ inline int match_specialised_tables(const M& m) {
     }
     if (ok) return kSpecKonnov;
   }
-  if (m.NI == gen_acetylene::kSpecN && m.R == gen_acetylene::kSpecR) {
+  if (m.NI == gen_acetylene::kSpecN && m.RM == gen_acetylene::kSpecR) {
     bool ok = true;
-    for (int r = 0; ok && r < m.R; ++r) {
+    for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_acetylene::kSpecNupd[r];
       for (int i = 0; ok && i < 3; ++i)
         ok = m.left[r][i] == gen_acetylene::kSpecLeft[r][i] && m.right[r][i] == gen_acetylene::kSpecRight[r][i];

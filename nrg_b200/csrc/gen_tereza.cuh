@@ -303,647 +303,498 @@ __device__ __forceinline__ void spec_rhs(S& c) {
   c.zd(9) = d9;
 }
 
-// I + factor * J written into the LU storage: c.a(j, i) = A(i+1, j+1)
-template <class S, typename LUT>
-__device__ __forceinline__ void spec_matrix(S& c, double factor) {
-  const double z0 = c.z(0);
-  const double z1 = c.z(1);
-  const double z2 = c.z(2);
-  const double z3 = c.z(3);
-  const double z4 = c.z(4);
-  const double z5 = c.z(5);
-  const double z6 = c.z(6);
-  const double z7 = c.z(7);
-  const double z8 = c.z(8);
-  const double z9 = c.z(9);
+// Column J of I + factor * J: v[i] = A(i+1, J+1), each element's terms in
+// reaction order.
+template <int J, class S, typename LUT>
+__device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[10]) {
   const double msf = -factor;
-  LUT a0_0 = (LUT)0, a0_1 = (LUT)0, a0_2 = (LUT)0, a0_3 = (LUT)0, a0_4 = (LUT)0, a0_5 = (LUT)0, a0_6 = (LUT)0, a0_7 = (LUT)0, a0_8 = (LUT)0, a0_9 = (LUT)0, a1_0 = (LUT)0, a1_1 = (LUT)0, a1_2 = (LUT)0, a1_3 = (LUT)0, a1_4 = (LUT)0, a1_5 = (LUT)0, a1_6 = (LUT)0, a1_7 = (LUT)0, a1_8 = (LUT)0, a1_9 = (LUT)0, a2_0 = (LUT)0, a2_1 = (LUT)0, a2_2 = (LUT)0, a2_3 = (LUT)0, a2_4 = (LUT)0, a2_5 = (LUT)0, a2_6 = (LUT)0, a2_7 = (LUT)0, a2_8 = (LUT)0, a2_9 = (LUT)0, a3_0 = (LUT)0, a3_1 = (LUT)0, a3_2 = (LUT)0, a3_3 = (LUT)0, a3_4 = (LUT)0, a3_5 = (LUT)0, a3_6 = (LUT)0, a3_7 = (LUT)0, a3_8 = (LUT)0, a3_9 = (LUT)0, a4_0 = (LUT)0, a4_1 = (LUT)0, a4_2 = (LUT)0, a4_3 = (LUT)0, a4_4 = (LUT)0, a4_5 = (LUT)0, a4_6 = (LUT)0, a4_7 = (LUT)0, a4_8 = (LUT)0, a4_9 = (LUT)0, a5_0 = (LUT)0, a5_1 = (LUT)0, a5_2 = (LUT)0, a5_3 = (LUT)0, a5_4 = (LUT)0, a5_5 = (LUT)0, a5_6 = (LUT)0, a5_7 = (LUT)0, a5_8 = (LUT)0, a5_9 = (LUT)0, a6_0 = (LUT)0, a6_1 = (LUT)0, a6_2 = (LUT)0, a6_3 = (LUT)0, a6_4 = (LUT)0, a6_5 = (LUT)0, a6_6 = (LUT)0, a6_7 = (LUT)0, a6_8 = (LUT)0, a6_9 = (LUT)0, a7_0 = (LUT)0, a7_1 = (LUT)0, a7_2 = (LUT)0, a7_3 = (LUT)0, a7_4 = (LUT)0, a7_5 = (LUT)0, a7_6 = (LUT)0, a7_7 = (LUT)0, a7_8 = (LUT)0, a7_9 = (LUT)0, a8_0 = (LUT)0, a8_1 = (LUT)0, a8_2 = (LUT)0, a8_3 = (LUT)0, a8_4 = (LUT)0, a8_5 = (LUT)0, a8_6 = (LUT)0, a8_7 = (LUT)0, a8_8 = (LUT)0, a8_9 = (LUT)0, a9_0 = (LUT)0, a9_1 = (LUT)0, a9_2 = (LUT)0, a9_3 = (LUT)0, a9_4 = (LUT)0, a9_5 = (LUT)0, a9_6 = (LUT)0, a9_7 = (LUT)0, a9_8 = (LUT)0, a9_9 = (LUT)0;
   double d;
-  d = __dmul_rn(c.kf(0), z1);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  d = __dmul_rn(c.kf(0), z3);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  a1_8 = (LUT)__dadd_rn((double)a1_8, d);
-  d = __dmul_rn(c.kr(0), z8);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_8 = (LUT)__dadd_rn((double)a4_8, d);
-  d = __dmul_rn(c.kr(0), z4);
-  d = __dmul_rn(d, msf);
-  a8_1 = (LUT)__dsub_rn((double)a8_1, d);
-  a8_3 = (LUT)__dsub_rn((double)a8_3, d);
-  a8_4 = (LUT)__dadd_rn((double)a8_4, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kf(1), z4);
-  d = __dmul_rn(d, factor);
-  a9_1 = (LUT)__dadd_rn((double)a9_1, d);
-  a9_4 = (LUT)__dsub_rn((double)a9_4, d);
-  a9_8 = (LUT)__dadd_rn((double)a9_8, d);
-  a9_9 = (LUT)__dsub_rn((double)a9_9, d);
-  d = __dmul_rn(c.kf(1), z9);
-  d = __dmul_rn(d, factor);
-  a4_1 = (LUT)__dadd_rn((double)a4_1, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_8 = (LUT)__dadd_rn((double)a4_8, d);
-  a4_9 = (LUT)__dsub_rn((double)a4_9, d);
-  d = __dmul_rn(c.kr(1), z1);
-  d = __dmul_rn(d, msf);
-  a8_1 = (LUT)__dadd_rn((double)a8_1, d);
-  a8_4 = (LUT)__dsub_rn((double)a8_4, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_9 = (LUT)__dsub_rn((double)a8_9, d);
-  d = __dmul_rn(c.kr(1), z8);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_4 = (LUT)__dsub_rn((double)a1_4, d);
-  a1_8 = (LUT)__dadd_rn((double)a1_8, d);
-  a1_9 = (LUT)__dsub_rn((double)a1_9, d);
-  d = __dmul_rn(c.kf(2), z3);
-  d = __dmul_rn(d, factor);
-  a9_3 = (LUT)__dsub_rn((double)a9_3, d);
-  a9_8 = (LUT)__dadd_rn((double)a9_8, d);
-  a9_8 = (LUT)__dadd_rn((double)a9_8, d);
-  a9_9 = (LUT)__dsub_rn((double)a9_9, d);
-  d = __dmul_rn(c.kf(2), z9);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  a3_9 = (LUT)__dsub_rn((double)a3_9, d);
-  d = __dmul_rn(c.kr(2), z8);
-  d = __dmul_rn(d, msf);
-  a8_3 = (LUT)__dsub_rn((double)a8_3, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_9 = (LUT)__dsub_rn((double)a8_9, d);
-  d = __dmul_rn(c.kr(2), z8);
-  d = __dmul_rn(d, msf);
-  a8_3 = (LUT)__dsub_rn((double)a8_3, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_9 = (LUT)__dsub_rn((double)a8_9, d);
-  d = __dmul_rn(c.kf(3), z3);
-  d = __dmul_rn(d, factor);
-  a9_3 = (LUT)__dsub_rn((double)a9_3, d);
-  a9_4 = (LUT)__dadd_rn((double)a9_4, d);
-  a9_6 = (LUT)__dadd_rn((double)a9_6, d);
-  a9_9 = (LUT)__dsub_rn((double)a9_9, d);
-  d = __dmul_rn(c.kf(3), z9);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  a3_9 = (LUT)__dsub_rn((double)a3_9, d);
-  d = __dmul_rn(c.kr(3), z4);
-  d = __dmul_rn(d, msf);
-  a6_3 = (LUT)__dsub_rn((double)a6_3, d);
-  a6_4 = (LUT)__dadd_rn((double)a6_4, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_9 = (LUT)__dsub_rn((double)a6_9, d);
-  d = __dmul_rn(c.kr(3), z6);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_6 = (LUT)__dadd_rn((double)a4_6, d);
-  a4_9 = (LUT)__dsub_rn((double)a4_9, d);
-  d = __dmul_rn(c.kf(4), z4);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  a0_4 = (LUT)__dsub_rn((double)a0_4, d);
-  a0_8 = (LUT)__dadd_rn((double)a0_8, d);
-  d = __dmul_rn(c.kf(4), z0);
-  d = __dmul_rn(d, factor);
-  a4_0 = (LUT)__dsub_rn((double)a4_0, d);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_8 = (LUT)__dadd_rn((double)a4_8, d);
-  d = __dmul_rn(c.kr(4), z8);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  d = __dmul_rn(c.kr(4), z3);
-  d = __dmul_rn(d, msf);
-  a8_0 = (LUT)__dsub_rn((double)a8_0, d);
-  a8_3 = (LUT)__dadd_rn((double)a8_3, d);
-  a8_4 = (LUT)__dsub_rn((double)a8_4, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kf(5), z8);
-  d = __dmul_rn(d, factor);
-  a8_4 = (LUT)__dadd_rn((double)a8_4, d);
-  a8_6 = (LUT)__dadd_rn((double)a8_6, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  d = __dmul_rn(c.kf(5), z8);
-  d = __dmul_rn(d, factor);
-  a8_4 = (LUT)__dadd_rn((double)a8_4, d);
-  a8_6 = (LUT)__dadd_rn((double)a8_6, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(5), z4);
-  d = __dmul_rn(d, msf);
-  a6_4 = (LUT)__dadd_rn((double)a6_4, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_8 = (LUT)__dsub_rn((double)a6_8, d);
-  a6_8 = (LUT)__dsub_rn((double)a6_8, d);
-  d = __dmul_rn(c.kr(5), z6);
-  d = __dmul_rn(d, msf);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_6 = (LUT)__dadd_rn((double)a4_6, d);
-  a4_8 = (LUT)__dsub_rn((double)a4_8, d);
-  a4_8 = (LUT)__dsub_rn((double)a4_8, d);
-  d = __dmul_rn(c.kf(6), z8);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  a0_6 = (LUT)__dadd_rn((double)a0_6, d);
-  a0_8 = (LUT)__dsub_rn((double)a0_8, d);
-  d = __dmul_rn(c.kf(6), z0);
-  d = __dmul_rn(d, factor);
-  a8_0 = (LUT)__dsub_rn((double)a8_0, d);
-  a8_3 = (LUT)__dadd_rn((double)a8_3, d);
-  a8_6 = (LUT)__dadd_rn((double)a8_6, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(6), z3);
-  d = __dmul_rn(d, msf);
-  a6_0 = (LUT)__dsub_rn((double)a6_0, d);
-  a6_3 = (LUT)__dadd_rn((double)a6_3, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_8 = (LUT)__dsub_rn((double)a6_8, d);
-  d = __dmul_rn(c.kr(6), z6);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  a3_8 = (LUT)__dsub_rn((double)a3_8, d);
-  d = __dmul_rn(c.kf(7), z1);
-  d = __dmul_rn(d, factor);
-  a7_1 = (LUT)__dsub_rn((double)a7_1, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  a7_9 = (LUT)__dadd_rn((double)a7_9, d);
-  a7_9 = (LUT)__dadd_rn((double)a7_9, d);
-  d = __dmul_rn(c.kf(7), z7);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_7 = (LUT)__dsub_rn((double)a1_7, d);
-  a1_9 = (LUT)__dadd_rn((double)a1_9, d);
-  a1_9 = (LUT)__dadd_rn((double)a1_9, d);
-  d = __dmul_rn(c.kr(7), z9);
-  d = __dmul_rn(d, msf);
-  a9_1 = (LUT)__dsub_rn((double)a9_1, d);
-  a9_7 = (LUT)__dsub_rn((double)a9_7, d);
-  a9_9 = (LUT)__dadd_rn((double)a9_9, d);
-  a9_9 = (LUT)__dadd_rn((double)a9_9, d);
-  d = __dmul_rn(c.kr(7), z9);
-  d = __dmul_rn(d, msf);
-  a9_1 = (LUT)__dsub_rn((double)a9_1, d);
-  a9_7 = (LUT)__dsub_rn((double)a9_7, d);
-  a9_9 = (LUT)__dadd_rn((double)a9_9, d);
-  a9_9 = (LUT)__dadd_rn((double)a9_9, d);
-  d = __dmul_rn(c.kf(8), z8);
-  d = __dmul_rn(d, factor);
-  a7_6 = (LUT)__dadd_rn((double)a7_6, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  a7_8 = (LUT)__dsub_rn((double)a7_8, d);
-  a7_9 = (LUT)__dadd_rn((double)a7_9, d);
-  d = __dmul_rn(c.kf(8), z7);
-  d = __dmul_rn(d, factor);
-  a8_6 = (LUT)__dadd_rn((double)a8_6, d);
-  a8_7 = (LUT)__dsub_rn((double)a8_7, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  a8_9 = (LUT)__dadd_rn((double)a8_9, d);
-  d = __dmul_rn(c.kr(8), z9);
-  d = __dmul_rn(d, msf);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_7 = (LUT)__dsub_rn((double)a6_7, d);
-  a6_8 = (LUT)__dsub_rn((double)a6_8, d);
-  a6_9 = (LUT)__dadd_rn((double)a6_9, d);
-  d = __dmul_rn(c.kr(8), z6);
-  d = __dmul_rn(d, msf);
-  a9_6 = (LUT)__dadd_rn((double)a9_6, d);
-  a9_7 = (LUT)__dsub_rn((double)a9_7, d);
-  a9_8 = (LUT)__dsub_rn((double)a9_8, d);
-  a9_9 = (LUT)__dadd_rn((double)a9_9, d);
-  d = __dmul_rn(c.kf(9), z3);
-  d = __dmul_rn(d, factor);
-  a7_0 = (LUT)__dadd_rn((double)a7_0, d);
-  a7_3 = (LUT)__dsub_rn((double)a7_3, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  a7_9 = (LUT)__dadd_rn((double)a7_9, d);
-  d = __dmul_rn(c.kf(9), z7);
-  d = __dmul_rn(d, factor);
-  a3_0 = (LUT)__dadd_rn((double)a3_0, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_7 = (LUT)__dsub_rn((double)a3_7, d);
-  a3_9 = (LUT)__dadd_rn((double)a3_9, d);
-  d = __dmul_rn(c.kr(9), z0);
-  d = __dmul_rn(d, msf);
-  a9_0 = (LUT)__dadd_rn((double)a9_0, d);
-  a9_3 = (LUT)__dsub_rn((double)a9_3, d);
-  a9_7 = (LUT)__dsub_rn((double)a9_7, d);
-  a9_9 = (LUT)__dadd_rn((double)a9_9, d);
-  d = __dmul_rn(c.kr(9), z9);
-  d = __dmul_rn(d, msf);
-  a0_0 = (LUT)__dadd_rn((double)a0_0, d);
-  a0_3 = (LUT)__dsub_rn((double)a0_3, d);
-  a0_7 = (LUT)__dsub_rn((double)a0_7, d);
-  a0_9 = (LUT)__dadd_rn((double)a0_9, d);
-  d = __dmul_rn(c.kf(10), z3);
-  d = __dmul_rn(d, factor);
-  a7_3 = (LUT)__dsub_rn((double)a7_3, d);
-  a7_6 = (LUT)__dadd_rn((double)a7_6, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  a7_8 = (LUT)__dadd_rn((double)a7_8, d);
-  d = __dmul_rn(c.kf(10), z7);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  a3_7 = (LUT)__dsub_rn((double)a3_7, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  d = __dmul_rn(c.kr(10), z8);
-  d = __dmul_rn(d, msf);
-  a6_3 = (LUT)__dsub_rn((double)a6_3, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_7 = (LUT)__dsub_rn((double)a6_7, d);
-  a6_8 = (LUT)__dadd_rn((double)a6_8, d);
-  d = __dmul_rn(c.kr(10), z6);
-  d = __dmul_rn(d, msf);
-  a8_3 = (LUT)__dsub_rn((double)a8_3, d);
-  a8_6 = (LUT)__dadd_rn((double)a8_6, d);
-  a8_7 = (LUT)__dsub_rn((double)a8_7, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kf(11), z4);
-  d = __dmul_rn(d, factor);
-  a7_4 = (LUT)__dsub_rn((double)a7_4, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  a7_8 = (LUT)__dadd_rn((double)a7_8, d);
-  a7_9 = (LUT)__dadd_rn((double)a7_9, d);
-  d = __dmul_rn(c.kf(11), z7);
-  d = __dmul_rn(d, factor);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_7 = (LUT)__dsub_rn((double)a4_7, d);
-  a4_8 = (LUT)__dadd_rn((double)a4_8, d);
-  a4_9 = (LUT)__dadd_rn((double)a4_9, d);
-  d = __dmul_rn(c.kr(11), z8);
-  d = __dmul_rn(d, msf);
-  a9_4 = (LUT)__dsub_rn((double)a9_4, d);
-  a9_7 = (LUT)__dsub_rn((double)a9_7, d);
-  a9_8 = (LUT)__dadd_rn((double)a9_8, d);
-  a9_9 = (LUT)__dadd_rn((double)a9_9, d);
-  d = __dmul_rn(c.kr(11), z9);
-  d = __dmul_rn(d, msf);
-  a8_4 = (LUT)__dsub_rn((double)a8_4, d);
-  a8_7 = (LUT)__dsub_rn((double)a8_7, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_9 = (LUT)__dadd_rn((double)a8_9, d);
-  d = c.kf(12);
-  d = __dmul_rn(d, factor);
-  a6_3 = (LUT)__dadd_rn((double)a6_3, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_8 = (LUT)__dadd_rn((double)a6_8, d);
-  d = __dmul_rn(c.kr(12), z8);
-  d = __dmul_rn(d, msf);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_6 = (LUT)__dsub_rn((double)a3_6, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  d = __dmul_rn(c.kr(12), z3);
-  d = __dmul_rn(d, msf);
-  a8_3 = (LUT)__dadd_rn((double)a8_3, d);
-  a8_6 = (LUT)__dsub_rn((double)a8_6, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = c.kf(13);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  d = __dmul_rn(c.kr(13), z4);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  d = __dmul_rn(c.kr(13), z4);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  d = c.kf(14);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  d = __dmul_rn(c.kr(14), z3);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  d = __dmul_rn(c.kr(14), z3);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  d = __dmul_rn(c.kf(15), z3);
-  d = __dmul_rn(d, factor);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_8 = (LUT)__dadd_rn((double)a4_8, d);
-  d = __dmul_rn(c.kf(15), z4);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  d = c.kr(15);
-  d = __dmul_rn(d, msf);
-  a8_3 = (LUT)__dsub_rn((double)a8_3, d);
-  a8_4 = (LUT)__dsub_rn((double)a8_4, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kf(16), z4);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  a3_5 = (LUT)__dadd_rn((double)a3_5, d);
-  d = __dmul_rn(c.kf(16), z3);
-  d = __dmul_rn(d, factor);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  d = c.kr(16);
-  d = __dmul_rn(d, msf);
-  a5_3 = (LUT)__dsub_rn((double)a5_3, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  d = __dmul_rn(c.kf(17), z6);
-  d = __dmul_rn(d, factor);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_6 = (LUT)__dsub_rn((double)a5_6, d);
-  a5_6 = (LUT)__dadd_rn((double)a5_6, d);
-  a5_8 = (LUT)__dadd_rn((double)a5_8, d);
-  d = __dmul_rn(c.kf(17), z5);
-  d = __dmul_rn(d, factor);
-  a6_5 = (LUT)__dsub_rn((double)a6_5, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_8 = (LUT)__dadd_rn((double)a6_8, d);
-  d = __dmul_rn(c.kr(17), z6);
-  d = __dmul_rn(d, msf);
-  a8_5 = (LUT)__dsub_rn((double)a8_5, d);
-  a8_6 = (LUT)__dsub_rn((double)a8_6, d);
-  a8_6 = (LUT)__dadd_rn((double)a8_6, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(17), z8);
-  d = __dmul_rn(d, msf);
-  a6_5 = (LUT)__dsub_rn((double)a6_5, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_8 = (LUT)__dadd_rn((double)a6_8, d);
-  d = __dmul_rn(c.kf(18), z0);
-  d = __dmul_rn(d, factor);
-  a5_0 = (LUT)__dsub_rn((double)a5_0, d);
-  a5_0 = (LUT)__dadd_rn((double)a5_0, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_8 = (LUT)__dadd_rn((double)a5_8, d);
-  d = __dmul_rn(c.kf(18), z5);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_0 = (LUT)__dadd_rn((double)a0_0, d);
-  a0_5 = (LUT)__dsub_rn((double)a0_5, d);
-  a0_8 = (LUT)__dadd_rn((double)a0_8, d);
-  d = __dmul_rn(c.kr(18), z0);
-  d = __dmul_rn(d, msf);
-  a8_0 = (LUT)__dsub_rn((double)a8_0, d);
-  a8_0 = (LUT)__dadd_rn((double)a8_0, d);
-  a8_5 = (LUT)__dsub_rn((double)a8_5, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(18), z8);
-  d = __dmul_rn(d, msf);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_0 = (LUT)__dadd_rn((double)a0_0, d);
-  a0_5 = (LUT)__dsub_rn((double)a0_5, d);
-  a0_8 = (LUT)__dadd_rn((double)a0_8, d);
-  d = __dmul_rn(c.kf(19), z2);
-  d = __dmul_rn(d, factor);
-  a5_2 = (LUT)__dsub_rn((double)a5_2, d);
-  a5_2 = (LUT)__dadd_rn((double)a5_2, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_8 = (LUT)__dadd_rn((double)a5_8, d);
-  d = __dmul_rn(c.kf(19), z5);
-  d = __dmul_rn(d, factor);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_2 = (LUT)__dadd_rn((double)a2_2, d);
-  a2_5 = (LUT)__dsub_rn((double)a2_5, d);
-  a2_8 = (LUT)__dadd_rn((double)a2_8, d);
-  d = __dmul_rn(c.kr(19), z2);
-  d = __dmul_rn(d, msf);
-  a8_2 = (LUT)__dsub_rn((double)a8_2, d);
-  a8_2 = (LUT)__dadd_rn((double)a8_2, d);
-  a8_5 = (LUT)__dsub_rn((double)a8_5, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(19), z8);
-  d = __dmul_rn(d, msf);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_2 = (LUT)__dadd_rn((double)a2_2, d);
-  a2_5 = (LUT)__dsub_rn((double)a2_5, d);
-  a2_8 = (LUT)__dadd_rn((double)a2_8, d);
-  d = __dmul_rn(c.kf(20), z8);
-  d = __dmul_rn(d, factor);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_8 = (LUT)__dsub_rn((double)a5_8, d);
-  a5_8 = (LUT)__dadd_rn((double)a5_8, d);
-  a5_8 = (LUT)__dadd_rn((double)a5_8, d);
-  d = __dmul_rn(c.kf(20), z5);
-  d = __dmul_rn(d, factor);
-  a8_5 = (LUT)__dsub_rn((double)a8_5, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(20), z8);
-  d = __dmul_rn(d, msf);
-  a8_5 = (LUT)__dsub_rn((double)a8_5, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(20), z8);
-  d = __dmul_rn(d, msf);
-  a8_5 = (LUT)__dsub_rn((double)a8_5, d);
-  a8_8 = (LUT)__dsub_rn((double)a8_8, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kf(21), z3);
-  d = __dmul_rn(d, factor);
-  a5_3 = (LUT)__dsub_rn((double)a5_3, d);
-  a5_3 = (LUT)__dadd_rn((double)a5_3, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_8 = (LUT)__dadd_rn((double)a5_8, d);
-  d = __dmul_rn(c.kf(21), z5);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_5 = (LUT)__dsub_rn((double)a3_5, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  d = __dmul_rn(c.kr(21), z3);
-  d = __dmul_rn(d, msf);
-  a8_3 = (LUT)__dsub_rn((double)a8_3, d);
-  a8_3 = (LUT)__dadd_rn((double)a8_3, d);
-  a8_5 = (LUT)__dsub_rn((double)a8_5, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(21), z8);
-  d = __dmul_rn(d, msf);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_5 = (LUT)__dsub_rn((double)a3_5, d);
-  a3_8 = (LUT)__dadd_rn((double)a3_8, d);
-  d = c.kf(22);
-  d = __dmul_rn(d, factor);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_8 = (LUT)__dadd_rn((double)a5_8, d);
-  d = c.kr(22);
-  d = __dmul_rn(d, msf);
-  a8_5 = (LUT)__dsub_rn((double)a8_5, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kf(23), z1);
-  d = __dmul_rn(d, factor);
-  a5_1 = (LUT)__dsub_rn((double)a5_1, d);
-  a5_1 = (LUT)__dadd_rn((double)a5_1, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_8 = (LUT)__dadd_rn((double)a5_8, d);
-  d = __dmul_rn(c.kf(23), z5);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_5 = (LUT)__dsub_rn((double)a1_5, d);
-  a1_8 = (LUT)__dadd_rn((double)a1_8, d);
-  d = __dmul_rn(c.kr(23), z1);
-  d = __dmul_rn(d, msf);
-  a8_1 = (LUT)__dsub_rn((double)a8_1, d);
-  a8_1 = (LUT)__dadd_rn((double)a8_1, d);
-  a8_5 = (LUT)__dsub_rn((double)a8_5, d);
-  a8_8 = (LUT)__dadd_rn((double)a8_8, d);
-  d = __dmul_rn(c.kr(23), z8);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_5 = (LUT)__dsub_rn((double)a1_5, d);
-  a1_8 = (LUT)__dadd_rn((double)a1_8, d);
-  a0_0 = a0_0 + 1;
-  a1_1 = a1_1 + 1;
-  a2_2 = a2_2 + 1;
-  a3_3 = a3_3 + 1;
-  a4_4 = a4_4 + 1;
-  a5_5 = a5_5 + 1;
-  a6_6 = a6_6 + 1;
-  a7_7 = a7_7 + 1;
-  a8_8 = a8_8 + 1;
-  a9_9 = a9_9 + 1;
-  c.a(0, 0) = a0_0;
-  c.a(0, 1) = a0_1;
-  c.a(0, 2) = a0_2;
-  c.a(0, 3) = a0_3;
-  c.a(0, 4) = a0_4;
-  c.a(0, 5) = a0_5;
-  c.a(0, 6) = a0_6;
-  c.a(0, 7) = a0_7;
-  c.a(0, 8) = a0_8;
-  c.a(0, 9) = a0_9;
-  c.a(1, 0) = a1_0;
-  c.a(1, 1) = a1_1;
-  c.a(1, 2) = a1_2;
-  c.a(1, 3) = a1_3;
-  c.a(1, 4) = a1_4;
-  c.a(1, 5) = a1_5;
-  c.a(1, 6) = a1_6;
-  c.a(1, 7) = a1_7;
-  c.a(1, 8) = a1_8;
-  c.a(1, 9) = a1_9;
-  c.a(2, 0) = a2_0;
-  c.a(2, 1) = a2_1;
-  c.a(2, 2) = a2_2;
-  c.a(2, 3) = a2_3;
-  c.a(2, 4) = a2_4;
-  c.a(2, 5) = a2_5;
-  c.a(2, 6) = a2_6;
-  c.a(2, 7) = a2_7;
-  c.a(2, 8) = a2_8;
-  c.a(2, 9) = a2_9;
-  c.a(3, 0) = a3_0;
-  c.a(3, 1) = a3_1;
-  c.a(3, 2) = a3_2;
-  c.a(3, 3) = a3_3;
-  c.a(3, 4) = a3_4;
-  c.a(3, 5) = a3_5;
-  c.a(3, 6) = a3_6;
-  c.a(3, 7) = a3_7;
-  c.a(3, 8) = a3_8;
-  c.a(3, 9) = a3_9;
-  c.a(4, 0) = a4_0;
-  c.a(4, 1) = a4_1;
-  c.a(4, 2) = a4_2;
-  c.a(4, 3) = a4_3;
-  c.a(4, 4) = a4_4;
-  c.a(4, 5) = a4_5;
-  c.a(4, 6) = a4_6;
-  c.a(4, 7) = a4_7;
-  c.a(4, 8) = a4_8;
-  c.a(4, 9) = a4_9;
-  c.a(5, 0) = a5_0;
-  c.a(5, 1) = a5_1;
-  c.a(5, 2) = a5_2;
-  c.a(5, 3) = a5_3;
-  c.a(5, 4) = a5_4;
-  c.a(5, 5) = a5_5;
-  c.a(5, 6) = a5_6;
-  c.a(5, 7) = a5_7;
-  c.a(5, 8) = a5_8;
-  c.a(5, 9) = a5_9;
-  c.a(6, 0) = a6_0;
-  c.a(6, 1) = a6_1;
-  c.a(6, 2) = a6_2;
-  c.a(6, 3) = a6_3;
-  c.a(6, 4) = a6_4;
-  c.a(6, 5) = a6_5;
-  c.a(6, 6) = a6_6;
-  c.a(6, 7) = a6_7;
-  c.a(6, 8) = a6_8;
-  c.a(6, 9) = a6_9;
-  c.a(7, 0) = a7_0;
-  c.a(7, 1) = a7_1;
-  c.a(7, 2) = a7_2;
-  c.a(7, 3) = a7_3;
-  c.a(7, 4) = a7_4;
-  c.a(7, 5) = a7_5;
-  c.a(7, 6) = a7_6;
-  c.a(7, 7) = a7_7;
-  c.a(7, 8) = a7_8;
-  c.a(7, 9) = a7_9;
-  c.a(8, 0) = a8_0;
-  c.a(8, 1) = a8_1;
-  c.a(8, 2) = a8_2;
-  c.a(8, 3) = a8_3;
-  c.a(8, 4) = a8_4;
-  c.a(8, 5) = a8_5;
-  c.a(8, 6) = a8_6;
-  c.a(8, 7) = a8_7;
-  c.a(8, 8) = a8_8;
-  c.a(8, 9) = a8_9;
-  c.a(9, 0) = a9_0;
-  c.a(9, 1) = a9_1;
-  c.a(9, 2) = a9_2;
-  c.a(9, 3) = a9_3;
-  c.a(9, 4) = a9_4;
-  c.a(9, 5) = a9_5;
-  c.a(9, 6) = a9_6;
-  c.a(9, 7) = a9_7;
-  c.a(9, 8) = a9_8;
-  c.a(9, 9) = a9_9;
+  if constexpr (J == 0) {
+    const double z4 = c.z(4), z5 = c.z(5), z8 = c.z(8), z9 = c.z(9);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(4), z4), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(6), z8), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(9), z9), msf);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(c.kf(14), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(c.kf(18), z5), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(18), z8), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a0 = a0 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
+  if constexpr (J == 1) {
+    const double z3 = c.z(3), z5 = c.z(5), z7 = c.z(7), z8 = c.z(8);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(0), z3), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(1), z8), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(7), z7), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(c.kf(13), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(23), z5), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(23), z8), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a1 = a1 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
+  if constexpr (J == 2) {
+    const double z5 = c.z(5), z8 = c.z(8);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(19), z5), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(19), z8), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a2 = a2 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
+  if constexpr (J == 3) {
+    const double z1 = c.z(1), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6), z7 = c.z(7), z8 = c.z(8), z9 = c.z(9);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(0), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(2), z9), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(3), z9), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(4), z8), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(6), z6), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(9), z7), factor);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(10), z7), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(12), z8), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(14), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(c.kr(14), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(c.kf(15), z4), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(16), z4), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(21), z5), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(21), z8), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a3 = a3 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
+  if constexpr (J == 4) {
+    const double z0 = c.z(0), z3 = c.z(3), z4 = c.z(4), z6 = c.z(6), z7 = c.z(7), z8 = c.z(8), z9 = c.z(9);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(0), z8), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(1), z9), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(3), z6), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(4), z0), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(5), z6), msf);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(11), z7), factor);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(13), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(13), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(15), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(16), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a4 = a4 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
+  if constexpr (J == 5) {
+    const double z0 = c.z(0), z1 = c.z(1), z2 = c.z(2), z3 = c.z(3), z6 = c.z(6), z8 = c.z(8);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(c.kr(16), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(17), z6), factor);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(18), z0), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(19), z2), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(20), z8), factor);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(21), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(c.kf(22), factor);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(23), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a5 = a5 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
+  if constexpr (J == 6) {
+    const double z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z8 = c.z(8), z9 = c.z(9);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(3), z4), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(5), z4), msf);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(6), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(8), z9), msf);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(10), z8), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(c.kf(12), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(17), z5), factor);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(17), z8), msf);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a6 = a6 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
+  if constexpr (J == 7) {
+    const double z1 = c.z(1), z3 = c.z(3), z4 = c.z(4), z8 = c.z(8);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(7), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(8), z8), factor);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(9), z3), factor);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(10), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(11), z4), factor);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    a7 = a7 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
+  if constexpr (J == 8) {
+    const double z0 = c.z(0), z1 = c.z(1), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6), z7 = c.z(7), z8 = c.z(8), z9 = c.z(9);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(0), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(1), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(2), z8), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(2), z8), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(4), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(5), z8), factor);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(5), z8), factor);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(6), z0), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(8), z7), factor);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(10), z6), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(11), z9), msf);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(12), z3), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(c.kr(15), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(17), z6), msf);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(18), z0), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(19), z2), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kf(20), z5), factor);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(20), z8), msf);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(20), z8), msf);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(21), z3), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(c.kr(22), msf);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    d = __dmul_rn(__dmul_rn(c.kr(23), z1), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a8 = a8 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
+  if constexpr (J == 9) {
+    const double z0 = c.z(0), z3 = c.z(3), z4 = c.z(4), z6 = c.z(6), z8 = c.z(8), z9 = c.z(9);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(1), z4), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(2), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(3), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(7), z9), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(7), z9), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(8), z6), msf);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dsub_rn((double)a8, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(9), z0), msf);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kr(11), z8), msf);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a8 = (LUT)__dadd_rn((double)a8, d);
+    a9 = (LUT)__dadd_rn((double)a9, d);
+    a9 = a9 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7; v[8] = a8; v[9] = a9;
+  }
 }
 
 }  // namespace gen_tereza

@@ -1,6 +1,6 @@
 // Generated by nrg_b200/gen_mech.py from ZHANG.txt: do not edit.
 // Straight-line right-hand side and analytic iteration matrix over the
-// 8 reacting species and 28 reactions; same operation order as the
+// 8 reacting species and 25 reactions; same operation order as the
 // table-driven loops in chem_bdf.cuh, with the same explicitly rounded
 // (never fused) operations.
 #pragma once
@@ -8,8 +8,8 @@
 namespace nrg {
 namespace gen_zhang {
 
-constexpr int kSpecN = 8, kSpecR = 28;
-constexpr int kSpecLeft[28][3] = {
+constexpr int kSpecN = 8, kSpecR = 25;
+constexpr int kSpecLeft[25][3] = {
     {3, 1, -1},
     {2, 0, -1},
     {4, 0, -1},
@@ -25,21 +25,18 @@ constexpr int kSpecLeft[28][3] = {
     {5, 2, -1},
     {6, 2, -1},
     {6, 4, -1},
-    {6, 4, -1},
-    {6, 6, -1},
     {6, 6, -1},
     {7, -1, -1},
     {7, 3, -1},
     {7, 3, -1},
     {7, 2, -1},
     {7, 4, -1},
-    {7, 4, -1},
     {3, 1, 3},
     {3, 1, 3},
     {3, 1, 2},
     {3, 1, 4},
 };
-constexpr int kSpecRight[28][3] = {
+constexpr int kSpecRight[25][3] = {
     {2, 4, -1},
     {4, 3, -1},
     {3, 5, -1},
@@ -55,22 +52,19 @@ constexpr int kSpecRight[28][3] = {
     {3, 6, -1},
     {4, 1, -1},
     {5, 1, -1},
-    {5, 1, -1},
-    {7, 1, -1},
     {7, 1, -1},
     {4, 4, -1},
     {5, 4, -1},
     {6, 0, -1},
     {4, 6, -1},
     {5, 6, -1},
-    {5, 6, -1},
     {0, 1, -1},
     {4, 4, -1},
     {4, 1, -1},
     {5, 1, -1},
 };
-constexpr int kSpecNupd[28] = {4, 4, 4, 4, 3, 3, 3, 3, 5, 3, 4, 4, 4, 4, 4, 4, 4, 4, 3, 4, 4, 4, 4, 4, 5, 5, 5, 5};
-constexpr int kSpecUpdK[28][6] = {
+constexpr int kSpecNupd[25] = {4, 4, 4, 4, 3, 3, 3, 3, 5, 3, 4, 4, 4, 4, 4, 4, 3, 4, 4, 4, 4, 5, 5, 5, 5};
+constexpr int kSpecUpdK[25][6] = {
     {1, 2, 3, 4, 0, 0},
     {0, 2, 3, 4, 0, 0},
     {0, 3, 4, 5, 0, 0},
@@ -86,21 +80,18 @@ constexpr int kSpecUpdK[28][6] = {
     {2, 3, 5, 6, 0, 0},
     {1, 2, 4, 6, 0, 0},
     {1, 4, 5, 6, 0, 0},
-    {1, 4, 5, 6, 0, 0},
-    {1, 6, 6, 7, 0, 0},
     {1, 6, 6, 7, 0, 0},
     {4, 4, 7, 0, 0, 0},
     {3, 4, 5, 7, 0, 0},
     {0, 3, 6, 7, 0, 0},
     {2, 4, 6, 7, 0, 0},
     {4, 5, 6, 7, 0, 0},
-    {4, 5, 6, 7, 0, 0},
     {0, 1, 1, 3, 3, 0},
     {1, 3, 3, 4, 4, 0},
     {1, 1, 2, 3, 4, 0},
     {1, 1, 3, 4, 5, 0},
 };
-constexpr int kSpecUpdProd[28][6] = {
+constexpr int kSpecUpdProd[25][6] = {
     {0, 1, 0, 1, 0, 0},
     {0, 0, 1, 1, 0, 0},
     {0, 1, 0, 1, 0, 0},
@@ -116,13 +107,10 @@ constexpr int kSpecUpdProd[28][6] = {
     {0, 1, 0, 1, 0, 0},
     {1, 0, 1, 0, 0, 0},
     {1, 0, 1, 0, 0, 0},
-    {1, 0, 1, 0, 0, 0},
-    {1, 0, 0, 1, 0, 0},
     {1, 0, 0, 1, 0, 0},
     {1, 1, 0, 0, 0, 0},
     {0, 1, 1, 0, 0, 0},
     {1, 0, 1, 0, 0, 0},
-    {0, 1, 1, 0, 0, 0},
     {0, 1, 1, 0, 0, 0},
     {0, 1, 1, 0, 0, 0},
     {1, 0, 1, 0, 0, 0},
@@ -245,94 +233,73 @@ __device__ __forceinline__ void spec_rhs(S& c) {
   d4 = __dsub_rn(d4, q);
   d5 = __dadd_rn(d5, q);
   d6 = __dsub_rn(d6, q);
-  f = __dmul_rn(__dmul_rn(c.kf(15), z6), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(15), z5), z1);
-  q = __dsub_rn(f, b);
-  d1 = __dadd_rn(d1, q);
-  d4 = __dsub_rn(d4, q);
-  d5 = __dadd_rn(d5, q);
-  d6 = __dsub_rn(d6, q);
-  f = __dmul_rn(__dmul_rn(c.kf(16), z6), z6);
-  b = __dmul_rn(__dmul_rn(c.kr(16), z7), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(15), z6), z6);
+  b = __dmul_rn(__dmul_rn(c.kr(15), z7), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d6 = __dsub_rn(d6, q);
   d6 = __dsub_rn(d6, q);
   d7 = __dadd_rn(d7, q);
-  f = __dmul_rn(__dmul_rn(c.kf(17), z6), z6);
-  b = __dmul_rn(__dmul_rn(c.kr(17), z7), z1);
-  q = __dsub_rn(f, b);
-  d1 = __dadd_rn(d1, q);
-  d6 = __dsub_rn(d6, q);
-  d6 = __dsub_rn(d6, q);
-  d7 = __dadd_rn(d7, q);
-  f = __dmul_rn(c.kf(18), z7);
-  b = __dmul_rn(__dmul_rn(c.kr(18), z4), z4);
+  f = __dmul_rn(c.kf(16), z7);
+  b = __dmul_rn(__dmul_rn(c.kr(16), z4), z4);
   q = __dsub_rn(f, b);
   d4 = __dadd_rn(d4, q);
   d4 = __dadd_rn(d4, q);
   d7 = __dsub_rn(d7, q);
-  f = __dmul_rn(__dmul_rn(c.kf(19), z7), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(19), z5), z4);
+  f = __dmul_rn(__dmul_rn(c.kf(17), z7), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(17), z5), z4);
   q = __dsub_rn(f, b);
   d3 = __dsub_rn(d3, q);
   d4 = __dadd_rn(d4, q);
   d5 = __dadd_rn(d5, q);
   d7 = __dsub_rn(d7, q);
-  f = __dmul_rn(__dmul_rn(c.kf(20), z7), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(20), z6), z0);
+  f = __dmul_rn(__dmul_rn(c.kf(18), z7), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(18), z6), z0);
   q = __dsub_rn(f, b);
   d0 = __dadd_rn(d0, q);
   d3 = __dsub_rn(d3, q);
   d6 = __dadd_rn(d6, q);
   d7 = __dsub_rn(d7, q);
-  f = __dmul_rn(__dmul_rn(c.kf(21), z7), z2);
-  b = __dmul_rn(__dmul_rn(c.kr(21), z4), z6);
+  f = __dmul_rn(__dmul_rn(c.kf(19), z7), z2);
+  b = __dmul_rn(__dmul_rn(c.kr(19), z4), z6);
   q = __dsub_rn(f, b);
   d2 = __dsub_rn(d2, q);
   d4 = __dadd_rn(d4, q);
   d6 = __dadd_rn(d6, q);
   d7 = __dsub_rn(d7, q);
-  f = __dmul_rn(__dmul_rn(c.kf(22), z7), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(22), z5), z6);
+  f = __dmul_rn(__dmul_rn(c.kf(20), z7), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(20), z5), z6);
   q = __dsub_rn(f, b);
   d4 = __dsub_rn(d4, q);
   d5 = __dadd_rn(d5, q);
   d6 = __dadd_rn(d6, q);
   d7 = __dsub_rn(d7, q);
-  f = __dmul_rn(__dmul_rn(c.kf(23), z7), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(23), z5), z6);
-  q = __dsub_rn(f, b);
-  d4 = __dsub_rn(d4, q);
-  d5 = __dadd_rn(d5, q);
-  d6 = __dadd_rn(d6, q);
-  d7 = __dsub_rn(d7, q);
-  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(24), z3), z1), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(24), z0), z1);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(21), z3), z1), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(21), z0), z1);
   q = __dsub_rn(f, b);
   d0 = __dadd_rn(d0, q);
   d1 = __dsub_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d3 = __dsub_rn(d3, q);
   d3 = __dsub_rn(d3, q);
-  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(25), z3), z1), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(25), z4), z4);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(22), z3), z1), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(22), z4), z4);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d3 = __dsub_rn(d3, q);
   d3 = __dsub_rn(d3, q);
   d4 = __dadd_rn(d4, q);
   d4 = __dadd_rn(d4, q);
-  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(26), z3), z1), z2);
-  b = __dmul_rn(__dmul_rn(c.kr(26), z4), z1);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(23), z3), z1), z2);
+  b = __dmul_rn(__dmul_rn(c.kr(23), z4), z1);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d2 = __dsub_rn(d2, q);
   d3 = __dsub_rn(d3, q);
   d4 = __dadd_rn(d4, q);
-  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(27), z3), z1), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(27), z5), z1);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(24), z3), z1), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(24), z5), z1);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d1 = __dadd_rn(d1, q);
@@ -349,765 +316,562 @@ __device__ __forceinline__ void spec_rhs(S& c) {
   c.zd(7) = d7;
 }
 
-// I + factor * J written into the LU storage: c.a(j, i) = A(i+1, j+1)
-template <class S, typename LUT>
-__device__ __forceinline__ void spec_matrix(S& c, double factor) {
-  const double z0 = c.z(0);
-  const double z1 = c.z(1);
-  const double z2 = c.z(2);
-  const double z3 = c.z(3);
-  const double z4 = c.z(4);
-  const double z5 = c.z(5);
-  const double z6 = c.z(6);
-  const double z7 = c.z(7);
+// Column J of I + factor * J: v[i] = A(i+1, J+1), each element's terms in
+// reaction order.
+template <int J, class S, typename LUT>
+__device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[8]) {
   const double msf = -factor;
-  LUT a0_0 = (LUT)0, a0_1 = (LUT)0, a0_2 = (LUT)0, a0_3 = (LUT)0, a0_4 = (LUT)0, a0_5 = (LUT)0, a0_6 = (LUT)0, a0_7 = (LUT)0, a1_0 = (LUT)0, a1_1 = (LUT)0, a1_2 = (LUT)0, a1_3 = (LUT)0, a1_4 = (LUT)0, a1_5 = (LUT)0, a1_6 = (LUT)0, a1_7 = (LUT)0, a2_0 = (LUT)0, a2_1 = (LUT)0, a2_2 = (LUT)0, a2_3 = (LUT)0, a2_4 = (LUT)0, a2_5 = (LUT)0, a2_6 = (LUT)0, a2_7 = (LUT)0, a3_0 = (LUT)0, a3_1 = (LUT)0, a3_2 = (LUT)0, a3_3 = (LUT)0, a3_4 = (LUT)0, a3_5 = (LUT)0, a3_6 = (LUT)0, a3_7 = (LUT)0, a4_0 = (LUT)0, a4_1 = (LUT)0, a4_2 = (LUT)0, a4_3 = (LUT)0, a4_4 = (LUT)0, a4_5 = (LUT)0, a4_6 = (LUT)0, a4_7 = (LUT)0, a5_0 = (LUT)0, a5_1 = (LUT)0, a5_2 = (LUT)0, a5_3 = (LUT)0, a5_4 = (LUT)0, a5_5 = (LUT)0, a5_6 = (LUT)0, a5_7 = (LUT)0, a6_0 = (LUT)0, a6_1 = (LUT)0, a6_2 = (LUT)0, a6_3 = (LUT)0, a6_4 = (LUT)0, a6_5 = (LUT)0, a6_6 = (LUT)0, a6_7 = (LUT)0, a7_0 = (LUT)0, a7_1 = (LUT)0, a7_2 = (LUT)0, a7_3 = (LUT)0, a7_4 = (LUT)0, a7_5 = (LUT)0, a7_6 = (LUT)0, a7_7 = (LUT)0;
   double d;
-  d = __dmul_rn(c.kf(0), z1);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_2 = (LUT)__dadd_rn((double)a3_2, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  d = __dmul_rn(c.kf(0), z3);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_2 = (LUT)__dadd_rn((double)a1_2, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  d = __dmul_rn(c.kr(0), z4);
-  d = __dmul_rn(d, msf);
-  a2_1 = (LUT)__dsub_rn((double)a2_1, d);
-  a2_2 = (LUT)__dadd_rn((double)a2_2, d);
-  a2_3 = (LUT)__dsub_rn((double)a2_3, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  d = __dmul_rn(c.kr(0), z2);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_2 = (LUT)__dadd_rn((double)a4_2, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  d = __dmul_rn(c.kf(1), z0);
-  d = __dmul_rn(d, factor);
-  a2_0 = (LUT)__dsub_rn((double)a2_0, d);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_3 = (LUT)__dadd_rn((double)a2_3, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  d = __dmul_rn(c.kf(1), z2);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_2 = (LUT)__dsub_rn((double)a0_2, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  a0_4 = (LUT)__dadd_rn((double)a0_4, d);
-  d = __dmul_rn(c.kr(1), z3);
-  d = __dmul_rn(d, msf);
-  a4_0 = (LUT)__dsub_rn((double)a4_0, d);
-  a4_2 = (LUT)__dsub_rn((double)a4_2, d);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  d = __dmul_rn(c.kr(1), z4);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_2 = (LUT)__dsub_rn((double)a3_2, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  d = __dmul_rn(c.kf(2), z0);
-  d = __dmul_rn(d, factor);
-  a4_0 = (LUT)__dsub_rn((double)a4_0, d);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  d = __dmul_rn(c.kf(2), z4);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  a0_4 = (LUT)__dsub_rn((double)a0_4, d);
-  a0_5 = (LUT)__dadd_rn((double)a0_5, d);
-  d = __dmul_rn(c.kr(2), z5);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  a3_5 = (LUT)__dadd_rn((double)a3_5, d);
-  d = __dmul_rn(c.kr(2), z3);
-  d = __dmul_rn(d, msf);
-  a5_0 = (LUT)__dsub_rn((double)a5_0, d);
-  a5_3 = (LUT)__dadd_rn((double)a5_3, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  d = __dmul_rn(c.kf(3), z4);
-  d = __dmul_rn(d, factor);
-  a4_2 = (LUT)__dadd_rn((double)a4_2, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  d = __dmul_rn(c.kf(3), z4);
-  d = __dmul_rn(d, factor);
-  a4_2 = (LUT)__dadd_rn((double)a4_2, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  d = __dmul_rn(c.kr(3), z2);
-  d = __dmul_rn(d, msf);
-  a5_2 = (LUT)__dadd_rn((double)a5_2, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  d = __dmul_rn(c.kr(3), z5);
-  d = __dmul_rn(d, msf);
-  a2_2 = (LUT)__dadd_rn((double)a2_2, d);
-  a2_4 = (LUT)__dsub_rn((double)a2_4, d);
-  a2_4 = (LUT)__dsub_rn((double)a2_4, d);
-  a2_5 = (LUT)__dadd_rn((double)a2_5, d);
-  d = c.kf(4);
-  d = __dmul_rn(d, factor);
-  a0_0 = (LUT)__dsub_rn((double)a0_0, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  a0_3 = (LUT)__dadd_rn((double)a0_3, d);
-  d = __dmul_rn(c.kr(4), z3);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  d = __dmul_rn(c.kr(4), z3);
-  d = __dmul_rn(d, msf);
-  a3_0 = (LUT)__dsub_rn((double)a3_0, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  d = __dmul_rn(c.kf(5), z2);
-  d = __dmul_rn(d, factor);
-  a2_1 = (LUT)__dadd_rn((double)a2_1, d);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  d = __dmul_rn(c.kf(5), z2);
-  d = __dmul_rn(d, factor);
-  a2_1 = (LUT)__dadd_rn((double)a2_1, d);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  d = c.kr(5);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_2 = (LUT)__dsub_rn((double)a1_2, d);
-  a1_2 = (LUT)__dsub_rn((double)a1_2, d);
-  d = __dmul_rn(c.kf(6), z3);
-  d = __dmul_rn(d, factor);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_3 = (LUT)__dsub_rn((double)a2_3, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  d = __dmul_rn(c.kf(6), z2);
-  d = __dmul_rn(d, factor);
-  a3_2 = (LUT)__dsub_rn((double)a3_2, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  d = c.kr(6);
-  d = __dmul_rn(d, msf);
-  a4_2 = (LUT)__dsub_rn((double)a4_2, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  d = c.kf(7);
-  d = __dmul_rn(d, factor);
-  a5_3 = (LUT)__dadd_rn((double)a5_3, d);
-  a5_4 = (LUT)__dadd_rn((double)a5_4, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  d = __dmul_rn(c.kr(7), z4);
-  d = __dmul_rn(d, msf);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_5 = (LUT)__dsub_rn((double)a3_5, d);
-  d = __dmul_rn(c.kr(7), z3);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_5 = (LUT)__dsub_rn((double)a4_5, d);
-  d = __dmul_rn(c.kf(8), z5);
-  d = __dmul_rn(d, factor);
-  a5_3 = (LUT)__dadd_rn((double)a5_3, d);
-  a5_4 = (LUT)__dadd_rn((double)a5_4, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  d = __dmul_rn(c.kf(8), z5);
-  d = __dmul_rn(d, factor);
-  a5_3 = (LUT)__dadd_rn((double)a5_3, d);
-  a5_4 = (LUT)__dadd_rn((double)a5_4, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  d = __dmul_rn(__dmul_rn(c.kr(8), z4), z5);
-  d = __dmul_rn(d, msf);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_5 = (LUT)__dsub_rn((double)a3_5, d);
-  a3_5 = (LUT)__dsub_rn((double)a3_5, d);
-  a3_5 = (LUT)__dadd_rn((double)a3_5, d);
-  d = __dmul_rn(__dmul_rn(c.kr(8), z3), z5);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dadd_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_5 = (LUT)__dsub_rn((double)a4_5, d);
-  a4_5 = (LUT)__dsub_rn((double)a4_5, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  d = __dmul_rn(__dmul_rn(c.kr(8), z3), z4);
-  d = __dmul_rn(d, msf);
-  a5_3 = (LUT)__dadd_rn((double)a5_3, d);
-  a5_4 = (LUT)__dadd_rn((double)a5_4, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  d = __dmul_rn(c.kf(9), z1);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  d = __dmul_rn(c.kf(9), z3);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_6 = (LUT)__dadd_rn((double)a1_6, d);
-  d = c.kr(9);
-  d = __dmul_rn(d, msf);
-  a6_1 = (LUT)__dsub_rn((double)a6_1, d);
-  a6_3 = (LUT)__dsub_rn((double)a6_3, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  d = __dmul_rn(c.kf(10), z3);
-  d = __dmul_rn(d, factor);
-  a6_0 = (LUT)__dadd_rn((double)a6_0, d);
-  a6_1 = (LUT)__dadd_rn((double)a6_1, d);
-  a6_3 = (LUT)__dsub_rn((double)a6_3, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  d = __dmul_rn(c.kf(10), z6);
-  d = __dmul_rn(d, factor);
-  a3_0 = (LUT)__dadd_rn((double)a3_0, d);
-  a3_1 = (LUT)__dadd_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_6 = (LUT)__dsub_rn((double)a3_6, d);
-  d = __dmul_rn(c.kr(10), z1);
-  d = __dmul_rn(d, msf);
-  a0_0 = (LUT)__dadd_rn((double)a0_0, d);
-  a0_1 = (LUT)__dadd_rn((double)a0_1, d);
-  a0_3 = (LUT)__dsub_rn((double)a0_3, d);
-  a0_6 = (LUT)__dsub_rn((double)a0_6, d);
-  d = __dmul_rn(c.kr(10), z0);
-  d = __dmul_rn(d, msf);
-  a1_0 = (LUT)__dadd_rn((double)a1_0, d);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_6 = (LUT)__dsub_rn((double)a1_6, d);
-  d = __dmul_rn(c.kf(11), z3);
-  d = __dmul_rn(d, factor);
-  a6_3 = (LUT)__dsub_rn((double)a6_3, d);
-  a6_4 = (LUT)__dadd_rn((double)a6_4, d);
-  a6_4 = (LUT)__dadd_rn((double)a6_4, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  d = __dmul_rn(c.kf(11), z6);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_6 = (LUT)__dsub_rn((double)a3_6, d);
-  d = __dmul_rn(c.kr(11), z4);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_6 = (LUT)__dsub_rn((double)a4_6, d);
-  d = __dmul_rn(c.kr(11), z4);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_6 = (LUT)__dsub_rn((double)a4_6, d);
-  d = __dmul_rn(c.kf(12), z2);
-  d = __dmul_rn(d, factor);
-  a5_2 = (LUT)__dsub_rn((double)a5_2, d);
-  a5_3 = (LUT)__dadd_rn((double)a5_3, d);
-  a5_5 = (LUT)__dsub_rn((double)a5_5, d);
-  a5_6 = (LUT)__dadd_rn((double)a5_6, d);
-  d = __dmul_rn(c.kf(12), z5);
-  d = __dmul_rn(d, factor);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_3 = (LUT)__dadd_rn((double)a2_3, d);
-  a2_5 = (LUT)__dsub_rn((double)a2_5, d);
-  a2_6 = (LUT)__dadd_rn((double)a2_6, d);
-  d = __dmul_rn(c.kr(12), z6);
-  d = __dmul_rn(d, msf);
-  a3_2 = (LUT)__dsub_rn((double)a3_2, d);
-  a3_3 = (LUT)__dadd_rn((double)a3_3, d);
-  a3_5 = (LUT)__dsub_rn((double)a3_5, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  d = __dmul_rn(c.kr(12), z3);
-  d = __dmul_rn(d, msf);
-  a6_2 = (LUT)__dsub_rn((double)a6_2, d);
-  a6_3 = (LUT)__dadd_rn((double)a6_3, d);
-  a6_5 = (LUT)__dsub_rn((double)a6_5, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  d = __dmul_rn(c.kf(13), z2);
-  d = __dmul_rn(d, factor);
-  a6_1 = (LUT)__dadd_rn((double)a6_1, d);
-  a6_2 = (LUT)__dsub_rn((double)a6_2, d);
-  a6_4 = (LUT)__dadd_rn((double)a6_4, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  d = __dmul_rn(c.kf(13), z6);
-  d = __dmul_rn(d, factor);
-  a2_1 = (LUT)__dadd_rn((double)a2_1, d);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  a2_6 = (LUT)__dsub_rn((double)a2_6, d);
-  d = __dmul_rn(c.kr(13), z1);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dadd_rn((double)a4_1, d);
-  a4_2 = (LUT)__dsub_rn((double)a4_2, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_6 = (LUT)__dsub_rn((double)a4_6, d);
-  d = __dmul_rn(c.kr(13), z4);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_2 = (LUT)__dsub_rn((double)a1_2, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  a1_6 = (LUT)__dsub_rn((double)a1_6, d);
-  d = __dmul_rn(c.kf(14), z4);
-  d = __dmul_rn(d, factor);
-  a6_1 = (LUT)__dadd_rn((double)a6_1, d);
-  a6_4 = (LUT)__dsub_rn((double)a6_4, d);
-  a6_5 = (LUT)__dadd_rn((double)a6_5, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  d = __dmul_rn(c.kf(14), z6);
-  d = __dmul_rn(d, factor);
-  a4_1 = (LUT)__dadd_rn((double)a4_1, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  a4_6 = (LUT)__dsub_rn((double)a4_6, d);
-  d = __dmul_rn(c.kr(14), z1);
-  d = __dmul_rn(d, msf);
-  a5_1 = (LUT)__dadd_rn((double)a5_1, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  a5_6 = (LUT)__dsub_rn((double)a5_6, d);
-  d = __dmul_rn(c.kr(14), z5);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_4 = (LUT)__dsub_rn((double)a1_4, d);
-  a1_5 = (LUT)__dadd_rn((double)a1_5, d);
-  a1_6 = (LUT)__dsub_rn((double)a1_6, d);
-  d = __dmul_rn(c.kf(15), z4);
-  d = __dmul_rn(d, factor);
-  a6_1 = (LUT)__dadd_rn((double)a6_1, d);
-  a6_4 = (LUT)__dsub_rn((double)a6_4, d);
-  a6_5 = (LUT)__dadd_rn((double)a6_5, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  d = __dmul_rn(c.kf(15), z6);
-  d = __dmul_rn(d, factor);
-  a4_1 = (LUT)__dadd_rn((double)a4_1, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  a4_6 = (LUT)__dsub_rn((double)a4_6, d);
-  d = __dmul_rn(c.kr(15), z1);
-  d = __dmul_rn(d, msf);
-  a5_1 = (LUT)__dadd_rn((double)a5_1, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  a5_6 = (LUT)__dsub_rn((double)a5_6, d);
-  d = __dmul_rn(c.kr(15), z5);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_4 = (LUT)__dsub_rn((double)a1_4, d);
-  a1_5 = (LUT)__dadd_rn((double)a1_5, d);
-  a1_6 = (LUT)__dsub_rn((double)a1_6, d);
-  d = __dmul_rn(c.kf(16), z6);
-  d = __dmul_rn(d, factor);
-  a6_1 = (LUT)__dadd_rn((double)a6_1, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_7 = (LUT)__dadd_rn((double)a6_7, d);
-  d = __dmul_rn(c.kf(16), z6);
-  d = __dmul_rn(d, factor);
-  a6_1 = (LUT)__dadd_rn((double)a6_1, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_7 = (LUT)__dadd_rn((double)a6_7, d);
-  d = __dmul_rn(c.kr(16), z1);
-  d = __dmul_rn(d, msf);
-  a7_1 = (LUT)__dadd_rn((double)a7_1, d);
-  a7_6 = (LUT)__dsub_rn((double)a7_6, d);
-  a7_6 = (LUT)__dsub_rn((double)a7_6, d);
-  a7_7 = (LUT)__dadd_rn((double)a7_7, d);
-  d = __dmul_rn(c.kr(16), z7);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_6 = (LUT)__dsub_rn((double)a1_6, d);
-  a1_6 = (LUT)__dsub_rn((double)a1_6, d);
-  a1_7 = (LUT)__dadd_rn((double)a1_7, d);
-  d = __dmul_rn(c.kf(17), z6);
-  d = __dmul_rn(d, factor);
-  a6_1 = (LUT)__dadd_rn((double)a6_1, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_7 = (LUT)__dadd_rn((double)a6_7, d);
-  d = __dmul_rn(c.kf(17), z6);
-  d = __dmul_rn(d, factor);
-  a6_1 = (LUT)__dadd_rn((double)a6_1, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_6 = (LUT)__dsub_rn((double)a6_6, d);
-  a6_7 = (LUT)__dadd_rn((double)a6_7, d);
-  d = __dmul_rn(c.kr(17), z1);
-  d = __dmul_rn(d, msf);
-  a7_1 = (LUT)__dadd_rn((double)a7_1, d);
-  a7_6 = (LUT)__dsub_rn((double)a7_6, d);
-  a7_6 = (LUT)__dsub_rn((double)a7_6, d);
-  a7_7 = (LUT)__dadd_rn((double)a7_7, d);
-  d = __dmul_rn(c.kr(17), z7);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_6 = (LUT)__dsub_rn((double)a1_6, d);
-  a1_6 = (LUT)__dsub_rn((double)a1_6, d);
-  a1_7 = (LUT)__dadd_rn((double)a1_7, d);
-  d = c.kf(18);
-  d = __dmul_rn(d, factor);
-  a7_4 = (LUT)__dadd_rn((double)a7_4, d);
-  a7_4 = (LUT)__dadd_rn((double)a7_4, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  d = __dmul_rn(c.kr(18), z4);
-  d = __dmul_rn(d, msf);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_7 = (LUT)__dsub_rn((double)a4_7, d);
-  d = __dmul_rn(c.kr(18), z4);
-  d = __dmul_rn(d, msf);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_7 = (LUT)__dsub_rn((double)a4_7, d);
-  d = __dmul_rn(c.kf(19), z3);
-  d = __dmul_rn(d, factor);
-  a7_3 = (LUT)__dsub_rn((double)a7_3, d);
-  a7_4 = (LUT)__dadd_rn((double)a7_4, d);
-  a7_5 = (LUT)__dadd_rn((double)a7_5, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  d = __dmul_rn(c.kf(19), z7);
-  d = __dmul_rn(d, factor);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_5 = (LUT)__dadd_rn((double)a3_5, d);
-  a3_7 = (LUT)__dsub_rn((double)a3_7, d);
-  d = __dmul_rn(c.kr(19), z4);
-  d = __dmul_rn(d, msf);
-  a5_3 = (LUT)__dsub_rn((double)a5_3, d);
-  a5_4 = (LUT)__dadd_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  a5_7 = (LUT)__dsub_rn((double)a5_7, d);
-  d = __dmul_rn(c.kr(19), z5);
-  d = __dmul_rn(d, msf);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  a4_7 = (LUT)__dsub_rn((double)a4_7, d);
-  d = __dmul_rn(c.kf(20), z3);
-  d = __dmul_rn(d, factor);
-  a7_0 = (LUT)__dadd_rn((double)a7_0, d);
-  a7_3 = (LUT)__dsub_rn((double)a7_3, d);
-  a7_6 = (LUT)__dadd_rn((double)a7_6, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  d = __dmul_rn(c.kf(20), z7);
-  d = __dmul_rn(d, factor);
-  a3_0 = (LUT)__dadd_rn((double)a3_0, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_6 = (LUT)__dadd_rn((double)a3_6, d);
-  a3_7 = (LUT)__dsub_rn((double)a3_7, d);
-  d = __dmul_rn(c.kr(20), z0);
-  d = __dmul_rn(d, msf);
-  a6_0 = (LUT)__dadd_rn((double)a6_0, d);
-  a6_3 = (LUT)__dsub_rn((double)a6_3, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_7 = (LUT)__dsub_rn((double)a6_7, d);
-  d = __dmul_rn(c.kr(20), z6);
-  d = __dmul_rn(d, msf);
-  a0_0 = (LUT)__dadd_rn((double)a0_0, d);
-  a0_3 = (LUT)__dsub_rn((double)a0_3, d);
-  a0_6 = (LUT)__dadd_rn((double)a0_6, d);
-  a0_7 = (LUT)__dsub_rn((double)a0_7, d);
-  d = __dmul_rn(c.kf(21), z2);
-  d = __dmul_rn(d, factor);
-  a7_2 = (LUT)__dsub_rn((double)a7_2, d);
-  a7_4 = (LUT)__dadd_rn((double)a7_4, d);
-  a7_6 = (LUT)__dadd_rn((double)a7_6, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  d = __dmul_rn(c.kf(21), z7);
-  d = __dmul_rn(d, factor);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  a2_6 = (LUT)__dadd_rn((double)a2_6, d);
-  a2_7 = (LUT)__dsub_rn((double)a2_7, d);
-  d = __dmul_rn(c.kr(21), z6);
-  d = __dmul_rn(d, msf);
-  a4_2 = (LUT)__dsub_rn((double)a4_2, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_6 = (LUT)__dadd_rn((double)a4_6, d);
-  a4_7 = (LUT)__dsub_rn((double)a4_7, d);
-  d = __dmul_rn(c.kr(21), z4);
-  d = __dmul_rn(d, msf);
-  a6_2 = (LUT)__dsub_rn((double)a6_2, d);
-  a6_4 = (LUT)__dadd_rn((double)a6_4, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_7 = (LUT)__dsub_rn((double)a6_7, d);
-  d = __dmul_rn(c.kf(22), z4);
-  d = __dmul_rn(d, factor);
-  a7_4 = (LUT)__dsub_rn((double)a7_4, d);
-  a7_5 = (LUT)__dadd_rn((double)a7_5, d);
-  a7_6 = (LUT)__dadd_rn((double)a7_6, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  d = __dmul_rn(c.kf(22), z7);
-  d = __dmul_rn(d, factor);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  a4_6 = (LUT)__dadd_rn((double)a4_6, d);
-  a4_7 = (LUT)__dsub_rn((double)a4_7, d);
-  d = __dmul_rn(c.kr(22), z6);
-  d = __dmul_rn(d, msf);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  a5_6 = (LUT)__dadd_rn((double)a5_6, d);
-  a5_7 = (LUT)__dsub_rn((double)a5_7, d);
-  d = __dmul_rn(c.kr(22), z5);
-  d = __dmul_rn(d, msf);
-  a6_4 = (LUT)__dsub_rn((double)a6_4, d);
-  a6_5 = (LUT)__dadd_rn((double)a6_5, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_7 = (LUT)__dsub_rn((double)a6_7, d);
-  d = __dmul_rn(c.kf(23), z4);
-  d = __dmul_rn(d, factor);
-  a7_4 = (LUT)__dsub_rn((double)a7_4, d);
-  a7_5 = (LUT)__dadd_rn((double)a7_5, d);
-  a7_6 = (LUT)__dadd_rn((double)a7_6, d);
-  a7_7 = (LUT)__dsub_rn((double)a7_7, d);
-  d = __dmul_rn(c.kf(23), z7);
-  d = __dmul_rn(d, factor);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  a4_6 = (LUT)__dadd_rn((double)a4_6, d);
-  a4_7 = (LUT)__dsub_rn((double)a4_7, d);
-  d = __dmul_rn(c.kr(23), z6);
-  d = __dmul_rn(d, msf);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  a5_6 = (LUT)__dadd_rn((double)a5_6, d);
-  a5_7 = (LUT)__dsub_rn((double)a5_7, d);
-  d = __dmul_rn(c.kr(23), z5);
-  d = __dmul_rn(d, msf);
-  a6_4 = (LUT)__dsub_rn((double)a6_4, d);
-  a6_5 = (LUT)__dadd_rn((double)a6_5, d);
-  a6_6 = (LUT)__dadd_rn((double)a6_6, d);
-  a6_7 = (LUT)__dsub_rn((double)a6_7, d);
-  d = __dmul_rn(__dmul_rn(c.kf(24), z1), z3);
-  d = __dmul_rn(d, factor);
-  a3_0 = (LUT)__dadd_rn((double)a3_0, d);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_1 = (LUT)__dadd_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  d = __dmul_rn(__dmul_rn(c.kf(24), z3), z3);
-  d = __dmul_rn(d, factor);
-  a1_0 = (LUT)__dadd_rn((double)a1_0, d);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  d = __dmul_rn(__dmul_rn(c.kf(24), z3), z1);
-  d = __dmul_rn(d, factor);
-  a3_0 = (LUT)__dadd_rn((double)a3_0, d);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_1 = (LUT)__dadd_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  d = __dmul_rn(c.kr(24), z1);
-  d = __dmul_rn(d, msf);
-  a0_0 = (LUT)__dadd_rn((double)a0_0, d);
-  a0_1 = (LUT)__dsub_rn((double)a0_1, d);
-  a0_1 = (LUT)__dadd_rn((double)a0_1, d);
-  a0_3 = (LUT)__dsub_rn((double)a0_3, d);
-  a0_3 = (LUT)__dsub_rn((double)a0_3, d);
-  d = __dmul_rn(c.kr(24), z0);
-  d = __dmul_rn(d, msf);
-  a1_0 = (LUT)__dadd_rn((double)a1_0, d);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  d = __dmul_rn(__dmul_rn(c.kf(25), z1), z3);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  d = __dmul_rn(__dmul_rn(c.kf(25), z3), z3);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  d = __dmul_rn(__dmul_rn(c.kf(25), z3), z1);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  d = __dmul_rn(c.kr(25), z4);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  d = __dmul_rn(c.kr(25), z4);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  d = __dmul_rn(__dmul_rn(c.kf(26), z1), z2);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_1 = (LUT)__dadd_rn((double)a3_1, d);
-  a3_2 = (LUT)__dsub_rn((double)a3_2, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dadd_rn((double)a3_4, d);
-  d = __dmul_rn(__dmul_rn(c.kf(26), z3), z2);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_2 = (LUT)__dsub_rn((double)a1_2, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  d = __dmul_rn(__dmul_rn(c.kf(26), z3), z1);
-  d = __dmul_rn(d, factor);
-  a2_1 = (LUT)__dsub_rn((double)a2_1, d);
-  a2_1 = (LUT)__dadd_rn((double)a2_1, d);
-  a2_2 = (LUT)__dsub_rn((double)a2_2, d);
-  a2_3 = (LUT)__dsub_rn((double)a2_3, d);
-  a2_4 = (LUT)__dadd_rn((double)a2_4, d);
-  d = __dmul_rn(c.kr(26), z1);
-  d = __dmul_rn(d, msf);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_1 = (LUT)__dadd_rn((double)a4_1, d);
-  a4_2 = (LUT)__dsub_rn((double)a4_2, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dadd_rn((double)a4_4, d);
-  d = __dmul_rn(c.kr(26), z4);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_2 = (LUT)__dsub_rn((double)a1_2, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_4 = (LUT)__dadd_rn((double)a1_4, d);
-  d = __dmul_rn(__dmul_rn(c.kf(27), z1), z4);
-  d = __dmul_rn(d, factor);
-  a3_1 = (LUT)__dsub_rn((double)a3_1, d);
-  a3_1 = (LUT)__dadd_rn((double)a3_1, d);
-  a3_3 = (LUT)__dsub_rn((double)a3_3, d);
-  a3_4 = (LUT)__dsub_rn((double)a3_4, d);
-  a3_5 = (LUT)__dadd_rn((double)a3_5, d);
-  d = __dmul_rn(__dmul_rn(c.kf(27), z3), z4);
-  d = __dmul_rn(d, factor);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_4 = (LUT)__dsub_rn((double)a1_4, d);
-  a1_5 = (LUT)__dadd_rn((double)a1_5, d);
-  d = __dmul_rn(__dmul_rn(c.kf(27), z3), z1);
-  d = __dmul_rn(d, factor);
-  a4_1 = (LUT)__dsub_rn((double)a4_1, d);
-  a4_1 = (LUT)__dadd_rn((double)a4_1, d);
-  a4_3 = (LUT)__dsub_rn((double)a4_3, d);
-  a4_4 = (LUT)__dsub_rn((double)a4_4, d);
-  a4_5 = (LUT)__dadd_rn((double)a4_5, d);
-  d = __dmul_rn(c.kr(27), z1);
-  d = __dmul_rn(d, msf);
-  a5_1 = (LUT)__dsub_rn((double)a5_1, d);
-  a5_1 = (LUT)__dadd_rn((double)a5_1, d);
-  a5_3 = (LUT)__dsub_rn((double)a5_3, d);
-  a5_4 = (LUT)__dsub_rn((double)a5_4, d);
-  a5_5 = (LUT)__dadd_rn((double)a5_5, d);
-  d = __dmul_rn(c.kr(27), z5);
-  d = __dmul_rn(d, msf);
-  a1_1 = (LUT)__dsub_rn((double)a1_1, d);
-  a1_1 = (LUT)__dadd_rn((double)a1_1, d);
-  a1_3 = (LUT)__dsub_rn((double)a1_3, d);
-  a1_4 = (LUT)__dsub_rn((double)a1_4, d);
-  a1_5 = (LUT)__dadd_rn((double)a1_5, d);
-  a0_0 = a0_0 + 1;
-  a1_1 = a1_1 + 1;
-  a2_2 = a2_2 + 1;
-  a3_3 = a3_3 + 1;
-  a4_4 = a4_4 + 1;
-  a5_5 = a5_5 + 1;
-  a6_6 = a6_6 + 1;
-  a7_7 = a7_7 + 1;
-  c.a(0, 0) = a0_0;
-  c.a(0, 1) = a0_1;
-  c.a(0, 2) = a0_2;
-  c.a(0, 3) = a0_3;
-  c.a(0, 4) = a0_4;
-  c.a(0, 5) = a0_5;
-  c.a(0, 6) = a0_6;
-  c.a(0, 7) = a0_7;
-  c.a(1, 0) = a1_0;
-  c.a(1, 1) = a1_1;
-  c.a(1, 2) = a1_2;
-  c.a(1, 3) = a1_3;
-  c.a(1, 4) = a1_4;
-  c.a(1, 5) = a1_5;
-  c.a(1, 6) = a1_6;
-  c.a(1, 7) = a1_7;
-  c.a(2, 0) = a2_0;
-  c.a(2, 1) = a2_1;
-  c.a(2, 2) = a2_2;
-  c.a(2, 3) = a2_3;
-  c.a(2, 4) = a2_4;
-  c.a(2, 5) = a2_5;
-  c.a(2, 6) = a2_6;
-  c.a(2, 7) = a2_7;
-  c.a(3, 0) = a3_0;
-  c.a(3, 1) = a3_1;
-  c.a(3, 2) = a3_2;
-  c.a(3, 3) = a3_3;
-  c.a(3, 4) = a3_4;
-  c.a(3, 5) = a3_5;
-  c.a(3, 6) = a3_6;
-  c.a(3, 7) = a3_7;
-  c.a(4, 0) = a4_0;
-  c.a(4, 1) = a4_1;
-  c.a(4, 2) = a4_2;
-  c.a(4, 3) = a4_3;
-  c.a(4, 4) = a4_4;
-  c.a(4, 5) = a4_5;
-  c.a(4, 6) = a4_6;
-  c.a(4, 7) = a4_7;
-  c.a(5, 0) = a5_0;
-  c.a(5, 1) = a5_1;
-  c.a(5, 2) = a5_2;
-  c.a(5, 3) = a5_3;
-  c.a(5, 4) = a5_4;
-  c.a(5, 5) = a5_5;
-  c.a(5, 6) = a5_6;
-  c.a(5, 7) = a5_7;
-  c.a(6, 0) = a6_0;
-  c.a(6, 1) = a6_1;
-  c.a(6, 2) = a6_2;
-  c.a(6, 3) = a6_3;
-  c.a(6, 4) = a6_4;
-  c.a(6, 5) = a6_5;
-  c.a(6, 6) = a6_6;
-  c.a(6, 7) = a6_7;
-  c.a(7, 0) = a7_0;
-  c.a(7, 1) = a7_1;
-  c.a(7, 2) = a7_2;
-  c.a(7, 3) = a7_3;
-  c.a(7, 4) = a7_4;
-  c.a(7, 5) = a7_5;
-  c.a(7, 6) = a7_6;
-  c.a(7, 7) = a7_7;
+  if constexpr (J == 0) {
+    const double z1 = c.z(1), z2 = c.z(2), z4 = c.z(4), z6 = c.z(6);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(1), z2), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(2), z4), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(c.kf(4), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(c.kr(10), z1), msf);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(18), z6), msf);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(21), z1), msf);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a0 = a0 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7;
+  }
+  if constexpr (J == 1) {
+    const double z0 = c.z(0), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z7 = c.z(7);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(0), z3), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(c.kr(5), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    d = __dmul_rn(__dmul_rn(c.kf(9), z3), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(10), z0), msf);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(13), z4), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(14), z5), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(15), z7), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a7 = (LUT)__dadd_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(21), z3), z3), factor);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(c.kr(21), z0), msf);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(22), z3), z3), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(23), z3), z2), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(23), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(24), z3), z4), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(24), z5), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a1 = a1 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7;
+  }
+  if constexpr (J == 2) {
+    const double z0 = c.z(0), z1 = c.z(1), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6), z7 = c.z(7);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(0), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(1), z0), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(3), z5), msf);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(5), z2), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    d = __dmul_rn(__dmul_rn(c.kf(5), z2), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    d = __dmul_rn(__dmul_rn(c.kf(6), z3), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(12), z5), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(13), z6), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(19), z7), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(23), z3), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a2 = a2 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7;
+  }
+  if constexpr (J == 3) {
+    const double z1 = c.z(1), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6), z7 = c.z(7);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kf(0), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(1), z4), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(2), z5), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(4), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(c.kr(4), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(c.kf(6), z2), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(7), z4), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(8), z4), z5), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(9), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(10), z6), factor);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(11), z6), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(12), z6), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(17), z7), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(18), z7), factor);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(21), z1), z3), factor);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(21), z3), z1), factor);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(22), z1), z3), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(22), z3), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(23), z1), z2), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(24), z1), z4), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a3 = a3 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7;
+  }
+  if constexpr (J == 4) {
+    const double z0 = c.z(0), z1 = c.z(1), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6), z7 = c.z(7);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(0), z2), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(1), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kf(2), z0), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(3), z4), factor);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(3), z4), factor);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(c.kr(6), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(7), z3), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(8), z3), z5), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(11), z4), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(11), z4), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(13), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(14), z6), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(16), z4), msf);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(16), z4), msf);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(17), z5), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(19), z6), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(20), z7), factor);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(22), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(22), z4), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(c.kr(23), z1), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(24), z3), z1), factor);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a4 = a4 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7;
+  }
+  if constexpr (J == 5) {
+    const double z1 = c.z(1), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(2), z3), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kr(3), z2), msf);
+    a2 = (LUT)__dadd_rn((double)a2, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(c.kf(7), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(8), z5), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(8), z5), factor);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(8), z3), z4), msf);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(c.kf(12), z2), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(14), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(17), z4), msf);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(20), z6), msf);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(24), z1), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a5 = a5 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7;
+  }
+  if constexpr (J == 6) {
+    const double z0 = c.z(0), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0;
+    d = __dmul_rn(c.kr(9), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(10), z3), factor);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(11), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kr(12), z3), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a5 = (LUT)__dsub_rn((double)a5, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(13), z2), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(14), z4), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    d = __dmul_rn(__dmul_rn(c.kf(15), z6), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a7 = (LUT)__dadd_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(15), z6), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a7 = (LUT)__dadd_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(18), z0), msf);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(19), z4), msf);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kr(20), z5), msf);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a6 = a6 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7;
+  }
+  if constexpr (J == 7) {
+    const double z1 = c.z(1), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4);
+    LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0;
+    d = __dmul_rn(__dmul_rn(c.kr(15), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a6 = (LUT)__dsub_rn((double)a6, d);
+    a7 = (LUT)__dadd_rn((double)a7, d);
+    d = __dmul_rn(c.kf(16), factor);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(17), z3), factor);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(18), z3), factor);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(19), z2), factor);
+    a2 = (LUT)__dsub_rn((double)a2, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    d = __dmul_rn(__dmul_rn(c.kf(20), z4), factor);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a6 = (LUT)__dadd_rn((double)a6, d);
+    a7 = (LUT)__dsub_rn((double)a7, d);
+    a7 = a7 + 1;
+    v[0] = a0; v[1] = a1; v[2] = a2; v[3] = a3; v[4] = a4; v[5] = a5; v[6] = a6; v[7] = a7;
+  }
 }
 
 }  // namespace gen_zhang

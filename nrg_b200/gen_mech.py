@@ -11,7 +11,7 @@ both paths give the same bits.  The tables of the specialised code are
 emitted too; nrg_chem_create compares them with the parsed mechanism and uses
 the specialised kernels only on an exact match.
 
-    python nrg_b200/gen_mech.py            # the four reference decks, writes the headers
+    python nrg_b200/gen_mech.py            # the five reference decks, writes the headers
 
 Needs a built libnrg_chem.so (it parses the decks with the library's own
 reader, nrg_mech_tables).
@@ -22,6 +22,9 @@ import os
 import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
+
+# as kMergeUpTo in csrc/chem_device.cuh
+MERGE_UP_TO = 8
 
 
 def reduced_structure(t: dict):
@@ -50,6 +53,12 @@ def reduced_structure(t: dict):
     left = [[int_of[s] if s >= 0 else -1 for s in row] for row in left]
     right = [[int_of[s] if s >= 0 else -1 for s in row] for row in right]
     upd = [[(int_of[k], p) for k, p in u] for u in upd]
+    if len(reacts) <= MERGE_UP_TO:
+        # reactions with equal lists are one reaction of the right-hand side
+        # (their rate constants are added once per cell)
+        first = [r for r in range(R) if (left[r], right[r]) not in list(zip(left[:r], right[:r]))]
+        left, right, upd = ([x[r] for r in first] for x in (left, right, upd))
+        R = len(first)
     return len(reacts), R, left, right, upd
 
 
@@ -106,39 +115,36 @@ def emit(name: str, ns: str, NI: int, R: int, left, right, upd) -> str:
         w(f"  c.zd({k}) = d{k};")
     w("}")
     w("")
-    # analytic iteration matrix
-    touched = set()
-    body = []
-    for r in range(R):
-        for side in (0, 1):
-            parts = right[r] if side else left[r]
-            k = f"c.kr({r})" if side else f"c.kf({r})"
-            sgn = "msf" if side else "factor"
-            for p in range(3):
-                sp = parts[p]
-                if sp < 0:
-                    continue
-                d = mul_chain(k, [parts[q] for q in range(3) if q != p and parts[q] >= 0])
-                body.append(f"  d = {d};")
-                body.append(f"  d = __dmul_rn(d, {sgn});")
-                for k2, pr in upd[r]:
-                    touched.add((sp, k2))
-                    body.append(f"  a{sp}_{k2} = (LUT){'__dadd_rn' if pr else '__dsub_rn'}((double)a{sp}_{k2}, d);")
-    w("// I + factor * J written into the LU storage: c.a(j, i) = A(i+1, j+1)")
-    w("template <class S, typename LUT>")
-    w("__device__ __forceinline__ void spec_matrix(S& c, double factor) {")
-    for k in range(NI):
-        w(f"  const double z{k} = c.z({k});")
+    # analytic iteration matrix, column by column
+    w("// Column J of I + factor * J: v[i] = A(i+1, J+1), each element's terms in")
+    w("// reaction order.")
+    w("template <int J, class S, typename LUT>")
+    w(f"__device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[{NI}]) {{")
     w("  const double msf = -factor;")
-    names = [f"a{j}_{i}" for j in range(NI) for i in range(NI)]
-    w("  LUT " + ", ".join(f"{n} = (LUT)0" for n in names) + ";")
     w("  double d;")
-    o.extend(body)
-    for i in range(NI):
-        w(f"  a{i}_{i} = a{i}_{i} + 1;")
     for j in range(NI):
-        for i in range(NI):
-            w(f"  c.a({j}, {i}) = a{j}_{i};")
+        names = set()
+        body = []
+        for r in range(R):
+            for side in (0, 1):
+                parts = right[r] if side else left[r]
+                k = f"c.kr({r})" if side else f"c.kf({r})"
+                for p in range(3):
+                    if parts[p] != j:
+                        continue
+                    others = [parts[q] for q in range(3) if q != p and parts[q] >= 0]
+                    names.update(others)
+                    body.append(f"    d = __dmul_rn({mul_chain(k, others)}, {'msf' if side else 'factor'});")
+                    for k2, pr in upd[r]:
+                        body.append(f"    a{k2} = (LUT){'__dadd_rn' if pr else '__dsub_rn'}((double)a{k2}, d);")
+        w(f"  if constexpr (J == {j}) {{")
+        if names:
+            w("    const double " + ", ".join(f"z{k} = c.z({k})" for k in sorted(names)) + ";")
+        w("    LUT " + ", ".join(f"a{i} = (LUT)0" for i in range(NI)) + ";")
+        o.extend(body)
+        w(f"    a{j} = a{j} + 1;")
+        w("    " + " ".join(f"v[{i}] = a{i};" for i in range(NI)))
+        w("  }")
     w("}")
     w("")
     w(f"}}  // namespace {ns}")
@@ -161,14 +167,15 @@ def emit_index(names) -> str:
         o += ["template <>", f"struct SpecOf<kSpec{n.capitalize()}> {{",
               f"  static constexpr int kN = {ns}::kSpecN, kR = {ns}::kSpecR;",
               "  template <class S>", f"  __device__ static void rhs(S& c) {{ {ns}::spec_rhs(c); }}",
-              "  template <class S, typename LUT>",
-              f"  __device__ static void matrix(S& c, double f) {{ {ns}::spec_matrix<S, LUT>(c, f); }}", "};"]
+              "  template <int J, class S, typename LUT>",
+              f"  __device__ static void column(const S& c, double f, LUT (&v)[{ns}::kSpecN]) {{",
+              f"    {ns}::spec_column<J>(c, f, v);", "  }", "};"]
     o += ["", "// 0 when the reduced reaction lists match none of the generated codes.",
           "template <class M>", "inline int match_specialised_tables(const M& m) {"]
     for n in names:
         ns = f"gen_{n.lower()}"
-        o += [f"  if (m.NI == {ns}::kSpecN && m.R == {ns}::kSpecR) {{", "    bool ok = true;",
-              "    for (int r = 0; ok && r < m.R; ++r) {",
+        o += [f"  if (m.NI == {ns}::kSpecN && m.RM == {ns}::kSpecR) {{", "    bool ok = true;",
+              "    for (int r = 0; ok && r < m.RM; ++r) {",
               f"      ok = m.nupd[r] == {ns}::kSpecNupd[r];",
               "      for (int i = 0; ok && i < 3; ++i)",
               f"        ok = m.left[r][i] == {ns}::kSpecLeft[r][i] && m.right[r][i] == {ns}::kSpecRight[r][i];",
