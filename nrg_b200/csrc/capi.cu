@@ -1302,16 +1302,23 @@ extern "C" int nrg_chem_load_transport(nrg_chem* h, const char* transport_path) 
   d.N = N;
   for (int k = 0; k < N; ++k) d.W[k] = h->mech.molar_mass[k];
   int q = 0;
+  double uniq[nrg::kDiffMaxPairs];
   for (int i = 0; i < N - 1; ++i)
     for (int j = i + 1; j < N; ++j, ++q) {
       const double eps_i = h->mech.well_depth[i], eps_j = h->mech.well_depth[j];
-      d.bdc[q] = h->mech.binary_diffusivity[(size_t)i * N + j];
-      d.pair_ok[q] = d.bdc[q] > 0.0 && eps_i > 0.0 && eps_j > 0.0;
-      if (!d.pair_ok[q]) continue;
-      const double sq = std::sqrt(eps_i * eps_j);  // the reference's per-call value, bit for bit
+      const double bdc = h->mech.binary_diffusivity[(size_t)i * N + j];
+      if (!(bdc > 0.0 && eps_i > 0.0 && eps_j > 0.0)) continue;
+      d.ibdc[q] = 1.0 / bdc;
+      const double sq = std::sqrt(eps_i * eps_j);
       int u = 0;
-      while (u < d.n_uniq && d.uniq_sq[u] != sq) ++u;
-      if (u == d.n_uniq) d.uniq_sq[d.n_uniq++] = sq;
+      while (u < d.n_uniq && uniq[u] != sq) ++u;
+      if (u == d.n_uniq) {
+        uniq[d.n_uniq++] = sq;
+        d.uniq_isq[u] = 1.0 / sq;
+        const long double c = 1.06036L * powl(sq / 1024.0L, 0.15610L);
+        d.uniq_pow[u] = (double)c;
+        d.uniq_pow_lo[u] = (double)(c - d.uniq_pow[u]);
+      }
       d.pair_u[q] = (unsigned char)u;
     }
   h->has_transport = true;

@@ -11,10 +11,13 @@ constexpr int kDiffMaxSpecies = 16;
 constexpr int kDiffMaxPairs = kDiffMaxSpecies * (kDiffMaxSpecies - 1) / 2;
 
 // Flat cells, species-major fields at [k * ld + c].  Pair tables in the order
-// (0,1), (0,2), ..., (1,2), ...: bdc = binary diffusivity constant,
-// pair_ok = bdc > 0 and both well depths > 0, pair_u = index of the pair's
-// sqrt(eps_i * eps_j) in uniq_sq (the distinct values, first-seen order):
-// pairs with equal values share one collision-integral evaluation.
+// (0,1), (0,2), ..., (1,2), ...: ibdc = 1 / binary diffusivity constant (0: the
+// pair has none, or a well depth that is not positive), pair_u = index of the
+// pair's sqrt(eps_i * eps_j) among the n_uniq distinct values (first-seen
+// order): pairs with equal values share one collision-integral evaluation.
+// uniq_isq: the values' reciprocals; uniq_pow + uniq_pow_lo: 1.06036
+// (value / 1024)^0.15610, the factor of (T / 1024)^-0.15610 in the fit's first
+// term.
 struct DiffusivityArgs {
   long n = 0, ld = 0;
   int N = 0;
@@ -25,10 +28,10 @@ struct DiffusivityArgs {
   const int8_t* bc = nullptr;
   double* D = nullptr;
   double W[kDiffMaxSpecies] = {};
-  double bdc[kDiffMaxPairs] = {};
-  double uniq_sq[kDiffMaxPairs] = {};
+  double ibdc[kDiffMaxPairs] = {};
+  double uniq_isq[kDiffMaxPairs] = {};
+  double uniq_pow[kDiffMaxPairs] = {}, uniq_pow_lo[kDiffMaxPairs] = {};
   int n_uniq = 0;
-  unsigned char pair_ok[kDiffMaxPairs] = {};
   unsigned char pair_u[kDiffMaxPairs] = {};
 };
 
