@@ -1358,22 +1358,31 @@ __device__ __forceinline__ double temperature_after_fast(double T0, const double
     s1 += X[k] * c_mech.invW[k];
   }
   const double W1 = 1.0 / s1;
-  double hc = 0.0, cp = 0.0;
-  double temp = NRG_FMIN(T0, 6000.0);
-  const int set = nasa_set(temp);
+  double hc = 0.0;
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     X[k] = X[k] * c_mech.invW[k] * W1;
     hc += c_mech.h_ref[k] * X[k];
-    const double* a = c_mech.a[k][set];
-    cp += fma(fma(fma(fma(a[4], temp, a[3]), temp, a[2]), temp, a[1]), temp, a[0]) * X[k];
   }
-  const double ei = e1 * W1, rcp = 1.0 / cp;
+  // the mixture's polynomial (coefficients weighted by the mole fractions, formed
+  // again when the iteration crosses 1000 K), one evaluation per iteration
+  double temp = NRG_FMIN(T0, 6000.0), m[6], rcp = 0.0;
+  const double ei = e1 * W1;
+  int set = -1;
   for (int it = 0; it < 1000; ++it) {
-    double e = 0.0;
+    const double t = NRG_FMIN(temp, 6000.0);
+    if (nasa_set(t) != set) {
+      set = nasa_set(t);
 #pragma unroll
-    for (int k = 0; k < N; ++k) e += nasa_enthalpy_fast(k, temp) * X[k];
-    e -= RG * temp;
+      for (int i = 0; i < 6; ++i) {
+        m[i] = 0.0;
+#pragma unroll
+        for (int k = 0; k < N; ++k) m[i] = fma(X[k], c_mech.a[k][set][i], m[i]);
+      }
+      if (it == 0) rcp = 1.0 / fma(fma(fma(fma(m[4], t, m[3]), t, m[2]), t, m[1]), t, m[0]);
+    }
+    const double hp = fma(fma(fma(fma(m[4] * 0.2, t, m[3] * 0.25), t, m[2] * (1.0 / 3.0)), t, m[1] * 0.5), t, m[0]);
+    const double e = fma(hp, t, m[5]) - RG * temp;
     const double res = (ei - (e - hc)) * rcp;
     temp += res;
     if (fabs(res) < (double)1e-08f) break;

@@ -382,83 +382,83 @@ __device__ __forceinline__ bool write_if_skipped(const StepArgs& a, long c, doub
   return true;
 }
 
-// Per-block copy of what the gate's energy closure reads: NASA-7 enthalpy
-// coefficients pre-divided by their powers (b_i = a_i / (i + 1), i < 5, and
-// a_5), cp coefficients a_0..a_4, both sets of each species, and 1 / W.
+// Per-block copy of what the gate's energy closure reads: the NASA-7 enthalpy
+// coefficients a_0..a_5 of both sets of each species, and 1 / W.
 struct GateThermo {
-  double h[9][2][6];
-  double cp[9][2][5];
+  double a[2][6][9];
   double invW[9];
 };
 
 __device__ void gate_thermo_init(GateThermo* g) {
-  for (int i = threadIdx.x; i < 9 * 2; i += blockDim.x) {
-    const int k = i >> 1, set = i & 1;
-    const double* a = c_mech.a[k][set];
-    for (int j = 0; j < 5; ++j) {
-      g->h[k][set][j] = a[j] / (double)(j + 1);
-      g->cp[k][set][j] = a[j];
-    }
-    g->h[k][set][5] = a[5];
-    if (set == 0) g->invW[k] = c_mech.invW[k];
+  for (int i = threadIdx.x; i < 2 * 6 * 9; i += blockDim.x)
+    g->a[i / 54][i / 9 % 6][i % 9] = c_mech.a[i % 9][i / 54][i / 9 % 6];
+  if (threadIdx.x < 9) g->invW[threadIdx.x] = c_mech.invW[threadIdx.x];
+}
+
+// NASA-7 coefficients of a mixture: the species' weighted by its mole fractions
+// (the reference's specie_enthalpy per mole, times R in the tables).
+__device__ __forceinline__ void gate_mixture(const GateThermo& g, int set, const double (&X)[9], double (&m)[6]) {
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    m[i] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) m[i] = fma(X[k], g.a[set][i][k], m[i]);
   }
 }
 
-// h_k(T) * ... as the reference's specie_enthalpy (per mole, times R in the
-// tables): t (b0 + t (b1 + t (b2 + t (b3 + t b4)))) + a5, t = min(T, 6000 K).
-__device__ __forceinline__ double gate_enthalpy(const GateThermo& g, int k, double T) {
-  const double t = fmin(T, 6000.0);
-  const double* b = g.h[k][t >= 1000.0 ? 1 : 0];
-  return fma(t, fma(t, fma(t, fma(t, fma(t, b[4], b[3]), b[2]), b[1]), b[0]), b[5]);
+// t (a0 + t (a1/2 + t (a2/3 + t (a3/4 + t a4/5)))) + a5, t <= 6000 K.
+__device__ __forceinline__ double gate_enthalpy(const double (&m)[6], double t) {
+  const double p = fma(fma(fma(fma(m[4] * 0.2, t, m[3] * 0.25), t, m[2] * (1.0 / 3.0)), t, m[1] * 0.5), t, m[0]);
+  return fma(p, t, m[5]);
 }
 
 // Energy closure of the gate: the reference's constant-density closure
 // (cpm_solver.f90:517,549; calculate_temperature, thermophysical_properties_
 // class.f90:409-452 -- Newton with cp frozen at the start temperature, at
-// most 1000 iterations, |step| < 1e-8 K) unrolled over the nine species in
-// registers, started at T_start (the network's temperature).  The gate
-// compares its result with the network's temperature change within dT_tol,
-// so it agrees with the integrator's closure to far below that tolerance
-// rather than to its last bit.
+// most 1000 iterations, |step| < 1e-8 K), started at T_start (the network's
+// temperature), on the polynomial of the mixture.  The gate compares its
+// result with the network's temperature change within dT_tol, so it agrees
+// with the integrator's closure to far below that tolerance rather than to its
+// last bit.
 __device__ __forceinline__ double gate_closure(const GateThermo& g, double T0, double T_start,
                                                const double (&Y0)[9], const double (&dY)[9], double dE) {
   const double RG = 8.31446261815324;
-  double X[9], s0 = 0.0, s1 = 0.0;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) s0 += Y0[k] * g.invW[k];
-  const double W0 = 1.0 / s0;
-  double e0 = 0.0, h0 = 0.0;
+  double X[9], m[6], s0 = 0.0, s1 = 0.0, h0 = 0.0;
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
-    const double x = Y0[k] * g.invW[k] * W0;
-    e0 += gate_enthalpy(g, k, T0) * x;
-    h0 += c_mech.h_ref[k] * x;
+    X[k] = Y0[k] * g.invW[k];
+    s0 += X[k];
+    h0 += c_mech.h_ref[k] * X[k];
   }
-  e0 -= RG * T0;
-  const double e1 = (e0 - h0) / W0 + dE;
+  const double W0 = 1.0 / s0, tc0 = fmin(T0, 6000.0);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) X[k] *= W0;
+  gate_mixture(g, tc0 >= 1000.0 ? 1 : 0, X, m);
+  const double e1 = (gate_enthalpy(m, tc0) - RG * T0) * s0 - h0 + dE;
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     X[k] = Y0[k] + dY[k];
     s1 += X[k] * g.invW[k];
   }
   const double W1 = 1.0 / s1;
-  double hc = 0.0, cp = 0.0;
+  double hc = 0.0;
   double temp = fmin(T_start, 6000.0);
-  const int set = temp >= 1000.0 ? 1 : 0;
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     X[k] = X[k] * g.invW[k] * W1;
     hc += c_mech.h_ref[k] * X[k];
-    const double* a = g.cp[k][set];
-    cp += fma(temp, fma(temp, fma(temp, fma(temp, a[4], a[3]), a[2]), a[1]), a[0]) * X[k];
   }
-  const double ei = e1 * W1, rcp = 1.0 / cp;
+  int set = temp >= 1000.0 ? 1 : 0;
+  gate_mixture(g, set, X, m);
+  const double ei = e1 * W1;
+  const double rcp = 1.0 / fma(temp, fma(temp, fma(temp, fma(temp, m[4], m[3]), m[2]), m[1]), m[0]);
   for (int it = 0; it < 1000; ++it) {
-    double e = 0.0;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) e += gate_enthalpy(g, k, temp) * X[k];
-    e -= RG * temp;
-    const double res = (ei - (e - hc)) * rcp;
+    const double t = fmin(temp, 6000.0);
+    if ((t >= 1000.0 ? 1 : 0) != set) {
+      set ^= 1;
+      gate_mixture(g, set, X, m);
+    }
+    const double res = (ei - (gate_enthalpy(m, t) - RG * temp - hc)) * rcp;
     temp += res;
     if (fabs(res) < (double)1e-08f) break;
   }
