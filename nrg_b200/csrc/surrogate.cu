@@ -32,80 +32,107 @@
 namespace nrg {
 
 // ------------------------------------------------------------------ GEMM
-struct GemmArgs {
-  int M, N, K;
-  const __nv_bfloat16* A;
-  long sam, sak;
-  const __nv_bfloat16* B;
-  long sbk, sbn;
-  float* C;  // fp32 result (may be null)
-  long ldc;
-  const float* bias;   // per column (may be null)
-  __nv_bfloat16* H;    // bf16 activation output (may be null)
-  long ldh;
-  int gelu;            // H = bf16(gelu(C)) when set, else bf16(C)
-};
-
 __device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi) {
   return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
-// C[M, N] = sum_k A[m, k] B[k, n] (+ bias, GELU) on the tensor cores, for
-// training (forward, weight and activation gradients) and the GEMM-chain
-// inference path.  One 128-thread CTA per 128-row x BN-column tile (BN = N
-// rounded up to 16, at most 128): K advances in chunks of 64, each staged in
-// shared memory in the K-major no-swizzle core-matrix layout by all threads
-// (16-byte vector loads where K is the contiguous direction, element loads
-// that transpose otherwise), then multiplied by one thread with
-// tcgen05.mma (kind::f16, FP32 accumulator in 128 TMEM columns); two
-// buffers, so the next chunk is staged while the tensor core reads the
-// previous one.  gridDim.z > 1 splits K (the weight gradients, K = batch):
-// each CTA adds its partial tile to C with atomics (C zeroed beforehand, no
-// bias or GELU then).  Every mbarrier wait is bounded; a timeout sets *err
-// and the CTA stops.
-constexpr uint64_t kTcWaitNs = 1000000000ull;  // 1 s per MMA wait (this GEMM and k_mlp_tc)
-constexpr int kTgBK = 64;
-constexpr uint32_t kTgBuf = 128 * kTgBK * 2;  // one operand chunk: 128 rows x 64 bf16 = 16 KB
-constexpr uint32_t kTgSmem = 4 * kTgBuf + 64;  // A0 A1 B0 B1, barriers, TMEM slot
+// One contraction C[m, n] = sum_k A(m, k) B(n, k) of the training and the GEMM
+// chain's inference, N = 16 or 128:
+//   kFwd: Z = A W^T + b (fp32, may be null), H = bf16(gelu(Z)) (may be null)
+//   kDH:  dZ = (A W) gelu'(Z), bf16, and its column sums added to db
+//   kDW:  C += A B, K split over CTAs (C zeroed beforehand)
+// a_mn / b_mn: the operand is stored with its M or N index contiguous ([K][ld],
+// the gradients' operands as the forward pass left them), else K contiguous.
+enum { kFwd = 0, kDH, kDW };
+struct GemmJob {
+  int mode;
+  int M, N, K;
+  const __nv_bfloat16 *A, *B;
+  int lda, ldb;
+  int a_mn, b_mn;
+  float* C;            // fp32 result (kFwd: may be null), ldc = N
+  const float* bias;   // kFwd, per column
+  __nv_bfloat16* H;    // bf16 result (kFwd: may be null), N columns
+  const float* Z;      // kDH: pre-activations, N columns
+  float* db;           // kDH
+  int k_per_cta;       // kDW; else K
+  int tiles;           // CTAs
+};
 
-__device__ __forceinline__ void tg_stage(unsigned char* dst, const __nv_bfloat16* src, long s_row, long s_k,
-                                         long row0, long rows, long k0, long kend) {
-  // dst: 128 rows x kTgBK, row r = operand row row0 + r, column kk = k0 + kk
-  const __nv_bfloat16 zero = __float2bfloat16(0.f);
-  const bool vec = s_k == 1 && (s_row % 8) == 0 && ((reinterpret_cast<uintptr_t>(src) & 15) == 0) &&
-                   k0 + kTgBK <= kend;
-  if (vec) {
-    for (int e = threadIdx.x; e < 128 * (kTgBK / 8); e += blockDim.x) {
-      const int r = e / (kTgBK / 8), kc = e % (kTgBK / 8);
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (row0 + r < rows) v = *reinterpret_cast<const uint4*>(src + (row0 + r) * s_row + k0 + kc * 8);
-      *reinterpret_cast<uint4*>(dst + tc::kmajor_off(r, kc, kTgBK)) = v;
+// A 256-thread CTA takes a 128-row tile (kDW: all of M and a range of K).  K
+// advances in chunks of 128: all threads copy the chunk of both operands with
+// 16-byte loads into the K-major or MN-major no-swizzle layout, whichever the
+// operand has in memory (the tensor core reads either, so nothing is
+// transposed), then one thread issues tcgen05.mma (kind::f16, FP32
+// accumulator in 128 TMEM columns).  In training K <= 128 per CTA, one chunk.
+// The result goes from TMEM through shared memory, so that rows are written,
+// read or added (16-byte reductions) as whole lines.  A launch holds one or two
+// jobs (the weight gradient of a layer and the gradient of its input need
+// only that layer's output gradient).  What bounds a training step of 4,096
+// rows is the latency of its 14 launches, not the tensor pipe: 0.70 -> 0.13
+// ms per step against element-wise transposing copies and results written and
+// added row by row from the accumulator's lanes.  Every mbarrier wait is
+// bounded; a timeout sets *err and the CTA stops.
+constexpr uint64_t kTcWaitNs = 1000000000ull;  // 1 s per MMA wait (this GEMM and k_mlp_tc)
+constexpr int kTgK = 128;
+constexpr int kTgThreads = 256;
+constexpr uint32_t kTgBuf = 128 * kTgK * 2;      // one operand chunk, 32 KB
+constexpr int kTgRow = 132;                      // floats per staged result row (padded)
+constexpr uint32_t kTgMisc = 128 * kTgRow * 4;   // after the result, which covers the operands
+constexpr uint32_t kTgSmem = kTgMisc + 8 * 128 * 4 + 64;
+static_assert(2 * kTgBuf <= kTgMisc, "the staged result covers the operand buffers");
+
+// rows [row0, row0 + 128) x columns [k0, k0 + 128) of the operand, zero outside
+// (rows, kend); kc: columns of the shared layout (16 or 128).
+__device__ __forceinline__ void tg_stage(unsigned char* dst, const __nv_bfloat16* src, int ld, bool mn, long row0,
+                                         long rows, long k0, long kend, int kc) {
+  const int lane8 = threadIdx.x & 7, grp = threadIdx.x >> 3;  // 8 lanes fill one core matrix
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  if (mn) {
+#pragma unroll 8
+    for (int e = grp; e < 16 * (kc / 8); e += kTgThreads / 8) {
+      const int ch = e % 16, k = e / 16 * 8 + lane8;
+      uint4 v = zero;
+      if (k0 + k < kend && row0 + ch * 8 < rows)
+        v = *reinterpret_cast<const uint4*>(src + (k0 + k) * ld + row0 + ch * 8);
+      *reinterpret_cast<uint4*>(dst + tc::mnmajor_off(k, ch)) = v;
     }
   } else {
-    // consecutive threads take consecutive rows (coalesced when rows are the
-    // contiguous direction, as in the transposed operands of the gradients)
-    for (int e = threadIdx.x; e < 128 * kTgBK; e += blockDim.x) {
-      const int r = e % 128, kk = e / 128;
-      const long row = row0 + r, k = k0 + kk;
-      const __nv_bfloat16 v = (row < rows && k < kend) ? src[row * s_row + k * s_k] : zero;
-      *reinterpret_cast<__nv_bfloat16*>(dst + tc::kmajor_off(r, kk >> 3, kTgBK) + (kk & 7) * 2) = v;
+    const int nc = kc / 8;
+#pragma unroll 8
+    for (int e = grp; e < 16 * nc; e += kTgThreads / 8) {
+      const int ch = e % nc, r = e / nc * 8 + lane8;
+      uint4 v = zero;
+      if (row0 + r < rows && k0 + ch * 8 < kend)
+        v = *reinterpret_cast<const uint4*>(src + (row0 + r) * ld + k0 + ch * 8);
+      *reinterpret_cast<uint4*>(dst + tc::kmajor_off(r, ch, kc)) = v;
     }
   }
 }
 
-__global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmArgs g, long k_per_cta, unsigned int* err) {
+__device__ __forceinline__ void red_add4(float* p, float4 v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kTgThreads, 2) k_gemm_tc(const __grid_constant__ GemmJob j0,
+                                                           const __grid_constant__ GemmJob j1, unsigned int* err) {
   extern __shared__ __align__(1024) unsigned char sm[];
-  unsigned char* bufA[2] = {sm, sm + kTgBuf};
-  unsigned char* bufB[2] = {sm + 2 * kTgBuf, sm + 3 * kTgBuf};
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + 4 * kTgBuf);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + 4 * kTgBuf + 32);
-  const int tid = threadIdx.x, wq = tid >> 5;
-  const long m0 = (long)blockIdx.x * 128, n0 = (long)blockIdx.y * 128;
-  const long kb = (long)blockIdx.z * k_per_cta, ke = min((long)g.K, kb + k_per_cta);
-  const int bn = (int)(((min(128L, (long)g.N - n0) + 15) / 16) * 16);
+  const bool second = (int)blockIdx.x >= j0.tiles;
+  const GemmJob& g = second ? j1 : j0;
+  const int tile = second ? (int)blockIdx.x - j0.tiles : (int)blockIdx.x;
+  unsigned char *bufA = sm, *bufB = sm + kTgBuf;
+  float* res = reinterpret_cast<float*>(sm);
+  float* colsum = reinterpret_cast<float*>(sm + kTgMisc);  // [warp][128]
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kTgMisc + 8 * 128 * 4);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kTgMisc + 8 * 128 * 4 + 16);
+  const int tid = threadIdx.x, wq = tid >> 5, lane = tid & 31;
+  const long m0 = g.mode == kDW ? 0 : (long)tile * 128;
+  const long kb = g.mode == kDW ? (long)tile * g.k_per_cta : 0, ke = min((long)g.K, kb + g.k_per_cta);
+  const int kc = g.K <= 16 ? 16 : kTgK;
+  const bool a_mn = g.a_mn, b_mn = g.b_mn;
   if (tid == 0) {
-    tc::mbar_init(tc::smem_u32(&mbar[0]), 1);
-    tc::mbar_init(tc::smem_u32(&mbar[1]), 1);
+    tc::mbar_init(tc::smem_u32(mbar), 1);
     tc::mbar_init_fence();
   }
   if (tid < 32) tc::tmem_alloc(tc::smem_u32(tslot), 128);
@@ -113,62 +140,88 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmArgs g, long k_per_cta, 
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *tslot;
-  // B operand rows are the output columns n: element (n, k) = B[k * sbk + n * sbn]
-  const uint32_t idesc = tc::idesc_bf16_f32(128, (uint32_t)bn);
-  const long nch = (ke - kb + kTgBK - 1) / kTgBK;
-  uint32_t parity[2] = {0u, 0u};
+  const uint32_t idesc = tc::idesc_bf16_f32(128, (uint32_t)g.N, a_mn, b_mn);
   bool ok = true;
-  for (long c = 0; c < nch && ok; ++c) {
-    const int b = (int)(c & 1);
-    if (c >= 2) {  // the MMAs that read this buffer two chunks ago are done
-      ok = tc::bar_and(1, 128, tc::mbar_wait(tc::smem_u32(&mbar[b]), parity[b], kTcWaitNs));
-      parity[b] ^= 1u;
+  uint32_t parity = 0;
+  for (long k0 = kb; k0 < ke && ok; k0 += kc) {
+    if (k0 > kb) {  // the MMAs that read the buffers are done
+      ok = __syncthreads_and(tc::mbar_wait(tc::smem_u32(mbar), parity, kTcWaitNs));
+      parity ^= 1u;
       if (!ok) break;
     }
-    const long k0 = kb + c * kTgBK;
-    tg_stage(bufA[b], g.A, g.sam, g.sak, m0, g.M, k0, ke);
-    tg_stage(bufB[b], g.B, g.sbn, g.sbk, n0, g.N, k0, ke);
+    tg_stage(bufA, g.A, g.lda, a_mn, m0, g.M, k0, ke, kc);
+    tg_stage(bufB, g.B, g.ldb, b_mn, 0, g.N, k0, ke, kc);
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     if (tid == 0) {
       tc::fence_after_sync();
-      const uint32_t a = tc::smem_u32(bufA[b]), bb = tc::smem_u32(bufB[b]);
-#pragma unroll
-      for (int s = 0; s < kTgBK / 16; ++s)
-        tc::mma_bf16(tbase, tc::smem_desc(a + s * 256, 128, kTgBK * 16), tc::smem_desc(bb + s * 256, 128, kTgBK * 16),
-                     idesc, (c > 0 || s > 0) ? 1u : 0u);
-      tc::commit(tc::smem_u32(&mbar[b]));
+      const uint32_t a = tc::smem_u32(bufA), b = tc::smem_u32(bufB);
+      for (int s = 0; s < kc / 16; ++s) {
+        const uint64_t da = a_mn ? tc::smem_desc(a + s * 2 * tc::kMnGroup, tc::kMnGroup, 128)
+                                 : tc::smem_desc(a + s * 256, 128, kc * 16);
+        const uint64_t db = b_mn ? tc::smem_desc(b + s * 2 * tc::kMnGroup, tc::kMnGroup, 128)
+                                 : tc::smem_desc(b + s * 256, 128, kc * 16);
+        tc::mma_bf16(tbase, da, db, idesc, (k0 > kb || s > 0) ? 1u : 0u);
+      }
+      tc::commit(tc::smem_u32(mbar));
     }
   }
-  // the last chunk's MMAs (and with them all earlier ones) complete
-  if (ok && nch > 0) {
-    const int b = (int)((nch - 1) & 1);
-    ok = tc::bar_and(1, 128, tc::mbar_wait(tc::smem_u32(&mbar[b]), parity[b], kTcWaitNs));
-  }
+  const bool any = ke > kb;
+  if (any && ok) ok = __syncthreads_and(tc::mbar_wait(tc::smem_u32(mbar), parity, kTcWaitNs));
   if (!ok) {
     if (tid == 0) atomicOr(err, 1u);
-  } else if (nch > 0) {
+  } else if (any) {
     tc::fence_after_sync();
-    const long m = m0 + tid;
-    const bool split = gridDim.z > 1;
-    for (int j0 = 0; j0 < bn; j0 += 16) {
+    // accumulator rows (lanes) to shared memory: warp w has lanes 32 (w % 4)..,
+    // and of 128 columns the half w / 4
+    const int row = (wq & 3) * 32 + lane;
+    const int c0 = g.N == 128 ? (wq >> 2) * 64 : 0, c1 = g.N == 128 ? c0 + 64 : (wq < 4 ? 16 : 0);
+    for (int c = c0; c < c1; c += 16) {
       uint32_t r[16];
-      tc::tmem_ld16(tbase + ((uint32_t)(wq * 32) << 16) + (uint32_t)j0, r);
+      tc::tmem_ld16(tbase + ((uint32_t)((wq & 3) * 32) << 16) + (uint32_t)c, r);
       tc::tmem_ld_wait();
-      if (m >= g.M) continue;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const long n = n0 + j0 + j;
-        if (n >= g.N) continue;
-        float v = __uint_as_float(r[j]);
-        if (split) {
-          atomicAdd(&g.C[m * g.ldc + n], v);
-          continue;
-        }
-        if (g.bias) v += g.bias[n];
-        if (g.C) g.C[m * g.ldc + n] = v;
-        if (g.H) g.H[m * g.ldh + n] = __float2bfloat16(g.gelu ? gelu_f(v) : v);
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(res + row * kTgRow + c + 4 * q) =
+            make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+    }
+    __syncthreads();
+    const int q4 = g.N / 4;  // 16-byte pieces of a row: 4 or 32
+    const int cq = tid % q4, n = 4 * cq;
+    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), sum = bias;
+    if (g.mode == kFwd) bias = *reinterpret_cast<const float4*>(g.bias + n);
+    const long rows = min(128L, (long)g.M - m0);
+    for (long r = tid / q4; r < rows; r += kTgThreads / q4) {
+      float4 v = *reinterpret_cast<const float4*>(res + r * kTgRow + n);
+      const long o = (m0 + r) * g.N + n;
+      if (g.mode == kDW) {
+        red_add4(g.C + o, v);
+        continue;
+      }
+      if (g.mode == kFwd) {
+        v = make_float4(v.x + bias.x, v.y + bias.y, v.z + bias.z, v.w + bias.w);
+        if (g.C) *reinterpret_cast<float4*>(g.C + o) = v;
+        if (!g.H) continue;
+        v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
+      } else {
+        const float4 z = *reinterpret_cast<const float4*>(g.Z + o);
+        v = make_float4(v.x * gelu_grad_f(z.x), v.y * gelu_grad_f(z.y), v.z * gelu_grad_f(z.z),
+                        v.w * gelu_grad_f(z.w));
+        sum = make_float4(sum.x + v.x, sum.y + v.y, sum.z + v.z, sum.w + v.w);
+      }
+      *reinterpret_cast<uint2*>(g.H + o) =
+          make_uint2(pack_bf16(__float2bfloat16(v.x), __float2bfloat16(v.y)),
+                     pack_bf16(__float2bfloat16(v.z), __float2bfloat16(v.w)));
+    }
+    if (g.mode == kDH) {  // N = 128: a warp has whole rows
+      *reinterpret_cast<float4*>(colsum + wq * 128 + n) = sum;
+      __syncthreads();
+      if (tid < 128) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < kTgThreads / 32; ++w) s += colsum[w * 128 + tid];
+        atomicAdd(g.db + tid, s);
       }
     }
   }
@@ -180,73 +233,63 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmArgs g, long k_per_cta, 
   }
 }
 
-// Launches the tensor-core GEMM; K split over CTAs when the output is a
-// single tile and K is long (the weight gradients).
-static cudaError_t gemm(const GemmArgs& g, cudaStream_t st, unsigned int* err) {
-  if (g.M <= 0 || g.N <= 0) return cudaSuccess;
-  dim3 grid((unsigned)((g.M + 127) / 128), (unsigned)((g.N + 127) / 128), 1);
-  long kpc = g.K;
-  if (grid.x * grid.y < 16 && g.K > 4 * kTgBK) {
-    if (g.bias || g.H || !g.C) return cudaErrorInvalidValue;  // split K adds partial tiles only
-    const long chunks = (g.K + kTgBK - 1) / kTgBK;
-    const long z = std::min<long>(chunks, 64);
-    kpc = ((chunks + z - 1) / z) * kTgBK;
-    grid.z = (unsigned)((g.K + kpc - 1) / kpc);
-    cudaError_t e = cudaSuccess;
-    if (g.ldc == g.N) {
-      e = cudaMemsetAsync(g.C, 0, sizeof(float) * (size_t)g.N * (size_t)g.M, st);
-    } else {
-      for (long m = 0; m < g.M && e == cudaSuccess; ++m)
-        e = cudaMemsetAsync(g.C + m * g.ldc, 0, sizeof(float) * (size_t)g.N, st);
+static cudaError_t launch_gemm(GemmJob a, GemmJob b, cudaStream_t st, unsigned int* err) {
+  for (GemmJob* g : {&a, &b}) {
+    if (g->M <= 0 || g->N <= 0) {
+      g->tiles = 0;
+      continue;
     }
-    if (e != cudaSuccess) return e;
+    if (g->mode == kDW) {  // K over up to 148 CTAs, in chunks of 128
+      const long chunks = (g->K + kTgK - 1) / kTgK, per = (chunks + 147) / 148;
+      g->k_per_cta = (int)per * kTgK;
+      g->tiles = (int)((chunks + per - 1) / per);
+    } else {
+      g->k_per_cta = g->K;
+      g->tiles = (g->M + 127) / 128;
+    }
   }
-  k_gemm_tc<<<grid, 128, kTgSmem, st>>>(g, kpc, err);
+  if (a.tiles + b.tiles <= 0) return cudaSuccess;
+  k_gemm_tc<<<(unsigned)(a.tiles + b.tiles), kTgThreads, kTgSmem, st>>>(a, b, err);
   return cudaGetLastError();
 }
 
 // ------------------------------------------------------- small kernels
-__global__ void k_loss_grad(long B, const float* O, const float* Y, float* dOf, __nv_bfloat16* dOb,
-                            double* loss) {
+// dO of the mean squared error, its column sums (the last layer's bias gradient)
+// added to db, and the loss.  256-thread blocks: a thread keeps its column.
+__global__ void __launch_bounds__(256) k_loss_grad(long B, const float* O, const float* Y, __nv_bfloat16* dOb, float* db,
+                                                   double* loss) {
   double part = 0.0;
+  float col = 0.f;
   const float scale = 2.0f / (float)(B * kMlpOut);
+  const int j = threadIdx.x % kMlpOutPad;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < B * kMlpOutPad; i += (long)gridDim.x * blockDim.x) {
     const long b = i / kMlpOutPad;
-    const int j = (int)(i % kMlpOutPad);
     float d = 0.f;
     if (j < kMlpOut) {
       const float e = O[b * kMlpOutPad + j] - Y[b * kMlpOut + j];
       part += (double)e * e;
       d = scale * e;
     }
-    dOf[i] = d;
     dOb[i] = __float2bfloat16(d);
+    col += d;
   }
+  __shared__ double sp[8];
+  __shared__ float sc[8][kMlpOutPad];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
-  if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, part / (double)(B * kMlpOut));
-}
-
-__global__ void k_gelu_back(long n, const float* dH, const float* Z, float* dZf, __nv_bfloat16* dZb) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const float d = dH[i] * gelu_grad_f(Z[i]);
-    dZf[i] = d;
-    dZb[i] = __float2bfloat16(d);
-  }
-}
-
-// db[c] = sum over rows of M[r][c] (one block per column)
-__global__ void k_colsum(long rows, int ncols, const float* M, float* db) {
-  const int c = blockIdx.x;
-  float s = 0.f;
-  for (long r = threadIdx.x; r < rows; r += blockDim.x) s += M[r * ncols + c];
-  __shared__ float red[32];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  col += __shfl_down_sync(0xffffffffu, col, 16);
+  if (lane == 0) sp[w] = part;
+  if (lane < kMlpOutPad) sc[w][lane] = col;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.f;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) db[c] = s;
+  if (threadIdx.x < kMlpOutPad) {
+    float s = 0.f;
+    for (int q = 0; q < 8; ++q) s += sc[q][threadIdx.x];
+    atomicAdd(db + threadIdx.x, s);
+  }
+  if (threadIdx.x == 32 && loss) {
+    double s = 0.0;
+    for (int q = 0; q < 8; ++q) s += sp[q];
+    atomicAdd(loss, s / (double)(B * kMlpOut));
   }
 }
 
@@ -269,14 +312,18 @@ __global__ void k_to_bf16(long n, const float* x, __nv_bfloat16* y) {
     y[i] = __float2bfloat16(x[i]);
 }
 
+// Rows idx[0..nb) of X (32 bytes each) and Y (40 bytes): a thread per 16-byte or
+// 4-byte piece.
 __global__ void k_gather_rows(long nb, const int* idx, const __nv_bfloat16* X, const float* Y,
                               __nv_bfloat16* Xb, float* Yb) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nb; i += (long)gridDim.x * blockDim.x) {
-    const long r = idx[i];
-#pragma unroll
-    for (int j = 0; j < kMlpInPad; ++j) Xb[i * kMlpInPad + j] = X[r * kMlpInPad + j];
-#pragma unroll
-    for (int j = 0; j < kMlpOut; ++j) Yb[i * kMlpOut + j] = Y[r * kMlpOut + j];
+  constexpr int kPieces = 2 + kMlpOut;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nb * kPieces; i += (long)gridDim.x * blockDim.x) {
+    const long b = i / kPieces, r = idx[b];
+    const int q = (int)(i % kPieces);
+    if (q < 2)
+      reinterpret_cast<uint4*>(Xb + b * kMlpInPad)[q] = reinterpret_cast<const uint4*>(X + r * kMlpInPad)[q];
+    else
+      Yb[b * kMlpOut + q - 2] = Y[r * kMlpOut + q - 2];
   }
 }
 
@@ -1080,8 +1127,8 @@ struct Surrogate {
   long step = 0;
   // activation buffers (grow-only)
   long cap = 0;
-  __nv_bfloat16 *X = nullptr, *H[kMlpLayers] = {}, *dHb = nullptr;
-  float *Z[kMlpLayers] = {}, *O = nullptr, *dOf = nullptr, *dHf = nullptr, *dZf = nullptr;
+  __nv_bfloat16 *X = nullptr, *H[kMlpLayers] = {}, *dHb[2] = {};  // dHb: gradients of alternate layers
+  float *Z[kMlpLayers] = {}, *O = nullptr;
   __nv_bfloat16* dOb = nullptr;
   float* Yb = nullptr;
   int* idx = nullptr;
@@ -1216,10 +1263,10 @@ static void free_act(Surrogate* s) {
     s->H[l] = nullptr;
     s->Z[l] = nullptr;
   }
-  cudaFree(s->dHb); cudaFree(s->O); cudaFree(s->dOf); cudaFree(s->dHf); cudaFree(s->dZf); cudaFree(s->dOb);
+  cudaFree(s->dHb[0]); cudaFree(s->dHb[1]); cudaFree(s->O); cudaFree(s->dOb);
   cudaFree(s->Yb); cudaFree(s->idx);
-  s->X = s->dHb = s->dOb = nullptr;
-  s->O = s->dOf = s->dHf = s->dZf = s->Yb = nullptr;
+  s->X = s->dHb[0] = s->dHb[1] = s->dOb = nullptr;
+  s->O = s->Yb = nullptr;
   s->idx = nullptr;
   s->cap = 0;
 }
@@ -1297,11 +1344,9 @@ static std::string ensure_act(Surrogate* s, long n) {
     if ((e = ck(cudaMalloc(&s->Z[l], np * mlp_out(l) * 4), "alloc Z")).size()) return e;
   }
   if ((e = ck(cudaMalloc(&s->O, np * kMlpOutPad * 4), "alloc O")).size()) return e;
-  if ((e = ck(cudaMalloc(&s->dOf, np * kMlpOutPad * 4), "alloc dO")).size()) return e;
   if ((e = ck(cudaMalloc(&s->dOb, np * kMlpOutPad * 2), "alloc dO")).size()) return e;
-  if ((e = ck(cudaMalloc(&s->dHf, np * kMlpHid * 4), "alloc dH")).size()) return e;
-  if ((e = ck(cudaMalloc(&s->dHb, np * kMlpHid * 2), "alloc dH")).size()) return e;
-  if ((e = ck(cudaMalloc(&s->dZf, np * kMlpHid * 4), "alloc dZ")).size()) return e;
+  for (auto& d : s->dHb)
+    if ((e = ck(cudaMalloc(&d, np * kMlpHid * 2), "alloc dH")).size()) return e;
   if ((e = ck(cudaMalloc(&s->Yb, np * kMlpOut * 4), "alloc Y")).size()) return e;
   if ((e = ck(cudaMalloc(&s->idx, np * 4), "alloc idx")).size()) return e;
   s->cap = np;
@@ -1402,28 +1447,27 @@ std::string surrogate_features(Surrogate* s, long n, long ld, double dt, const d
   return ck(cudaGetLastError(), "features");
 }
 
+static GemmJob fwd_job(const Surrogate* s, int l, long n, const __nv_bfloat16* in, float* z, __nv_bfloat16* h) {
+  GemmJob g{};
+  g.mode = kFwd;
+  g.M = (int)n;
+  g.N = mlp_out(l);
+  g.K = g.lda = g.ldb = mlp_in(l);
+  g.A = in;
+  g.B = s->wb + s->offW[l];
+  g.C = z;
+  g.bias = s->w + s->offb[l];
+  g.H = h;
+  return g;
+}
+
 // Forward over n rows of bf16 features; keeps H/Z for backward.
 static cudaError_t forward(Surrogate* s, long n, const __nv_bfloat16* x, float* out, cudaStream_t st) {
   const __nv_bfloat16* in = x;
   for (int l = 0; l < kMlpLayers; ++l) {
-    GemmArgs g{};
-    g.M = (int)n;
-    g.N = mlp_out(l);
-    g.K = mlp_in(l);
-    g.A = in;
-    g.sam = mlp_in(l);
-    g.sak = 1;
-    g.B = s->wb + s->offW[l];
-    g.sbk = 1;
-    g.sbn = mlp_in(l);
-    g.bias = s->w + s->offb[l];
     const bool last = l == kMlpLayers - 1;
-    g.C = last ? out : s->Z[l];
-    g.ldc = mlp_out(l);
-    g.H = last ? nullptr : s->H[l];
-    g.ldh = mlp_out(l);
-    g.gelu = 1;
-    cudaError_t e = gemm(g, st, s->d_err);
+    cudaError_t e = launch_gemm(fwd_job(s, l, n, in, last ? out : s->Z[l], last ? nullptr : s->H[l]), GemmJob{}, st,
+                                s->d_err);
     if (e != cudaSuccess) return e;
     in = s->H[l];
   }
@@ -1442,24 +1486,9 @@ std::string surrogate_forward(Surrogate* s, long n, const __nv_bfloat16* x, floa
 static cudaError_t forward_infer(Surrogate* s, long n, const __nv_bfloat16* x, float* out, cudaStream_t st) {
   const __nv_bfloat16* in = x;
   for (int l = 0; l < kMlpLayers; ++l) {
-    GemmArgs g{};
-    g.M = (int)n;
-    g.N = mlp_out(l);
-    g.K = mlp_in(l);
-    g.A = in;
-    g.sam = mlp_in(l);
-    g.sak = 1;
-    g.B = s->wb + s->offW[l];
-    g.sbk = 1;
-    g.sbn = mlp_in(l);
-    g.bias = s->w + s->offb[l];
     const bool last = l == kMlpLayers - 1;
-    g.C = last ? out : nullptr;
-    g.ldc = mlp_out(l);
-    g.H = last ? nullptr : s->iH[l & 1];
-    g.ldh = mlp_out(l);
-    g.gelu = 1;
-    cudaError_t e = gemm(g, st, s->d_err);
+    cudaError_t e = launch_gemm(fwd_job(s, l, n, in, last ? out : nullptr, last ? nullptr : s->iH[l & 1]), GemmJob{},
+                                st, s->d_err);
     if (e != cudaSuccess) return e;
     in = s->iH[l & 1];
   }
@@ -1468,49 +1497,39 @@ static cudaError_t forward_infer(Surrogate* s, long n, const __nv_bfloat16* x, f
 
 // Gradients of the MSE over B rows (x in s->X-like layout, y normalised).
 static cudaError_t backward(Surrogate* s, long B, const __nv_bfloat16* x, const float* y, cudaStream_t st) {
-  cudaError_t e = forward(s, B, x, s->O, st);
+  cudaError_t e = cudaMemsetAsync(s->gr, 0, sizeof(float) * (size_t)s->n_params, st);
+  if (e == cudaSuccess) e = forward(s, B, x, s->O, st);
   if (e != cudaSuccess) return e;
-  k_loss_grad<<<std::min<long>((B * kMlpOutPad + 255) / 256, 1024), 256, 0, st>>>(B, s->O, y, s->dOf, s->dOb,
-                                                                                   s->d_loss);
-  const __nv_bfloat16* dZb = s->dOb;
-  const float* dZf = s->dOf;
+  k_loss_grad<<<std::min<long>((B * kMlpOutPad + 255) / 256, 256), 256, 0, st>>>(
+      B, s->O, y, s->dOb, s->gr + s->offb[kMlpLayers - 1], s->d_loss);
+  const __nv_bfloat16* dZ = s->dOb;
   for (int l = kMlpLayers - 1; l >= 0; --l) {
-    const __nv_bfloat16* Hin = l == 0 ? x : s->H[l - 1];
     // dW[out][in] = sum_b dZ[b][out] Hin[b][in]
-    GemmArgs g{};
-    g.M = mlp_out(l);
-    g.N = mlp_in(l);
-    g.K = (int)B;
-    g.A = dZb;
-    g.sam = 1;
-    g.sak = mlp_out(l);
-    g.B = Hin;
-    g.sbk = mlp_in(l);
-    g.sbn = 1;
-    g.C = s->gr + s->offW[l];
-    g.ldc = mlp_in(l);
-    if ((e = gemm(g, st, s->d_err)) != cudaSuccess) return e;
-    k_colsum<<<mlp_out(l), 256, 0, st>>>(B, mlp_out(l), dZf, s->gr + s->offb[l]);
-    if (l == 0) break;
-    // dH[b][in] = sum_out dZ[b][out] W[out][in]
-    GemmArgs h{};
-    h.M = (int)B;
-    h.N = mlp_in(l);
-    h.K = mlp_out(l);
-    h.A = dZb;
-    h.sam = mlp_out(l);
-    h.sak = 1;
-    h.B = s->wb + s->offW[l];
-    h.sbk = mlp_in(l);
-    h.sbn = 1;
-    h.C = s->dHf;
-    h.ldc = mlp_in(l);
-    if ((e = gemm(h, st, s->d_err)) != cudaSuccess) return e;
-    const long cnt = B * kMlpHid;
-    k_gelu_back<<<std::min<long>((cnt + 255) / 256, 4096), 256, 0, st>>>(cnt, s->dHf, s->Z[l - 1], s->dZf,
-                                                                         s->dHb);
-    dZb = s->dHb;
-    dZf = s->dZf;
+    GemmJob w{}, h{};
+    w.mode = kDW;
+    w.M = w.lda = mlp_out(l);
+    w.N = w.ldb = mlp_in(l);
+    w.K = (int)B;
+    w.A = dZ;
+    w.B = l == 0 ? x : s->H[l - 1];
+    w.a_mn = w.b_mn = 1;
+    w.C = s->gr + s->offW[l];
+    __nv_bfloat16* dH = s->dHb[l & 1];
+    if (l > 0) {
+      // dZ of the layer below: (sum_out dZ[b][out] W[out][in]) gelu'(Z[b][in])
+      h.mode = kDH;
+      h.M = (int)B;
+      h.N = h.ldb = mlp_in(l);
+      h.K = h.lda = mlp_out(l);
+      h.A = dZ;
+      h.B = s->wb + s->offW[l];
+      h.b_mn = 1;
+      h.H = dH;
+      h.Z = s->Z[l - 1];
+      h.db = s->gr + s->offb[l - 1];
+    }
+    if ((e = launch_gemm(h, w, st, s->d_err)) != cudaSuccess) return e;
+    dZ = dH;
   }
   return cudaGetLastError();
 }
@@ -1552,7 +1571,7 @@ std::string surrogate_train(Surrogate* s, long n, const __nv_bfloat16* x, const 
     const int* cur = d_perm + (ep & 1) * n;
     cudaMemsetAsync(s->d_loss, 0, sizeof(double), st);
     for (long it = 0; it < steps; ++it) {
-      k_gather_rows<<<(batch + 255) / 256, 256, 0, st>>>(batch, cur + it * batch, x, y, Xb, s->Yb);
+      k_gather_rows<<<(batch * 12 + 255) / 256, 256, 0, st>>>(batch, cur + it * batch, x, y, Xb, s->Yb);
       cudaError_t ce = backward(s, batch, Xb, s->Yb, st);
       if (ce != cudaSuccess) {
         cudaFree(d_perm);
@@ -1565,7 +1584,7 @@ std::string surrogate_train(Surrogate* s, long n, const __nv_bfloat16* x, const 
       const float lr_t = (float)(lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(3.141592653589793 * frac))));
       const float b1 = 0.9f, b2 = 0.999f;
       const float bc1 = 1.f - std::pow(b1, (float)s->step), bc2 = 1.f - std::pow(b2, (float)s->step);
-      k_adam<<<64, 256, 0, st>>>(s->n_params, s->w, s->gr, s->m, s->v, s->wb, lr_t, b1, b2, 1e-8f, bc1, bc2);
+      k_adam<<<(unsigned)((s->n_params + 255) / 256), 256, 0, st>>>(s->n_params, s->w, s->gr, s->m, s->v, s->wb, lr_t, b1, b2, 1e-8f, bc1, bc2);
     }
     if (ep + 1 < epochs) {  // the next epoch's order, drawn while this one runs
       std::shuffle(perm.begin(), perm.end(), rng);

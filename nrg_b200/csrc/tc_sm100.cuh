@@ -33,9 +33,21 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// Instruction descriptor of kind::f16 with BF16 A/B, FP32 D, both K-major.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(uint32_t M, uint32_t N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
+// Byte offset of the 16-byte chunk (8 rows from 8 mnchunk on, column k) of an
+// MN-major operand of up to 128 rows, no swizzle: a core matrix is 8 columns of
+// 16 bytes (column k at +16 k), core matrices adjacent in MN are 128 bytes
+// apart (SBO), 8-column groups kMnGroup bytes (LBO); the K = 16 slice s starts
+// 2 kMnGroup s bytes into the operand.
+constexpr uint32_t kMnGroup = 16 * 128;
+__host__ __device__ constexpr uint32_t mnmajor_off(uint32_t k, uint32_t mnchunk) {
+  return (k >> 3) * kMnGroup + mnchunk * 128u + (k & 7u) * 16u;
+}
+
+// Instruction descriptor of kind::f16 with BF16 A/B, FP32 D; a_mn, b_mn: the
+// operand is MN-major (else K-major).
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(uint32_t M, uint32_t N, bool a_mn = false, bool b_mn = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u) | ((N >> 3) << 17) |
+         ((M >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
