@@ -775,7 +775,7 @@ extern "C" int nrg_chem_create(const char* mechanism_path, const char* thermo_pa
     return fail(nullptr, NRG_ERR_CUDA, msg);
   }
   reduce_dev_mech(h->dm, &h->dmr);
-  h->spec = nrg::match_specialised(h->dmr);
+  h->spec = nrg::match_specialised(h->dmr, h->dm);
   for (int i = 0; i < nrg::kMaxNets; ++i) h->sur_net[i] = nrg::surrogate_create(h->dm);
   if ((ce = use_tables(h)) != cudaSuccess) {
     std::string msg = std::string("mechanism upload failed: ") + cudaGetErrorString(ce);
@@ -835,7 +835,7 @@ extern "C" int nrg_chem_set_mode(nrg_chem* h, int mode) {
 
 extern "C" int nrg_chem_set_specialised(nrg_chem* h, int enable) {
   if (!h) return NRG_ERR_ARG;
-  const int id = nrg::match_specialised(h->dmr);
+  const int id = nrg::match_specialised(h->dmr, h->dm);
   if (enable && id == 0)
     return fail(h, NRG_ERR_UNSUPPORTED, "the mechanism matches none of the generated specialised codes");
   h->spec = enable ? id : 0;

@@ -716,8 +716,13 @@ __device__ __noinline__ void nl_rhs(double* d, LUT* f) {
   s.d = d;
   s.f = f;
   if constexpr (SPEC != 0) {
-    static_assert(N == SpecOf<SPEC>::kN && R == SpecOf<SPEC>::kR, "specialised code is for another mechanism size");
-    SpecOf<SPEC>::rhs(s);
+    // the reference mode integrates all species, the others the reacting ones
+    if constexpr (N == SpecOf<SPEC>::kFullN && R == SpecOf<SPEC>::kFullR) {
+      SpecOf<SPEC>::rhs_full(s);
+    } else {
+      static_assert(N == SpecOf<SPEC>::kN && R == SpecOf<SPEC>::kR, "specialised code is for another mechanism size");
+      SpecOf<SPEC>::rhs(s);
+    }
   } else {
     rhs<N>(s, R);
   }
@@ -874,7 +879,7 @@ __device__ void ddpst(CS& c) {
   c.nje += 1;
   c.ier = 0;
   const double el1h = EL(1, c.nq) * c.h;
-  if (JAC == kJacFD) {
+  if constexpr (JAC == kJacFD) {
     const double FACMAX = 0.5, BU = 0.5;
     const double br = c_mech.br, bl = c_mech.bl, bp = c_mech.bp, facmin = c_mech.facmin;
 #pragma unroll

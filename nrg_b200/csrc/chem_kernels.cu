@@ -14,7 +14,8 @@ void upload_mechanism_ref(const DevMech& m, cudaStream_t s);
 void upload_mechanism_fast(const DevMech& m, cudaStream_t s);
 void upload_mechanism_mixed(const DevMech& m, cudaStream_t s);
 bool supported_mechanism(int n_species, int n_reactions);
-cudaError_t launch_chem_ref(const StepArgs&, const LaunchCfg&, int*, unsigned long long*, cudaStream_t, int, int);
+cudaError_t launch_chem_ref(const StepArgs&, const LaunchCfg&, int*, unsigned long long*, cudaStream_t, int, int,
+                            int);
 cudaError_t launch_chem_fast(const StepArgs&, const LaunchCfg&, int*, unsigned long long*, cudaStream_t, int, int,
                              int, int);
 cudaError_t launch_chem_mixed(const StepArgs&, const LaunchCfg&, int*, unsigned long long*, cudaStream_t, int, int,
@@ -221,7 +222,7 @@ cudaError_t launch_chem(int n_species, int n_int, int spec, int n_reactions, int
                         cudaStream_t s) {
   if (!supported_mechanism(n_species, n_reactions)) return cudaErrorNotSupported;
   if (mixed) return launch_chem_mixed(a, cfg, queue, counters, s, n_int, spec, n_species, n_reactions);
-  return jac == kJacFD ? launch_chem_ref(a, cfg, queue, counters, s, n_species, n_reactions)
+  return jac == kJacFD ? launch_chem_ref(a, cfg, queue, counters, s, spec, n_species, n_reactions)
                        : launch_chem_fast(a, cfg, queue, counters, s, n_int, spec, n_species, n_reactions);
 }
 
@@ -231,7 +232,7 @@ bool supported_mechanism(int n_species, int n_reactions) {
          (n_species == 17 && n_reactions == 25);
 }
 
-int match_specialised(const DevMech& reduced) { return match_specialised_tables(reduced); }
+int match_specialised(const DevMech& reduced, const DevMech& full) { return match_specialised_tables(reduced, full); }
 
 int smem_bytes_per_cell(int n_species, int n_reactions, bool mixed) {
   if (n_species == 9 && n_reactions == 24)

@@ -21,8 +21,11 @@ struct SpecOf;
 template <>
 struct SpecOf<kSpecKeromnes> {
   static constexpr int kN = gen_keromnes::kSpecN, kR = gen_keromnes::kSpecR;
+  static constexpr int kFullN = gen_keromnes::kFullN, kFullR = gen_keromnes::kFullR;
   template <class S>
   __device__ static void rhs(S& c) { gen_keromnes::spec_rhs(c); }
+  template <class S>
+  __device__ static void rhs_full(S& c) { gen_keromnes::full_rhs(c); }
   template <int J, class S, typename LUT>
   __device__ static void column(const S& c, double f, LUT (&v)[gen_keromnes::kSpecN]) {
     gen_keromnes::spec_column<J>(c, f, v);
@@ -31,8 +34,11 @@ struct SpecOf<kSpecKeromnes> {
 template <>
 struct SpecOf<kSpecZhang> {
   static constexpr int kN = gen_zhang::kSpecN, kR = gen_zhang::kSpecR;
+  static constexpr int kFullN = gen_zhang::kFullN, kFullR = gen_zhang::kFullR;
   template <class S>
   __device__ static void rhs(S& c) { gen_zhang::spec_rhs(c); }
+  template <class S>
+  __device__ static void rhs_full(S& c) { gen_zhang::full_rhs(c); }
   template <int J, class S, typename LUT>
   __device__ static void column(const S& c, double f, LUT (&v)[gen_zhang::kSpecN]) {
     gen_zhang::spec_column<J>(c, f, v);
@@ -41,8 +47,11 @@ struct SpecOf<kSpecZhang> {
 template <>
 struct SpecOf<kSpecTereza> {
   static constexpr int kN = gen_tereza::kSpecN, kR = gen_tereza::kSpecR;
+  static constexpr int kFullN = gen_tereza::kFullN, kFullR = gen_tereza::kFullR;
   template <class S>
   __device__ static void rhs(S& c) { gen_tereza::spec_rhs(c); }
+  template <class S>
+  __device__ static void rhs_full(S& c) { gen_tereza::full_rhs(c); }
   template <int J, class S, typename LUT>
   __device__ static void column(const S& c, double f, LUT (&v)[gen_tereza::kSpecN]) {
     gen_tereza::spec_column<J>(c, f, v);
@@ -51,8 +60,11 @@ struct SpecOf<kSpecTereza> {
 template <>
 struct SpecOf<kSpecKonnov> {
   static constexpr int kN = gen_konnov::kSpecN, kR = gen_konnov::kSpecR;
+  static constexpr int kFullN = gen_konnov::kFullN, kFullR = gen_konnov::kFullR;
   template <class S>
   __device__ static void rhs(S& c) { gen_konnov::spec_rhs(c); }
+  template <class S>
+  __device__ static void rhs_full(S& c) { gen_konnov::full_rhs(c); }
   template <int J, class S, typename LUT>
   __device__ static void column(const S& c, double f, LUT (&v)[gen_konnov::kSpecN]) {
     gen_konnov::spec_column<J>(c, f, v);
@@ -61,18 +73,21 @@ struct SpecOf<kSpecKonnov> {
 template <>
 struct SpecOf<kSpecAcetylene> {
   static constexpr int kN = gen_acetylene::kSpecN, kR = gen_acetylene::kSpecR;
+  static constexpr int kFullN = gen_acetylene::kFullN, kFullR = gen_acetylene::kFullR;
   template <class S>
   __device__ static void rhs(S& c) { gen_acetylene::spec_rhs(c); }
+  template <class S>
+  __device__ static void rhs_full(S& c) { gen_acetylene::full_rhs(c); }
   template <int J, class S, typename LUT>
   __device__ static void column(const S& c, double f, LUT (&v)[gen_acetylene::kSpecN]) {
     gen_acetylene::spec_column<J>(c, f, v);
   }
 };
 
-// 0 when the reduced reaction lists match none of the generated codes.
+// 0 when the reaction lists, reduced or full, match none of the generated codes.
 template <class M>
-inline int match_specialised_tables(const M& m) {
-  if (m.NI == gen_keromnes::kSpecN && m.RM == gen_keromnes::kSpecR) {
+inline int match_specialised_tables(const M& m, const M& full) {
+  if (m.NI == gen_keromnes::kSpecN && m.RM == gen_keromnes::kSpecR && full.N == gen_keromnes::kFullN && full.R == gen_keromnes::kFullR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_keromnes::kSpecNupd[r];
@@ -81,9 +96,16 @@ inline int match_specialised_tables(const M& m) {
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_keromnes::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_keromnes::kSpecUpdProd[r][u];
     }
+    for (int r = 0; ok && r < full.R; ++r) {
+      ok = full.nupd[r] == gen_keromnes::kFullNupd[r];
+      for (int i = 0; ok && i < 3; ++i)
+        ok = full.left[r][i] == gen_keromnes::kFullLeft[r][i] && full.right[r][i] == gen_keromnes::kFullRight[r][i];
+      for (int u = 0; ok && u < full.nupd[r]; ++u)
+        ok = full.upd_k[r][u] == gen_keromnes::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_keromnes::kFullUpdProd[r][u];
+    }
     if (ok) return kSpecKeromnes;
   }
-  if (m.NI == gen_zhang::kSpecN && m.RM == gen_zhang::kSpecR) {
+  if (m.NI == gen_zhang::kSpecN && m.RM == gen_zhang::kSpecR && full.N == gen_zhang::kFullN && full.R == gen_zhang::kFullR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_zhang::kSpecNupd[r];
@@ -92,9 +114,16 @@ inline int match_specialised_tables(const M& m) {
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_zhang::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_zhang::kSpecUpdProd[r][u];
     }
+    for (int r = 0; ok && r < full.R; ++r) {
+      ok = full.nupd[r] == gen_zhang::kFullNupd[r];
+      for (int i = 0; ok && i < 3; ++i)
+        ok = full.left[r][i] == gen_zhang::kFullLeft[r][i] && full.right[r][i] == gen_zhang::kFullRight[r][i];
+      for (int u = 0; ok && u < full.nupd[r]; ++u)
+        ok = full.upd_k[r][u] == gen_zhang::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_zhang::kFullUpdProd[r][u];
+    }
     if (ok) return kSpecZhang;
   }
-  if (m.NI == gen_tereza::kSpecN && m.RM == gen_tereza::kSpecR) {
+  if (m.NI == gen_tereza::kSpecN && m.RM == gen_tereza::kSpecR && full.N == gen_tereza::kFullN && full.R == gen_tereza::kFullR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_tereza::kSpecNupd[r];
@@ -103,9 +132,16 @@ inline int match_specialised_tables(const M& m) {
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_tereza::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_tereza::kSpecUpdProd[r][u];
     }
+    for (int r = 0; ok && r < full.R; ++r) {
+      ok = full.nupd[r] == gen_tereza::kFullNupd[r];
+      for (int i = 0; ok && i < 3; ++i)
+        ok = full.left[r][i] == gen_tereza::kFullLeft[r][i] && full.right[r][i] == gen_tereza::kFullRight[r][i];
+      for (int u = 0; ok && u < full.nupd[r]; ++u)
+        ok = full.upd_k[r][u] == gen_tereza::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_tereza::kFullUpdProd[r][u];
+    }
     if (ok) return kSpecTereza;
   }
-  if (m.NI == gen_konnov::kSpecN && m.RM == gen_konnov::kSpecR) {
+  if (m.NI == gen_konnov::kSpecN && m.RM == gen_konnov::kSpecR && full.N == gen_konnov::kFullN && full.R == gen_konnov::kFullR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_konnov::kSpecNupd[r];
@@ -114,9 +150,16 @@ inline int match_specialised_tables(const M& m) {
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_konnov::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_konnov::kSpecUpdProd[r][u];
     }
+    for (int r = 0; ok && r < full.R; ++r) {
+      ok = full.nupd[r] == gen_konnov::kFullNupd[r];
+      for (int i = 0; ok && i < 3; ++i)
+        ok = full.left[r][i] == gen_konnov::kFullLeft[r][i] && full.right[r][i] == gen_konnov::kFullRight[r][i];
+      for (int u = 0; ok && u < full.nupd[r]; ++u)
+        ok = full.upd_k[r][u] == gen_konnov::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_konnov::kFullUpdProd[r][u];
+    }
     if (ok) return kSpecKonnov;
   }
-  if (m.NI == gen_acetylene::kSpecN && m.RM == gen_acetylene::kSpecR) {
+  if (m.NI == gen_acetylene::kSpecN && m.RM == gen_acetylene::kSpecR && full.N == gen_acetylene::kFullN && full.R == gen_acetylene::kFullR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_acetylene::kSpecNupd[r];
@@ -124,6 +167,13 @@ inline int match_specialised_tables(const M& m) {
         ok = m.left[r][i] == gen_acetylene::kSpecLeft[r][i] && m.right[r][i] == gen_acetylene::kSpecRight[r][i];
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_acetylene::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_acetylene::kSpecUpdProd[r][u];
+    }
+    for (int r = 0; ok && r < full.R; ++r) {
+      ok = full.nupd[r] == gen_acetylene::kFullNupd[r];
+      for (int i = 0; ok && i < 3; ++i)
+        ok = full.left[r][i] == gen_acetylene::kFullLeft[r][i] && full.right[r][i] == gen_acetylene::kFullRight[r][i];
+      for (int u = 0; ok && u < full.nupd[r]; ++u)
+        ok = full.upd_k[r][u] == gen_acetylene::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_acetylene::kFullUpdProd[r][u];
     }
     if (ok) return kSpecAcetylene;
   }

@@ -1,6 +1,7 @@
 // Generated by nrg_b200/gen_mech.py from TEREZA.txt: do not edit.
 // Straight-line right-hand side and analytic iteration matrix over the
-// 10 reacting species and 24 reactions; same operation order as the
+// 10 reacting species and 24 distinct reactions, and the right-hand side
+// over all 10 species and 24 reactions; same operation order as the
 // table-driven loops in chem_bdf.cuh, with the same explicitly rounded
 // (never fused) operations.
 #pragma once
@@ -118,6 +119,301 @@ constexpr int kSpecUpdProd[24][6] = {
 // zd = dC/dt at z (shared scratch in, shared scratch out)
 template <class S>
 __device__ __forceinline__ void spec_rhs(S& c) {
+  const double z0 = c.z(0);
+  const double z1 = c.z(1);
+  const double z2 = c.z(2);
+  const double z3 = c.z(3);
+  const double z4 = c.z(4);
+  const double z5 = c.z(5);
+  const double z6 = c.z(6);
+  const double z7 = c.z(7);
+  const double z8 = c.z(8);
+  const double z9 = c.z(9);
+  double d0 = 0.0, d1 = 0.0, d2 = 0.0, d3 = 0.0, d4 = 0.0, d5 = 0.0, d6 = 0.0, d7 = 0.0, d8 = 0.0, d9 = 0.0;
+  double f, b, q;
+  f = __dmul_rn(__dmul_rn(c.kf(0), z3), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(0), z4), z8);
+  q = __dsub_rn(f, b);
+  d1 = __dsub_rn(d1, q);
+  d3 = __dsub_rn(d3, q);
+  d4 = __dadd_rn(d4, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(1), z9), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(1), z8), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dadd_rn(d1, q);
+  d4 = __dsub_rn(d4, q);
+  d8 = __dadd_rn(d8, q);
+  d9 = __dsub_rn(d9, q);
+  f = __dmul_rn(__dmul_rn(c.kf(2), z9), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(2), z8), z8);
+  q = __dsub_rn(f, b);
+  d3 = __dsub_rn(d3, q);
+  d8 = __dadd_rn(d8, q);
+  d8 = __dadd_rn(d8, q);
+  d9 = __dsub_rn(d9, q);
+  f = __dmul_rn(__dmul_rn(c.kf(3), z9), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(3), z6), z4);
+  q = __dsub_rn(f, b);
+  d3 = __dsub_rn(d3, q);
+  d4 = __dadd_rn(d4, q);
+  d6 = __dadd_rn(d6, q);
+  d9 = __dsub_rn(d9, q);
+  f = __dmul_rn(__dmul_rn(c.kf(4), z0), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(4), z3), z8);
+  q = __dsub_rn(f, b);
+  d0 = __dsub_rn(d0, q);
+  d3 = __dadd_rn(d3, q);
+  d4 = __dsub_rn(d4, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(5), z8), z8);
+  b = __dmul_rn(__dmul_rn(c.kr(5), z6), z4);
+  q = __dsub_rn(f, b);
+  d4 = __dadd_rn(d4, q);
+  d6 = __dadd_rn(d6, q);
+  d8 = __dsub_rn(d8, q);
+  d8 = __dsub_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(6), z0), z8);
+  b = __dmul_rn(__dmul_rn(c.kr(6), z6), z3);
+  q = __dsub_rn(f, b);
+  d0 = __dsub_rn(d0, q);
+  d3 = __dadd_rn(d3, q);
+  d6 = __dadd_rn(d6, q);
+  d8 = __dsub_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(7), z7), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(7), z9), z9);
+  q = __dsub_rn(f, b);
+  d1 = __dsub_rn(d1, q);
+  d7 = __dsub_rn(d7, q);
+  d9 = __dadd_rn(d9, q);
+  d9 = __dadd_rn(d9, q);
+  f = __dmul_rn(__dmul_rn(c.kf(8), z7), z8);
+  b = __dmul_rn(__dmul_rn(c.kr(8), z6), z9);
+  q = __dsub_rn(f, b);
+  d6 = __dadd_rn(d6, q);
+  d7 = __dsub_rn(d7, q);
+  d8 = __dsub_rn(d8, q);
+  d9 = __dadd_rn(d9, q);
+  f = __dmul_rn(__dmul_rn(c.kf(9), z7), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(9), z9), z0);
+  q = __dsub_rn(f, b);
+  d0 = __dadd_rn(d0, q);
+  d3 = __dsub_rn(d3, q);
+  d7 = __dsub_rn(d7, q);
+  d9 = __dadd_rn(d9, q);
+  f = __dmul_rn(__dmul_rn(c.kf(10), z7), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(10), z6), z8);
+  q = __dsub_rn(f, b);
+  d3 = __dsub_rn(d3, q);
+  d6 = __dadd_rn(d6, q);
+  d7 = __dsub_rn(d7, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(11), z7), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(11), z9), z8);
+  q = __dsub_rn(f, b);
+  d4 = __dsub_rn(d4, q);
+  d7 = __dsub_rn(d7, q);
+  d8 = __dadd_rn(d8, q);
+  d9 = __dadd_rn(d9, q);
+  f = __dmul_rn(c.kf(12), z6);
+  b = __dmul_rn(__dmul_rn(c.kr(12), z3), z8);
+  q = __dsub_rn(f, b);
+  d3 = __dadd_rn(d3, q);
+  d6 = __dsub_rn(d6, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(c.kf(13), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(13), z4), z4);
+  q = __dsub_rn(f, b);
+  d1 = __dsub_rn(d1, q);
+  d4 = __dadd_rn(d4, q);
+  d4 = __dadd_rn(d4, q);
+  f = __dmul_rn(c.kf(14), z0);
+  b = __dmul_rn(__dmul_rn(c.kr(14), z3), z3);
+  q = __dsub_rn(f, b);
+  d0 = __dsub_rn(d0, q);
+  d3 = __dadd_rn(d3, q);
+  d3 = __dadd_rn(d3, q);
+  f = __dmul_rn(__dmul_rn(c.kf(15), z4), z3);
+  b = __dmul_rn(c.kr(15), z8);
+  q = __dsub_rn(f, b);
+  d3 = __dsub_rn(d3, q);
+  d4 = __dsub_rn(d4, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(16), z3), z4);
+  b = __dmul_rn(c.kr(16), z5);
+  q = __dsub_rn(f, b);
+  d3 = __dsub_rn(d3, q);
+  d4 = __dsub_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  f = __dmul_rn(__dmul_rn(c.kf(17), z5), z6);
+  b = __dmul_rn(__dmul_rn(c.kr(17), z8), z6);
+  q = __dsub_rn(f, b);
+  d5 = __dsub_rn(d5, q);
+  d6 = __dsub_rn(d6, q);
+  d6 = __dadd_rn(d6, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(18), z5), z0);
+  b = __dmul_rn(__dmul_rn(c.kr(18), z8), z0);
+  q = __dsub_rn(f, b);
+  d0 = __dsub_rn(d0, q);
+  d0 = __dadd_rn(d0, q);
+  d5 = __dsub_rn(d5, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(19), z5), z2);
+  b = __dmul_rn(__dmul_rn(c.kr(19), z8), z2);
+  q = __dsub_rn(f, b);
+  d2 = __dsub_rn(d2, q);
+  d2 = __dadd_rn(d2, q);
+  d5 = __dsub_rn(d5, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(20), z5), z8);
+  b = __dmul_rn(__dmul_rn(c.kr(20), z8), z8);
+  q = __dsub_rn(f, b);
+  d5 = __dsub_rn(d5, q);
+  d8 = __dsub_rn(d8, q);
+  d8 = __dadd_rn(d8, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(21), z5), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(21), z8), z3);
+  q = __dsub_rn(f, b);
+  d3 = __dsub_rn(d3, q);
+  d3 = __dadd_rn(d3, q);
+  d5 = __dsub_rn(d5, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(c.kf(22), z5);
+  b = __dmul_rn(c.kr(22), z8);
+  q = __dsub_rn(f, b);
+  d5 = __dsub_rn(d5, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(23), z5), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(23), z8), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dsub_rn(d1, q);
+  d1 = __dadd_rn(d1, q);
+  d5 = __dsub_rn(d5, q);
+  d8 = __dadd_rn(d8, q);
+  c.zd(0) = d0;
+  c.zd(1) = d1;
+  c.zd(2) = d2;
+  c.zd(3) = d3;
+  c.zd(4) = d4;
+  c.zd(5) = d5;
+  c.zd(6) = d6;
+  c.zd(7) = d7;
+  c.zd(8) = d8;
+  c.zd(9) = d9;
+}
+
+constexpr int kFullN = 10, kFullR = 24;
+constexpr int kFullLeft[24][3] = {
+    {3, 1, -1},
+    {9, 4, -1},
+    {9, 3, -1},
+    {9, 3, -1},
+    {0, 4, -1},
+    {8, 8, -1},
+    {0, 8, -1},
+    {7, 1, -1},
+    {7, 8, -1},
+    {7, 3, -1},
+    {7, 3, -1},
+    {7, 4, -1},
+    {6, -1, -1},
+    {1, -1, -1},
+    {0, -1, -1},
+    {4, 3, -1},
+    {3, 4, -1},
+    {5, 6, -1},
+    {5, 0, -1},
+    {5, 2, -1},
+    {5, 8, -1},
+    {5, 3, -1},
+    {5, -1, -1},
+    {5, 1, -1},
+};
+constexpr int kFullRight[24][3] = {
+    {4, 8, -1},
+    {8, 1, -1},
+    {8, 8, -1},
+    {6, 4, -1},
+    {3, 8, -1},
+    {6, 4, -1},
+    {6, 3, -1},
+    {9, 9, -1},
+    {6, 9, -1},
+    {9, 0, -1},
+    {6, 8, -1},
+    {9, 8, -1},
+    {3, 8, -1},
+    {4, 4, -1},
+    {3, 3, -1},
+    {8, -1, -1},
+    {-1, 5, -1},
+    {8, 6, -1},
+    {8, 0, -1},
+    {8, 2, -1},
+    {8, 8, -1},
+    {8, 3, -1},
+    {8, -1, -1},
+    {8, 1, -1},
+};
+constexpr int kFullNupd[24] = {4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 3, 3, 3, 3, 3, 4, 4, 4, 4, 4, 2, 4};
+constexpr int kFullUpdK[24][6] = {
+    {1, 3, 4, 8, 0, 0},
+    {1, 4, 8, 9, 0, 0},
+    {3, 8, 8, 9, 0, 0},
+    {3, 4, 6, 9, 0, 0},
+    {0, 3, 4, 8, 0, 0},
+    {4, 6, 8, 8, 0, 0},
+    {0, 3, 6, 8, 0, 0},
+    {1, 7, 9, 9, 0, 0},
+    {6, 7, 8, 9, 0, 0},
+    {0, 3, 7, 9, 0, 0},
+    {3, 6, 7, 8, 0, 0},
+    {4, 7, 8, 9, 0, 0},
+    {3, 6, 8, 0, 0, 0},
+    {1, 4, 4, 0, 0, 0},
+    {0, 3, 3, 0, 0, 0},
+    {3, 4, 8, 0, 0, 0},
+    {3, 4, 5, 0, 0, 0},
+    {5, 6, 6, 8, 0, 0},
+    {0, 0, 5, 8, 0, 0},
+    {2, 2, 5, 8, 0, 0},
+    {5, 8, 8, 8, 0, 0},
+    {3, 3, 5, 8, 0, 0},
+    {5, 8, 0, 0, 0, 0},
+    {1, 1, 5, 8, 0, 0},
+};
+constexpr int kFullUpdProd[24][6] = {
+    {0, 0, 1, 1, 0, 0},
+    {1, 0, 1, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {0, 1, 0, 1, 0, 0},
+    {1, 1, 0, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {0, 0, 1, 1, 0, 0},
+    {1, 0, 0, 1, 0, 0},
+    {1, 0, 0, 1, 0, 0},
+    {0, 1, 0, 1, 0, 0},
+    {0, 0, 1, 1, 0, 0},
+    {1, 0, 1, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {0, 0, 1, 0, 0, 0},
+    {0, 0, 1, 0, 0, 0},
+    {0, 0, 1, 1, 0, 0},
+    {0, 1, 0, 1, 0, 0},
+    {0, 1, 0, 1, 0, 0},
+    {0, 0, 1, 1, 0, 0},
+    {0, 1, 0, 1, 0, 0},
+    {0, 1, 0, 0, 0, 0},
+    {0, 1, 0, 1, 0, 0},
+};
+
+// zd = dC/dt at z (shared scratch in, shared scratch out)
+template <class S>
+__device__ __forceinline__ void full_rhs(S& c) {
   const double z0 = c.z(0);
   const double z1 = c.z(1);
   const double z2 = c.z(2);

@@ -1,6 +1,7 @@
 // Generated by nrg_b200/gen_mech.py from ZHANG.txt: do not edit.
 // Straight-line right-hand side and analytic iteration matrix over the
-// 8 reacting species and 25 reactions; same operation order as the
+// 8 reacting species and 25 distinct reactions, and the right-hand side
+// over all 9 species and 28 reactions; same operation order as the
 // table-driven loops in chem_bdf.cuh, with the same explicitly rounded
 // (never fused) operations.
 #pragma once
@@ -314,6 +315,348 @@ __device__ __forceinline__ void spec_rhs(S& c) {
   c.zd(5) = d5;
   c.zd(6) = d6;
   c.zd(7) = d7;
+}
+
+constexpr int kFullN = 9, kFullR = 28;
+constexpr int kFullLeft[28][3] = {
+    {4, 1, -1},
+    {3, 0, -1},
+    {5, 0, -1},
+    {5, 5, -1},
+    {0, -1, -1},
+    {3, 3, -1},
+    {3, 4, -1},
+    {6, -1, -1},
+    {6, 6, -1},
+    {4, 1, -1},
+    {7, 4, -1},
+    {7, 4, -1},
+    {6, 3, -1},
+    {7, 3, -1},
+    {7, 5, -1},
+    {7, 5, -1},
+    {7, 7, -1},
+    {7, 7, -1},
+    {8, -1, -1},
+    {8, 4, -1},
+    {8, 4, -1},
+    {8, 3, -1},
+    {8, 5, -1},
+    {8, 5, -1},
+    {4, 1, 4},
+    {4, 1, 4},
+    {4, 1, 3},
+    {4, 1, 5},
+};
+constexpr int kFullRight[28][3] = {
+    {3, 5, -1},
+    {5, 4, -1},
+    {4, 6, -1},
+    {6, 3, -1},
+    {4, 4, -1},
+    {1, -1, -1},
+    {5, -1, -1},
+    {4, 5, -1},
+    {4, 5, 6},
+    {7, -1, -1},
+    {0, 1, -1},
+    {5, 5, -1},
+    {4, 7, -1},
+    {5, 1, -1},
+    {6, 1, -1},
+    {6, 1, -1},
+    {8, 1, -1},
+    {8, 1, -1},
+    {5, 5, -1},
+    {6, 5, -1},
+    {7, 0, -1},
+    {5, 7, -1},
+    {6, 7, -1},
+    {6, 7, -1},
+    {0, 1, -1},
+    {5, 5, -1},
+    {5, 1, -1},
+    {6, 1, -1},
+};
+constexpr int kFullNupd[28] = {4, 4, 4, 4, 3, 3, 3, 3, 5, 3, 4, 4, 4, 4, 4, 4, 4, 4, 3, 4, 4, 4, 4, 4, 5, 5, 5, 5};
+constexpr int kFullUpdK[28][6] = {
+    {1, 3, 4, 5, 0, 0},
+    {0, 3, 4, 5, 0, 0},
+    {0, 4, 5, 6, 0, 0},
+    {3, 5, 5, 6, 0, 0},
+    {0, 4, 4, 0, 0, 0},
+    {1, 3, 3, 0, 0, 0},
+    {3, 4, 5, 0, 0, 0},
+    {4, 5, 6, 0, 0, 0},
+    {4, 5, 6, 6, 6, 0},
+    {1, 4, 7, 0, 0, 0},
+    {0, 1, 4, 7, 0, 0},
+    {4, 5, 5, 7, 0, 0},
+    {3, 4, 6, 7, 0, 0},
+    {1, 3, 5, 7, 0, 0},
+    {1, 5, 6, 7, 0, 0},
+    {1, 5, 6, 7, 0, 0},
+    {1, 7, 7, 8, 0, 0},
+    {1, 7, 7, 8, 0, 0},
+    {5, 5, 8, 0, 0, 0},
+    {4, 5, 6, 8, 0, 0},
+    {0, 4, 7, 8, 0, 0},
+    {3, 5, 7, 8, 0, 0},
+    {5, 6, 7, 8, 0, 0},
+    {5, 6, 7, 8, 0, 0},
+    {0, 1, 1, 4, 4, 0},
+    {1, 4, 4, 5, 5, 0},
+    {1, 1, 3, 4, 5, 0},
+    {1, 1, 4, 5, 6, 0},
+};
+constexpr int kFullUpdProd[28][6] = {
+    {0, 1, 0, 1, 0, 0},
+    {0, 0, 1, 1, 0, 0},
+    {0, 1, 0, 1, 0, 0},
+    {1, 0, 0, 1, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {1, 0, 0, 0, 0, 0},
+    {0, 0, 1, 0, 0, 0},
+    {1, 1, 0, 0, 0, 0},
+    {1, 1, 0, 0, 1, 0},
+    {0, 0, 1, 0, 0, 0},
+    {1, 1, 0, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {0, 1, 0, 1, 0, 0},
+    {1, 0, 1, 0, 0, 0},
+    {1, 0, 1, 0, 0, 0},
+    {1, 0, 1, 0, 0, 0},
+    {1, 0, 0, 1, 0, 0},
+    {1, 0, 0, 1, 0, 0},
+    {1, 1, 0, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {1, 0, 1, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {0, 1, 1, 0, 0, 0},
+    {1, 0, 1, 0, 0, 0},
+    {0, 0, 0, 1, 1, 0},
+    {0, 1, 0, 0, 1, 0},
+    {0, 1, 0, 0, 1, 0},
+};
+
+// zd = dC/dt at z (shared scratch in, shared scratch out)
+template <class S>
+__device__ __forceinline__ void full_rhs(S& c) {
+  const double z0 = c.z(0);
+  const double z1 = c.z(1);
+  const double z3 = c.z(3);
+  const double z4 = c.z(4);
+  const double z5 = c.z(5);
+  const double z6 = c.z(6);
+  const double z7 = c.z(7);
+  const double z8 = c.z(8);
+  double d0 = 0.0, d1 = 0.0, d2 = 0.0, d3 = 0.0, d4 = 0.0, d5 = 0.0, d6 = 0.0, d7 = 0.0, d8 = 0.0;
+  double f, b, q;
+  f = __dmul_rn(__dmul_rn(c.kf(0), z4), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(0), z3), z5);
+  q = __dsub_rn(f, b);
+  d1 = __dsub_rn(d1, q);
+  d3 = __dadd_rn(d3, q);
+  d4 = __dsub_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  f = __dmul_rn(__dmul_rn(c.kf(1), z3), z0);
+  b = __dmul_rn(__dmul_rn(c.kr(1), z5), z4);
+  q = __dsub_rn(f, b);
+  d0 = __dsub_rn(d0, q);
+  d3 = __dsub_rn(d3, q);
+  d4 = __dadd_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  f = __dmul_rn(__dmul_rn(c.kf(2), z5), z0);
+  b = __dmul_rn(__dmul_rn(c.kr(2), z4), z6);
+  q = __dsub_rn(f, b);
+  d0 = __dsub_rn(d0, q);
+  d4 = __dadd_rn(d4, q);
+  d5 = __dsub_rn(d5, q);
+  d6 = __dadd_rn(d6, q);
+  f = __dmul_rn(__dmul_rn(c.kf(3), z5), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(3), z6), z3);
+  q = __dsub_rn(f, b);
+  d3 = __dadd_rn(d3, q);
+  d5 = __dsub_rn(d5, q);
+  d5 = __dsub_rn(d5, q);
+  d6 = __dadd_rn(d6, q);
+  f = __dmul_rn(c.kf(4), z0);
+  b = __dmul_rn(__dmul_rn(c.kr(4), z4), z4);
+  q = __dsub_rn(f, b);
+  d0 = __dsub_rn(d0, q);
+  d4 = __dadd_rn(d4, q);
+  d4 = __dadd_rn(d4, q);
+  f = __dmul_rn(__dmul_rn(c.kf(5), z3), z3);
+  b = __dmul_rn(c.kr(5), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dadd_rn(d1, q);
+  d3 = __dsub_rn(d3, q);
+  d3 = __dsub_rn(d3, q);
+  f = __dmul_rn(__dmul_rn(c.kf(6), z3), z4);
+  b = __dmul_rn(c.kr(6), z5);
+  q = __dsub_rn(f, b);
+  d3 = __dsub_rn(d3, q);
+  d4 = __dsub_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  f = __dmul_rn(c.kf(7), z6);
+  b = __dmul_rn(__dmul_rn(c.kr(7), z4), z5);
+  q = __dsub_rn(f, b);
+  d4 = __dadd_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  d6 = __dsub_rn(d6, q);
+  f = __dmul_rn(__dmul_rn(c.kf(8), z6), z6);
+  b = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(8), z4), z5), z6);
+  q = __dsub_rn(f, b);
+  d4 = __dadd_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  d6 = __dsub_rn(d6, q);
+  d6 = __dsub_rn(d6, q);
+  d6 = __dadd_rn(d6, q);
+  f = __dmul_rn(__dmul_rn(c.kf(9), z4), z1);
+  b = __dmul_rn(c.kr(9), z7);
+  q = __dsub_rn(f, b);
+  d1 = __dsub_rn(d1, q);
+  d4 = __dsub_rn(d4, q);
+  d7 = __dadd_rn(d7, q);
+  f = __dmul_rn(__dmul_rn(c.kf(10), z7), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(10), z0), z1);
+  q = __dsub_rn(f, b);
+  d0 = __dadd_rn(d0, q);
+  d1 = __dadd_rn(d1, q);
+  d4 = __dsub_rn(d4, q);
+  d7 = __dsub_rn(d7, q);
+  f = __dmul_rn(__dmul_rn(c.kf(11), z7), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(11), z5), z5);
+  q = __dsub_rn(f, b);
+  d4 = __dsub_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  d5 = __dadd_rn(d5, q);
+  d7 = __dsub_rn(d7, q);
+  f = __dmul_rn(__dmul_rn(c.kf(12), z6), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(12), z4), z7);
+  q = __dsub_rn(f, b);
+  d3 = __dsub_rn(d3, q);
+  d4 = __dadd_rn(d4, q);
+  d6 = __dsub_rn(d6, q);
+  d7 = __dadd_rn(d7, q);
+  f = __dmul_rn(__dmul_rn(c.kf(13), z7), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(13), z5), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dadd_rn(d1, q);
+  d3 = __dsub_rn(d3, q);
+  d5 = __dadd_rn(d5, q);
+  d7 = __dsub_rn(d7, q);
+  f = __dmul_rn(__dmul_rn(c.kf(14), z7), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(14), z6), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dadd_rn(d1, q);
+  d5 = __dsub_rn(d5, q);
+  d6 = __dadd_rn(d6, q);
+  d7 = __dsub_rn(d7, q);
+  f = __dmul_rn(__dmul_rn(c.kf(15), z7), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(15), z6), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dadd_rn(d1, q);
+  d5 = __dsub_rn(d5, q);
+  d6 = __dadd_rn(d6, q);
+  d7 = __dsub_rn(d7, q);
+  f = __dmul_rn(__dmul_rn(c.kf(16), z7), z7);
+  b = __dmul_rn(__dmul_rn(c.kr(16), z8), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dadd_rn(d1, q);
+  d7 = __dsub_rn(d7, q);
+  d7 = __dsub_rn(d7, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(17), z7), z7);
+  b = __dmul_rn(__dmul_rn(c.kr(17), z8), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dadd_rn(d1, q);
+  d7 = __dsub_rn(d7, q);
+  d7 = __dsub_rn(d7, q);
+  d8 = __dadd_rn(d8, q);
+  f = __dmul_rn(c.kf(18), z8);
+  b = __dmul_rn(__dmul_rn(c.kr(18), z5), z5);
+  q = __dsub_rn(f, b);
+  d5 = __dadd_rn(d5, q);
+  d5 = __dadd_rn(d5, q);
+  d8 = __dsub_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(19), z8), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(19), z6), z5);
+  q = __dsub_rn(f, b);
+  d4 = __dsub_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  d6 = __dadd_rn(d6, q);
+  d8 = __dsub_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(20), z8), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(20), z7), z0);
+  q = __dsub_rn(f, b);
+  d0 = __dadd_rn(d0, q);
+  d4 = __dsub_rn(d4, q);
+  d7 = __dadd_rn(d7, q);
+  d8 = __dsub_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(21), z8), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(21), z5), z7);
+  q = __dsub_rn(f, b);
+  d3 = __dsub_rn(d3, q);
+  d5 = __dadd_rn(d5, q);
+  d7 = __dadd_rn(d7, q);
+  d8 = __dsub_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(22), z8), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(22), z6), z7);
+  q = __dsub_rn(f, b);
+  d5 = __dsub_rn(d5, q);
+  d6 = __dadd_rn(d6, q);
+  d7 = __dadd_rn(d7, q);
+  d8 = __dsub_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(c.kf(23), z8), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(23), z6), z7);
+  q = __dsub_rn(f, b);
+  d5 = __dsub_rn(d5, q);
+  d6 = __dadd_rn(d6, q);
+  d7 = __dadd_rn(d7, q);
+  d8 = __dsub_rn(d8, q);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(24), z4), z1), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(24), z0), z1);
+  q = __dsub_rn(f, b);
+  d0 = __dadd_rn(d0, q);
+  d1 = __dsub_rn(d1, q);
+  d1 = __dadd_rn(d1, q);
+  d4 = __dsub_rn(d4, q);
+  d4 = __dsub_rn(d4, q);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(25), z4), z1), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(25), z5), z5);
+  q = __dsub_rn(f, b);
+  d1 = __dsub_rn(d1, q);
+  d4 = __dsub_rn(d4, q);
+  d4 = __dsub_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  d5 = __dadd_rn(d5, q);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(26), z4), z1), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(26), z5), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dsub_rn(d1, q);
+  d1 = __dadd_rn(d1, q);
+  d3 = __dsub_rn(d3, q);
+  d4 = __dsub_rn(d4, q);
+  d5 = __dadd_rn(d5, q);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(27), z4), z1), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(27), z6), z1);
+  q = __dsub_rn(f, b);
+  d1 = __dsub_rn(d1, q);
+  d1 = __dadd_rn(d1, q);
+  d4 = __dsub_rn(d4, q);
+  d5 = __dsub_rn(d5, q);
+  d6 = __dadd_rn(d6, q);
+  c.zd(0) = d0;
+  c.zd(1) = d1;
+  c.zd(2) = d2;
+  c.zd(3) = d3;
+  c.zd(4) = d4;
+  c.zd(5) = d5;
+  c.zd(6) = d6;
+  c.zd(7) = d7;
+  c.zd(8) = d8;
 }
 
 // Column J of I + factor * J: v[i] = A(i+1, J+1), each element's terms in

@@ -27,9 +27,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 MERGE_UP_TO = 8
 
 
-def reduced_structure(t: dict):
+def reduced_structure(t: dict, full: bool = False):
     """Reaction lists over the reacting species, built exactly as the host
-    builds the device tables (build_dev_mech + reduce_dev_mech in capi.cu)."""
+    builds the device tables (build_dev_mech + reduce_dev_mech in capi.cu);
+    full: over all species and reactions (build_dev_mech alone)."""
     N, R = t["n_species"], t["n_reactions"]
     co = t["coeffs"]
     left, right, upd = [], [], []
@@ -48,6 +49,8 @@ def reduced_structure(t: dict):
                 if raw_r[i] == k:
                     u.append((k - 1, 1))
         upd.append(u)
+    if full:
+        return N, R, left, right, upd
     reacts = sorted({s for r in range(R) for s in left[r] + right[r] if s >= 0})
     int_of = {k: i for i, k in enumerate(reacts)}
     left = [[int_of[s] if s >= 0 else -1 for s in row] for row in left]
@@ -70,20 +73,9 @@ def mul_chain(first: str, species) -> str:
     return e
 
 
-def emit(name: str, ns: str, NI: int, R: int, left, right, upd) -> str:
-    o = []
-    w = o.append
-    w(f"// Generated by nrg_b200/gen_mech.py from {name}.txt: do not edit.")
-    w("// Straight-line right-hand side and analytic iteration matrix over the")
-    w(f"// {NI} reacting species and {R} reactions; same operation order as the")
-    w("// table-driven loops in chem_bdf.cuh, with the same explicitly rounded")
-    w("// (never fused) operations.")
-    w("#pragma once")
-    w("")
-    w("namespace nrg {")
-    w(f"namespace {ns} {{")
-    w("")
-    w(f"constexpr int kSpecN = {NI}, kSpecR = {R};")
+def emit_tables_rhs(w, prefix: str, fn: str, N: int, R: int, left, right, upd) -> None:
+    """The reaction lists and the right-hand side over N species and R reactions."""
+    w(f"constexpr int {prefix}N = {N}, {prefix}R = {R};")
 
     def arr(nm, rows, width):
         w(f"constexpr int {nm}[{R}][{width}] = {{")
@@ -91,19 +83,20 @@ def emit(name: str, ns: str, NI: int, R: int, left, right, upd) -> str:
             w("    {" + ", ".join(str(x) for x in row) + "},")
         w("};")
 
-    arr("kSpecLeft", left, 3)
-    arr("kSpecRight", right, 3)
-    w(f"constexpr int kSpecNupd[{R}] = {{" + ", ".join(str(len(u)) for u in upd) + "};")
-    arr("kSpecUpdK", [[k for k, _ in u] + [0] * (6 - len(u)) for u in upd], 6)
-    arr("kSpecUpdProd", [[p for _, p in u] + [0] * (6 - len(u)) for u in upd], 6)
+    arr(f"{prefix}Left", left, 3)
+    arr(f"{prefix}Right", right, 3)
+    w(f"constexpr int {prefix}Nupd[{R}] = {{" + ", ".join(str(len(u)) for u in upd) + "};")
+    arr(f"{prefix}UpdK", [[k for k, _ in u] + [0] * (6 - len(u)) for u in upd], 6)
+    arr(f"{prefix}UpdProd", [[p for _, p in u] + [0] * (6 - len(u)) for u in upd], 6)
     w("")
-    # right-hand side
     w("// zd = dC/dt at z (shared scratch in, shared scratch out)")
     w("template <class S>")
-    w("__device__ __forceinline__ void spec_rhs(S& c) {")
-    for k in range(NI):
-        w(f"  const double z{k} = c.z({k});")
-    w("  double " + ", ".join(f"d{k} = 0.0" for k in range(NI)) + ";")
+    w(f"__device__ __forceinline__ void {fn}(S& c) {{")
+    used = {s for row in left + right for s in row if s >= 0}
+    for k in range(N):
+        if k in used:
+            w(f"  const double z{k} = c.z({k});")
+    w("  double " + ", ".join(f"d{k} = 0.0" for k in range(N)) + ";")
     w("  double f, b, q;")
     for r in range(R):
         w(f"  f = {mul_chain('c.kf(%d)' % r, [s for s in left[r] if s >= 0])};")
@@ -111,10 +104,29 @@ def emit(name: str, ns: str, NI: int, R: int, left, right, upd) -> str:
         w("  q = __dsub_rn(f, b);")
         for k, p in upd[r]:
             w(f"  d{k} = {'__dadd_rn' if p else '__dsub_rn'}(d{k}, q);")
-    for k in range(NI):
+    for k in range(N):
         w(f"  c.zd({k}) = d{k};")
     w("}")
     w("")
+
+
+def emit(name: str, ns: str, reduced, full) -> str:
+    NI, R, left, right, upd = reduced
+    o = []
+    w = o.append
+    w(f"// Generated by nrg_b200/gen_mech.py from {name}.txt: do not edit.")
+    w("// Straight-line right-hand side and analytic iteration matrix over the")
+    w(f"// {NI} reacting species and {R} distinct reactions, and the right-hand side")
+    w(f"// over all {full[0]} species and {full[1]} reactions; same operation order as the")
+    w("// table-driven loops in chem_bdf.cuh, with the same explicitly rounded")
+    w("// (never fused) operations.")
+    w("#pragma once")
+    w("")
+    w("namespace nrg {")
+    w(f"namespace {ns} {{")
+    w("")
+    emit_tables_rhs(w, "kSpec", "spec_rhs", NI, R, left, right, upd)
+    emit_tables_rhs(w, "kFull", "full_rhs", *full)
     # analytic iteration matrix, column by column
     w("// Column J of I + factor * J: v[i] = A(i+1, J+1), each element's terms in")
     w("// reaction order.")
@@ -166,22 +178,27 @@ def emit_index(names) -> str:
         ns = f"gen_{n.lower()}"
         o += ["template <>", f"struct SpecOf<kSpec{n.capitalize()}> {{",
               f"  static constexpr int kN = {ns}::kSpecN, kR = {ns}::kSpecR;",
+              f"  static constexpr int kFullN = {ns}::kFullN, kFullR = {ns}::kFullR;",
               "  template <class S>", f"  __device__ static void rhs(S& c) {{ {ns}::spec_rhs(c); }}",
+              "  template <class S>", f"  __device__ static void rhs_full(S& c) {{ {ns}::full_rhs(c); }}",
               "  template <int J, class S, typename LUT>",
               f"  __device__ static void column(const S& c, double f, LUT (&v)[{ns}::kSpecN]) {{",
               f"    {ns}::spec_column<J>(c, f, v);", "  }", "};"]
-    o += ["", "// 0 when the reduced reaction lists match none of the generated codes.",
-          "template <class M>", "inline int match_specialised_tables(const M& m) {"]
+    o += ["", "// 0 when the reaction lists, reduced or full, match none of the generated codes.",
+          "template <class M>", "inline int match_specialised_tables(const M& m, const M& full) {"]
     for n in names:
         ns = f"gen_{n.lower()}"
-        o += [f"  if (m.NI == {ns}::kSpecN && m.RM == {ns}::kSpecR) {{", "    bool ok = true;",
-              "    for (int r = 0; ok && r < m.RM; ++r) {",
-              f"      ok = m.nupd[r] == {ns}::kSpecNupd[r];",
-              "      for (int i = 0; ok && i < 3; ++i)",
-              f"        ok = m.left[r][i] == {ns}::kSpecLeft[r][i] && m.right[r][i] == {ns}::kSpecRight[r][i];",
-              "      for (int u = 0; ok && u < m.nupd[r]; ++u)",
-              f"        ok = m.upd_k[r][u] == {ns}::kSpecUpdK[r][u] && m.upd_prod[r][u] == {ns}::kSpecUpdProd[r][u];",
-              "    }", f"    if (ok) return kSpec{n.capitalize()};", "  }"]
+        o += [f"  if (m.NI == {ns}::kSpecN && m.RM == {ns}::kSpecR && full.N == {ns}::kFullN && full.R == {ns}::kFullR) {{",
+              "    bool ok = true;"]
+        for t, r, p in (("m", "m.RM", "kSpec"), ("full", "full.R", "kFull")):
+            o += [f"    for (int r = 0; ok && r < {r}; ++r) {{",
+                  f"      ok = {t}.nupd[r] == {ns}::{p}Nupd[r];",
+                  "      for (int i = 0; ok && i < 3; ++i)",
+                  f"        ok = {t}.left[r][i] == {ns}::{p}Left[r][i] && {t}.right[r][i] == {ns}::{p}Right[r][i];",
+                  f"      for (int u = 0; ok && u < {t}.nupd[r]; ++u)",
+                  f"        ok = {t}.upd_k[r][u] == {ns}::{p}UpdK[r][u] && {t}.upd_prod[r][u] == {ns}::{p}UpdProd[r][u];",
+                  "    }"]
+        o += [f"    if (ok) return kSpec{n.capitalize()};", "  }"]
     o += ["  return 0;", "}", "", "}  // namespace nrg", ""]
     return "\n".join(o)
 
@@ -192,11 +209,11 @@ def main() -> int:
     from nrg_b200.chemistry import mechanism_tables
     for name in MECHANISMS:
         t = mechanism_tables(*mechanism_paths(name))
-        NI, R, left, right, upd = reduced_structure(t)
+        reduced, full = reduced_structure(t), reduced_structure(t, True)
         out = os.path.join(HERE, "csrc", f"gen_{name.lower()}.cuh")
         with open(out, "w") as fh:
-            fh.write(emit(name, f"gen_{name.lower()}", NI, R, left, right, upd))
-        print(f"wrote {out}: {NI} reacting species, {R} reactions")
+            fh.write(emit(name, f"gen_{name.lower()}", reduced, full))
+        print(f"wrote {out}: {reduced[0]} reacting species, {reduced[1]} distinct reactions")
     with open(os.path.join(HERE, "csrc", "gen_mechanisms.cuh"), "w") as fh:
         fh.write(emit_index(MECHANISMS))
     return 0
