@@ -278,9 +278,9 @@ NRG_API int nrg_chem_set_mode(nrg_chem* h, int mode);
  * queue, 2 = one warp per cell pulling cells from the work queue.  block: 32
  * (default) or 64 for kernels 0/1, 128 or 256 for kernel 2.  grid: persistent
  * grid size (0 = fill the GPU).  chunk: cells reserved per queue fetch (1..64).
- * The analytic-Jacobian and mixed kernels of mechanisms with up to 8 reacting
- * species choose their blocks by the number of cells whatever `block` says, and
- * with kernel 1 their warps reserve `chunk` groups of 32 cells at a time. */
+ * The analytic-Jacobian and mixed kernels choose their blocks by the number of
+ * cells whatever `block` says, and with kernel 1 their warps reserve `chunk`
+ * groups of 32 cells at a time. */
 NRG_API int nrg_chem_set_launch(nrg_chem* h, int kernel, int block, int grid, int chunk);
 NRG_API int nrg_chem_get_launch(nrg_chem* h, int* kernel, int* block, int* grid, int* chunk);
 /* Form of the LU factorisation in the thread-per-cell kernels: 0 (default)
@@ -288,8 +288,7 @@ NRG_API int nrg_chem_get_launch(nrg_chem* h, int* kernel, int* block, int* grid,
  * unrolled form is faster where neighbouring cells take alike BDF paths
  * (the flame field), the loop, with a quarter of the code, where they vary
  * (ignition and wide-range fields).  nrg_chem_autotune tries both.  Without
- * effect on the analytic-Jacobian and mixed kernels of mechanisms with up to 8
- * reacting species, which have one form. */
+ * effect on the analytic-Jacobian and mixed kernels, which have one form. */
 NRG_API int nrg_chem_set_lu_form(nrg_chem* h, int rolled);
 NRG_API int nrg_chem_get_lu_form(nrg_chem* h, int* rolled);
 

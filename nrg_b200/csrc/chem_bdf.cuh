@@ -110,7 +110,7 @@ struct RowPerm {
 // register-resident vectors are never forced to local memory by the call.
 template <int N, int R, typename LUT, int BS, int SPEC>
 __device__ __noinline__ void nl_rhs(double* d, LUT* f);
-template <int N, int R, typename LUT, int BS, int SPEC>
+template <int N, int R, typename LUT, int BS>
 __device__ __noinline__ void nl_analytic_matrix(double* d, LUT* f, double factor);
 template <int N, int R, typename LUT, int BS, bool RECIP>
 __device__ __noinline__ RowPerm<N> nl_dgefa(double* d, LUT* f, int* info, int rolled);
@@ -715,41 +715,20 @@ __device__ __noinline__ void nl_rhs(double* d, LUT* f) {
   SmemStore<N, R, LUT, BS> s;
   s.d = d;
   s.f = f;
-  if constexpr (SPEC != 0) {
-    // the reference mode integrates all species, the others the reacting ones
-    if constexpr (N == SpecOf<SPEC>::kFullN && R == SpecOf<SPEC>::kFullR) {
-      SpecOf<SPEC>::rhs_full(s);
-    } else {
-      static_assert(N == SpecOf<SPEC>::kN && R == SpecOf<SPEC>::kR, "specialised code is for another mechanism size");
-      SpecOf<SPEC>::rhs(s);
-    }
+  if constexpr (SPEC != 0) {  // the reference mode, which integrates all species
+    static_assert(N == SpecOf<SPEC>::kFullN && R == SpecOf<SPEC>::kFullR, "specialised code of another mechanism");
+    SpecOf<SPEC>::rhs_full(s);
   } else {
     rhs<N>(s, R);
   }
 }
 
-// The generated iteration matrix into the LU storage, one column in registers
-// at a time.
-template <int SPEC, int N, typename LUT, int J, class S>
-__device__ __forceinline__ void spec_store_columns(const S& s, double factor) {
-  LUT v[N];
-  SpecOf<SPEC>::template column<J>(s, factor, v);
-#pragma unroll
-  for (int i = 0; i < N; ++i) s.a(J, i) = v[i];
-  if constexpr (J + 1 < N) spec_store_columns<SPEC, N, LUT, J + 1>(s, factor);
-}
-
-template <int N, int R, typename LUT, int BS, int SPEC>
+template <int N, int R, typename LUT, int BS>
 __device__ __noinline__ void nl_analytic_matrix(double* d, LUT* f, double factor) {
   SmemStore<N, R, LUT, BS> s;
   s.d = d;
   s.f = f;
-  if constexpr (SPEC != 0) {
-    static_assert(N == SpecOf<SPEC>::kN && R == SpecOf<SPEC>::kR, "specialised code is for another mechanism size");
-    spec_store_columns<SPEC, N, LUT, 0>(s, factor);
-  } else {
-    analytic_iteration_matrix<N>(s, factor, R);
-  }
+  analytic_iteration_matrix<N>(s, factor, R);
 }
 
 template <int N, int R, typename LUT, int BS, bool RECIP>
@@ -929,7 +908,7 @@ __device__ void ddpst(CS& c) {
   } else {
 #pragma unroll
     for (int k = 0; k < N; ++k) c.z(k) = c.y[k];
-    nl_analytic_matrix<N, R, typename CS::lut_t, CS::kBS, CS::kSpec>(c.d, c.f, -el1h);
+    nl_analytic_matrix<N, R, typename CS::lut_t, CS::kBS>(c.d, c.f, -el1h);
   }
   int info = 0;
   c.piv = nl_dgefa<N, R, typename CS::lut_t, CS::kBS, JAC != kJacFD>(c.d, c.f, &info, c.lu_rolled);

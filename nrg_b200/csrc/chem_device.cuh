@@ -16,7 +16,7 @@ namespace nrg {
 constexpr int kMaxSpecies = 24;
 constexpr int kMaxReactions = 96;
 constexpr int kMaxOrd = 5;  // MXORD for Gear (MINT = 2)
-constexpr int kMergeUpTo = 8;  // integrated species up to which equal reactions are merged
+constexpr int kMergeUpTo = 16;  // integrated species up to which equal reactions are merged
 constexpr int kMaxSpecUpd = 64;  // reactions touching one species
 
 // Per-reaction update list entry: species (0-based) and whether the
@@ -65,7 +65,7 @@ struct DevMech {
   // The first RM reactions have distinct reactant and product lists; reaction
   // r >= RM repeats the lists of reaction m_of[r], so the right-hand side and
   // the iteration matrix walk RM reactions with the sums of the rate constants.
-  // (Full tables and tables of more than kMergeUpTo species: RM = R.)
+  // (Full tables: RM = R.)
   int RM;
   int m_of[kMaxReactions];
 };

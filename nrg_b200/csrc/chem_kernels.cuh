@@ -2,7 +2,7 @@
 // translation units chem_k_*.cu, which instantiate them).
 //
 //   k_chem_pass   -- one thread per cell in passes (chem_pass.cuh): analytic
-//                    Jacobian, up to 8 integrated species.
+//                    Jacobian.
 //   k_chem_plain  -- one thread per cell, grid covers all cells.
 //   k_chem_queue  -- persistent grid; every lane pulls cells from a device
 //                    work queue and is refilled as soon as its cell reaches
@@ -139,16 +139,28 @@ static cudaError_t launch_bs(const StepArgs& a, const LaunchCfg& cfg, int* queue
 // the block go through the passes together, so that the loop's 50 to 80 KB of
 // code are fetched once for all of them.  QUEUE: the warps pull groups of 32
 // cells from the work queue; else the grid covers the cells.
-template <int N, int R, typename LUT, int BS, int NF, int SPEC, bool LOCK, bool QUEUE>
-__global__ void __launch_bounds__(BS, 256 / BS) k_chem_pass(StepArgs a, int* queue, int chunk,
+// TM: the cells' rate constants in tensor memory (lockstep blocks of 128 threads:
+// warp w has lanes 32 w).
+template <int N, int R, typename LUT, int BS, int NF, int SPEC, bool LOCK, bool QUEUE, bool TM>
+__global__ void __launch_bounds__(BS, BS > 128 ? 1 : 256 / BS) k_chem_pass(StepArgs a, int* queue, int chunk,
                                                             unsigned long long* counters) {
   static_assert(!(LOCK && QUEUE), "the work queue serves warps on their own");
+  static_assert(!TM || (LOCK && BS == 128), "one warp per quarter of the tensor memory's lanes");
   extern __shared__ __align__(16) char smem[];
   const long nl = a.cell_list ? (long)(a.n_list_dev ? *a.n_list_dev : a.n_list) : a.n;
   if (!QUEUE && (long)blockIdx.x * BS >= nl) return;
   unsigned long long v[kCntSlots] = {0, 0, 0, 0, 0, 0};
-  PassStore<N, RateSlots<R, SPEC>::value, LUT, SPEC == 0> st;
+  using Store = PassStore<N, RateSlots<R, SPEC>::value, LUT, SPEC == 0, TM>;
+  Store st;
   st.bind(smem, threadIdx.x);
+  __shared__ uint32_t tslot;
+  if constexpr (TM) {
+    if (threadIdx.x < 32) tc::tmem_alloc(tc::smem_u32(&tslot), Store::kTmCols);
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    st.tm = tslot + ((threadIdx.x & ~31u) << 16);
+  }
   const int lane = threadIdx.x & 31;
   long base = ((long)blockIdx.x * BS + threadIdx.x) & ~31L;
   int left = 0;
@@ -177,6 +189,7 @@ __global__ void __launch_bounds__(BS, 256 / BS) k_chem_pass(StepArgs a, int* que
       live = pass_begin<N, R, NF>(st, a, cid, res.y);
       if (a.dt_cells) res.tout = a.dt_cells[cid];
     }
+    if constexpr (TM) pass_rates_to_tm<N>(st);
     const int status = pass_integrate<N, R, NF, SPEC, LOCK>(st, a, live, res.tout, res.y, v);
     if (live) {
       cell_finish<N, kJacAnalytic>(res, a, cid, status);
@@ -185,16 +198,25 @@ __global__ void __launch_bounds__(BS, 256 / BS) k_chem_pass(StepArgs a, int* que
     }
     if (!QUEUE) break;
   }
+  if constexpr (TM) {
+    __syncthreads();
+    if (threadIdx.x < 32) tc::tmem_dealloc(tslot, Store::kTmCols);
+  }
   if (counters) block_flush_counters(counters, v);
 }
 
-template <int N, int R, typename LUT, int BS, int NF, int SPEC, bool LOCK, bool QUEUE>
+template <int N, int R, typename LUT, int BS, int NF, int SPEC, bool LOCK, bool QUEUE, bool TM = false>
 static cudaError_t launch_pass_bs(const StepArgs& a, long grid, int* queue, int chunk, unsigned long long* counters,
                                   cudaStream_t s) {
-  const auto kern = k_chem_pass<N, R, LUT, BS, NF, SPEC, LOCK, QUEUE>;
-  const int smem = BS * PassStore<N, RateSlots<R, SPEC>::value, LUT, SPEC == 0>::kBytesPerThread;
+  const auto kern = k_chem_pass<N, R, LUT, BS, NF, SPEC, LOCK, QUEUE, TM>;
+  const int smem = BS * PassStore<N, RateSlots<R, SPEC>::value, LUT, SPEC == 0, TM>::kBytesPerThread;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  // lockstep blocks of larger mechanisms spill part of the Nordsieck array: what
+  // shared memory their one or two blocks per SM leave goes to the L1 cache
+  // (KONNOV flame of 196,608 cells 26.9 -> 22.8 ms)
+  const int used = (smem + 1024) * (smem < 115000 ? 2 : 1);
+  const int carveout = N > 8 && LOCK ? (100 * used + 233471) / 233472 : 100;
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
   if (e != cudaSuccess) return e;
   if (grid > 0) kern<<<(unsigned)grid, BS, smem, s>>>(a, queue, chunk, counters);
   return cudaGetLastError();
@@ -210,13 +232,35 @@ constexpr long kLockstepCells = 148L * 2 * 128;
 template <int N, int R, typename LUT, int NF, int SPEC>
 static cudaError_t launch_pass(const StepArgs& a, const LaunchCfg& cfg, int* queue, unsigned long long* counters,
                                cudaStream_t s) {
-  if (cfg.kernel == kKernelThreadQueue)
-    return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, true>(a, cfg.grid > 0 ? cfg.grid : 148, queue, cfg.chunk,
-                                                                counters, s);
+  if constexpr (N <= 8) {
+    if (cfg.kernel == kKernelThreadQueue)
+      return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, true>(a, cfg.grid > 0 ? cfg.grid : 148, queue, cfg.chunk,
+                                                                  counters, s);
+  }
   const long nl = a.cell_list ? (long)a.n_list : a.n;
-  if (nl < kLockstepCells)
-    return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, false>(a, (nl + 63) / 64, queue, 0, counters, s);
-  return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false>(a, (nl + 127) / 128, queue, 0, counters, s);
+  if constexpr (N <= 8) {
+    if (nl < kLockstepCells)
+      return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, false>(a, (nl + 63) / 64, queue, 0, counters, s);
+    return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false>(a, (nl + 127) / 128, queue, 0, counters, s);
+  } else {
+    // as many warps as the cells' shared memory allows, one block per SM; with the
+    // generated code in blocks of 128 threads with the rate constants in tensor
+    // memory, where more warps fit that way (KONNOV 2 -> 4 warps, TEREZA 5 -> 8;
+    // flame of 196,608 cells 46.4 -> 26.9 ms and 11.7 -> 9.0 ms)
+    constexpr int RS = RateSlots<R, SPEC>::value;
+    constexpr int kWarpBytes = 32 * PassStore<N, RS, LUT, SPEC == 0>::kBytesPerThread;
+    constexpr int W = 232448 / kWarpBytes < 8 ? 232448 / kWarpBytes : 8;
+    if (nl < 148L * 32 * W)
+      return launch_pass_bs<N, R, LUT, 32, NF, SPEC, false, false>(a, (nl + 31) / 32, queue, 0, counters, s);
+    if constexpr (SPEC != 0) {
+      constexpr int kTmBytes = 128 * PassStore<N, RS, LUT, false, true>::kBytesPerThread;
+      constexpr int kTmWarps = kTmBytes > 232448 ? 0 : kTmBytes > 115000 ? 4 : 8;
+      if constexpr (kTmWarps > W)
+        return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false, true>(a, (nl + 127) / 128, queue, 0, counters, s);
+    }
+    return launch_pass_bs<N, R, LUT, 32 * W, NF, SPEC, true, false>(a, (nl + 32 * W - 1) / (32 * W), queue, 0,
+                                                                    counters, s);
+  }
 }
 
 __host__ __device__ constexpr size_t warp_tables_bytes() { return (sizeof(DevMech) + 15) / 16 * 16; }
@@ -293,13 +337,14 @@ static cudaError_t launch_warp(const StepArgs& a, const LaunchCfg& cfg, int* que
   return cudaGetLastError();
 }
 
-// The thread-per-cell kernels: in passes where the Nordsieck array fits the
-// registers (up to 8 integrated species, analytic Jacobian; these choose their
-// blocks themselves), else routine by routine.
+// The thread-per-cell kernels: in passes for the analytic Jacobian (these choose
+// their blocks themselves; above 8 species part of the Nordsieck array spills
+// to the L1 cache), routine by routine for the reference mode and for mechanisms
+// of nine species that all react, which no generated code covers.
 template <int NF, int NI, int R, int JAC, typename LUT, int SPEC>
 static cudaError_t launch_thread(const StepArgs& a, const LaunchCfg& cfg, int* queue, unsigned long long* counters,
                                  cudaStream_t s) {
-  if constexpr (JAC == kJacAnalytic && NI <= 8) {
+  if constexpr (JAC == kJacAnalytic && NI != 9) {
     return launch_pass<NI, R, LUT, NF, SPEC>(a, cfg, queue, counters, s);
   } else {
     switch (cfg.block) {

@@ -17,7 +17,8 @@
 // shared memory a cell took 1,408 B there, so an SM held 4 warps, one per
 // scheduler, and the kernel waited on dependent FP64 and shared-memory
 // latency (issue slots 22 % used, FP64 pipe 19 %).  Here the Nordsieck array
-// (6 N doubles) is in registers with compile-time column numbers: columns
+// (6 N doubles; above 8 species part of it spills to the L1 cache) is in
+// registers with compile-time column numbers: columns
 // above a cell's order hold zeros, so lanes of different order run the same
 // predictor, update and interpolation code (adding, scaling or multiplying
 // zeros changes no value).  Shared memory keeps what is indexed at run time
@@ -27,10 +28,13 @@
 // slots at two warps per scheduler, FP64 pipe 37 %) and instruction fetch:
 // the loop is about 4,000 instructions, so the warps of a block go through it
 // in lockstep (k_chem_pass).  2048 x 2048 flame 72.0 -> 28.7 ms, 512 x 512
-// ignition field 79.7 -> 16.2 ms, 64 x 64 random cells 2.49 -> 1.10 ms.
+// ignition field 79.7 -> 16.1 ms, 64 x 64 random cells 2.49 -> 1.10 ms; flames of
+// 196,608 cells with the larger mechanisms: TEREZA 21.6 -> 9.1 ms, KONNOV 42.3
+// -> 22.8 ms, ACETYLENE 30.9 -> 24.8 ms.
 #pragma once
 
 #include "chem_bdf.cuh"
+#include "tc_sm100.cuh"
 
 namespace nrg {
 
@@ -50,19 +54,32 @@ struct RateSlots<R, 0> {
 // lane covers factors of other lanes, but of no other warp); TAB: the
 // table-driven right-hand side also indexes z and zd at run time and keeps its
 // own copies.
-template <int N, int R, typename LUT, bool TAB>
+//
+// TM: the rate constants live in tensor memory instead, lane = cell, four
+// 32-bit columns per reaction (k_f, k_r), next to the 227 KB of shared memory
+// and of the same size.  They are what a cell of a larger mechanism has most
+// of, and the right-hand side reads them in order, sixteen columns at a time.
+// (Tensor memory is read and written by whole warps at warp-uniform columns,
+// so nothing that a lane indexes on its own can go there.)
+template <int N, int R, typename LUT, bool TAB, bool TM = false>
 struct PassStore {
+  static_assert(!(TAB && TM), "the table walk indexes the rate constants in shared memory");
   static constexpr int BS = 32;
-  static constexpr int kSlots = R;
+  static constexpr bool kTM = TM;
+  static constexpr int kRates = R;
+  static constexpr int kSlots = TM ? 0 : R;  // in shared memory
+  static constexpr int kTmCols = 4 * R <= 128 ? 128 : 4 * R <= 256 ? 256 : 512;
+  static_assert(!TM || 4 * R <= 512, "tensor memory columns");
   static constexpr int kKF = 0;
-  static constexpr int kKR = R;
-  static constexpr int kS = 2 * R;               // permutation scratch / z
+  static constexpr int kKR = kSlots;
+  static constexpr int kS = 2 * kSlots;          // permutation scratch / z
   static constexpr int kZD = kS + N;             // TAB only
   static constexpr int kDoubles = kS + (TAB ? 2 : 1) * N;
   static constexpr int kBytesPerThread = kDoubles * 8 + N * N * (int)sizeof(LUT);
   using lut_t = LUT;
   double* d;
   LUT* f;
+  uint32_t tm;  // TM: the warp's lanes of column 0
   __device__ __forceinline__ void bind(char* smem, int tid) {
     smem += (size_t)(tid / BS) * BS * kBytesPerThread;
     d = reinterpret_cast<double*>(smem) + tid % BS;
@@ -101,6 +118,32 @@ struct RegView {
   __device__ __forceinline__ double& zd(int k) const { return out[k]; }
 };
 
+// RegView with the rate constants from tensor memory: four reactions in
+// registers, the next four on their way.  The generated code asks for k_f then
+// k_r of reactions 0, 1, 2, ...
+template <class S, int N>
+struct TmView {
+  const S& st;
+  const double (&zin)[N];
+  double (&out)[N];
+  uint32_t cur[16], nxt[16];
+  __device__ __forceinline__ void start() { tc::tmem_ld16(st.tm, nxt); }
+  __device__ __forceinline__ double kf(int r) {
+    if ((r & 3) == 0) {
+      tc::tmem_ld_wait(nxt);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) cur[i] = nxt[i];
+      if (r + 4 < S::kRates) tc::tmem_ld16(st.tm + 4 * (r + 4), nxt);
+    }
+    return __hiloint2double((int)cur[4 * (r & 3) + 1], (int)cur[4 * (r & 3)]);
+  }
+  __device__ __forceinline__ double kr(int r) const {
+    return __hiloint2double((int)cur[4 * (r & 3) + 3], (int)cur[4 * (r & 3) + 2]);
+  }
+  __device__ __forceinline__ double z(int k) const { return zin[k]; }
+  __device__ __forceinline__ double& zd(int k) const { return out[k]; }
+};
+
 // The store as the generated columns see it.  The rate constants are read
 // again for each column (volatile): kept from one column to the next they
 // would take the registers the Nordsieck array needs.
@@ -108,8 +151,17 @@ template <class S, int N>
 struct ColumnView {
   const S& st;
   const double (&zin)[N];
-  __device__ __forceinline__ double kf(int r) const { return *(const volatile double*)&st.kf(r); }
-  __device__ __forceinline__ double kr(int r) const { return *(const volatile double*)&st.kr(r); }
+  __device__ __forceinline__ double rate(int q) const {
+    if constexpr (S::kTM) {
+      uint32_t v[2];
+      tc::tmem_ld2(st.tm + 2 * q, v);
+      return __hiloint2double((int)v[1], (int)v[0]);
+    } else {
+      return *(const volatile double*)&((q & 1) ? st.kr(q >> 1) : st.kf(q >> 1));
+    }
+  }
+  __device__ __forceinline__ double kf(int r) const { return rate(2 * r); }
+  __device__ __forceinline__ double kr(int r) const { return rate(2 * r + 1); }
   __device__ __forceinline__ double z(int k) const { return zin[k]; }
 };
 
@@ -129,8 +181,15 @@ template <int N, int R, int SPEC, class S>
 __device__ __forceinline__ void pass_rhs(const S& st, const double (&y)[N], double (&out)[N]) {
   if constexpr (SPEC != 0) {
     static_assert(N == SpecOf<SPEC>::kN, "specialised code is for another mechanism size");
-    RegView<S, N> v{st, y, out};
-    SpecOf<SPEC>::rhs(v);
+    if constexpr (S::kTM) {
+      TmView<S, N> v{st, y, out};
+      __syncwarp();
+      v.start();
+      SpecOf<SPEC>::rhs(v);
+    } else {
+      RegView<S, N> v{st, y, out};
+      SpecOf<SPEC>::rhs(v);
+    }
   } else {
     TabView<S, N> v{st};
 #pragma unroll
@@ -148,14 +207,17 @@ __device__ __forceinline__ void pass_rhs(const S& st, const double (&y)[N], doub
 // right-looking dgefa<RECIP> in the same order, but the matrix never exists
 // in memory before it is factored: 64 stores and 28 loads of elements instead
 // of a store, a load and 3 to 4 updates of each.
+// commit: the lane keeps the factors (with rates in tensor memory the whole warp
+// goes through the columns).
 template <int N, int SPEC, int J, class V, class S>
 __device__ __forceinline__ void pass_factor_columns(const V& view, const S& st, double factor, RowPerm<N>& perm,
-                                                    bool& ok) {
+                                                    bool& ok, bool commit) {
   using LUT = typename S::lut_t;
   LUT v[N];
   // one column at a time: without this the loads of later columns are moved up
   // and 250 bytes of registers per thread spill
   asm volatile("" ::: "memory");
+  if constexpr (S::kTM) __syncwarp();
   SpecOf<SPEC>::template column<J>(view, factor, v);
   if constexpr (J > 0) {
 #pragma unroll
@@ -183,11 +245,13 @@ __device__ __forceinline__ void pass_factor_columns(const V& view, const S& st, 
       for (int i = J + 1; i < N; ++i)
         if (i == l) v[i] = v[J];
       v[J] = piv;
+      if (commit) {
 #pragma unroll
-      for (int k = 0; k < J; ++k) {
-        const LUT m = st.a(k, l);
-        st.a(k, l) = st.a(k, J);
-        st.a(k, J) = m;
+        for (int k = 0; k < J; ++k) {
+          const LUT m = st.a(k, l);
+          st.a(k, l) = st.a(k, J);
+          st.a(k, J) = m;
+        }
       }
       const int pk = perm.get(J);
       perm.set(J, perm.get(l));
@@ -203,9 +267,11 @@ __device__ __forceinline__ void pass_factor_columns(const V& view, const S& st, 
   }
 #pragma unroll
   for (int i = 0; i < J; ++i) v[i] = v[i] * v[J];  // U scaled by its pivots (pass_solve)
+  if (commit) {
 #pragma unroll
-  for (int i = 0; i < N; ++i) st.a(J, i) = v[i];
-  if constexpr (J + 1 < N) pass_factor_columns<N, SPEC, J + 1>(view, st, factor, perm, ok);
+    for (int i = 0; i < N; ++i) st.a(J, i) = v[i];
+  }
+  if constexpr (J + 1 < N) pass_factor_columns<N, SPEC, J + 1>(view, st, factor, perm, ok, commit);
 }
 
 // dgefa<RECIP> on the LU storage as two loops over whole columns (rows above
@@ -261,12 +327,13 @@ __device__ __forceinline__ bool pass_lu_loop(const S& st, RowPerm<N>& perm) {
 
 // Factors of I + factor * J(y); false when singular.
 template <int N, int R, int SPEC, class S>
-__device__ __forceinline__ bool pass_factor(const S& st, const double (&y)[N], double factor, RowPerm<N>& perm) {
+__device__ __forceinline__ bool pass_factor(const S& st, const double (&y)[N], double factor, RowPerm<N>& perm,
+                                            bool commit) {
   if constexpr (SPEC != 0) {
     ColumnView<S, N> v{st, y};
     perm.identity();
     bool ok = true;
-    pass_factor_columns<N, SPEC, 0>(v, st, factor, perm, ok);
+    pass_factor_columns<N, SPEC, 0>(v, st, factor, perm, ok, commit);
     return ok;
   } else {
     TabView<S, N> v{st};
@@ -343,6 +410,22 @@ __device__ __forceinline__ double pass_rcp(double x) {
   return fma(r, fma(-w, r, 1.0), r);
 }
 
+// The rate constants of a warp's cells from the set-up scratch (pass_begin) into
+// tensor memory; all lanes.
+template <int N, class S>
+__device__ __forceinline__ void pass_rates_to_tm(const S& st) {
+  const int lane = threadIdx.x % S::BS;
+  SetupView<S, N, 0> v{st, reinterpret_cast<double*>(st.f - lane) + lane};
+  __syncwarp();
+#pragma unroll 4
+  for (int r = 0; r < S::kRates; ++r) {
+    const double f = v.kf(r), b = v.kr(r);
+    tc::tmem_st4(st.tm + 4 * r, (uint32_t)__double2loint(f), (uint32_t)__double2hiint(f), (uint32_t)__double2loint(b),
+                 (uint32_t)__double2hiint(b));
+  }
+  tc::tmem_st_wait();
+}
+
 // x^p, 0 < p < 1, for the step-size choices: 2^(p log2 x) with the logarithm's
 // fraction and the power in single precision (relative error about 1e-6, as
 // ratio_pow) over the whole range of x >= 0; NaN and infinity pass through.
@@ -401,7 +484,7 @@ __device__ __forceinline__ bool pass_begin(const S& st, const StepArgs& a, long 
   double conc[NF];
 #pragma unroll
   for (int k = 0; k < NF; ++k) conc[k] = a.Y[k * a.ld + cid] * rho / c_mech.W[k];
-  constexpr int RS = S::kSlots;
+  constexpr int RS = S::kSlots;  // none with rates in tensor memory: pass_rates_to_tm moves them there
   static_assert(2 * N + 2 * (R - RS) <= N * N * (int)sizeof(typename S::lut_t) / 8, "set-up scratch");
   const int lane = threadIdx.x % S::BS;
   SetupView<S, N, RS> v{st, reinterpret_cast<double*>(st.f - lane) + lane};
@@ -415,8 +498,8 @@ __device__ __forceinline__ bool pass_begin(const S& st, const StepArgs& a, long 
   rate_constants_fast<N, R>(v, Tc);
   for (int r = c_mech.RM; r < R; ++r) {
     const int m = c_mech.m_of[r];
-    st.kf(m) += v.kf(r);
-    st.kr(m) += v.kr(r);
+    v.kf(m) += v.kf(r);
+    v.kr(m) += v.kr(r);
   }
   // mechanism order to integrated order (the inert species drop out); the
   // index is a table read, so through the scratch unless nothing drops out
@@ -572,9 +655,17 @@ __device__ __forceinline__ int pass_integrate(const S& st, const StepArgs& a, bo
         const bool make = 2 * pass_count<LOCK>(due) >= nrun;
     const bool need = due && make;
     if (due) phase = make ? kPredict : kWait;
+    const double jac_factor = -(EL(1, nq) * h);
+    RowPerm<N> made;
+    bool factored = false;
+    if constexpr (S::kTM) {
+      if (__any_sync(kAll, need)) factored = pass_factor<N, R, SPEC>(st, yh[0], jac_factor, made, need);
+    }
     if (need) {
       nje += 1;
-      ier = !pass_factor<N, R, SPEC>(st, yh[0], -(EL(1, nq) * h), piv);
+      if constexpr (S::kTM) piv = made;
+      else factored = pass_factor<N, R, SPEC>(st, yh[0], jac_factor, piv, true);
+      ier = !factored;
       if (!ier) {
         convrg = false;
         rc = 1.0;

@@ -1,6 +1,6 @@
 // Generated by nrg_b200/gen_mech.py from KONNOV.txt: do not edit.
 // Straight-line right-hand side and analytic iteration matrix over the
-// 13 reacting species and 71 distinct reactions, and the right-hand side
+// 13 reacting species and 67 distinct reactions, and the right-hand side
 // over all 13 species and 71 reactions; same operation order as the
 // table-driven loops in chem_bdf.cuh, with the same explicitly rounded
 // (never fused) operations.
@@ -9,8 +9,8 @@
 namespace nrg {
 namespace gen_konnov {
 
-constexpr int kSpecN = 13, kSpecR = 71;
-constexpr int kSpecLeft[71][3] = {
+constexpr int kSpecN = 13, kSpecR = 67;
+constexpr int kSpecLeft[67][3] = {
     {4, 4, -1},
     {4, 4, 0},
     {4, 4, 2},
@@ -30,15 +30,11 @@ constexpr int kSpecLeft[71][3] = {
     {6, 3, -1},
     {0, 1, -1},
     {7, 5, -1},
-    {7, 5, -1},
-    {7, 7, -1},
     {7, 7, -1},
     {8, 4, -1},
     {8, 4, -1},
     {8, 3, -1},
     {8, 5, -1},
-    {8, 5, -1},
-    {1, 3, -1},
     {1, 3, -1},
     {12, 3, -1},
     {12, 3, -1},
@@ -83,7 +79,7 @@ constexpr int kSpecLeft[71][3] = {
     {4, 1, 3},
     {4, 1, 5},
 };
-constexpr int kSpecRight[71][3] = {
+constexpr int kSpecRight[67][3] = {
     {0, -1, -1},
     {0, 0, -1},
     {0, 2, -1},
@@ -103,15 +99,11 @@ constexpr int kSpecRight[71][3] = {
     {4, 7, -1},
     {4, 7, -1},
     {6, 1, -1},
-    {6, 1, -1},
-    {8, 1, -1},
     {8, 1, -1},
     {7, 0, -1},
     {6, 5, -1},
     {7, 5, -1},
     {7, 6, -1},
-    {7, 6, -1},
-    {12, -1, -1},
     {12, -1, -1},
     {1, 1, -1},
     {11, 1, -1},
@@ -156,8 +148,8 @@ constexpr int kSpecRight[71][3] = {
     {5, 1, -1},
     {6, 1, -1},
 };
-constexpr int kSpecNupd[71] = {3, 5, 5, 5, 3, 3, 3, 5, 3, 3, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 3, 3, 4, 4, 3, 2, 4, 4, 4, 5, 4, 4, 4, 2, 4, 5, 4, 4, 4, 3, 4, 4, 4, 4, 5, 4, 4, 4, 3, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 5, 5, 5, 5};
-constexpr int kSpecUpdK[71][6] = {
+constexpr int kSpecNupd[67] = {3, 5, 5, 5, 3, 3, 3, 5, 3, 3, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 3, 4, 4, 3, 2, 4, 4, 4, 5, 4, 4, 4, 2, 4, 5, 4, 4, 4, 3, 4, 4, 4, 4, 5, 4, 4, 4, 3, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 4, 5, 5, 5, 5};
+constexpr int kSpecUpdK[67][6] = {
     {0, 4, 4, 0, 0, 0},
     {0, 0, 0, 4, 4, 0},
     {0, 2, 2, 4, 4, 0},
@@ -177,15 +169,11 @@ constexpr int kSpecUpdK[71][6] = {
     {3, 4, 6, 7, 0, 0},
     {0, 1, 4, 7, 0, 0},
     {1, 5, 6, 7, 0, 0},
-    {1, 5, 6, 7, 0, 0},
-    {1, 7, 7, 8, 0, 0},
     {1, 7, 7, 8, 0, 0},
     {0, 4, 7, 8, 0, 0},
     {4, 5, 6, 8, 0, 0},
     {3, 5, 7, 8, 0, 0},
     {5, 6, 7, 8, 0, 0},
-    {5, 6, 7, 8, 0, 0},
-    {1, 3, 12, 0, 0, 0},
     {1, 3, 12, 0, 0, 0},
     {1, 1, 3, 12, 0, 0},
     {1, 3, 11, 12, 0, 0},
@@ -230,7 +218,7 @@ constexpr int kSpecUpdK[71][6] = {
     {1, 1, 3, 4, 5, 0},
     {1, 1, 4, 5, 6, 0},
 };
-constexpr int kSpecUpdProd[71][6] = {
+constexpr int kSpecUpdProd[67][6] = {
     {1, 0, 0, 0, 0, 0},
     {0, 1, 1, 0, 0, 0},
     {1, 0, 1, 0, 0, 0},
@@ -250,15 +238,11 @@ constexpr int kSpecUpdProd[71][6] = {
     {0, 1, 0, 1, 0, 0},
     {0, 0, 1, 1, 0, 0},
     {1, 0, 1, 0, 0, 0},
-    {1, 0, 1, 0, 0, 0},
-    {1, 0, 0, 1, 0, 0},
     {1, 0, 0, 1, 0, 0},
     {1, 0, 1, 0, 0, 0},
     {0, 1, 1, 0, 0, 0},
     {0, 1, 1, 0, 0, 0},
     {0, 1, 1, 0, 0, 0},
-    {0, 1, 1, 0, 0, 0},
-    {0, 0, 1, 0, 0, 0},
     {0, 0, 1, 0, 0, 0},
     {1, 1, 0, 0, 0, 0},
     {1, 0, 1, 0, 0, 0},
@@ -453,362 +437,335 @@ __device__ __forceinline__ void spec_rhs(S& c) {
   d5 = __dsub_rn(d5, q);
   d6 = __dadd_rn(d6, q);
   d7 = __dsub_rn(d7, q);
-  f = __dmul_rn(__dmul_rn(c.kf(19), z7), z5);
-  b = __dmul_rn(__dmul_rn(c.kr(19), z6), z1);
-  q = __dsub_rn(f, b);
-  d1 = __dadd_rn(d1, q);
-  d5 = __dsub_rn(d5, q);
-  d6 = __dadd_rn(d6, q);
-  d7 = __dsub_rn(d7, q);
-  f = __dmul_rn(__dmul_rn(c.kf(20), z7), z7);
-  b = __dmul_rn(__dmul_rn(c.kr(20), z8), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(19), z7), z7);
+  b = __dmul_rn(__dmul_rn(c.kr(19), z8), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d7 = __dsub_rn(d7, q);
   d7 = __dsub_rn(d7, q);
   d8 = __dadd_rn(d8, q);
-  f = __dmul_rn(__dmul_rn(c.kf(21), z7), z7);
-  b = __dmul_rn(__dmul_rn(c.kr(21), z8), z1);
-  q = __dsub_rn(f, b);
-  d1 = __dadd_rn(d1, q);
-  d7 = __dsub_rn(d7, q);
-  d7 = __dsub_rn(d7, q);
-  d8 = __dadd_rn(d8, q);
-  f = __dmul_rn(__dmul_rn(c.kf(22), z8), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(22), z7), z0);
+  f = __dmul_rn(__dmul_rn(c.kf(20), z8), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(20), z7), z0);
   q = __dsub_rn(f, b);
   d0 = __dadd_rn(d0, q);
   d4 = __dsub_rn(d4, q);
   d7 = __dadd_rn(d7, q);
   d8 = __dsub_rn(d8, q);
-  f = __dmul_rn(__dmul_rn(c.kf(23), z8), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(23), z6), z5);
+  f = __dmul_rn(__dmul_rn(c.kf(21), z8), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(21), z6), z5);
   q = __dsub_rn(f, b);
   d4 = __dsub_rn(d4, q);
   d5 = __dadd_rn(d5, q);
   d6 = __dadd_rn(d6, q);
   d8 = __dsub_rn(d8, q);
-  f = __dmul_rn(__dmul_rn(c.kf(24), z8), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(24), z7), z5);
+  f = __dmul_rn(__dmul_rn(c.kf(22), z8), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(22), z7), z5);
   q = __dsub_rn(f, b);
   d3 = __dsub_rn(d3, q);
   d5 = __dadd_rn(d5, q);
   d7 = __dadd_rn(d7, q);
   d8 = __dsub_rn(d8, q);
-  f = __dmul_rn(__dmul_rn(c.kf(25), z8), z5);
-  b = __dmul_rn(__dmul_rn(c.kr(25), z7), z6);
+  f = __dmul_rn(__dmul_rn(c.kf(23), z8), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(23), z7), z6);
   q = __dsub_rn(f, b);
   d5 = __dsub_rn(d5, q);
   d6 = __dadd_rn(d6, q);
   d7 = __dadd_rn(d7, q);
   d8 = __dsub_rn(d8, q);
-  f = __dmul_rn(__dmul_rn(c.kf(26), z8), z5);
-  b = __dmul_rn(__dmul_rn(c.kr(26), z7), z6);
-  q = __dsub_rn(f, b);
-  d5 = __dsub_rn(d5, q);
-  d6 = __dadd_rn(d6, q);
-  d7 = __dadd_rn(d7, q);
-  d8 = __dsub_rn(d8, q);
-  f = __dmul_rn(__dmul_rn(c.kf(27), z1), z3);
-  b = __dmul_rn(c.kr(27), z12);
+  f = __dmul_rn(__dmul_rn(c.kf(24), z1), z3);
+  b = __dmul_rn(c.kr(24), z12);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d3 = __dsub_rn(d3, q);
   d12 = __dadd_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(28), z1), z3);
-  b = __dmul_rn(c.kr(28), z12);
-  q = __dsub_rn(f, b);
-  d1 = __dsub_rn(d1, q);
-  d3 = __dsub_rn(d3, q);
-  d12 = __dadd_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(29), z12), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(29), z1), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(25), z12), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(25), z1), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d3 = __dsub_rn(d3, q);
   d12 = __dsub_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(30), z12), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(30), z11), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(26), z12), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(26), z11), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d3 = __dsub_rn(d3, q);
   d11 = __dadd_rn(d11, q);
   d12 = __dsub_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(31), z3), z3);
-  b = __dmul_rn(c.kr(31), z11);
+  f = __dmul_rn(__dmul_rn(c.kf(27), z3), z3);
+  b = __dmul_rn(c.kr(27), z11);
   q = __dsub_rn(f, b);
   d3 = __dsub_rn(d3, q);
   d3 = __dsub_rn(d3, q);
   d11 = __dadd_rn(d11, q);
-  f = __dmul_rn(c.kf(32), z11);
-  b = __dmul_rn(c.kr(32), z1);
+  f = __dmul_rn(c.kf(28), z11);
+  b = __dmul_rn(c.kr(28), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d11 = __dsub_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(33), z11), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(33), z1), z3);
+  f = __dmul_rn(__dmul_rn(c.kf(29), z11), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(29), z1), z3);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d3 = __dsub_rn(d3, q);
   d3 = __dadd_rn(d3, q);
   d11 = __dsub_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(34), z11), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(34), z1), z4);
+  f = __dmul_rn(__dmul_rn(c.kf(30), z11), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(30), z1), z4);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d4 = __dsub_rn(d4, q);
   d4 = __dadd_rn(d4, q);
   d11 = __dsub_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(35), z11), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(35), z3), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(31), z11), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(31), z3), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d3 = __dsub_rn(d3, q);
   d3 = __dadd_rn(d3, q);
   d11 = __dsub_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(36), z11), z12);
-  b = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(36), z1), z1), z3);
+  f = __dmul_rn(__dmul_rn(c.kf(32), z11), z12);
+  b = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(32), z1), z1), z3);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d3 = __dadd_rn(d3, q);
   d11 = __dsub_rn(d11, q);
   d12 = __dsub_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(37), z9), z11);
-  b = __dmul_rn(__dmul_rn(c.kr(37), z3), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(33), z9), z11);
+  b = __dmul_rn(__dmul_rn(c.kr(33), z3), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d3 = __dadd_rn(d3, q);
   d9 = __dsub_rn(d9, q);
   d11 = __dsub_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(38), z9), z1);
-  b = __dmul_rn(__dmul_rn(c.kr(38), z3), z11);
+  f = __dmul_rn(__dmul_rn(c.kf(34), z9), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(34), z3), z11);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d3 = __dadd_rn(d3, q);
   d9 = __dsub_rn(d9, q);
   d11 = __dadd_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(39), z9), z1);
-  b = __dmul_rn(__dmul_rn(c.kr(39), z3), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(35), z9), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(35), z3), z1);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d3 = __dadd_rn(d3, q);
   d9 = __dsub_rn(d9, q);
-  f = __dmul_rn(c.kf(40), z9);
-  b = __dmul_rn(c.kr(40), z3);
+  f = __dmul_rn(c.kf(36), z9);
+  b = __dmul_rn(c.kr(36), z3);
   q = __dsub_rn(f, b);
   d3 = __dadd_rn(d3, q);
   d9 = __dsub_rn(d9, q);
-  f = __dmul_rn(__dmul_rn(c.kf(41), z9), z2);
-  b = __dmul_rn(__dmul_rn(c.kr(41), z3), z2);
+  f = __dmul_rn(__dmul_rn(c.kf(37), z9), z2);
+  b = __dmul_rn(__dmul_rn(c.kr(37), z3), z2);
   q = __dsub_rn(f, b);
   d2 = __dsub_rn(d2, q);
   d2 = __dadd_rn(d2, q);
   d3 = __dadd_rn(d3, q);
   d9 = __dsub_rn(d9, q);
-  f = __dmul_rn(__dmul_rn(c.kf(42), z9), z12);
-  b = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(42), z1), z3), z3);
+  f = __dmul_rn(__dmul_rn(c.kf(38), z9), z12);
+  b = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(38), z1), z3), z3);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d3 = __dadd_rn(d3, q);
   d3 = __dadd_rn(d3, q);
   d9 = __dsub_rn(d9, q);
   d12 = __dsub_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(43), z9), z12);
-  b = __dmul_rn(__dmul_rn(c.kr(43), z1), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(39), z9), z12);
+  b = __dmul_rn(__dmul_rn(c.kr(39), z1), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d9 = __dsub_rn(d9, q);
   d12 = __dsub_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(44), z0), z11);
-  b = __dmul_rn(__dmul_rn(c.kr(44), z4), z7);
+  f = __dmul_rn(__dmul_rn(c.kf(40), z0), z11);
+  b = __dmul_rn(__dmul_rn(c.kr(40), z4), z7);
   q = __dsub_rn(f, b);
   d0 = __dsub_rn(d0, q);
   d4 = __dadd_rn(d4, q);
   d7 = __dadd_rn(d7, q);
   d11 = __dsub_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(45), z4), z11);
-  b = __dmul_rn(__dmul_rn(c.kr(45), z5), z3);
+  f = __dmul_rn(__dmul_rn(c.kf(41), z4), z11);
+  b = __dmul_rn(__dmul_rn(c.kr(41), z5), z3);
   q = __dsub_rn(f, b);
   d3 = __dadd_rn(d3, q);
   d4 = __dsub_rn(d4, q);
   d5 = __dadd_rn(d5, q);
   d11 = __dsub_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(46), z4), z11);
-  b = __dmul_rn(c.kr(46), z7);
+  f = __dmul_rn(__dmul_rn(c.kf(42), z4), z11);
+  b = __dmul_rn(c.kr(42), z7);
   q = __dsub_rn(f, b);
   d4 = __dsub_rn(d4, q);
   d7 = __dadd_rn(d7, q);
   d11 = __dsub_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(47), z7), z5);
-  b = __dmul_rn(__dmul_rn(c.kr(47), z6), z11);
+  f = __dmul_rn(__dmul_rn(c.kf(43), z7), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(43), z6), z11);
   q = __dsub_rn(f, b);
   d5 = __dsub_rn(d5, q);
   d6 = __dadd_rn(d6, q);
   d7 = __dsub_rn(d7, q);
   d11 = __dadd_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(48), z5), z11);
-  b = __dmul_rn(__dmul_rn(c.kr(48), z3), z7);
+  f = __dmul_rn(__dmul_rn(c.kf(44), z5), z11);
+  b = __dmul_rn(__dmul_rn(c.kr(44), z3), z7);
   q = __dsub_rn(f, b);
   d3 = __dadd_rn(d3, q);
   d5 = __dsub_rn(d5, q);
   d7 = __dadd_rn(d7, q);
   d11 = __dsub_rn(d11, q);
-  f = __dmul_rn(__dmul_rn(c.kf(49), z12), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(49), z5), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(45), z12), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(45), z5), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d4 = __dsub_rn(d4, q);
   d5 = __dadd_rn(d5, q);
   d12 = __dsub_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(50), z12), z5);
-  b = __dmul_rn(__dmul_rn(c.kr(50), z7), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(46), z12), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(46), z7), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d5 = __dsub_rn(d5, q);
   d7 = __dadd_rn(d7, q);
   d12 = __dsub_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(51), z12), z7);
-  b = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(51), z5), z1), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(47), z12), z7);
+  b = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(47), z5), z1), z1);
   q = __dsub_rn(f, b);
   d1 = __dadd_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d5 = __dadd_rn(d5, q);
   d7 = __dsub_rn(d7, q);
   d12 = __dsub_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(52), z4), z7);
-  b = __dmul_rn(__dmul_rn(c.kr(52), z6), z9);
+  f = __dmul_rn(__dmul_rn(c.kf(48), z4), z7);
+  b = __dmul_rn(__dmul_rn(c.kr(48), z6), z9);
   q = __dsub_rn(f, b);
   d4 = __dsub_rn(d4, q);
   d6 = __dadd_rn(d6, q);
   d7 = __dsub_rn(d7, q);
   d9 = __dadd_rn(d9, q);
-  f = __dmul_rn(__dmul_rn(c.kf(53), z9), z0);
-  b = __dmul_rn(__dmul_rn(c.kr(53), z5), z4);
+  f = __dmul_rn(__dmul_rn(c.kf(49), z9), z0);
+  b = __dmul_rn(__dmul_rn(c.kr(49), z5), z4);
   q = __dsub_rn(f, b);
   d0 = __dsub_rn(d0, q);
   d4 = __dadd_rn(d4, q);
   d5 = __dadd_rn(d5, q);
   d9 = __dsub_rn(d9, q);
-  f = __dmul_rn(__dmul_rn(c.kf(54), z9), z6);
-  b = __dmul_rn(__dmul_rn(c.kr(54), z5), z5);
+  f = __dmul_rn(__dmul_rn(c.kf(50), z9), z6);
+  b = __dmul_rn(__dmul_rn(c.kr(50), z5), z5);
   q = __dsub_rn(f, b);
   d5 = __dadd_rn(d5, q);
   d5 = __dadd_rn(d5, q);
   d6 = __dsub_rn(d6, q);
   d9 = __dsub_rn(d9, q);
-  f = __dmul_rn(__dmul_rn(c.kf(55), z3), z4);
-  b = __dmul_rn(c.kr(55), z10);
+  f = __dmul_rn(__dmul_rn(c.kf(51), z3), z4);
+  b = __dmul_rn(c.kr(51), z10);
   q = __dsub_rn(f, b);
   d3 = __dsub_rn(d3, q);
   d4 = __dsub_rn(d4, q);
   d10 = __dadd_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(56), z10), z1);
-  b = __dmul_rn(__dmul_rn(c.kr(56), z5), z1);
+  f = __dmul_rn(__dmul_rn(c.kf(52), z10), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(52), z5), z1);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d5 = __dadd_rn(d5, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(57), z10), z2);
-  b = __dmul_rn(__dmul_rn(c.kr(57), z5), z2);
+  f = __dmul_rn(__dmul_rn(c.kf(53), z10), z2);
+  b = __dmul_rn(__dmul_rn(c.kr(53), z5), z2);
   q = __dsub_rn(f, b);
   d2 = __dsub_rn(d2, q);
   d2 = __dadd_rn(d2, q);
   d5 = __dadd_rn(d5, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(58), z10), z6);
-  b = __dmul_rn(__dmul_rn(c.kr(58), z5), z6);
+  f = __dmul_rn(__dmul_rn(c.kf(54), z10), z6);
+  b = __dmul_rn(__dmul_rn(c.kr(54), z5), z6);
   q = __dsub_rn(f, b);
   d5 = __dadd_rn(d5, q);
   d6 = __dsub_rn(d6, q);
   d6 = __dadd_rn(d6, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(59), z10), z0);
-  b = __dmul_rn(__dmul_rn(c.kr(59), z5), z0);
+  f = __dmul_rn(__dmul_rn(c.kf(55), z10), z0);
+  b = __dmul_rn(__dmul_rn(c.kr(55), z5), z0);
   q = __dsub_rn(f, b);
   d0 = __dsub_rn(d0, q);
   d0 = __dadd_rn(d0, q);
   d5 = __dadd_rn(d5, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(60), z10), z5);
-  b = __dmul_rn(__dmul_rn(c.kr(60), z5), z5);
+  f = __dmul_rn(__dmul_rn(c.kf(56), z10), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(56), z5), z5);
   q = __dsub_rn(f, b);
   d5 = __dsub_rn(d5, q);
   d5 = __dadd_rn(d5, q);
   d5 = __dadd_rn(d5, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(61), z10), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(61), z5), z4);
+  f = __dmul_rn(__dmul_rn(c.kf(57), z10), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(57), z5), z4);
   q = __dsub_rn(f, b);
   d4 = __dsub_rn(d4, q);
   d4 = __dadd_rn(d4, q);
   d5 = __dadd_rn(d5, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(62), z10), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(62), z5), z3);
+  f = __dmul_rn(__dmul_rn(c.kf(58), z10), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(58), z5), z3);
   q = __dsub_rn(f, b);
   d3 = __dsub_rn(d3, q);
   d3 = __dadd_rn(d3, q);
   d5 = __dadd_rn(d5, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(63), z10), z0);
-  b = __dmul_rn(__dmul_rn(c.kr(63), z6), z4);
+  f = __dmul_rn(__dmul_rn(c.kf(59), z10), z0);
+  b = __dmul_rn(__dmul_rn(c.kr(59), z6), z4);
   q = __dsub_rn(f, b);
   d0 = __dsub_rn(d0, q);
   d4 = __dadd_rn(d4, q);
   d6 = __dadd_rn(d6, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(64), z10), z1);
-  b = __dmul_rn(__dmul_rn(c.kr(64), z12), z4);
+  f = __dmul_rn(__dmul_rn(c.kf(60), z10), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(60), z12), z4);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d4 = __dadd_rn(d4, q);
   d10 = __dsub_rn(d10, q);
   d12 = __dadd_rn(d12, q);
-  f = __dmul_rn(__dmul_rn(c.kf(65), z10), z1);
-  b = __dmul_rn(__dmul_rn(c.kr(65), z7), z3);
+  f = __dmul_rn(__dmul_rn(c.kf(61), z10), z1);
+  b = __dmul_rn(__dmul_rn(c.kr(61), z7), z3);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d3 = __dadd_rn(d3, q);
   d7 = __dadd_rn(d7, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(c.kf(66), z10), z6);
-  b = __dmul_rn(__dmul_rn(c.kr(66), z8), z4);
+  f = __dmul_rn(__dmul_rn(c.kf(62), z10), z6);
+  b = __dmul_rn(__dmul_rn(c.kr(62), z8), z4);
   q = __dsub_rn(f, b);
   d4 = __dadd_rn(d4, q);
   d6 = __dsub_rn(d6, q);
   d8 = __dadd_rn(d8, q);
   d10 = __dsub_rn(d10, q);
-  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(67), z4), z1), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(67), z0), z1);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(63), z4), z1), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(63), z0), z1);
   q = __dsub_rn(f, b);
   d0 = __dadd_rn(d0, q);
   d1 = __dsub_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d4 = __dsub_rn(d4, q);
   d4 = __dsub_rn(d4, q);
-  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(68), z4), z1), z4);
-  b = __dmul_rn(__dmul_rn(c.kr(68), z5), z5);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(64), z4), z1), z4);
+  b = __dmul_rn(__dmul_rn(c.kr(64), z5), z5);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d4 = __dsub_rn(d4, q);
   d4 = __dsub_rn(d4, q);
   d5 = __dadd_rn(d5, q);
   d5 = __dadd_rn(d5, q);
-  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(69), z4), z1), z3);
-  b = __dmul_rn(__dmul_rn(c.kr(69), z5), z1);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(65), z4), z1), z3);
+  b = __dmul_rn(__dmul_rn(c.kr(65), z5), z1);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d1 = __dadd_rn(d1, q);
   d3 = __dsub_rn(d3, q);
   d4 = __dsub_rn(d4, q);
   d5 = __dadd_rn(d5, q);
-  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(70), z4), z1), z5);
-  b = __dmul_rn(__dmul_rn(c.kr(70), z6), z1);
+  f = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(66), z4), z1), z5);
+  b = __dmul_rn(__dmul_rn(c.kr(66), z6), z1);
   q = __dsub_rn(f, b);
   d1 = __dsub_rn(d1, q);
   d1 = __dadd_rn(d1, q);
@@ -1709,37 +1666,37 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kr(22), z7), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(20), z7), msf);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(44), z11), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(40), z11), factor);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(53), z9), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(49), z9), factor);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
+    d = __dmul_rn(__dmul_rn(c.kf(55), z10), factor);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a10 = (LUT)__dsub_rn((double)a10, d);
+    d = __dmul_rn(__dmul_rn(c.kr(55), z5), msf);
+    a0 = (LUT)__dsub_rn((double)a0, d);
+    a0 = (LUT)__dadd_rn((double)a0, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    a10 = (LUT)__dsub_rn((double)a10, d);
     d = __dmul_rn(__dmul_rn(c.kf(59), z10), factor);
-    a0 = (LUT)__dsub_rn((double)a0, d);
-    a0 = (LUT)__dadd_rn((double)a0, d);
-    a5 = (LUT)__dadd_rn((double)a5, d);
-    a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(59), z5), msf);
-    a0 = (LUT)__dsub_rn((double)a0, d);
-    a0 = (LUT)__dadd_rn((double)a0, d);
-    a5 = (LUT)__dadd_rn((double)a5, d);
-    a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(63), z10), factor);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(67), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(63), z1), msf);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
@@ -1779,189 +1736,175 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kr(19), z6), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a5 = (LUT)__dsub_rn((double)a5, d);
-    a6 = (LUT)__dadd_rn((double)a6, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kr(20), z8), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(19), z8), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a8 = (LUT)__dadd_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(21), z8), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    a8 = (LUT)__dadd_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(27), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(24), z3), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a12 = (LUT)__dadd_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(28), z3), factor);
-    a1 = (LUT)__dsub_rn((double)a1, d);
-    a3 = (LUT)__dsub_rn((double)a3, d);
-    a12 = (LUT)__dadd_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(29), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(25), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(29), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(25), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(30), z11), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(26), z11), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(c.kr(32), msf);
+    d = __dmul_rn(c.kr(28), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kr(29), z3), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kr(30), z4), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a4 = (LUT)__dadd_rn((double)a4, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kr(31), z3), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(32), z1), z3), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(32), z1), z3), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
     d = __dmul_rn(__dmul_rn(c.kr(33), z3), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
-    a3 = (LUT)__dsub_rn((double)a3, d);
-    a3 = (LUT)__dadd_rn((double)a3, d);
-    a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(34), z4), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a4 = (LUT)__dsub_rn((double)a4, d);
-    a4 = (LUT)__dadd_rn((double)a4, d);
-    a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(35), z3), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a3 = (LUT)__dsub_rn((double)a3, d);
-    a3 = (LUT)__dadd_rn((double)a3, d);
-    a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(36), z1), z3), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a3 = (LUT)__dadd_rn((double)a3, d);
-    a11 = (LUT)__dsub_rn((double)a11, d);
-    a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(36), z1), z3), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a3 = (LUT)__dadd_rn((double)a3, d);
-    a11 = (LUT)__dsub_rn((double)a11, d);
-    a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(37), z3), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(38), z9), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(34), z9), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(39), z9), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(35), z9), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kr(39), z3), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(35), z3), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(42), z3), z3), msf);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(38), z3), z3), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(43), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(39), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(43), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(39), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(49), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(45), z5), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(50), z7), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(46), z7), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(51), z5), z1), msf);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(47), z5), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(51), z5), z1), msf);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(47), z5), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(56), z10), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(52), z10), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(56), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(52), z5), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(64), z10), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(60), z10), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
     a12 = (LUT)__dadd_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(65), z10), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(61), z10), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(67), z4), z4), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(63), z4), z4), factor);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
-    d = __dmul_rn(__dmul_rn(c.kr(67), z0), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(63), z0), msf);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(68), z4), z4), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(64), z4), z4), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(69), z4), z3), factor);
-    a1 = (LUT)__dsub_rn((double)a1, d);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a3 = (LUT)__dsub_rn((double)a3, d);
-    a4 = (LUT)__dsub_rn((double)a4, d);
-    a5 = (LUT)__dadd_rn((double)a5, d);
-    d = __dmul_rn(__dmul_rn(c.kr(69), z5), msf);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(65), z4), z3), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(70), z4), z5), factor);
+    d = __dmul_rn(__dmul_rn(c.kr(65), z5), msf);
+    a1 = (LUT)__dsub_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a4 = (LUT)__dsub_rn((double)a4, d);
+    a5 = (LUT)__dadd_rn((double)a5, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(66), z4), z5), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
-    d = __dmul_rn(__dmul_rn(c.kr(70), z6), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(66), z6), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
@@ -1985,22 +1928,22 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
     a2 = (LUT)__dadd_rn((double)a2, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
-    d = __dmul_rn(__dmul_rn(c.kf(41), z9), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(37), z9), factor);
     a2 = (LUT)__dsub_rn((double)a2, d);
     a2 = (LUT)__dadd_rn((double)a2, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kr(41), z3), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(37), z3), msf);
     a2 = (LUT)__dsub_rn((double)a2, d);
     a2 = (LUT)__dadd_rn((double)a2, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kf(57), z10), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(53), z10), factor);
     a2 = (LUT)__dsub_rn((double)a2, d);
     a2 = (LUT)__dadd_rn((double)a2, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(57), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(53), z5), msf);
     a2 = (LUT)__dsub_rn((double)a2, d);
     a2 = (LUT)__dadd_rn((double)a2, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
@@ -2048,128 +1991,124 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
     a4 = (LUT)__dadd_rn((double)a4, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kf(24), z8), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(22), z8), factor);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(27), z1), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(24), z1), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a12 = (LUT)__dadd_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(28), z1), factor);
-    a1 = (LUT)__dsub_rn((double)a1, d);
-    a3 = (LUT)__dsub_rn((double)a3, d);
-    a12 = (LUT)__dadd_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(29), z12), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(25), z12), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(30), z12), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(26), z12), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(31), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(27), z3), factor);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(31), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(27), z3), factor);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(33), z11), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(29), z11), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kr(29), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kf(31), z11), factor);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(c.kr(31), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dsub_rn((double)a3, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(32), z1), z1), msf);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a1 = (LUT)__dadd_rn((double)a1, d);
+    a3 = (LUT)__dadd_rn((double)a3, d);
+    a11 = (LUT)__dsub_rn((double)a11, d);
+    a12 = (LUT)__dsub_rn((double)a12, d);
     d = __dmul_rn(__dmul_rn(c.kr(33), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
-    a3 = (LUT)__dsub_rn((double)a3, d);
-    a3 = (LUT)__dadd_rn((double)a3, d);
-    a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(35), z11), factor);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a3 = (LUT)__dsub_rn((double)a3, d);
-    a3 = (LUT)__dadd_rn((double)a3, d);
-    a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(35), z1), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a3 = (LUT)__dsub_rn((double)a3, d);
-    a3 = (LUT)__dadd_rn((double)a3, d);
-    a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(36), z1), z1), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a3 = (LUT)__dadd_rn((double)a3, d);
-    a11 = (LUT)__dsub_rn((double)a11, d);
-    a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(37), z1), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(38), z11), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(34), z11), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(39), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(35), z1), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(c.kr(40), msf);
+    d = __dmul_rn(c.kr(36), msf);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kr(41), z2), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(37), z2), msf);
     a2 = (LUT)__dsub_rn((double)a2, d);
     a2 = (LUT)__dadd_rn((double)a2, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(42), z1), z3), msf);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(38), z1), z3), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(42), z1), z3), msf);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(38), z1), z3), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(45), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(41), z5), msf);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(48), z7), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(44), z7), msf);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(55), z4), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(51), z4), factor);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a10 = (LUT)__dadd_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(62), z10), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(58), z10), factor);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(62), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(58), z5), msf);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(65), z7), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(61), z7), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(69), z4), z1), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(65), z4), z1), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
@@ -2285,115 +2224,115 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kf(22), z8), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(20), z8), factor);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(23), z8), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(21), z8), factor);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(34), z11), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(30), z11), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(34), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(30), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(44), z7), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(40), z7), msf);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(45), z11), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(41), z11), factor);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(46), z11), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(42), z11), factor);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(49), z12), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(45), z12), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(52), z7), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(48), z7), factor);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a9 = (LUT)__dadd_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kr(53), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(49), z5), msf);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kf(55), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(51), z3), factor);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a10 = (LUT)__dadd_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(61), z10), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(57), z10), factor);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(61), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(57), z5), msf);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(63), z6), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(59), z6), msf);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(64), z12), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(60), z12), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
     a12 = (LUT)__dadd_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(66), z8), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(62), z8), msf);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a8 = (LUT)__dadd_rn((double)a8, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(67), z1), z4), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(63), z1), z4), factor);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(67), z4), z1), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(63), z4), z1), factor);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(68), z1), z4), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(64), z1), z4), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(68), z4), z1), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(64), z4), z1), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(69), z1), z3), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(65), z1), z3), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(70), z1), z5), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(66), z1), z5), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
@@ -2472,141 +2411,131 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kf(19), z7), factor);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a5 = (LUT)__dsub_rn((double)a5, d);
-    a6 = (LUT)__dadd_rn((double)a6, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kr(23), z6), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(21), z6), msf);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(24), z7), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(22), z7), msf);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(25), z8), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(23), z8), factor);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(26), z8), factor);
-    a5 = (LUT)__dsub_rn((double)a5, d);
-    a6 = (LUT)__dadd_rn((double)a6, d);
-    a7 = (LUT)__dadd_rn((double)a7, d);
-    a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(45), z3), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(41), z3), msf);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(47), z7), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(43), z7), factor);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(48), z11), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(44), z11), factor);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(49), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(45), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(50), z12), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(46), z12), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(51), z1), z1), msf);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kr(47), z1), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(53), z4), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(49), z4), msf);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kr(54), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(50), z5), msf);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kr(54), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(50), z5), msf);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kr(56), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(52), z1), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(57), z2), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(53), z2), msf);
     a2 = (LUT)__dsub_rn((double)a2, d);
     a2 = (LUT)__dadd_rn((double)a2, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(58), z6), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(54), z6), msf);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(59), z0), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(55), z0), msf);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(60), z10), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(56), z10), factor);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(60), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(56), z5), msf);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(60), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(56), z5), msf);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(61), z4), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(57), z4), msf);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(62), z3), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(58), z3), msf);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(68), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(64), z5), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
-    d = __dmul_rn(__dmul_rn(c.kr(68), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(64), z5), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
-    d = __dmul_rn(__dmul_rn(c.kr(69), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(65), z1), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
-    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(70), z4), z1), factor);
+    d = __dmul_rn(__dmul_rn(__dmul_rn(c.kf(66), z4), z1), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
@@ -2660,62 +2589,52 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kr(19), z1), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a5 = (LUT)__dsub_rn((double)a5, d);
-    a6 = (LUT)__dadd_rn((double)a6, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kr(23), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(21), z5), msf);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(25), z7), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(23), z7), msf);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(26), z7), msf);
-    a5 = (LUT)__dsub_rn((double)a5, d);
-    a6 = (LUT)__dadd_rn((double)a6, d);
-    a7 = (LUT)__dadd_rn((double)a7, d);
-    a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(47), z11), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(43), z11), msf);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(52), z9), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(48), z9), msf);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a9 = (LUT)__dadd_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kf(54), z9), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(50), z9), factor);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kf(58), z10), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(54), z10), factor);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(58), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(54), z5), msf);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(63), z4), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(59), z4), msf);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(66), z10), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(62), z10), factor);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a8 = (LUT)__dadd_rn((double)a8, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kr(70), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(66), z1), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
@@ -2756,87 +2675,67 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kf(19), z5), factor);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a5 = (LUT)__dsub_rn((double)a5, d);
-    a6 = (LUT)__dadd_rn((double)a6, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    d = __dmul_rn(__dmul_rn(c.kf(20), z7), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(19), z7), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a8 = (LUT)__dadd_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(20), z7), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(19), z7), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a8 = (LUT)__dadd_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(21), z7), factor);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    a8 = (LUT)__dadd_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(21), z7), factor);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    a8 = (LUT)__dadd_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(22), z0), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(20), z0), msf);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(24), z5), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(22), z5), msf);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(25), z6), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(23), z6), msf);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(26), z6), msf);
-    a5 = (LUT)__dsub_rn((double)a5, d);
-    a6 = (LUT)__dadd_rn((double)a6, d);
-    a7 = (LUT)__dadd_rn((double)a7, d);
-    a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(44), z4), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(40), z4), msf);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(c.kr(46), msf);
+    d = __dmul_rn(c.kr(42), msf);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(47), z5), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(43), z5), factor);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(48), z3), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(44), z3), msf);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(50), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(46), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(51), z12), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(47), z12), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(52), z4), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(48), z4), factor);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a9 = (LUT)__dadd_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kr(65), z3), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(61), z3), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
@@ -2851,42 +2750,32 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(20), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(19), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a8 = (LUT)__dadd_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(21), z1), msf);
-    a1 = (LUT)__dadd_rn((double)a1, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    a7 = (LUT)__dsub_rn((double)a7, d);
-    a8 = (LUT)__dadd_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(22), z4), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(20), z4), factor);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(23), z4), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(21), z4), factor);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(24), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(22), z3), factor);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(25), z5), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(23), z5), factor);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kf(26), z5), factor);
-    a5 = (LUT)__dsub_rn((double)a5, d);
-    a6 = (LUT)__dadd_rn((double)a6, d);
-    a7 = (LUT)__dadd_rn((double)a7, d);
-    a8 = (LUT)__dsub_rn((double)a8, d);
-    d = __dmul_rn(__dmul_rn(c.kr(66), z4), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(62), z4), msf);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a8 = (LUT)__dadd_rn((double)a8, d);
@@ -2897,51 +2786,51 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
   if constexpr (J == 9) {
     const double z0 = c.z(0), z1 = c.z(1), z2 = c.z(2), z6 = c.z(6), z11 = c.z(11), z12 = c.z(12);
     LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0;
-    d = __dmul_rn(__dmul_rn(c.kf(37), z11), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(33), z11), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(38), z1), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(34), z1), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(39), z1), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(35), z1), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(c.kf(40), factor);
+    d = __dmul_rn(c.kf(36), factor);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kf(41), z2), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(37), z2), factor);
     a2 = (LUT)__dsub_rn((double)a2, d);
     a2 = (LUT)__dadd_rn((double)a2, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kf(42), z12), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(38), z12), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(43), z12), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(39), z12), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(52), z6), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(48), z6), msf);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a9 = (LUT)__dadd_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kf(53), z0), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(49), z0), factor);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
-    d = __dmul_rn(__dmul_rn(c.kf(54), z6), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(50), z6), factor);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
@@ -2952,61 +2841,61 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
   if constexpr (J == 10) {
     const double z0 = c.z(0), z1 = c.z(1), z2 = c.z(2), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6);
     LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0;
-    d = __dmul_rn(c.kr(55), msf);
+    d = __dmul_rn(c.kr(51), msf);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a10 = (LUT)__dadd_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(56), z1), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(52), z1), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(57), z2), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(53), z2), factor);
     a2 = (LUT)__dsub_rn((double)a2, d);
     a2 = (LUT)__dadd_rn((double)a2, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(58), z6), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(54), z6), factor);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(59), z0), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(55), z0), factor);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a0 = (LUT)__dadd_rn((double)a0, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(60), z5), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(56), z5), factor);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(61), z4), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(57), z4), factor);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(62), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(58), z3), factor);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(63), z0), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(59), z0), factor);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(64), z1), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(60), z1), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
     a12 = (LUT)__dadd_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(65), z1), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(61), z1), factor);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a10 = (LUT)__dsub_rn((double)a10, d);
-    d = __dmul_rn(__dmul_rn(c.kf(66), z6), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(62), z6), factor);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a6 = (LUT)__dsub_rn((double)a6, d);
     a8 = (LUT)__dadd_rn((double)a8, d);
@@ -3017,69 +2906,69 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
   if constexpr (J == 11) {
     const double z0 = c.z(0), z1 = c.z(1), z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z6 = c.z(6), z9 = c.z(9), z12 = c.z(12);
     LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0;
-    d = __dmul_rn(__dmul_rn(c.kr(30), z1), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(26), z1), msf);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(c.kr(31), msf);
+    d = __dmul_rn(c.kr(27), msf);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(c.kf(32), factor);
+    d = __dmul_rn(c.kf(28), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(33), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(29), z3), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(34), z4), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(30), z4), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(35), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(31), z3), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(36), z12), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(32), z12), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(37), z9), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(33), z9), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(38), z3), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(34), z3), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(44), z0), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(40), z0), factor);
     a0 = (LUT)__dsub_rn((double)a0, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(45), z4), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(41), z4), factor);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(46), z4), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(42), z4), factor);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kr(47), z6), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(43), z6), msf);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a6 = (LUT)__dadd_rn((double)a6, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
-    d = __dmul_rn(__dmul_rn(c.kf(48), z5), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(44), z5), factor);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
@@ -3090,58 +2979,54 @@ __device__ __forceinline__ void spec_column(const S& c, double factor, LUT (&v)[
   if constexpr (J == 12) {
     const double z3 = c.z(3), z4 = c.z(4), z5 = c.z(5), z7 = c.z(7), z9 = c.z(9), z11 = c.z(11);
     LUT a0 = (LUT)0, a1 = (LUT)0, a2 = (LUT)0, a3 = (LUT)0, a4 = (LUT)0, a5 = (LUT)0, a6 = (LUT)0, a7 = (LUT)0, a8 = (LUT)0, a9 = (LUT)0, a10 = (LUT)0, a11 = (LUT)0, a12 = (LUT)0;
-    d = __dmul_rn(c.kr(27), msf);
+    d = __dmul_rn(c.kr(24), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a12 = (LUT)__dadd_rn((double)a12, d);
-    d = __dmul_rn(c.kr(28), msf);
-    a1 = (LUT)__dsub_rn((double)a1, d);
-    a3 = (LUT)__dsub_rn((double)a3, d);
-    a12 = (LUT)__dadd_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(29), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(25), z3), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(30), z3), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(26), z3), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dsub_rn((double)a3, d);
     a11 = (LUT)__dadd_rn((double)a11, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(36), z11), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(32), z11), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a11 = (LUT)__dsub_rn((double)a11, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(42), z9), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(38), z9), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a3 = (LUT)__dadd_rn((double)a3, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(43), z9), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(39), z9), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a9 = (LUT)__dsub_rn((double)a9, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(49), z4), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(45), z4), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a4 = (LUT)__dsub_rn((double)a4, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(50), z5), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(46), z5), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dsub_rn((double)a5, d);
     a7 = (LUT)__dadd_rn((double)a7, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kf(51), z7), factor);
+    d = __dmul_rn(__dmul_rn(c.kf(47), z7), factor);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a1 = (LUT)__dadd_rn((double)a1, d);
     a5 = (LUT)__dadd_rn((double)a5, d);
     a7 = (LUT)__dsub_rn((double)a7, d);
     a12 = (LUT)__dsub_rn((double)a12, d);
-    d = __dmul_rn(__dmul_rn(c.kr(64), z4), msf);
+    d = __dmul_rn(__dmul_rn(c.kr(60), z4), msf);
     a1 = (LUT)__dsub_rn((double)a1, d);
     a4 = (LUT)__dadd_rn((double)a4, d);
     a10 = (LUT)__dsub_rn((double)a10, d);

@@ -24,7 +24,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 # as kMergeUpTo in csrc/chem_device.cuh
-MERGE_UP_TO = 8
+MERGE_UP_TO = 16
 
 
 def reduced_structure(t: dict, full: bool = False):
