@@ -511,7 +511,7 @@ def time_diffusivity(solver, tables, args, dev, field, T, Y) -> dict:
     return {"ms": ms, "cells_per_s": n / (ms * 1e-3), "bytes_per_cell": bpc,
             "algorithmic_GB_s": bpc * n / (ms * 1e-3) * 1e-9, "pairs_per_cell": N * (N - 1) // 2,
             "what": "nrg_mixture_diffusivity_device: Chapman-Enskog binary coefficients (Neufeld collision "
-                    "integral: one pow and three exp per species pair) and the mixture-averaged coefficient "
+                    "integral: one pow per cell, up to three exp per distinct pair scale) and the mixture-averaged coefficient "
                     "of every species, every cell of the field"}
 
 
