@@ -395,6 +395,9 @@ NRG_API int nrg_surrogate_prepare(nrg_chem* h, long n, long ld, double dt, const
 NRG_API int nrg_surrogate_features(nrg_chem* h, long n, long ld, double dt, const double* dt_cells,
                                    const double* T, const double* rho, const double* Y, float* xraw,
                                    void* x_bf16);
+/* Device arrays x_bf16 (n x 16), y (n x 10) and out (n x 16) of these calls may
+ * start at any element: rows off a 16-byte boundary go through a buffer of
+ * the library. */
 NRG_API int nrg_surrogate_forward(nrg_chem* h, long n, const void* x_bf16, float* out);
 /* Mean-squared-error gradient over n rows into host memory (no update). */
 NRG_API int nrg_surrogate_grad(nrg_chem* h, long n, const void* x_bf16, const float* y, float* grads_host,

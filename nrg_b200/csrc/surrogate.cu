@@ -312,18 +312,26 @@ __global__ void k_to_bf16(long n, const float* x, __nv_bfloat16* y) {
     y[i] = __float2bfloat16(x[i]);
 }
 
+// The contraction copies its operands and stores its result in 16-byte pieces.
+// A caller's array may start at any element.
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 // Rows idx[0..nb) of X (32 bytes each) and Y (40 bytes): a thread per 16-byte or
-// 4-byte piece.
+// 4-byte piece.  vec: X starts on a 16-byte boundary.
 __global__ void k_gather_rows(long nb, const int* idx, const __nv_bfloat16* X, const float* Y,
-                              __nv_bfloat16* Xb, float* Yb) {
+                              __nv_bfloat16* Xb, float* Yb, bool vec) {
   constexpr int kPieces = 2 + kMlpOut;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nb * kPieces; i += (long)gridDim.x * blockDim.x) {
     const long b = i / kPieces, r = idx[b];
     const int q = (int)(i % kPieces);
-    if (q < 2)
-      reinterpret_cast<uint4*>(Xb + b * kMlpInPad)[q] = reinterpret_cast<const uint4*>(X + r * kMlpInPad)[q];
-    else
+    if (q >= 2) {
       Yb[b * kMlpOut + q - 2] = Y[r * kMlpOut + q - 2];
+    } else if (vec) {
+      reinterpret_cast<uint4*>(Xb + b * kMlpInPad)[q] = reinterpret_cast<const uint4*>(X + r * kMlpInPad)[q];
+    } else {
+#pragma unroll
+      for (int j = 8 * q; j < 8 * q + 8; ++j) Xb[b * kMlpInPad + j] = X[r * kMlpInPad + j];
+    }
   }
 }
 
@@ -1474,11 +1482,25 @@ static cudaError_t forward(Surrogate* s, long n, const __nv_bfloat16* x, float* 
   return cudaSuccess;
 }
 
+// The caller's n rows of features as the contraction can read them: where they
+// are, or copied to the library's own (aligned) buffer.
+static std::string aligned_rows(Surrogate* s, long n, const __nv_bfloat16** x, cudaStream_t st) {
+  if (aligned16(*x)) return "";
+  const std::string e = ck(cudaMemcpyAsync(s->X, *x, n * kMlpInPad * 2, cudaMemcpyDeviceToDevice, st), "copy X");
+  *x = s->X;
+  return e;
+}
+
 std::string surrogate_forward(Surrogate* s, long n, const __nv_bfloat16* x, float* out, cudaStream_t st) {
   std::string e = ensure_act(s, n);
   if (!e.empty()) return e;
-  e = ck(forward(s, n, x, out, st), "forward");
+  if ((e = aligned_rows(s, n, &x, st)).size()) return e;
+  float* res = aligned16(out) ? out : s->O;
+  e = ck(forward(s, n, x, res, st), "forward");
   if (!e.empty()) return e;
+  if (res != out &&
+      (e = ck(cudaMemcpyAsync(out, res, n * kMlpOutPad * 4, cudaMemcpyDeviceToDevice, st), "copy out")).size())
+    return e;
   return ck(cudaStreamSynchronize(st), "forward");
 }
 
@@ -1538,6 +1560,7 @@ std::string surrogate_grad(Surrogate* s, long n, const __nv_bfloat16* x, const f
                            double* loss, cudaStream_t st) {
   std::string e = ensure_act(s, n);
   if (!e.empty()) return e;
+  if ((e = aligned_rows(s, n, &x, st)).size()) return e;
   cudaMemsetAsync(s->d_loss, 0, sizeof(double), st);
   if ((e = ck(backward(s, n, x, y, st), "backward")).size()) return e;
   if (grads_host) cudaMemcpyAsync(grads_host, s->gr, s->n_params * 4, cudaMemcpyDeviceToHost, st);
@@ -1571,7 +1594,8 @@ std::string surrogate_train(Surrogate* s, long n, const __nv_bfloat16* x, const 
     const int* cur = d_perm + (ep & 1) * n;
     cudaMemsetAsync(s->d_loss, 0, sizeof(double), st);
     for (long it = 0; it < steps; ++it) {
-      k_gather_rows<<<(batch * 12 + 255) / 256, 256, 0, st>>>(batch, cur + it * batch, x, y, Xb, s->Yb);
+      k_gather_rows<<<(batch * 12 + 255) / 256, 256, 0, st>>>(batch, cur + it * batch, x, y, Xb, s->Yb,
+                                                              aligned16(x));
       cudaError_t ce = backward(s, batch, Xb, s->Yb, st);
       if (ce != cudaSuccess) {
         cudaFree(d_perm);
