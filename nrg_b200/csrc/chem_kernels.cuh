@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(BS, BS > 128 ? 1 : 256 / BS) k_chem_pass(StepA
       if (a.dt_cells) res.tout = a.dt_cells[cid];
     }
     if constexpr (TM) pass_rates_to_tm<N>(st);
+    else __syncwarp();  // the set-up scratch covers other lanes' factors when these are floats
     const int status = pass_integrate<N, R, NF, SPEC, LOCK>(st, a, live, res.tout, res.y, v);
     if (live) {
       cell_finish<N, kJacAnalytic>(res, a, cid, status);
@@ -197,6 +198,7 @@ __global__ void __launch_bounds__(BS, BS > 128 ? 1 : 256 / BS) k_chem_pass(StepA
       v[kCntBad] += status != kCellOk;
     }
     if (!QUEUE) break;
+    __syncwarp();  // the factors of this group, before the next group's set-up scratch
   }
   if constexpr (TM) {
     __syncthreads();
