@@ -41,7 +41,9 @@ struct nrg_chem {
   nrg::Mechanism mech;
   DevMech dm;   // tables over all species
   DevMech dmr;  // reaction lists over the reacting species (fast / mixed thread kernels)
-  int spec = 0;  // generated mechanism-specialised RHS / iteration matrix in use (0: tables)
+  // generated mechanism-specialised code in use (0: tables): right-hand side and
+  // iteration matrix over the reacting species, right-hand side over all (reference mode)
+  int spec = 0, spec_full = 0;
   bool has_transport = false;
   nrg::DiffusivityArgs diff;  // pair tables of the loaded transport deck
   int device = 0;
@@ -527,6 +529,7 @@ int ensure_staging(nrg_chem* h, size_t n) {
 }
 
 int jac_of(int mode) { return mode == NRG_MODE_REFERENCE ? 0 : 1; }
+int spec_of(const nrg_chem* h) { return h->mode == NRG_MODE_REFERENCE ? h->spec_full : h->spec; }
 
 // Enqueue the plain integrator (no surrogate) on stream s.
 cudaError_t enqueue_integrator(nrg_chem* h, const StepArgs& a, const LaunchCfg& cfg, cudaStream_t s) {
@@ -551,7 +554,7 @@ cudaError_t enqueue_integrator(nrg_chem* h, const StepArgs& a, const LaunchCfg& 
     b.n_list = (int)a.n;
     b.n_list_dev = nullptr;
   }
-  return nrg::launch_chem(h->mech.n(), h->dmr.NI, h->spec, h->mech.r(), jac_of(h->mode), h->mode == NRG_MODE_MIXED, b, c,
+  return nrg::launch_chem(h->mech.n(), h->dmr.NI, spec_of(h), h->mech.r(), jac_of(h->mode), h->mode == NRG_MODE_MIXED, b, c,
                           h->d_queue, h->d_counters, s);
 }
 
@@ -775,7 +778,8 @@ extern "C" int nrg_chem_create(const char* mechanism_path, const char* thermo_pa
     return fail(nullptr, NRG_ERR_CUDA, msg);
   }
   reduce_dev_mech(h->dm, &h->dmr);
-  h->spec = nrg::match_specialised(h->dmr, h->dm);
+  h->spec = nrg::match_specialised(h->dmr);
+  h->spec_full = nrg::match_specialised_full(h->dm);
   for (int i = 0; i < nrg::kMaxNets; ++i) h->sur_net[i] = nrg::surrogate_create(h->dm);
   if ((ce = use_tables(h)) != cudaSuccess) {
     std::string msg = std::string("mechanism upload failed: ") + cudaGetErrorString(ce);
@@ -835,10 +839,11 @@ extern "C" int nrg_chem_set_mode(nrg_chem* h, int mode) {
 
 extern "C" int nrg_chem_set_specialised(nrg_chem* h, int enable) {
   if (!h) return NRG_ERR_ARG;
-  const int id = nrg::match_specialised(h->dmr, h->dm);
+  const int id = nrg::match_specialised(h->dmr);  // full lists that match reduce to lists that match
   if (enable && id == 0)
     return fail(h, NRG_ERR_UNSUPPORTED, "the mechanism matches none of the generated specialised codes");
   h->spec = enable ? id : 0;
+  h->spec_full = enable ? nrg::match_specialised_full(h->dm) : 0;
   return NRG_OK;
 }
 
@@ -2030,7 +2035,7 @@ extern "C" int nrg_chem_step_device_noalloc(nrg_chem* h, double time_step, long 
   fa.n_list_dev = n_list;
   LaunchCfg cfg = h->cfg;
   if (cfg.kernel == nrg::kKernelThreadQueue && cfg.grid <= 0) cfg.grid = h->num_sms;
-  const cudaError_t le = nrg::launch_chem(h->mech.n(), h->dmr.NI, h->spec, h->mech.r(), jac_of(h->mode), h->mode == NRG_MODE_MIXED,
+  const cudaError_t le = nrg::launch_chem(h->mech.n(), h->dmr.NI, spec_of(h), h->mech.r(), jac_of(h->mode), h->mode == NRG_MODE_MIXED,
                                           fa, cfg, queue, counters, s);
   if (le != cudaSuccess) return cuda_fail(h, le, "no-allocation integrator launch");
   CK(h, cudaEventRecord(h->ev1, s));

@@ -232,7 +232,8 @@ bool supported_mechanism(int n_species, int n_reactions) {
          (n_species == 17 && n_reactions == 25);
 }
 
-int match_specialised(const DevMech& reduced, const DevMech& full) { return match_specialised_tables(reduced, full); }
+int match_specialised(const DevMech& reduced) { return match_specialised_tables(reduced); }
+int match_specialised_full(const DevMech& full) { return match_specialised_full_tables(full); }
 
 int smem_bytes_per_cell(int n_species, int n_reactions, bool mixed) {
   if (n_species == 9 && n_reactions == 24)

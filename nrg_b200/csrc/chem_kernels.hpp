@@ -79,8 +79,10 @@ void upload_mechanism(const DevMech& full, const DevMech& reduced, cudaStream_t 
 // (13, 71) (thread-per-cell grid, reference and analytic-Jacobian modes).
 bool supported_mechanism(int n_species, int n_reactions);
 // The number (1..) of the generated mechanism-specialised code whose reaction
-// lists equal the reduced and the full ones, 0 when none does.
-int match_specialised(const DevMech& reduced, const DevMech& full);
+// lists equal the reduced ones (fast and mixed modes) or the full ones
+// (reference mode), 0 when none does.
+int match_specialised(const DevMech& reduced);
+int match_specialised_full(const DevMech& full);
 cudaError_t launch_chem(int n_species, int n_int, int spec, int n_reactions, int jac, bool mixed, const StepArgs& a,
                         const LaunchCfg& cfg, int* queue, unsigned long long* counters,
                         cudaStream_t s);

@@ -84,10 +84,10 @@ struct SpecOf<kSpecAcetylene> {
   }
 };
 
-// 0 when the reaction lists, reduced or full, match none of the generated codes.
+// 0 when the reduced reaction lists match none of the generated codes.
 template <class M>
-inline int match_specialised_tables(const M& m, const M& full) {
-  if (m.NI == gen_keromnes::kSpecN && m.RM == gen_keromnes::kSpecR && full.N == gen_keromnes::kFullN && full.R == gen_keromnes::kFullR) {
+inline int match_specialised_tables(const M& m) {
+  if (m.NI == gen_keromnes::kSpecN && m.RM == gen_keromnes::kSpecR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_keromnes::kSpecNupd[r];
@@ -96,16 +96,9 @@ inline int match_specialised_tables(const M& m, const M& full) {
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_keromnes::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_keromnes::kSpecUpdProd[r][u];
     }
-    for (int r = 0; ok && r < full.R; ++r) {
-      ok = full.nupd[r] == gen_keromnes::kFullNupd[r];
-      for (int i = 0; ok && i < 3; ++i)
-        ok = full.left[r][i] == gen_keromnes::kFullLeft[r][i] && full.right[r][i] == gen_keromnes::kFullRight[r][i];
-      for (int u = 0; ok && u < full.nupd[r]; ++u)
-        ok = full.upd_k[r][u] == gen_keromnes::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_keromnes::kFullUpdProd[r][u];
-    }
     if (ok) return kSpecKeromnes;
   }
-  if (m.NI == gen_zhang::kSpecN && m.RM == gen_zhang::kSpecR && full.N == gen_zhang::kFullN && full.R == gen_zhang::kFullR) {
+  if (m.NI == gen_zhang::kSpecN && m.RM == gen_zhang::kSpecR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_zhang::kSpecNupd[r];
@@ -114,16 +107,9 @@ inline int match_specialised_tables(const M& m, const M& full) {
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_zhang::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_zhang::kSpecUpdProd[r][u];
     }
-    for (int r = 0; ok && r < full.R; ++r) {
-      ok = full.nupd[r] == gen_zhang::kFullNupd[r];
-      for (int i = 0; ok && i < 3; ++i)
-        ok = full.left[r][i] == gen_zhang::kFullLeft[r][i] && full.right[r][i] == gen_zhang::kFullRight[r][i];
-      for (int u = 0; ok && u < full.nupd[r]; ++u)
-        ok = full.upd_k[r][u] == gen_zhang::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_zhang::kFullUpdProd[r][u];
-    }
     if (ok) return kSpecZhang;
   }
-  if (m.NI == gen_tereza::kSpecN && m.RM == gen_tereza::kSpecR && full.N == gen_tereza::kFullN && full.R == gen_tereza::kFullR) {
+  if (m.NI == gen_tereza::kSpecN && m.RM == gen_tereza::kSpecR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_tereza::kSpecNupd[r];
@@ -132,16 +118,9 @@ inline int match_specialised_tables(const M& m, const M& full) {
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_tereza::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_tereza::kSpecUpdProd[r][u];
     }
-    for (int r = 0; ok && r < full.R; ++r) {
-      ok = full.nupd[r] == gen_tereza::kFullNupd[r];
-      for (int i = 0; ok && i < 3; ++i)
-        ok = full.left[r][i] == gen_tereza::kFullLeft[r][i] && full.right[r][i] == gen_tereza::kFullRight[r][i];
-      for (int u = 0; ok && u < full.nupd[r]; ++u)
-        ok = full.upd_k[r][u] == gen_tereza::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_tereza::kFullUpdProd[r][u];
-    }
     if (ok) return kSpecTereza;
   }
-  if (m.NI == gen_konnov::kSpecN && m.RM == gen_konnov::kSpecR && full.N == gen_konnov::kFullN && full.R == gen_konnov::kFullR) {
+  if (m.NI == gen_konnov::kSpecN && m.RM == gen_konnov::kSpecR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_konnov::kSpecNupd[r];
@@ -150,16 +129,9 @@ inline int match_specialised_tables(const M& m, const M& full) {
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_konnov::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_konnov::kSpecUpdProd[r][u];
     }
-    for (int r = 0; ok && r < full.R; ++r) {
-      ok = full.nupd[r] == gen_konnov::kFullNupd[r];
-      for (int i = 0; ok && i < 3; ++i)
-        ok = full.left[r][i] == gen_konnov::kFullLeft[r][i] && full.right[r][i] == gen_konnov::kFullRight[r][i];
-      for (int u = 0; ok && u < full.nupd[r]; ++u)
-        ok = full.upd_k[r][u] == gen_konnov::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_konnov::kFullUpdProd[r][u];
-    }
     if (ok) return kSpecKonnov;
   }
-  if (m.NI == gen_acetylene::kSpecN && m.RM == gen_acetylene::kSpecR && full.N == gen_acetylene::kFullN && full.R == gen_acetylene::kFullR) {
+  if (m.NI == gen_acetylene::kSpecN && m.RM == gen_acetylene::kSpecR) {
     bool ok = true;
     for (int r = 0; ok && r < m.RM; ++r) {
       ok = m.nupd[r] == gen_acetylene::kSpecNupd[r];
@@ -168,12 +140,66 @@ inline int match_specialised_tables(const M& m, const M& full) {
       for (int u = 0; ok && u < m.nupd[r]; ++u)
         ok = m.upd_k[r][u] == gen_acetylene::kSpecUpdK[r][u] && m.upd_prod[r][u] == gen_acetylene::kSpecUpdProd[r][u];
     }
-    for (int r = 0; ok && r < full.R; ++r) {
-      ok = full.nupd[r] == gen_acetylene::kFullNupd[r];
+    if (ok) return kSpecAcetylene;
+  }
+  return 0;
+}
+
+// 0 when the full reaction lists match none of the generated codes.
+template <class M>
+inline int match_specialised_full_tables(const M& m) {
+  if (m.N == gen_keromnes::kFullN && m.R == gen_keromnes::kFullR) {
+    bool ok = true;
+    for (int r = 0; ok && r < m.R; ++r) {
+      ok = m.nupd[r] == gen_keromnes::kFullNupd[r];
       for (int i = 0; ok && i < 3; ++i)
-        ok = full.left[r][i] == gen_acetylene::kFullLeft[r][i] && full.right[r][i] == gen_acetylene::kFullRight[r][i];
-      for (int u = 0; ok && u < full.nupd[r]; ++u)
-        ok = full.upd_k[r][u] == gen_acetylene::kFullUpdK[r][u] && full.upd_prod[r][u] == gen_acetylene::kFullUpdProd[r][u];
+        ok = m.left[r][i] == gen_keromnes::kFullLeft[r][i] && m.right[r][i] == gen_keromnes::kFullRight[r][i];
+      for (int u = 0; ok && u < m.nupd[r]; ++u)
+        ok = m.upd_k[r][u] == gen_keromnes::kFullUpdK[r][u] && m.upd_prod[r][u] == gen_keromnes::kFullUpdProd[r][u];
+    }
+    if (ok) return kSpecKeromnes;
+  }
+  if (m.N == gen_zhang::kFullN && m.R == gen_zhang::kFullR) {
+    bool ok = true;
+    for (int r = 0; ok && r < m.R; ++r) {
+      ok = m.nupd[r] == gen_zhang::kFullNupd[r];
+      for (int i = 0; ok && i < 3; ++i)
+        ok = m.left[r][i] == gen_zhang::kFullLeft[r][i] && m.right[r][i] == gen_zhang::kFullRight[r][i];
+      for (int u = 0; ok && u < m.nupd[r]; ++u)
+        ok = m.upd_k[r][u] == gen_zhang::kFullUpdK[r][u] && m.upd_prod[r][u] == gen_zhang::kFullUpdProd[r][u];
+    }
+    if (ok) return kSpecZhang;
+  }
+  if (m.N == gen_tereza::kFullN && m.R == gen_tereza::kFullR) {
+    bool ok = true;
+    for (int r = 0; ok && r < m.R; ++r) {
+      ok = m.nupd[r] == gen_tereza::kFullNupd[r];
+      for (int i = 0; ok && i < 3; ++i)
+        ok = m.left[r][i] == gen_tereza::kFullLeft[r][i] && m.right[r][i] == gen_tereza::kFullRight[r][i];
+      for (int u = 0; ok && u < m.nupd[r]; ++u)
+        ok = m.upd_k[r][u] == gen_tereza::kFullUpdK[r][u] && m.upd_prod[r][u] == gen_tereza::kFullUpdProd[r][u];
+    }
+    if (ok) return kSpecTereza;
+  }
+  if (m.N == gen_konnov::kFullN && m.R == gen_konnov::kFullR) {
+    bool ok = true;
+    for (int r = 0; ok && r < m.R; ++r) {
+      ok = m.nupd[r] == gen_konnov::kFullNupd[r];
+      for (int i = 0; ok && i < 3; ++i)
+        ok = m.left[r][i] == gen_konnov::kFullLeft[r][i] && m.right[r][i] == gen_konnov::kFullRight[r][i];
+      for (int u = 0; ok && u < m.nupd[r]; ++u)
+        ok = m.upd_k[r][u] == gen_konnov::kFullUpdK[r][u] && m.upd_prod[r][u] == gen_konnov::kFullUpdProd[r][u];
+    }
+    if (ok) return kSpecKonnov;
+  }
+  if (m.N == gen_acetylene::kFullN && m.R == gen_acetylene::kFullR) {
+    bool ok = true;
+    for (int r = 0; ok && r < m.R; ++r) {
+      ok = m.nupd[r] == gen_acetylene::kFullNupd[r];
+      for (int i = 0; ok && i < 3; ++i)
+        ok = m.left[r][i] == gen_acetylene::kFullLeft[r][i] && m.right[r][i] == gen_acetylene::kFullRight[r][i];
+      for (int u = 0; ok && u < m.nupd[r]; ++u)
+        ok = m.upd_k[r][u] == gen_acetylene::kFullUpdK[r][u] && m.upd_prod[r][u] == gen_acetylene::kFullUpdProd[r][u];
     }
     if (ok) return kSpecAcetylene;
   }

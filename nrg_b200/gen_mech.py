@@ -166,7 +166,10 @@ def emit(name: str, ns: str, reduced, full) -> str:
 
 def emit_index(names) -> str:
     """gen_mechanisms.cuh: the generated mechanisms, numbered from 1, and the
-    host-side match of a parsed mechanism's reduced tables against them."""
+    host-side match of a parsed mechanism's tables against them: the reduced
+    ones (the integrators that skip inert species) and the full ones (the
+    reference mode) each on their own, for a deck that only lists an inert
+    species elsewhere still has the reduced lists."""
     o = ["// Generated by nrg_b200/gen_mech.py: do not edit.",
          "// The mechanism-specialised codes, numbered from 1 (0 = table-driven).",
          "#pragma once", ""]
@@ -184,22 +187,25 @@ def emit_index(names) -> str:
               "  template <int J, class S, typename LUT>",
               f"  __device__ static void column(const S& c, double f, LUT (&v)[{ns}::kSpecN]) {{",
               f"    {ns}::spec_column<J>(c, f, v);", "  }", "};"]
-    o += ["", "// 0 when the reaction lists, reduced or full, match none of the generated codes.",
-          "template <class M>", "inline int match_specialised_tables(const M& m, const M& full) {"]
-    for n in names:
-        ns = f"gen_{n.lower()}"
-        o += [f"  if (m.NI == {ns}::kSpecN && m.RM == {ns}::kSpecR && full.N == {ns}::kFullN && full.R == {ns}::kFullR) {{",
-              "    bool ok = true;"]
-        for t, r, p in (("m", "m.RM", "kSpec"), ("full", "full.R", "kFull")):
-            o += [f"    for (int r = 0; ok && r < {r}; ++r) {{",
-                  f"      ok = {t}.nupd[r] == {ns}::{p}Nupd[r];",
+    for fn, doc, count, species, prefix in (
+            ("match_specialised_tables", "reduced", "m.RM", "m.NI", "kSpec"),
+            ("match_specialised_full_tables", "full", "m.R", "m.N", "kFull")):
+        o += ["", f"// 0 when the {doc} reaction lists match none of the generated codes.",
+              "template <class M>", f"inline int {fn}(const M& m) {{"]
+        for n in names:
+            ns = f"gen_{n.lower()}"
+            o += [f"  if ({species} == {ns}::{prefix}N && {count} == {ns}::{prefix}R) {{",
+                  "    bool ok = true;",
+                  f"    for (int r = 0; ok && r < {count}; ++r) {{",
+                  f"      ok = m.nupd[r] == {ns}::{prefix}Nupd[r];",
                   "      for (int i = 0; ok && i < 3; ++i)",
-                  f"        ok = {t}.left[r][i] == {ns}::{p}Left[r][i] && {t}.right[r][i] == {ns}::{p}Right[r][i];",
-                  f"      for (int u = 0; ok && u < {t}.nupd[r]; ++u)",
-                  f"        ok = {t}.upd_k[r][u] == {ns}::{p}UpdK[r][u] && {t}.upd_prod[r][u] == {ns}::{p}UpdProd[r][u];",
-                  "    }"]
-        o += [f"    if (ok) return kSpec{n.capitalize()};", "  }"]
-    o += ["  return 0;", "}", "", "}  // namespace nrg", ""]
+                  f"        ok = m.left[r][i] == {ns}::{prefix}Left[r][i] && m.right[r][i] == {ns}::{prefix}Right[r][i];",
+                  "      for (int u = 0; ok && u < m.nupd[r]; ++u)",
+                  f"        ok = m.upd_k[r][u] == {ns}::{prefix}UpdK[r][u] && m.upd_prod[r][u] == {ns}::{prefix}UpdProd[r][u];",
+                  "    }",
+                  f"    if (ok) return kSpec{n.capitalize()};", "  }"]
+        o += ["  return 0;", "}"]
+    o += ["", "}  // namespace nrg", ""]
     return "\n".join(o)
 
 
