@@ -39,7 +39,7 @@ __device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi
 // One contraction C[m, n] = sum_k A(m, k) B(n, k) of the training and the GEMM
 // chain's inference, N = 16 or 128:
 //   kFwd: Z = A W^T + b (fp32, may be null), H = bf16(gelu(Z)) (may be null)
-//   kDH:  dZ = (A W) gelu'(Z), bf16, and its column sums added to db
+//   kDH:  dZ = (A W) gelu'(Z), bf16, and its column sums in db
 //   kDW:  C += A B, K split over CTAs (C zeroed beforehand)
 // a_mn / b_mn: the operand is stored with its M or N index contiguous ([K][ld],
 // the gradients' operands as the forward pass left them), else K contiguous.
@@ -55,6 +55,8 @@ struct GemmJob {
   __nv_bfloat16* H;    // bf16 result (kFwd: may be null), N columns
   const float* Z;      // kDH: pre-activations, N columns
   float* db;           // kDH
+  float* part;         // kDH: column sums of the tiles, [tile][128]
+  unsigned int* tick;  // kDH: tiles done, zero between launches
   int k_per_cta;       // kDW; else K
   int tiles;           // CTAs
 };
@@ -108,6 +110,18 @@ __device__ __forceinline__ void tg_stage(unsigned char* dst, const __nv_bfloat16
       *reinterpret_cast<uint4*>(dst + tc::kmajor_off(r, ch, kc)) = v;
     }
   }
+}
+
+// One more block of `blocks` is done; true in the block that is the last, which
+// then sees what the others wrote before.  The count ends at zero.
+__device__ __forceinline__ bool last_block(unsigned int* tick, int blocks) {
+  __threadfence();
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(tick, (unsigned)blocks - 1u) == (unsigned)blocks - 1u;
+  __syncthreads();
+  __threadfence();
+  return last;
 }
 
 __device__ __forceinline__ void red_add4(float* p, float4 v) {
@@ -171,6 +185,7 @@ __global__ void __launch_bounds__(kTgThreads, 2) k_gemm_tc(const __grid_constant
   if (any && ok) ok = __syncthreads_and(tc::mbar_wait(tc::smem_u32(mbar), parity, kTcWaitNs));
   if (!ok) {
     if (tid == 0) atomicOr(err, 1u);
+    if (g.mode == kDH && tid < 128) g.part[tile * 128 + tid] = 0.f;
   } else if (any) {
     tc::fence_after_sync();
     // accumulator rows (lanes) to shared memory: warp w has lanes 32 (w % 4)..,
@@ -221,9 +236,19 @@ __global__ void __launch_bounds__(kTgThreads, 2) k_gemm_tc(const __grid_constant
         float s = 0.f;
 #pragma unroll
         for (int w = 0; w < kTgThreads / 32; ++w) s += colsum[w * 128 + tid];
-        atomicAdd(g.db + tid, s);
+        g.part[tile * 128 + tid] = s;
       }
     }
+  }
+  // the tiles' sums in tile order, by the block that finishes last: the bias
+  // gradients repeat bit for bit
+  if (g.mode == kDH && last_block(g.tick, g.tiles)) {
+    float s = 0.f;
+#pragma unroll 4
+    for (int t = tid >> 7; t < g.tiles; t += 2) s += __ldcg(g.part + t * 128 + (tid & 127));
+    colsum[tid] = s;
+    __syncthreads();
+    if (tid < 128) g.db[tid] = colsum[tid] + colsum[128 + tid];
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -255,10 +280,13 @@ static cudaError_t launch_gemm(GemmJob a, GemmJob b, cudaStream_t st, unsigned i
 
 // ------------------------------------------------------- small kernels
 // dO of the mean squared error, its column sums (the last layer's bias gradient)
-// added to db, and the loss.  256-thread blocks: a thread keeps its column.
+// in db, and the loss added to *loss.  256-thread blocks: a thread keeps its
+// column.  The last block to finish adds the blocks' sums (part, lpart) in
+// block order.
+constexpr int kLossBlocks = 256;
 __global__ void __launch_bounds__(256) k_loss_grad(long B, const float* O, const float* Y, __nv_bfloat16* dOb, float* db,
-                                                   double* loss) {
-  double part = 0.0;
+                                                   double* loss, float* part, double* lpart, unsigned int* tick) {
+  double sq = 0.0;
   float col = 0.f;
   const float scale = 2.0f / (float)(B * kMlpOut);
   const int j = threadIdx.x % kMlpOutPad;
@@ -267,7 +295,7 @@ __global__ void __launch_bounds__(256) k_loss_grad(long B, const float* O, const
     float d = 0.f;
     if (j < kMlpOut) {
       const float e = O[b * kMlpOutPad + j] - Y[b * kMlpOut + j];
-      part += (double)e * e;
+      sq += (double)e * e;
       d = scale * e;
     }
     dOb[i] = __float2bfloat16(d);
@@ -276,20 +304,33 @@ __global__ void __launch_bounds__(256) k_loss_grad(long B, const float* O, const
   __shared__ double sp[8];
   __shared__ float sc[8][kMlpOutPad];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
+  for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
   col += __shfl_down_sync(0xffffffffu, col, 16);
-  if (lane == 0) sp[w] = part;
+  if (lane == 0) sp[w] = sq;
   if (lane < kMlpOutPad) sc[w][lane] = col;
   __syncthreads();
   if (threadIdx.x < kMlpOutPad) {
     float s = 0.f;
     for (int q = 0; q < 8; ++q) s += sc[q][threadIdx.x];
-    atomicAdd(db + threadIdx.x, s);
+    part[blockIdx.x * kMlpOutPad + threadIdx.x] = s;
   }
-  if (threadIdx.x == 32 && loss) {
+  if (threadIdx.x == 32) {
     double s = 0.0;
     for (int q = 0; q < 8; ++q) s += sp[q];
-    atomicAdd(loss, s / (double)(B * kMlpOut));
+    lpart[blockIdx.x] = s;
+  }
+  if (!last_block(tick, gridDim.x)) return;
+  if (threadIdx.x < kMlpOutPad) {
+    float s = 0.f;
+#pragma unroll 8
+    for (int t = 0; t < (int)gridDim.x; ++t) s += __ldcg(part + t * kMlpOutPad + threadIdx.x);
+    db[threadIdx.x] = s;
+  }
+  if (threadIdx.x == 32) {
+    double s = 0.0;
+#pragma unroll 8
+    for (int t = 0; t < (int)gridDim.x; ++t) s += __ldcg(lpart + t);
+    *loss += s / (double)(B * kMlpOut);
   }
 }
 
@@ -1139,6 +1180,9 @@ struct Surrogate {
   float *Z[kMlpLayers] = {}, *O = nullptr;
   __nv_bfloat16* dOb = nullptr;
   float* Yb = nullptr;
+  float* part = nullptr;          // sums of the training blocks (bias gradients)
+  double* lpart = nullptr;        // and of the loss
+  unsigned int* tick = nullptr;   // blocks done, zero between launches
   int* idx = nullptr;
   double* d_loss = nullptr;
   // inference buffers (features, two activation buffers, outputs)
@@ -1272,9 +1316,11 @@ static void free_act(Surrogate* s) {
     s->Z[l] = nullptr;
   }
   cudaFree(s->dHb[0]); cudaFree(s->dHb[1]); cudaFree(s->O); cudaFree(s->dOb);
-  cudaFree(s->Yb); cudaFree(s->idx);
+  cudaFree(s->Yb); cudaFree(s->idx); cudaFree(s->part); cudaFree(s->lpart); cudaFree(s->tick);
   s->X = s->dHb[0] = s->dHb[1] = s->dOb = nullptr;
-  s->O = s->Yb = nullptr;
+  s->O = s->Yb = s->part = nullptr;
+  s->lpart = nullptr;
+  s->tick = nullptr;
   s->idx = nullptr;
   s->cap = 0;
 }
@@ -1357,6 +1403,12 @@ static std::string ensure_act(Surrogate* s, long n) {
     if ((e = ck(cudaMalloc(&d, np * kMlpHid * 2), "alloc dH")).size()) return e;
   if ((e = ck(cudaMalloc(&s->Yb, np * kMlpOut * 4), "alloc Y")).size()) return e;
   if ((e = ck(cudaMalloc(&s->idx, np * 4), "alloc idx")).size()) return e;
+  const long rows = std::max<long>((np + 127) / 128 * 128, kLossBlocks * kMlpOutPad);
+  if ((e = ck(cudaMalloc(&s->part, rows * 4), "alloc sums")).size()) return e;
+  if ((e = ck(cudaMalloc(&s->lpart, kLossBlocks * 8), "alloc sums")).size()) return e;
+  if ((e = ck(cudaMalloc(&s->tick, 4), "alloc count")).size()) return e;
+  if ((e = ck(cudaMemset(s->tick, 0, 4), "clear count")).size()) return e;
+  if ((e = ck(cudaStreamSynchronize(nullptr), "clear count")).size()) return e;
   s->cap = np;
   return "";
 }
@@ -1522,8 +1574,8 @@ static cudaError_t backward(Surrogate* s, long B, const __nv_bfloat16* x, const 
   cudaError_t e = cudaMemsetAsync(s->gr, 0, sizeof(float) * (size_t)s->n_params, st);
   if (e == cudaSuccess) e = forward(s, B, x, s->O, st);
   if (e != cudaSuccess) return e;
-  k_loss_grad<<<std::min<long>((B * kMlpOutPad + 255) / 256, 256), 256, 0, st>>>(
-      B, s->O, y, s->dOb, s->gr + s->offb[kMlpLayers - 1], s->d_loss);
+  k_loss_grad<<<std::min<long>((B * kMlpOutPad + 255) / 256, kLossBlocks), 256, 0, st>>>(
+      B, s->O, y, s->dOb, s->gr + s->offb[kMlpLayers - 1], s->d_loss, s->part, s->lpart, s->tick);
   const __nv_bfloat16* dZ = s->dOb;
   for (int l = kMlpLayers - 1; l >= 0; --l) {
     // dW[out][in] = sum_b dZ[b][out] Hin[b][in]
@@ -1549,6 +1601,8 @@ static cudaError_t backward(Surrogate* s, long B, const __nv_bfloat16* x, const 
       h.H = dH;
       h.Z = s->Z[l - 1];
       h.db = s->gr + s->offb[l - 1];
+      h.part = s->part;
+      h.tick = s->tick;
     }
     if ((e = launch_gemm(h, w, st, s->d_err)) != cudaSuccess) return e;
     dZ = dH;

@@ -70,3 +70,29 @@ def test_arrays_off_a_16_byte_boundary(sur, off):
         res.append(sur.params())
     sur.init(seed=7)
     assert np.linalg.norm(res[0] - res[1]) <= 1e-5 * np.linalg.norm(res[0])
+
+
+def test_sums_repeat_bit_for_bit(sur):
+    """Batches of up to two 128-row tiles train to the same parameters and
+    losses every time (two tiles' weight gradients add to zero in either order
+    alike); bias gradients and the loss repeat at any batch (155 tiles here, 256
+    blocks of the loss)."""
+    for batch in (64, 128, 192, 256):
+        xt, yt, _, _ = rand_batch(4 * batch + 3, 50 + batch)
+        runs = []
+        for _ in range(4):
+            sur.init(seed=7)
+            losses = sur.train(xt, yt, epochs=3, batch=batch, lr=1e-3, seed=2)
+            runs.append((sur.params(), losses))
+        for p, losses in runs[1:]:
+            np.testing.assert_array_equal(p, runs[0][0], err_msg=str(batch))
+            np.testing.assert_array_equal(losses, runs[0][1], err_msg=str(batch))
+    sur.init(seed=7)
+    xt, yt, _, _ = rand_batch(154 * 128 + 9, 60)
+    runs = [sur.grad(xt, yt) for _ in range(4)]
+    off = 0
+    for o, i in mlp_ref.SHAPES:
+        for g, loss in runs[1:]:
+            np.testing.assert_array_equal(g[off + o * i:off + o * i + o], runs[0][0][off + o * i:off + o * i + o])
+            assert loss == runs[0][1]
+        off += o * i + o
