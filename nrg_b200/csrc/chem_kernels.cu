@@ -56,9 +56,17 @@ __global__ void k_fp64_peak(double* out, int iters) {
 // 102 registers (five blocks per SM): 0.79 ms with the state's copies against
 // 0.89 ms at 144 and 0.81 ms at 80.
 
+// |x| in (2^-lo, 2^hi): finite, and far from where quotients and their
+// remainders leave the normal range.
+template <int LO, int HI>
+__device__ __forceinline__ bool within(double x) {
+  const unsigned e = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  return e - ((1023u - LO) << 20) < (unsigned)(LO + HI) << 20;
+}
+
 // x / d from r, the correctly rounded 1 / d: the remainder of x r corrects it
-// (Markstein's theorem: correctly rounded unless x, d or the remainder leave
-// the normal range).
+// (Markstein's theorem: correctly rounded while x, d and the remainder are in
+// the normal range; an infinite x or a zero d would give NaN).
 __device__ __forceinline__ double div_known(double x, double d, double r) {
   const double q = x * r;
   return fma(fma(-q, d, x), r, q);
@@ -94,8 +102,73 @@ __device__ __forceinline__ double state_cp(const StateTables<N>& s, int set, int
   return cp * t + s.a[set][0][k];
 }
 
+// The cells whose operands leave the range of div_known (infinite or NaN
+// fields, a vanishing density or mixture, an iteration that diverged): the
+// reference's operations with its divisions.  sources: the chemistry sources
+// are still to be applied.
 template <int N>
-__global__ void __launch_bounds__(128, N <= 10 ? 5 : 2) k_apply_state(ApplyStateArgs a) {
+__device__ __noinline__ void state_plain(const ApplyStateArgs& a, long c, bool sources) {
+  const double RG = 8.31446261815324;
+  const double rho = a.rho[c];
+  double X[N], avg = 0.0;
+  double Ef = a.E_f[c];
+  if (sources && a.E_f_prod) {
+    Ef = Ef + a.E_f_prod[c] * a.dt / rho;
+    a.E_f[c] = Ef;
+  }
+#pragma unroll 1
+  for (int k = 0; k < N; ++k) {
+    double y = a.Y[k * a.ld + c];
+    if (sources && a.Y_prod) {
+      y = y + a.Y_prod[k * a.ld + c] * a.dt / rho;
+      a.Y[k * a.ld + c] = y;
+    }
+    X[k] = ddiv(y, c_mech.W[k]);
+    avg = avg + X[k];
+  }
+  avg = ddiv(1.0, avg);
+  double e_i = Ef, h_ref = 0.0;
+  for (int d = 0; d < a.dims; ++d) {
+    const double vd = a.v[d * a.ld + c];
+    e_i = e_i - __dmul_rn(0.5, __dmul_rn(vd, vd));
+  }
+  e_i = e_i * avg;
+  double t = NRG_FMIN(a.T[c], 6000.0), cp = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < N; ++k) {
+    X[k] = X[k] * avg;
+    h_ref = h_ref + c_mech.h_ref[k] * X[k];
+    cp = cp + d_cp(t, k) * X[k];
+  }
+  for (int iter = 0; iter < 1000; ++iter) {
+    double e = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < N; ++k) e = e + (d_enthalpy(t, k) - RG * t) * X[k];
+    const double residual = ddiv(e_i - (e - h_ref), cp);
+    t = t + residual;
+    if (fabs(residual) < (double)1e-08f) break;
+  }
+  double h = 0.0;
+  cp = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < N; ++k) {
+    cp = cp + d_cp(t, k) * X[k];
+    h = h + d_enthalpy(t, k) * X[k];
+  }
+  const double p = ddiv(t * rho * RG, avg), gamma = ddiv(cp, cp - RG);
+  a.T[c] = t;
+  a.p[c] = p;
+  a.gamma[c] = gamma;
+  if (a.h_s) a.h_s[c] = ddiv(h - h_ref, avg);
+  if (a.h_full) a.h_full[c] = ddiv(h, avg);
+  if (a.cp_mass) a.cp_mass[c] = ddiv(cp, avg);
+  if (a.mix_mol_mass) a.mix_mol_mass[c] = avg;
+  if (a.v_s) a.v_s[c] = sqrt(ddiv(gamma * p, rho));
+  if (a.status) a.status[c] = (gamma < 0.0 || p < 0.0 || rho < 0.0) ? 2 : 1;
+}
+
+template <int N>
+__global__ void __launch_bounds__(128, N <= 10 ? 5 : 2) k_apply_state(const __grid_constant__ ApplyStateArgs a) {
   const double RG = 8.31446261815324;
   __shared__ StateTables<N> tab;
   for (int i = threadIdx.x; i < 2 * 6 * N; i += blockDim.x) {
@@ -120,19 +193,13 @@ __global__ void __launch_bounds__(128, N <= 10 ? 5 : 2) k_apply_state(ApplyState
 #pragma unroll
     for (int k = 0; k < N; ++k) S[k] = a.Y_prod[k * a.ld + c];
   }
-  const bool exact_r = fabs(rho) > 1e-280 && fabs(rho) < 1e280;
   const double rrho = 1.0 / rho;
-  auto over_rho = [&](double x) { return exact_r ? div_known(x, rho, rrho) : x / rho; };
-  if (a.E_f_prod) {
-    Ef = Ef + over_rho(a.E_f_prod[c] * a.dt);
-    a.E_f[c] = Ef;
-  }
+  auto over_rho = [&](double x) { return within<500, 500>(x) || x == 0.0 ? div_known(x, rho, rrho) : ddiv(x, rho); };
+  bool known = within<300, 300>(rho);
+  if (a.E_f_prod) Ef = Ef + over_rho(a.E_f_prod[c] * a.dt);
   if (a.Y_prod) {
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-      Y[k] = Y[k] + over_rho(S[k] * a.dt);
-      a.Y[k * a.ld + c] = Y[k];
-    }
+    for (int k = 0; k < N; ++k) Y[k] = Y[k] + over_rho(S[k] * a.dt);
   }
   double e_i = Ef;
   for (int d = 0; d < a.dims; ++d) {
@@ -142,10 +209,20 @@ __global__ void __launch_bounds__(128, N <= 10 ? 5 : 2) k_apply_state(ApplyState
   double X[N], avg = 0.0, h_ref = 0.0;
 #pragma unroll
   for (int k = 0; k < N; ++k) {
+    known = known && within<1023, 400>(Y[k]);  // a quotient that underflows adds nothing to the others
     X[k] = div_known(Y[k], c_mech.W[k], c_mech.invW[k]);
     avg = avg + X[k];
   }
   avg = 1.0 / avg;
+  if (!known || !within<300, 300>(avg)) {
+    state_plain<N>(a, c, true);
+    return;
+  }
+  if (a.E_f_prod) a.E_f[c] = Ef;
+  if (a.Y_prod) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) a.Y[k * a.ld + c] = Y[k];
+  }
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     X[k] = X[k] * avg;
@@ -167,6 +244,10 @@ __global__ void __launch_bounds__(128, N <= 10 ? 5 : 2) k_apply_state(ApplyState
     const double residual = div_known(e_i - (e - h_ref), cp, rcp);
     t = t + residual;
     if (fabs(residual) < (double)1e-08f) break;  // single-precision literal in the reference
+  }
+  if (!(t > -1e4 && within<300, 300>(t))) {
+    state_plain<N>(a, c, false);
+    return;
   }
   const double tt = NRG_FMIN(t, 6000.0), rt = 1.0 / tt, ravg = 1.0 / avg;
   const int set = nasa_set(tt);

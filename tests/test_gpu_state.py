@@ -98,3 +98,48 @@ def test_acetylene_state_equation_matches_oracle():
     np.testing.assert_array_equal(g["status"], o["status"])
     for k in KEYS:
         np.testing.assert_allclose(g[k], o[k], rtol=1e-13, atol=0, err_msg=k)
+
+
+def test_state_equation_gives_the_reference_bits(solver, oracle_mech, W):
+    """Quotients formed from reciprocals are the divisions' bits: every output
+    of a field with sources equals the oracle's exactly, mass fractions from
+    1e-300 up and sources that underflow among them."""
+    f = fields.slice_field(fields.wide_range_field(W, n_side=64), 4000)
+    rng = np.random.default_rng(11)
+    f.Y[4:, ::5] *= 10.0 ** rng.uniform(-290.0, 0.0, (5, f.Y[4:, ::5].shape[1]))
+    v = rng.uniform(-500.0, 500.0, (2, f.n))
+    E = _energy_per_mass(oracle_mech, f.T, f.Y, W, v)
+    Yp = 2e-3 * rng.uniform(-1.0, 1.0, f.Y.shape) * f.Y * f.rho / f.dt
+    Yp[:, ::3] *= 10.0 ** rng.uniform(-300.0, 0.0, Yp[:, ::3].shape)
+    Ep = rng.uniform(-1e9, 1e9, f.n)
+    T0 = f.T * rng.uniform(0.8, 1.2, f.n)
+    g = _device_state(solver, f, E, v, T0, Y_prod=Yp, E_f_prod=Ep)
+    o = oracle_mech.apply_state(f.rho, f.Y, E, T0, v=v, dt=f.dt, Y_prod=Yp, E_f_prod=Ep)
+    for k in KEYS + ("Y", "E_f", "status"):
+        np.testing.assert_array_equal(g[k], o[k], err_msg=k)
+
+
+def test_state_equation_outside_the_normal_range(solver, oracle_mech, W):
+    """Infinite and NaN fields and sources, vanishing and denormal densities,
+    mixtures and temperatures: the values the reference's divisions give,
+    infinities and NaN included."""
+    f = fields.slice_field(fields.wide_range_field(W, n_side=64), 40)
+    inf, nan, tiny = np.inf, np.nan, 1e-310
+    E = _energy_per_mass(oracle_mech, f.T, f.Y, W, np.zeros((0, f.n)))
+    T0, Yp, Ep = f.T.copy(), np.zeros_like(f.Y), np.zeros(f.n)
+    E[:4] = inf, -inf, nan, 1e300
+    f.Y[0, 4:8] = inf, -inf, nan, 1e200
+    f.Y[:, 8] = 0.0
+    f.Y[:, 9] *= 1e-250
+    f.Y[:, 10] = tiny
+    f.rho[11:17] = 0.0, inf, nan, tiny, -1.0, 1e200
+    T0[17:24] = 0.0, -5.0, inf, nan, tiny, -1e300, 1e-200
+    Ep[24:28] = inf, -inf, nan, 1e305
+    Yp[3, 28:32] = inf, -inf, nan, 1e-300
+    v = np.zeros((1, f.n))
+    v[0, 32:35] = 1e200, inf, nan
+    with np.errstate(all="ignore"):
+        g = _device_state(solver, f, E, v, T0, Y_prod=Yp, E_f_prod=Ep)
+        o = oracle_mech.apply_state(f.rho, f.Y, E, T0, v=v, dt=f.dt, Y_prod=Yp, E_f_prod=Ep)
+    for k in KEYS + ("Y", "E_f", "status"):
+        np.testing.assert_array_equal(g[k], o[k], err_msg=k)
