@@ -39,7 +39,7 @@ __device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi
 // One contraction C[m, n] = sum_k A(m, k) B(n, k) of the training and the GEMM
 // chain's inference, N = 16 or 128:
 //   kFwd: Z = A W^T + b (fp32, may be null), H = bf16(gelu(Z)) (may be null)
-//   kDH:  dZ = (A W) gelu'(Z), bf16, and its column sums in db
+//   kDH:  dZ = (A W) gelu'(Z), bf16, and each tile's column sums
 //   kDW:  C += A B, K split over CTAs (C zeroed beforehand)
 // a_mn / b_mn: the operand is stored with its M or N index contiguous ([K][ld],
 // the gradients' operands as the forward pass left them), else K contiguous.
@@ -54,11 +54,21 @@ struct GemmJob {
   const float* bias;   // kFwd, per column
   __nv_bfloat16* H;    // bf16 result (kFwd: may be null), N columns
   const float* Z;      // kDH: pre-activations, N columns
-  float* db;           // kDH
   float* part;         // kDH: column sums of the tiles, [tile][128]
-  unsigned int* tick;  // kDH: tiles done, zero between launches
   int k_per_cta;       // kDW; else K
   int tiles;           // CTAs
+};
+
+// Sums of the blocks of an earlier launch, added in block order by one more CTA:
+// a bias gradient's column sums, and the loss.
+struct SumJob {
+  int blocks;          // 0: none
+  int cols;            // 16 or 128
+  const float* part;   // [block][cols]
+  float* db;
+  const double* lpart; // [block], at most 256 blocks (may be null)
+  double* loss;
+  double lscale;
 };
 
 // A 256-thread CTA takes a 128-row tile (kDW: all of M and a range of K).  K
@@ -112,16 +122,28 @@ __device__ __forceinline__ void tg_stage(unsigned char* dst, const __nv_bfloat16
   }
 }
 
-// One more block of `blocks` is done; true in the block that is the last, which
-// then sees what the others wrote before.  The count ends at zero.
-__device__ __forceinline__ bool last_block(unsigned int* tick, int blocks) {
-  __threadfence();
-  __shared__ bool last;
+// 256 threads; sm: 2 KB.  Thread (g, c) adds the blocks g, g + G, ... of column c.
+__device__ __forceinline__ void sum_blocks(const SumJob& j, void* sm) {
+  const int c = threadIdx.x % j.cols, g = threadIdx.x / j.cols, G = blockDim.x / j.cols;
+  float s = 0.f;
+#pragma unroll 16
+  for (int b = g; b < j.blocks; b += G) s += j.part[(long)b * j.cols + c];
+  float* f = static_cast<float*>(sm);
+  f[threadIdx.x] = s;
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicInc(tick, (unsigned)blocks - 1u) == (unsigned)blocks - 1u;
+  if (g == 0) {
+    for (int q = 1; q < G; ++q) s += f[q * j.cols + c];
+    j.db[c] = s;
+  }
+  if (!j.lpart) return;
   __syncthreads();
-  __threadfence();
-  return last;
+  double* d = static_cast<double*>(sm);
+  d[threadIdx.x] = (int)threadIdx.x < j.blocks ? j.lpart[threadIdx.x] : 0.0;
+  for (int o = blockDim.x / 2; o > 0; o /= 2) {
+    __syncthreads();
+    if ((int)threadIdx.x < o) d[threadIdx.x] += d[threadIdx.x + o];
+  }
+  if (threadIdx.x == 0) *j.loss += d[0] * j.lscale;
 }
 
 __device__ __forceinline__ void red_add4(float* p, float4 v) {
@@ -130,8 +152,13 @@ __device__ __forceinline__ void red_add4(float* p, float4 v) {
 }
 
 __global__ void __launch_bounds__(kTgThreads, 2) k_gemm_tc(const __grid_constant__ GemmJob j0,
-                                                           const __grid_constant__ GemmJob j1, unsigned int* err) {
+                                                           const __grid_constant__ GemmJob j1,
+                                                           const __grid_constant__ SumJob jsum, unsigned int* err) {
   extern __shared__ __align__(1024) unsigned char sm[];
+  if ((int)blockIdx.x == j0.tiles + j1.tiles) {
+    sum_blocks(jsum, sm);
+    return;
+  }
   const bool second = (int)blockIdx.x >= j0.tiles;
   const GemmJob& g = second ? j1 : j0;
   const int tile = second ? (int)blockIdx.x - j0.tiles : (int)blockIdx.x;
@@ -240,16 +267,6 @@ __global__ void __launch_bounds__(kTgThreads, 2) k_gemm_tc(const __grid_constant
       }
     }
   }
-  // the tiles' sums in tile order, by the block that finishes last: the bias
-  // gradients repeat bit for bit
-  if (g.mode == kDH && last_block(g.tick, g.tiles)) {
-    float s = 0.f;
-#pragma unroll 4
-    for (int t = tid >> 7; t < g.tiles; t += 2) s += __ldcg(g.part + t * 128 + (tid & 127));
-    colsum[tid] = s;
-    __syncthreads();
-    if (tid < 128) g.db[tid] = colsum[tid] + colsum[128 + tid];
-  }
   tc::fence_before_sync();
   __syncthreads();
   if (tid < 32) {
@@ -258,7 +275,7 @@ __global__ void __launch_bounds__(kTgThreads, 2) k_gemm_tc(const __grid_constant
   }
 }
 
-static cudaError_t launch_gemm(GemmJob a, GemmJob b, cudaStream_t st, unsigned int* err) {
+static cudaError_t launch_gemm(GemmJob a, GemmJob b, const SumJob& sum, cudaStream_t st, unsigned int* err) {
   for (GemmJob* g : {&a, &b}) {
     if (g->M <= 0 || g->N <= 0) {
       g->tiles = 0;
@@ -273,19 +290,19 @@ static cudaError_t launch_gemm(GemmJob a, GemmJob b, cudaStream_t st, unsigned i
       g->tiles = (g->M + 127) / 128;
     }
   }
-  if (a.tiles + b.tiles <= 0) return cudaSuccess;
-  k_gemm_tc<<<(unsigned)(a.tiles + b.tiles), kTgThreads, kTgSmem, st>>>(a, b, err);
+  const int grid = a.tiles + b.tiles + (sum.blocks > 0 ? 1 : 0);
+  if (grid <= 0) return cudaSuccess;
+  k_gemm_tc<<<(unsigned)grid, kTgThreads, kTgSmem, st>>>(a, b, sum, err);
   return cudaGetLastError();
 }
 
 // ------------------------------------------------------- small kernels
-// dO of the mean squared error, its column sums (the last layer's bias gradient)
-// in db, and the loss added to *loss.  256-thread blocks: a thread keeps its
-// column.  The last block to finish adds the blocks' sums (part, lpart) in
-// block order.
+// dO of the mean squared error and each block's column sums of it (part) and of
+// the squared errors (lpart); the next launch adds them up (SumJob).  256-thread
+// blocks: a thread keeps its column.
 constexpr int kLossBlocks = 256;
-__global__ void __launch_bounds__(256) k_loss_grad(long B, const float* O, const float* Y, __nv_bfloat16* dOb, float* db,
-                                                   double* loss, float* part, double* lpart, unsigned int* tick) {
+__global__ void __launch_bounds__(256) k_loss_grad(long B, const float* O, const float* Y, __nv_bfloat16* dOb,
+                                                   float* part, double* lpart) {
   double sq = 0.0;
   float col = 0.f;
   const float scale = 2.0f / (float)(B * kMlpOut);
@@ -318,19 +335,6 @@ __global__ void __launch_bounds__(256) k_loss_grad(long B, const float* O, const
     double s = 0.0;
     for (int q = 0; q < 8; ++q) s += sp[q];
     lpart[blockIdx.x] = s;
-  }
-  if (!last_block(tick, gridDim.x)) return;
-  if (threadIdx.x < kMlpOutPad) {
-    float s = 0.f;
-#pragma unroll 8
-    for (int t = 0; t < (int)gridDim.x; ++t) s += __ldcg(part + t * kMlpOutPad + threadIdx.x);
-    db[threadIdx.x] = s;
-  }
-  if (threadIdx.x == 32) {
-    double s = 0.0;
-#pragma unroll 8
-    for (int t = 0; t < (int)gridDim.x; ++t) s += __ldcg(lpart + t);
-    *loss += s / (double)(B * kMlpOut);
   }
 }
 
@@ -1180,9 +1184,8 @@ struct Surrogate {
   float *Z[kMlpLayers] = {}, *O = nullptr;
   __nv_bfloat16* dOb = nullptr;
   float* Yb = nullptr;
-  float* part = nullptr;          // sums of the training blocks (bias gradients)
-  double* lpart = nullptr;        // and of the loss
-  unsigned int* tick = nullptr;   // blocks done, zero between launches
+  float* part[2] = {};      // the training blocks' column sums (alternate launches)
+  double* lpart = nullptr;  // and squared errors
   int* idx = nullptr;
   double* d_loss = nullptr;
   // inference buffers (features, two activation buffers, outputs)
@@ -1316,11 +1319,11 @@ static void free_act(Surrogate* s) {
     s->Z[l] = nullptr;
   }
   cudaFree(s->dHb[0]); cudaFree(s->dHb[1]); cudaFree(s->O); cudaFree(s->dOb);
-  cudaFree(s->Yb); cudaFree(s->idx); cudaFree(s->part); cudaFree(s->lpart); cudaFree(s->tick);
+  cudaFree(s->Yb); cudaFree(s->idx); cudaFree(s->part[0]); cudaFree(s->part[1]);
+  cudaFree(s->lpart);
   s->X = s->dHb[0] = s->dHb[1] = s->dOb = nullptr;
-  s->O = s->Yb = s->part = nullptr;
+  s->O = s->Yb = s->part[0] = s->part[1] = nullptr;
   s->lpart = nullptr;
-  s->tick = nullptr;
   s->idx = nullptr;
   s->cap = 0;
 }
@@ -1404,11 +1407,9 @@ static std::string ensure_act(Surrogate* s, long n) {
   if ((e = ck(cudaMalloc(&s->Yb, np * kMlpOut * 4), "alloc Y")).size()) return e;
   if ((e = ck(cudaMalloc(&s->idx, np * 4), "alloc idx")).size()) return e;
   const long rows = std::max<long>((np + 127) / 128 * 128, kLossBlocks * kMlpOutPad);
-  if ((e = ck(cudaMalloc(&s->part, rows * 4), "alloc sums")).size()) return e;
+  for (auto& p : s->part)
+    if ((e = ck(cudaMalloc(&p, rows * 4), "alloc sums")).size()) return e;
   if ((e = ck(cudaMalloc(&s->lpart, kLossBlocks * 8), "alloc sums")).size()) return e;
-  if ((e = ck(cudaMalloc(&s->tick, 4), "alloc count")).size()) return e;
-  if ((e = ck(cudaMemset(s->tick, 0, 4), "clear count")).size()) return e;
-  if ((e = ck(cudaStreamSynchronize(nullptr), "clear count")).size()) return e;
   s->cap = np;
   return "";
 }
@@ -1526,8 +1527,8 @@ static cudaError_t forward(Surrogate* s, long n, const __nv_bfloat16* x, float* 
   const __nv_bfloat16* in = x;
   for (int l = 0; l < kMlpLayers; ++l) {
     const bool last = l == kMlpLayers - 1;
-    cudaError_t e = launch_gemm(fwd_job(s, l, n, in, last ? out : s->Z[l], last ? nullptr : s->H[l]), GemmJob{}, st,
-                                s->d_err);
+    cudaError_t e = launch_gemm(fwd_job(s, l, n, in, last ? out : s->Z[l], last ? nullptr : s->H[l]), GemmJob{}, SumJob{},
+                                st, s->d_err);
     if (e != cudaSuccess) return e;
     in = s->H[l];
   }
@@ -1562,7 +1563,7 @@ static cudaError_t forward_infer(Surrogate* s, long n, const __nv_bfloat16* x, f
   for (int l = 0; l < kMlpLayers; ++l) {
     const bool last = l == kMlpLayers - 1;
     cudaError_t e = launch_gemm(fwd_job(s, l, n, in, last ? out : nullptr, last ? nullptr : s->iH[l & 1]), GemmJob{},
-                                st, s->d_err);
+                                SumJob{}, st, s->d_err);
     if (e != cudaSuccess) return e;
     in = s->iH[l & 1];
   }
@@ -1574,8 +1575,11 @@ static cudaError_t backward(Surrogate* s, long B, const __nv_bfloat16* x, const 
   cudaError_t e = cudaMemsetAsync(s->gr, 0, sizeof(float) * (size_t)s->n_params, st);
   if (e == cudaSuccess) e = forward(s, B, x, s->O, st);
   if (e != cudaSuccess) return e;
-  k_loss_grad<<<std::min<long>((B * kMlpOutPad + 255) / 256, kLossBlocks), 256, 0, st>>>(
-      B, s->O, y, s->dOb, s->gr + s->offb[kMlpLayers - 1], s->d_loss, s->part, s->lpart, s->tick);
+  const int lb = (int)std::min<long>((B * kMlpOutPad + 255) / 256, kLossBlocks);
+  k_loss_grad<<<lb, 256, 0, st>>>(B, s->O, y, s->dOb, s->part[kMlpLayers & 1], s->lpart);
+  // each launch adds up the column sums that the one before left
+  SumJob sum{lb, kMlpOutPad, s->part[kMlpLayers & 1], s->gr + s->offb[kMlpLayers - 1],
+             s->lpart, s->d_loss, 1.0 / (double)(B * kMlpOut)};
   const __nv_bfloat16* dZ = s->dOb;
   for (int l = kMlpLayers - 1; l >= 0; --l) {
     // dW[out][in] = sum_b dZ[b][out] Hin[b][in]
@@ -1600,11 +1604,10 @@ static cudaError_t backward(Surrogate* s, long B, const __nv_bfloat16* x, const 
       h.b_mn = 1;
       h.H = dH;
       h.Z = s->Z[l - 1];
-      h.db = s->gr + s->offb[l - 1];
-      h.part = s->part;
-      h.tick = s->tick;
+      h.part = s->part[l & 1];
     }
-    if ((e = launch_gemm(h, w, st, s->d_err)) != cudaSuccess) return e;
+    if ((e = launch_gemm(h, w, sum, st, s->d_err)) != cudaSuccess) return e;
+    sum = SumJob{(int)((B + 127) / 128), kMlpHid, h.part, l > 0 ? s->gr + s->offb[l - 1] : nullptr, nullptr, nullptr, 0.0};
     dZ = dH;
   }
   return cudaGetLastError();
