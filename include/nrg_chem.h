@@ -287,13 +287,15 @@ NRG_API int nrg_chem_get_launch(nrg_chem* h, int* kernel, int* block, int* grid,
  * unrolled over the integrated species, 1 a loop.  Same results; the
  * unrolled form is faster where neighbouring cells take alike BDF paths
  * (the flame field), the loop, with a quarter of the code, where they vary
- * (ignition and wide-range fields).  nrg_chem_autotune tries both.  Without
- * effect on the analytic-Jacobian and mixed kernels, which have one form. */
+ * (ignition and wide-range fields).  Without effect on the analytic-Jacobian
+ * and mixed kernels, which have one form; for the others nrg_chem_autotune
+ * tries both. */
 NRG_API int nrg_chem_set_lu_form(nrg_chem* h, int rolled);
 NRG_API int nrg_chem_get_lu_form(nrg_chem* h, int* rolled);
 
 /* Times candidate launch shapes on the given device-resident inputs (outputs
- * are scratch) and keeps the fastest for this handle.  ms_best may be NULL. */
+ * are scratch) and keeps the fastest for this handle.  Where block and LU form
+ * have no effect the handle's stay as they are.  ms_best may be NULL. */
 NRG_API int nrg_chem_autotune(nrg_chem* h, double time_step, long n, long ld, const double* T,
                       const double* rho, const double* Y, const signed char* bc, double* Y_prod,
                       double* Y_prod2, double* E_f_prod, double* ms_best);

@@ -1172,7 +1172,11 @@ extern "C" int nrg_chem_autotune(nrg_chem* h, double time_step, long n, long ld,
   // candidate shapes: warp per cell (occupancy-derived persistent grid),
   // thread per cell from the work queue (1 or 2 blocks of 64 per SM, chunk 1
   // or 2) and thread per cell over the plain grid (32- or 64-thread blocks, LU
-  // unrolled or as a loop)
+  // unrolled or as a loop).  The integrator in passes chooses its blocks and
+  // has one LU form, so there the grid is one candidate, the caller's block and
+  // LU form are kept for the kernels they matter to, and the queue's blocks
+  // are the 2 or 4 of 64 that fit an SM.
+  const bool passes = nrg::integrates_in_passes(jac_of(h->mode), h->dmr.NI);
   std::vector<LaunchCfg> cands;
   for (int block : {128, 256}) {
     LaunchCfg c;
@@ -1182,8 +1186,9 @@ extern "C" int nrg_chem_autotune(nrg_chem* h, double time_step, long n, long ld,
     c.chunk = 1;
     cands.push_back(c);
   }
-  for (int per_sm : {1, 2})
+  for (int half : {1, 2})
     for (int chunk : {1, 2}) {
+      const int per_sm = passes ? 2 * half : half;
       LaunchCfg c;
       c.kernel = nrg::kKernelThreadQueue;
       c.block = 64;
@@ -1191,14 +1196,24 @@ extern "C" int nrg_chem_autotune(nrg_chem* h, double time_step, long n, long ld,
       c.chunk = chunk;
       cands.push_back(c);
     }
-  for (int block : {32, 64})
-    for (int rolled : {0, 1}) {
-      LaunchCfg c;
-      c.kernel = nrg::kKernelThreadGrid;
-      c.block = block;
-      c.lu_rolled = rolled;
-      cands.push_back(c);
+  if (passes) {
+    LaunchCfg c;
+    c.kernel = nrg::kKernelThreadGrid;
+    cands.push_back(c);
+    for (LaunchCfg& k : cands) {
+      k.lu_rolled = h->cfg.lu_rolled;
+      if (k.kernel != nrg::kKernelWarpQueue && h->cfg.kernel != nrg::kKernelWarpQueue) k.block = h->cfg.block;
     }
+  } else {
+    for (int block : {32, 64})
+      for (int rolled : {0, 1}) {
+        LaunchCfg c;
+        c.kernel = nrg::kKernelThreadGrid;
+        c.block = block;
+        c.lu_rolled = rolled;
+        cands.push_back(c);
+      }
+  }
   cudaStream_t s = h->stream;
   float best = 1e30f;
   LaunchCfg best_cfg = h->cfg;

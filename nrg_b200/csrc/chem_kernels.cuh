@@ -346,7 +346,7 @@ static cudaError_t launch_warp(const StepArgs& a, const LaunchCfg& cfg, int* que
 template <int NF, int NI, int R, int JAC, typename LUT, int SPEC>
 static cudaError_t launch_thread(const StepArgs& a, const LaunchCfg& cfg, int* queue, unsigned long long* counters,
                                  cudaStream_t s) {
-  if constexpr (JAC == kJacAnalytic && NI != 9) {
+  if constexpr (integrates_in_passes(JAC, NI)) {
     return launch_pass<NI, R, LUT, NF, SPEC>(a, cfg, queue, counters, s);
   } else {
     switch (cfg.block) {

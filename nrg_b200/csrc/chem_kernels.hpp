@@ -83,6 +83,10 @@ bool supported_mechanism(int n_species, int n_reactions);
 // (reference mode), 0 when none does.
 int match_specialised(const DevMech& reduced);
 int match_specialised_full(const DevMech& full);
+// Whether the thread-per-cell kernels of n_int integrated species run in passes
+// (they then choose their blocks themselves and have one LU form): analytic
+// Jacobian, but for the nine-species mechanisms that no generated code covers.
+constexpr bool integrates_in_passes(int jac, int n_int) { return jac != 0 && n_int != 9; }
 cudaError_t launch_chem(int n_species, int n_int, int spec, int n_reactions, int jac, bool mixed, const StepArgs& a,
                         const LaunchCfg& cfg, int* queue, unsigned long long* counters,
                         cudaStream_t s);

@@ -69,3 +69,22 @@ def test_launches_agree_and_match_the_oracle(name, mode, first, more):
     assert np.max(np.abs(whole["Y_prod"][:, :m] - o["Y_prod"]) * h.dt / h.rho) <= 1e-9
     assert np.max(np.abs(whole["T_after"][:m] - T1) / h.T) <= 1e-6
     np.testing.assert_array_equal(whole["status"][:m] != 0, h.T >= 305.0)
+
+
+def test_autotuner_keeps_what_has_no_effect(decks):
+    """In the fast mode the block and the LU form of the thread kernels select
+    nothing: the autotuner leaves them as they were set, for the reference mode
+    after it, and tries both there."""
+    import torch
+    from nrg_b200.chemistry import ChemicalKineticsSolver
+    f = fields.random_field(fields_W())
+    T, rho, Y = (torch.tensor(a, device="cuda") for a in (f.T, f.rho, f.Y))
+    s = ChemicalKineticsSolver(None, *decks, mode="fast")
+    try:
+        for block, rolled in ((32, True), (64, False), (64, True), (32, False)):
+            s.set_launch(kernel="thread", block=block, lu_rolled=rolled)
+            assert s.autotune(f.dt, T, rho, Y, torch.zeros_like(Y), torch.zeros_like(Y), torch.zeros_like(T)) > 0.0
+            d = s.get_launch()
+            assert d["kernel"] in ("thread", "thread_queue") and d["block"] == block and d["lu_rolled"] is rolled, d
+    finally:
+        s.close()
