@@ -14,6 +14,8 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "chem_bdf.cuh"
 #include "chem_kernels.hpp"
 #include "chem_pass.cuh"
@@ -112,6 +114,14 @@ __global__ void __launch_bounds__(BS, 1) k_chem_queue(StepArgs a, int* queue, in
   if (counters) block_flush_counters(counters, v);
 }
 
+// Blocks of a work-queue launch: no more than have a cell to start with, and
+// few enough that the reservations past the end (up to 64 cells from each of 64
+// lanes a block) leave the int queue head far from overflow.
+static int queue_blocks(int grid, const StepArgs& a, int cells_per_block) {
+  const long nl = a.cell_list ? (long)a.n_list : a.n;
+  return (int)std::max<long>(1, std::min<long>({(long)grid, (nl + cells_per_block - 1) / cells_per_block, 65536L}));
+}
+
 template <int N, int R, int JAC, typename LUT, int BS, int NF, int SPEC>
 static cudaError_t launch_bs(const StepArgs& a, const LaunchCfg& cfg, int* queue,
                              unsigned long long* counters, cudaStream_t s) {
@@ -121,7 +131,7 @@ static cudaError_t launch_bs(const StepArgs& a, const LaunchCfg& cfg, int* queue
     e = cudaFuncSetAttribute(k_chem_queue<N, R, JAC, LUT, BS, NF, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
     if (e != cudaSuccess) return e;
-    const int grid = cfg.grid > 0 ? cfg.grid : 148;
+    const int grid = queue_blocks(cfg.grid > 0 ? cfg.grid : 148, a, BS);
     k_chem_queue<N, R, JAC, LUT, BS, NF, SPEC><<<grid, BS, smem, s>>>(a, queue, cfg.chunk, counters);
   } else {
     e = cudaFuncSetAttribute(k_chem_plain<N, R, JAC, LUT, BS, NF, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -236,8 +246,8 @@ static cudaError_t launch_pass(const StepArgs& a, const LaunchCfg& cfg, int* que
                                cudaStream_t s) {
   if constexpr (N <= 8) {
     if (cfg.kernel == kKernelThreadQueue)
-      return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, true>(a, cfg.grid > 0 ? cfg.grid : 148, queue, cfg.chunk,
-                                                                  counters, s);
+      return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, true>(a, queue_blocks(cfg.grid > 0 ? cfg.grid : 148, a, 64),
+                                                                  queue, cfg.chunk, counters, s);
   }
   const long nl = a.cell_list ? (long)a.n_list : a.n;
   if constexpr (N <= 8) {
@@ -335,6 +345,7 @@ static cudaError_t launch_warp(const StepArgs& a, const LaunchCfg& cfg, int* que
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_chem_warp<N, R, JAC, LUT, WARPS>, WARPS * 32, smem);
     grid = sms * (per_sm > 0 ? per_sm : 1);
   }
+  grid = queue_blocks(grid, a, WARPS);
   k_chem_warp<N, R, JAC, LUT, WARPS><<<grid, WARPS * 32, smem, s>>>(a, queue, cfg.chunk, counters);
   return cudaGetLastError();
 }

@@ -88,3 +88,21 @@ def test_autotuner_keeps_what_has_no_effect(decks):
             assert d["kernel"] in ("thread", "thread_queue") and d["block"] == block and d["lu_rolled"] is rolled, d
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("mode,kernel,block", [("fast", "thread_queue", 64), ("reference", "thread_queue", 32),
+                                               ("fast", "warp_queue", 256)])
+def test_a_queue_of_more_blocks_than_cells(decks, mode, kernel, block):
+    """The largest grid that nrg_chem_set_launch takes: blocks without a cell are
+    not launched (their reservations would carry the queue head past the end
+    of an int), the cells' bits stay."""
+    from nrg_b200.chemistry import ChemicalKineticsSolver
+    f = fields.slice_field(fields.random_field(fields_W()), 200)
+    s = ChemicalKineticsSolver(None, *decks, mode=mode)
+    try:
+        a, b = (run_device(s, f, mode, launch=dict(kernel=kernel, block=block, grid=grid, chunk=64))[0]
+                for grid in (3, 2**31 - 1))
+    finally:
+        s.close()
+    for k in KEYS:
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)
