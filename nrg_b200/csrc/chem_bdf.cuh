@@ -360,42 +360,72 @@ __device__ void rate_constants_fast(CS& c, double Tin) {
   }
 }
 
+// The NU updates of reaction r by +-q: at(k) is the accumulator of species k.  All
+// are read before the first is written (a species that occurs twice has adjacent
+// entries and is carried on), so that a reaction's updates wait for shared
+// memory once and not one after the other, and one jump on their number takes
+// the place of a branch for each.
+template <int NU, typename T, class At>
+__device__ __forceinline__ void update_species(int r, double q, const At& at) {
+  int k[NU];
+  T v[NU];
+#pragma unroll
+  for (int u = 0; u < NU; ++u) {
+    k[u] = c_mech.upd_k[r][u];
+    v[u] = at(k[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < NU; ++u) {
+    if (u > 0) v[u] = k[u] == k[u - 1] ? v[u - 1] : v[u];
+    v[u] = (T)__dadd_rn((double)v[u], c_mech.upd_prod[r][u] ? q : -q);
+  }
+#pragma unroll
+  for (int u = 0; u < NU; ++u) at(k[u]) = v[u];
+}
+
+template <typename T, class At>
+__device__ __forceinline__ void update_species(int nu, int r, double q, const At& at) {
+  switch (nu) {
+    case 2: update_species<2, T>(r, q, at); break;
+    case 3: update_species<3, T>(r, q, at); break;
+    case 4: update_species<4, T>(r, q, at); break;
+    case 5: update_species<5, T>(r, q, at); break;
+    case 6: update_species<6, T>(r, q, at); break;
+    default:
+      if (nu == 1) update_species<1, T>(r, q, at);
+  }
+}
+
 // fun (chemical_kinetics_solver.f90:495-540): zd = dC/dt at z (both in the
 // cell's shared scratch), accumulated per reaction as the net rate f - b.
 template <int N, class CS>
 __device__ __forceinline__ void rhs(CS& c, int R) {
 #pragma unroll
   for (int k = 0; k < N; ++k) c.zd(k) = 0.0;
-// Fixed-trip inner loops (3 reactant and 3 product slots, unused and M
-// slots hold -1 and multiply by 1.0, which leaves every product unchanged; 6
-// update slots under a predicate): no data-dependent branches per reaction.
-// Explicitly rounded operations (never fused into FMAs) make the result
+// 3 reactant and 3 product slots: unused and M slots hold -1 and multiply by
+// 1.0, which leaves every product unchanged.  The walk waits for dependent
+// shared-memory reads, so a reaction's operands are read before the updates of
+// the one before it.  Explicitly rounded operations (never fused into FMAs) make the result
 // independent of how the compiler schedules this loop, so the generated
 // straight-line version (gen_keromnes.cuh) gives the same bits.
+  double f, b, zl[3], zr[3];
+  const auto load = [&](int r) {
+    f = c.kf(r);
+    b = c.kr(r);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int sl = c_mech.left[r][i], sr = c_mech.right[r][i];
+      zl[i] = sl >= 0 ? c.z(sl) : 1.0;
+      zr[i] = sr >= 0 ? c.z(sr) : 1.0;
+    }
+  };
+  load(0);
 #pragma unroll 1
   for (int r = 0; r < R; ++r) {
-    double f = c.kf(r);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const int sp = c_mech.left[r][i];
-      f = __dmul_rn(f, sp >= 0 ? c.z(sp) : 1.0);
-    }
-    double b = c.kr(r);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const int sp = c_mech.right[r][i];
-      b = __dmul_rn(b, sp >= 0 ? c.z(sp) : 1.0);
-    }
-    const double q = __dsub_rn(f, b);
-    const int nu = c_mech.nupd[r];
-#pragma unroll
-    for (int u = 0; u < 6; ++u) {
-      if (u < nu) {
-        const int k = c_mech.upd_k[r][u];
-        const double v = c.zd(k);
-        c.zd(k) = c_mech.upd_prod[r][u] ? __dadd_rn(v, q) : __dsub_rn(v, q);
-      }
-    }
+    const double q = __dsub_rn(__dmul_rn(__dmul_rn(__dmul_rn(f, zl[0]), zl[1]), zl[2]),
+                               __dmul_rn(__dmul_rn(__dmul_rn(b, zr[0]), zr[1]), zr[2]));
+    load(r + 1 < R ? r + 1 : r);
+    update_species<double>(c_mech.nupd[r], r, q, [&](int k) -> double& { return c.zd(k); });
   }
 }
 
@@ -418,35 +448,40 @@ __device__ void analytic_iteration_matrix(CS& c, double factor, int R) {
   for (int j = 0; j < N; ++j)
 #pragma unroll
     for (int i = 0; i < N; ++i) c.a(j, i) = 0;
+  double k[2], z[2][3];
+  int sp[2][3];
+  const auto load = [&](int r) {
+    k[0] = c.kf(r);
+    k[1] = c.kr(r);
+#pragma unroll
+    for (int side = 0; side < 2; ++side)
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        sp[side][p] = side ? c_mech.right[r][p] : c_mech.left[r][p];
+        z[side][p] = sp[side][p] >= 0 ? c.z(sp[side][p]) : 1.0;
+      }
+  };
+  load(0);
 #pragma unroll 1
   for (int r = 0; r < R; ++r) {
     const int nu = c_mech.nupd[r];
+    double d[2][3];  // d(f - b) / dz
+    int col[2][3];
 #pragma unroll
-    for (int side = 0; side < 2; ++side) {
-      const double k = side ? c.kr(r) : c.kf(r);
-      const double sgn = side ? -factor : factor;  // d(f - b)
+    for (int side = 0; side < 2; ++side)
 #pragma unroll
       for (int p = 0; p < 3; ++p) {
-        const int sp = side ? c_mech.right[r][p] : c_mech.left[r][p];
-        if (sp < 0) continue;
-        double d = k;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          if (q == p) continue;
-          const int sq = side ? c_mech.right[r][q] : c_mech.left[r][q];
-          d = __dmul_rn(d, sq >= 0 ? c.z(sq) : 1.0);
-        }
-        d = __dmul_rn(d, sgn);
-#pragma unroll
-        for (int u = 0; u < 6; ++u) {
-          if (u < nu) {
-            const int k2 = c_mech.upd_k[r][u];
-            const double v = (double)c.a(sp, k2);
-            c.a(sp, k2) = (LUT_T)(c_mech.upd_prod[r][u] ? __dadd_rn(v, d) : __dsub_rn(v, d));
-          }
-        }
+        d[side][p] = __dmul_rn(__dmul_rn(__dmul_rn(k[side], z[side][p == 0 ? 1 : 0]), z[side][p == 2 ? 1 : 2]),
+                               side ? -factor : factor);
+        col[side][p] = sp[side][p];
       }
-    }
+    load(r + 1 < R ? r + 1 : r);
+#pragma unroll
+    for (int side = 0; side < 2; ++side)
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        if (col[side][p] >= 0)
+          update_species<LUT_T>(nu, r, d[side][p], [&](int i) -> LUT_T& { return c.a(col[side][p], i); });
   }
 #pragma unroll
   for (int i = 0; i < N; ++i) c.a(i, i) += 1;

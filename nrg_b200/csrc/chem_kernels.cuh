@@ -223,22 +223,32 @@ static cudaError_t launch_pass_bs(const StepArgs& a, long grid, int* queue, int 
   const auto kern = k_chem_pass<N, R, LUT, BS, NF, SPEC, LOCK, QUEUE, TM>;
   const int smem = BS * PassStore<N, RateSlots<R, SPEC>::value, LUT, SPEC == 0, TM>::kBytesPerThread;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  // lockstep blocks of larger mechanisms spill part of the Nordsieck array: what
-  // shared memory their one or two blocks per SM leave goes to the L1 cache
-  // (KONNOV flame of 196,608 cells 26.9 -> 22.8 ms)
-  const int used = (smem + 1024) * (smem < 115000 ? 2 : 1);
-  const int carveout = N > 8 && LOCK ? (100 * used + 233471) / 233472 : 100;
+  // larger mechanisms spill part of the Nordsieck array: what shared memory the
+  // blocks of an SM leave goes to the L1 cache (KONNOV flame of 196,608 cells in
+  // lockstep 26.9 -> 22.8 ms; 9,472 random cells on their own 5.71 -> 4.84 ms).
+  const int fit = std::max(1, 232448 / (smem + 1024));
+  const int used = (smem + 1024) * fit;
+  const int carveout = N > 8 ? (100 * used + 233471) / 233472 : 100;
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
   if (e != cudaSuccess) return e;
   if (grid > 0) kern<<<(unsigned)grid, BS, smem, s>>>(a, queue, chunk, counters);
   return cudaGetLastError();
 }
 
-// Blocks of 128 threads in lockstep, two per SM, from kLockstepCells cells on
-// (one wave of them on 148 SMs); below, 64-thread blocks whose warps run on
-// their own: the cells then spread over more SMs and nothing waits for another
-// warp.  2048 x 2048 flame 32.1 ms on their own, 29.2 ms in lockstep; 512 x
-// 512 ignition field 22.1 and 18.8 ms; 64 x 64 random cells 1.15 and 1.29 ms.
+// Up to 8 integrated species with generated code: blocks of 128 threads in
+// lockstep from kLockstepCells cells on, the places of two such blocks on each
+// of 148 SMs (a list counts with its capacity, which the host knows); below,
+// 64-thread blocks whose warps run on their own: the cells then spread over more
+// SMs and nothing waits for another warp.  KEROMNES (880 B a cell, two blocks
+// fit): 37,888 random cells 1.90 ms on their own and 1.48 ms in lockstep, 196,608
+// 9.18 and 6.47 ms, a flame of 196,608 2.36 and 2.10 ms; 4,096 random cells 1.15
+// and 1.29 ms.  ZHANG (976 B, one block fits): 37,888 random cells 2.95 and 2.48
+// ms, a flame of 196,608 3.41 and 3.22 ms.
+//
+// Table walks are bound by the latency of their dependent reads, which more
+// warps of their own hide better: 64-thread blocks at any size (KEROMNES, three
+// fit: 196,608 random cells 26.5 ms against 29.9 ms in lockstep, a flame 8.0
+// against 10.2; 32-thread blocks above 8 species).
 constexpr long kLockstepCells = 148L * 2 * 128;
 
 template <int N, int R, typename LUT, int NF, int SPEC>
@@ -251,27 +261,31 @@ static cudaError_t launch_pass(const StepArgs& a, const LaunchCfg& cfg, int* que
   }
   const long nl = a.cell_list ? (long)a.n_list : a.n;
   if constexpr (N <= 8) {
-    if (nl < kLockstepCells)
-      return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, false>(a, (nl + 63) / 64, queue, 0, counters, s);
-    return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false>(a, (nl + 127) / 128, queue, 0, counters, s);
-  } else {
-    // as many warps as the cells' shared memory allows, one block per SM; with the
-    // generated code in blocks of 128 threads with the rate constants in tensor
-    // memory, where more warps fit that way (KONNOV 2 -> 4 warps, TEREZA 5 -> 8;
-    // flame of 196,608 cells 46.4 -> 26.9 ms and 11.7 -> 9.0 ms)
-    constexpr int RS = RateSlots<R, SPEC>::value;
-    constexpr int kWarpBytes = 32 * PassStore<N, RS, LUT, SPEC == 0>::kBytesPerThread;
-    constexpr int W = 232448 / kWarpBytes < 8 ? 232448 / kWarpBytes : 8;
-    if (nl < 148L * 32 * W)
-      return launch_pass_bs<N, R, LUT, 32, NF, SPEC, false, false>(a, (nl + 31) / 32, queue, 0, counters, s);
     if constexpr (SPEC != 0) {
+      if (nl >= kLockstepCells)
+        return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false>(a, (nl + 127) / 128, queue, 0, counters, s);
+    }
+    return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, false>(a, (nl + 63) / 64, queue, 0, counters, s);
+  } else {
+    if constexpr (SPEC != 0) {
+      // as many warps as the cells' shared memory allows, one block per SM, or blocks
+      // of 128 threads with the rate constants in tensor memory, where more warps fit
+      // that way (KONNOV 2 -> 4 warps, TEREZA 5 -> 8; flame of 196,608 cells 46.4 ->
+      // 26.9 ms and 11.7 -> 9.0 ms)
+      constexpr int RS = RateSlots<R, SPEC>::value;
+      constexpr int kWarpBytes = 32 * PassStore<N, RS, LUT, false>::kBytesPerThread;
+      constexpr int W = 232448 / kWarpBytes < 8 ? 232448 / kWarpBytes : 8;
       constexpr int kTmBytes = 128 * PassStore<N, RS, LUT, false, true>::kBytesPerThread;
       constexpr int kTmWarps = kTmBytes > 232448 ? 0 : kTmBytes > 115000 ? 4 : 8;
-      if constexpr (kTmWarps > W)
-        return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false, true>(a, (nl + 127) / 128, queue, 0, counters, s);
+      if constexpr (kTmWarps > W) {
+        if (nl >= 148L * 32 * W)
+          return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false, true>(a, (nl + 127) / 128, queue, 0, counters, s);
+      } else if (nl >= 148L * 32 * W) {
+        return launch_pass_bs<N, R, LUT, 32 * W, NF, SPEC, true, false>(a, (nl + 32 * W - 1) / (32 * W), queue, 0,
+                                                                        counters, s);
+      }
     }
-    return launch_pass_bs<N, R, LUT, 32 * W, NF, SPEC, true, false>(a, (nl + 32 * W - 1) / (32 * W), queue, 0,
-                                                                    counters, s);
+    return launch_pass_bs<N, R, LUT, 32, NF, SPEC, false, false>(a, (nl + 31) / 32, queue, 0, counters, s);
   }
 }
 

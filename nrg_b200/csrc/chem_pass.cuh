@@ -177,6 +177,17 @@ struct TabView {
   __device__ __forceinline__ lut_t& a(int j, int i) { return st.a(j, i); }
 };
 
+// The table walks are functions of their own: inlined they had the registers the
+// Nordsieck array leaves, and took 1.4 to 1.6 times as long (KONNOV, ACETYLENE).
+template <int N, class S>
+__device__ __noinline__ void pass_walk_rhs(double* d) {
+  S st;
+  st.d = d;
+  st.f = nullptr;
+  TabView<S, N> v{st};
+  rhs<N>(v, c_mech.RM);
+}
+
 template <int N, int R, int SPEC, class S>
 __device__ __forceinline__ void pass_rhs(const S& st, const double (&y)[N], double (&out)[N]) {
   if constexpr (SPEC != 0) {
@@ -194,7 +205,7 @@ __device__ __forceinline__ void pass_rhs(const S& st, const double (&y)[N], doub
     TabView<S, N> v{st};
 #pragma unroll
     for (int k = 0; k < N; ++k) v.z(k) = y[k];
-    rhs<N>(v, c_mech.RM);
+    pass_walk_rhs<N, S>(st.d);
 #pragma unroll
     for (int k = 0; k < N; ++k) out[k] = v.zd(k);
   }
@@ -274,9 +285,10 @@ __device__ __forceinline__ void pass_factor_columns(const V& view, const S& st, 
   if constexpr (J + 1 < N) pass_factor_columns<N, SPEC, J + 1>(view, st, factor, perm, ok, commit);
 }
 
-// dgefa<RECIP> on the LU storage as two loops over whole columns (rows above
-// the pivot get a zero multiplier, which changes nothing): the operations of
-// pass_factor_columns in a tenth of its code.
+// dgefa<RECIP> on the LU storage as two loops over columns (rows above the pivot
+// get a zero multiplier, which changes nothing): the operations of
+// pass_factor_columns in a tenth of its code.  A zero of the pivot row, where
+// the species' reactions do not meet, leaves its column as it is.
 template <int N, class S>
 __device__ __forceinline__ bool pass_lu_loop(const S& st, RowPerm<N>& perm) {
   using LUT = typename S::lut_t;
@@ -316,12 +328,30 @@ __device__ __forceinline__ bool pass_lu_loop(const S& st, RowPerm<N>& perm) {
       const LUT tj = cj[l * BS];
       cj[l * BS] = cj[k * BS];
       cj[k * BS] = tj;
-      if (j > k) {
+      if (j > k && tj != (LUT)0) {
+        constexpr int H = N / 2;  // rows 1..H-1 only while some lie below the pivot
+        if (k < H - 1) {
 #pragma unroll
-        for (int i = 1; i < N; ++i) cj[i * BS] = lu_axpy<LUT, true>(cj[i * BS], tj, c[i]);
+          for (int i = 1; i < H; ++i) cj[i * BS] = lu_axpy<LUT, true>(cj[i * BS], tj, c[i]);
+        }
+#pragma unroll
+        for (int i = H; i < N; ++i) cj[i * BS] = lu_axpy<LUT, true>(cj[i * BS], tj, c[i]);
       }
     }
   }
+  return ok;
+}
+
+template <int N, class S>
+__device__ __noinline__ bool pass_walk_factor(double* d, typename S::lut_t* f, double factor, RowPerm<N>* perm) {
+  S st;
+  st.d = d;
+  st.f = f;
+  TabView<S, N> v{st};
+  analytic_iteration_matrix<N>(v, factor, c_mech.RM);
+  RowPerm<N> p;
+  const bool ok = pass_lu_loop<N>(st, p);
+  *perm = p;
   return ok;
 }
 
@@ -339,8 +369,10 @@ __device__ __forceinline__ bool pass_factor(const S& st, const double (&y)[N], d
     TabView<S, N> v{st};
 #pragma unroll
     for (int k = 0; k < N; ++k) v.z(k) = y[k];
-    analytic_iteration_matrix<N>(v, factor, c_mech.RM);
-    return pass_lu_loop<N>(st, perm);
+    RowPerm<N> p;
+    const bool ok = pass_walk_factor<N, S>(st.d, st.f, factor, &p);
+    perm = p;
+    return ok;
   }
 }
 
@@ -650,9 +682,11 @@ __device__ __forceinline__ int pass_integrate(const S& st, const StepArgs& a, bo
     // ---- iteration matrix and its factors (DDPST) where due.  They cost more
     // than the rest of a pass, so they are made when half of the live lanes
     // (of the warp, or of the block in lockstep) wait for theirs; a waiting
-    // lane sits passes out.  The lanes' own sequences do not change.
+    // lane sits passes out.  The lanes' own sequences do not change.  Table
+    // walks: two thirds (196,608 random cells, KONNOV: half 255 ms, two thirds
+    // 244, all 319 before the walk read ahead; ACETYLENE 122.5 and 119.8 ms).
     const bool due = run && (pred || phase == kRedo || phase == kWait) && (evaljc || ier);
-        const bool make = 2 * pass_count<LOCK>(due) >= nrun;
+    const bool make = (SPEC == 0 ? 3 : 4) * pass_count<LOCK>(due) >= 2 * nrun;
     const bool need = due && make;
     if (due) phase = make ? kPredict : kWait;
     const double jac_factor = -(EL(1, nq) * h);

@@ -52,6 +52,12 @@ def test_launches_agree_and_match_the_oracle(name, mode, first, more):
             g, _ = run_device(s, fields.slice_field(f, part), mode)
             for k in KEYS:
                 np.testing.assert_array_equal(g[k], whole[k][..., :part], err_msg=f"{k} {part}")
+        s.set_specialised(False)  # the table walk, in blocks of its own at any size
+        for part in (129, f.n):
+            g, _ = run_device(s, fields.slice_field(f, part), mode)
+            for k in KEYS:
+                np.testing.assert_array_equal(g[k], whole[k][..., :part], err_msg=f"{k} tables {part}")
+        s.set_specialised(True)
         if name == "KEROMNES":
             # grid 1: each warp sets up some sixteen groups in the shared memory of the one before
             for grid, chunk in ((7, 3), (1, 1)):
