@@ -226,8 +226,11 @@ static cudaError_t launch_pass_bs(const StepArgs& a, long grid, int* queue, int 
   // larger mechanisms spill part of the Nordsieck array: what shared memory the
   // blocks of an SM leave goes to the L1 cache (KONNOV flame of 196,608 cells in
   // lockstep 26.9 -> 22.8 ms; 9,472 random cells on their own 5.71 -> 4.84 ms).
+  // Above 10 species (1 KB and more a thread) two blocks, though a third of
+  // ACETYLENE's fits (flame of 18,944 cells 3.31 -> 2.59 ms, random cells 9.46 ->
+  // 8.12 ms).
   const int fit = std::max(1, 232448 / (smem + 1024));
-  const int used = (smem + 1024) * fit;
+  const int used = (smem + 1024) * (N > 10 ? std::min(fit, 2) : fit);
   const int carveout = N > 8 ? (100 * used + 233471) / 233472 : 100;
   if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
   if (e != cudaSuccess) return e;
@@ -268,19 +271,23 @@ static cudaError_t launch_pass(const StepArgs& a, const LaunchCfg& cfg, int* que
     return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, false>(a, (nl + 63) / 64, queue, 0, counters, s);
   } else {
     if constexpr (SPEC != 0) {
-      // as many warps as the cells' shared memory allows, one block per SM, or blocks
-      // of 128 threads with the rate constants in tensor memory, where more warps fit
-      // that way (KONNOV 2 -> 4 warps, TEREZA 5 -> 8; flame of 196,608 cells 46.4 ->
-      // 26.9 ms and 11.7 -> 9.0 ms)
+      // W: the warps of a SM's shared memory.  More fit in blocks of 128 threads with
+      // the rate constants in tensor memory for KONNOV (2 -> 4) and TEREZA (5 -> 8):
+      // these from one more cell than the W warps take at once (KONNOV, 9,472 random
+      // cells 4.88 ms on their own and 5.37 ms, 14,208 7.86 and 5.42 ms; TEREZA,
+      // 23,680 cells 2.83 and 2.95 ms, 28,416 4.15 and 3.12 ms).  Otherwise
+      // (ACETYLENE) W warps in lockstep from twice as many cells on: a flame of
+      // 18,944 cells 2.59 ms on their own and 3.93 ms, of 28,416 3.20 and 3.80 ms, of
+      // 37,888 4.39 and 3.73 ms.
       constexpr int RS = RateSlots<R, SPEC>::value;
       constexpr int kWarpBytes = 32 * PassStore<N, RS, LUT, false>::kBytesPerThread;
       constexpr int W = 232448 / kWarpBytes < 8 ? 232448 / kWarpBytes : 8;
       constexpr int kTmBytes = 128 * PassStore<N, RS, LUT, false, true>::kBytesPerThread;
       constexpr int kTmWarps = kTmBytes > 232448 ? 0 : kTmBytes > 115000 ? 4 : 8;
       if constexpr (kTmWarps > W) {
-        if (nl >= 148L * 32 * W)
+        if (nl > 148L * 32 * W)
           return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false, true>(a, (nl + 127) / 128, queue, 0, counters, s);
-      } else if (nl >= 148L * 32 * W) {
+      } else if (nl > 2 * 148L * 32 * W) {
         return launch_pass_bs<N, R, LUT, 32 * W, NF, SPEC, true, false>(a, (nl + 32 * W - 1) / (32 * W), queue, 0,
                                                                         counters, s);
       }
