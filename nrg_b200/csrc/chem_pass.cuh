@@ -402,8 +402,8 @@ __device__ __forceinline__ void pass_pascal(double (&yh)[kMaxOrd + 1][N], double
 }
 
 // The weighted norms' squares of two vectors with the same weights
-// max(|y|, YWT), as weighted_norm forms them.  Sums that overflow or are NaN
-// pass no test: the attempt fails, and the cell's tries are counted.
+// max(|y|, YWT), as weighted_norm forms them.  An error norm that overflows
+// passes no test: the attempt fails, and the cell's tries are counted.
 template <int N>
 __device__ __forceinline__ void pass_norms2(const double (&x0)[N], const double (&x1)[N], const double (&y)[N],
                                             const double (&ywt)[N], double* n0, double* n1) {
@@ -723,11 +723,17 @@ __device__ __forceinline__ int pass_integrate(const S& st, const StepArgs& a, bo
     bool fail = singular, conv = false;
     double ctest = 0.0, e2 = 0.0;  // e2: the squared ratio of the error estimate to eps
     if (go && !singular) {
-      double x[N], d;
+      double x[N], d, unit = 1.0;
       if (first) {
+        // the squares of rates above 1e134 (densities far beyond any gas) are kept
+        // in range by a power of two
+        bool big = false;
+#pragma unroll
+        for (int i = 0; i < N; ++i) big = big || (__double2hiint(s2[i]) & 0x7fffffff) >= (1023 + 448) << 20;
+        unit = big ? 0x1p-448 : 1.0;
 #pragma unroll
         for (int i = 0; i < N; ++i) {
-          x[i] = s2[i];
+          x[i] = s2[i] * unit;
           y[i] = 1.0;
         }
       } else {
@@ -749,7 +755,9 @@ __device__ __forceinline__ int pass_integrate(const S& st, const StepArgs& a, bo
         trend = 1.0;
         nq = 1;
         nwait = 3;
-        const double hd = eps * pass_rcp(d);
+        // d is in units of 1 / unit; an infinite one (infinite rates) leaves a step
+        // whose attempts show it
+        const double hd = NRG_FMAX(eps * pass_rcp(d) * unit, 1e-309);
         if (hd < fabs(h)) h = copysign(hd, h);
 #pragma unroll
         for (int i = 0; i < N; ++i) {

@@ -112,3 +112,23 @@ def test_a_queue_of_more_blocks_than_cells(decks, mode, kernel, block):
         s.close()
     for k in KEYS:
         np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+@pytest.mark.parametrize("mode", ["fast", "mixed"])
+def test_norms_beyond_the_range_of_their_squares(decks, mode):
+    """Densities at which the first weighted norm of dy/dt is above 1e154, so that
+    its square overflows: the step size comes from the scaled norm, and the
+    cells end as the oracle's do, at the limit of steps with a finite state."""
+    from nrg_b200.chemistry import ChemicalKineticsSolver
+    from oracle import oracle_py as op
+    f = fields.slice_field(fields.random_field(fields_W()), 64)
+    f.rho = f.rho * 1e85
+    o = op.Mechanism(*decks, 1.0, "cal.mol").chem_step(f.dt, f.T, f.rho, f.Y)
+    assert np.all(np.isfinite(o["Y_prod"]))
+    s = ChemicalKineticsSolver(None, *decks, mode=mode)
+    try:
+        g, st = run_device(s, f, mode)
+    finally:
+        s.close()
+    assert np.all(g["status"] == 2) and np.all(np.isfinite(g["Y_prod"]))
+    assert st["steps"] == 10000 * f.n
