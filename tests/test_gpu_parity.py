@@ -435,10 +435,12 @@ def _check_eps(solver, oracle_mech, f, launch):
         np.testing.assert_array_equal(again[k], base[k])
 
 
-@pytest.mark.parametrize("mode", ["reference", "fast", "mixed"])
+@pytest.mark.parametrize("mode", ["reference"])
 def test_lu_forms_give_identical_results(solver, W, mode):
     """nrg_chem_set_lu_form: the unrolled and the looped LU factorisation of
-    the thread-per-cell kernels take the same operations in the same order."""
+    the thread-per-cell kernels take the same operations in the same order.
+    (The fast and mixed modes have one form; their generated and table-driven
+    factorisations are compared above.)"""
     f = fields.slice_field(fields.ignition_field(W, n_side=128), 4000, stride=3)
     try:
         outs = [run_device(solver, f, mode, launch=dict(kernel="thread", block=32, grid=0, chunk=1, lu_rolled=r))
