@@ -271,23 +271,26 @@ static cudaError_t launch_pass(const StepArgs& a, const LaunchCfg& cfg, int* que
     return launch_pass_bs<N, R, LUT, 64, NF, SPEC, false, false>(a, (nl + 63) / 64, queue, 0, counters, s);
   } else {
     if constexpr (SPEC != 0) {
-      // W: the warps of a SM's shared memory.  More fit in blocks of 128 threads with
-      // the rate constants in tensor memory for KONNOV (2 -> 4) and TEREZA (5 -> 8):
-      // these from one more cell than the W warps take at once (KONNOV, 9,472 random
-      // cells 4.88 ms on their own and 5.37 ms, 14,208 7.86 and 5.42 ms; TEREZA,
-      // 23,680 cells 2.83 and 2.95 ms, 28,416 4.15 and 3.12 ms).  Otherwise
-      // (ACETYLENE) W warps in lockstep from twice as many cells on: a flame of
-      // 18,944 cells 2.59 ms on their own and 3.93 ms, of 28,416 3.20 and 3.80 ms, of
-      // 37,888 4.39 and 3.73 ms.
+      // W: the warps of a SM's shared memory, at most two above 10 species, whose
+      // spilled state the L1 cache then holds.  More fit in blocks of 128 threads
+      // with the rate constants in tensor memory for KONNOV (2 -> 4) and TEREZA (5 ->
+      // 8): these from one more cell than the W warps take at once (KONNOV, 9,472
+      // random cells 4.88 ms on their own and 5.37 ms, 14,208 7.86 and 5.42 ms;
+      // TEREZA, 23,680 cells 2.83 and 2.95 ms, 28,416 4.15 and 3.12 ms).  Otherwise
+      // (ACETYLENE) W warps in lockstep from there on: 18,944 random cells 7.76 ms on
+      // their own and 6.42 ms, a flame of them 2.53 and 2.60 ms, of 196,608 18.4 and
+      // 15.9 ms.  Its three warps that fit took 14.6 ms there, but 66.3 against 57.5
+      // ms for random cells, and 3.70 against 2.57 ms for a flame of 4,096 cells,
+      // which a large field with few hot cells comes to.
       constexpr int RS = RateSlots<R, SPEC>::value;
       constexpr int kWarpBytes = 32 * PassStore<N, RS, LUT, false>::kBytesPerThread;
-      constexpr int W = 232448 / kWarpBytes < 8 ? 232448 / kWarpBytes : 8;
+      constexpr int W = std::min(232448 / kWarpBytes, N > 10 ? 2 : 8);
       constexpr int kTmBytes = 128 * PassStore<N, RS, LUT, false, true>::kBytesPerThread;
       constexpr int kTmWarps = kTmBytes > 232448 ? 0 : kTmBytes > 115000 ? 4 : 8;
       if constexpr (kTmWarps > W) {
         if (nl > 148L * 32 * W)
           return launch_pass_bs<N, R, LUT, 128, NF, SPEC, true, false, true>(a, (nl + 127) / 128, queue, 0, counters, s);
-      } else if (nl > 2 * 148L * 32 * W) {
+      } else if (nl > 148L * 32 * W) {
         return launch_pass_bs<N, R, LUT, 32 * W, NF, SPEC, true, false>(a, (nl + 32 * W - 1) / (32 * W), queue, 0,
                                                                         counters, s);
       }
