@@ -316,12 +316,6 @@ bool supported_mechanism(int n_species, int n_reactions) {
 int match_specialised(const DevMech& reduced) { return match_specialised_tables(reduced); }
 int match_specialised_full(const DevMech& full) { return match_specialised_full_tables(full); }
 
-int smem_bytes_per_cell(int n_species, int n_reactions, bool mixed) {
-  if (n_species == 9 && n_reactions == 24)
-    return mixed ? SmemStore<9, 24, float, 32>::kBytesPerThread : SmemStore<9, 24, double, 32>::kBytesPerThread;
-  return 0;
-}
-
 cudaError_t launch_fp64_peak(double* out, int blocks, int threads, int iters, cudaStream_t s) {
   k_fp64_peak<<<blocks, threads, 0, s>>>(out, iters);
   return cudaGetLastError();

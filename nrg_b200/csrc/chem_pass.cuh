@@ -10,8 +10,10 @@
 // while the other lanes go on with their own next step, so the warp runs as
 // many passes as its slowest cell has right-hand sides; the routine-by-routine
 // form makes every lane wait for each retry and iteration of any other.
-// Each routine has one call site and is inlined there: there is no call that
-// would spill the cell's registers.
+// The routines of a pass have one call site each and are inlined there, so that
+// no call spills the cell's registers in every pass; out of line are the
+// step-size ratios of the order choice (four uses, pass_ratio) and the table
+// walks of decks without generated code.
 //
 // What bounds it, and where the state lives: with the Nordsieck array in
 // shared memory a cell took 1,408 B there, so an SM held 4 warps, one per
@@ -23,14 +25,14 @@
 // predictor, update and interpolation code (adding, scaling or multiplying
 // zeros changes no value).  Shared memory keeps what is indexed at run time
 // (the LU factors, whose pivot row varies) and what is read once per right-hand
-// side (the rate constants, equal reactions merged): 880 B a cell, 8 warps on an
-// SM at 255 registers.  What bounds it now is instruction issue (45 % of the
-// slots at two warps per scheduler, FP64 pipe 37 %) and instruction fetch:
-// the loop is about 4,000 instructions, so the warps of a block go through it
-// in lockstep (k_chem_pass).  2048 x 2048 flame 72.0 -> 28.7 ms, 512 x 512
-// ignition field 79.7 -> 16.1 ms, 64 x 64 random cells 2.49 -> 1.10 ms; flames of
-// 196,608 cells with the larger mechanisms: TEREZA 21.6 -> 9.1 ms, KONNOV 42.3
-// -> 22.8 ms, ACETYLENE 30.9 -> 24.8 ms.
+// side (the rate constants, equal reactions merged): 880 B a cell of KEROMNES, 8
+// warps on an SM at 252 registers.  What bounds it now is instruction issue
+// (41 % of the slots at two warps per scheduler, FP64 pipe 38 %) and instruction
+// fetch: the loop is about 4,000 instructions, so the warps of a block go through
+// it in lockstep (k_chem_pass).  2048 x 2048 flame 72.0 -> 28.6 ms, 512 x 512
+// ignition field 79.7 -> 16.2 ms, 64 x 64 random cells 2.49 -> 1.10 ms; a flame of
+// 512 x 384 cells with the larger mechanisms: TEREZA 21.6 -> 9.1 ms, KONNOV 42.3
+// -> 21.1 ms, ACETYLENE 30.9 -> 24.8 ms.
 #pragma once
 
 #include "chem_bdf.cuh"
