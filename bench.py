@@ -54,7 +54,7 @@ def parse():
                    help="fix the integrator launch instead of autotuning it (with --block)")
     p.add_argument("--block", type=int, default=32)
     p.add_argument("--lu", choices=["unrolled", "loop"], default=None,
-                   help="with --kernel: the thread kernels' LU form (default: unrolled)")
+                   help="with --kernel: the LU form of the reference mode's thread kernels (default: unrolled)")
     p.add_argument("--no-train", dest="train", action="store_false",
                    help="skip the training leg (the 4M-pair set generated by the FP64 integrator, then seconds "
                         "per epoch of the tensor-core forward/backward/Adam kernels)")

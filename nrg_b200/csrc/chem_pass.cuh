@@ -27,12 +27,12 @@
 // (the LU factors, whose pivot row varies) and what is read once per right-hand
 // side (the rate constants, equal reactions merged): 880 B a cell of KEROMNES, 8
 // warps on an SM at 252 registers.  What bounds it now is instruction issue
-// (41 % of the slots at two warps per scheduler, FP64 pipe 38 %) and instruction
+// (40 % of the slots at two warps per scheduler, FP64 pipe 39 %) and instruction
 // fetch: the loop is about 4,000 instructions, so the warps of a block go through
 // it in lockstep (k_chem_pass).  2048 x 2048 flame 72.0 -> 28.6 ms, 512 x 512
-// ignition field 79.7 -> 16.2 ms, 64 x 64 random cells 2.49 -> 1.10 ms; a flame of
-// 512 x 384 cells with the larger mechanisms: TEREZA 21.6 -> 9.1 ms, KONNOV 42.3
-// -> 21.1 ms, ACETYLENE 30.9 -> 24.8 ms.
+// ignition field 79.7 -> 16.1 ms, 64 x 64 random cells 2.49 -> 1.10 ms; a flame of
+// 512 x 384 cells with the larger mechanisms: TEREZA 21.6 -> 8.3 ms, KONNOV 42.3
+// -> 21.1 ms, ACETYLENE 30.9 -> 25.9 ms.
 #pragma once
 
 #include "chem_bdf.cuh"
