@@ -40,6 +40,11 @@
 
 namespace nrg {
 
+// Whether U's columns are multiplied by their pivots' reciprocals (pass_solve):
+// not for float factors, where it would round each of them once more.
+template <typename LUT>
+constexpr bool kScaledU = std::is_same<LUT, double>::value;
+
 // Slots of rate constants a cell keeps: the distinct reactions of the generated
 // code, all of them in table-driven kernels.
 template <int R, int SPEC>
@@ -278,8 +283,10 @@ __device__ __forceinline__ void pass_factor_columns(const V& view, const S& st, 
     ok = ok && v[J] != (LUT)0;
     v[J] = (LUT)1 / v[J];
   }
+  if constexpr (kScaledU<LUT>) {
 #pragma unroll
-  for (int i = 0; i < J; ++i) v[i] = v[i] * v[J];  // U scaled by its pivots (pass_solve)
+    for (int i = 0; i < J; ++i) v[i] = v[i] * v[J];
+  }
   if (commit) {
 #pragma unroll
     for (int i = 0; i < N; ++i) st.a(J, i) = v[i];
@@ -316,8 +323,9 @@ __device__ __forceinline__ bool pass_lu_loop(const S& st, RowPerm<N>& perm) {
     const LUT t = (LUT)-1 / piv;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
+      const LUT u = c[i];
       c[i] = t * (i > k && i == l ? ckk : c[i]);
-      ck[i * BS] = i > k ? c[i] : i < k ? -c[i] : -t;  // U scaled by its pivots (pass_solve)
+      ck[i * BS] = i > k ? c[i] : i < k ? (kScaledU<LUT> ? -c[i] : u) : -t;
       c[i] = i > k ? c[i] : (LUT)0;
     }
     const int pk = perm.get(k);
@@ -475,9 +483,9 @@ __device__ __forceinline__ double pass_pow(double x, float p) {
 
 // Corrector solve: the row permutation through the cell's scratch, then the two
 // sweeps without tests for zero multipliers (adding a zero product changes
-// nothing).  The factors hold the pivots' reciprocals on the diagonal and U's
-// columns multiplied by them, so that the backward sweep is a chain of one
-// fused multiply-add per row instead of a multiply and one.
+// nothing).  The factors hold the pivots' reciprocals on the diagonal and, in
+// double, U's columns multiplied by them, so that the backward sweep is a chain
+// of one fused multiply-add per row instead of a multiply and one.
 template <int N, class S>
 __device__ __forceinline__ void pass_solve(const S& st, const RowPerm<N>& piv, double (&b)[N]) {
 #pragma unroll
@@ -488,12 +496,17 @@ __device__ __forceinline__ void pass_solve(const S& st, const RowPerm<N>& piv, d
   for (int k = 0; k < N - 1; ++k)
 #pragma unroll
     for (int i = k + 1; i < N; ++i) b[i] = b[i] + b[k] * (double)st.a(k, i);
+  constexpr bool kScaled = kScaledU<typename S::lut_t>;
 #pragma unroll
-  for (int k = N - 1; k > 0; --k)
+  for (int k = N - 1; k >= 0; --k) {
+    if constexpr (!kScaled) b[k] = b[k] * (double)st.a(k, k);
 #pragma unroll
     for (int i = 0; i < k; ++i) b[i] = b[i] - b[k] * (double)st.a(k, i);
+  }
+  if constexpr (kScaled) {
 #pragma unroll
-  for (int k = 0; k < N; ++k) b[k] = b[k] * (double)st.a(k, k);
+    for (int k = 0; k < N; ++k) b[k] = b[k] * (double)st.a(k, k);
+  }
 }
 
 // The state a finished cell hands to cell_finish.
